@@ -343,7 +343,7 @@ def run_ours(a):
                             + ("" if world == 1 else " (experts are sharded: one touched by several GPUs' batches is streamed once, by its owner; the exchanges are inside the timed region)")},
         "cases": r["detail"],
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                     "traffic": traffic if world == 1 else None, "peak_source": peak_src, "kernel": "k_moe_decode_tc" if world == 1 else "k_prefill_gemm_r<3>",
+                     "traffic": traffic if world == 1 else None, "peak_source": peak_src, "kernel": "k_moe_decode_tc" if world == 1 else "k_grouped_gemm<3>",
                      "bytes_per_launch": round(r["step_bytes"] / world / (r["cases"] * a.layers)), "per_gpu": world > 1},
         "e2e": {"value": round(r["step_bytes"] / (r["e2e_ms"] * 1e-3) / 1e9, 1), "unit": "GB/s", "ms_per_step": round(r["e2e_ms"], 3),
                 "h2d_bytes_per_step": r["io"]["h2d"] * world, "d2h_bytes_per_step": r["io"]["d2h"] * world,

@@ -22,9 +22,9 @@ FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-li
 
 DIAG = "--diag" in sys.argv or os.environ.get("B200MOE_DIAG") == "1"
 if DIAG:
-    # diagnostic build (libb200moe_diag.so, loaded with B200MOE_LIB=<path>): per-worker cycle counters in the decode kernel,
-    # ablation switches of the prefill GEMM, and the entry points of include/b200moe_diag.h. Not the library that ships.
-    FLAGS += ["-DB200_TIMERS", "-DB200_PF_ABLATE", "-DB200_DIAGNOSTICS"]
+    # diagnostic build (libb200moe_diag.so, loaded with B200MOE_LIB=<path>): per-worker cycle counters in the decode kernel and
+    # the entry points of include/b200moe_diag.h. Not the library that ships.
+    FLAGS += ["-DB200_TIMERS", "-DB200_DIAGNOSTICS"]
     LIB = PKG / "libb200moe_diag.so"
 
 

@@ -36,3 +36,19 @@ inline int cuda_fail(cudaError_t e) {
     cudaError_t _e = cudaGetLastError();                      \
     if (_e != cudaSuccess) return ::b200::cuda_fail(_e);      \
   } while (0)
+
+namespace b200 {
+// Launch of `fn` on `st`. chained: programmatically behind the kernel before it in the stream - it may start when every block of
+// that kernel has called grid_launch_dependents (or has ended) and waits with grid_dependency_wait before it touches that
+// kernel's results.
+inline int launch_kernel(const void* fn, int grid, int block, int smem, bool chained, void** args, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid), cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = (size_t)smem, cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = chained ? 1 : 0;
+  B200_CUDA_TRY(cudaLaunchKernelExC(&cfg, fn, args));
+  return B200MOE_OK;
+}
+}  // namespace b200

@@ -74,7 +74,6 @@ __global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* __res
                               // whatever ran before it in the stream until that has completed
   uint8_t* xsf = xb + (long long)KB1 * N * 128;
   __shared__ float wm[4];
-  __shared__ float s_g1;
   // each thread keeps its (at most two) 16-value blocks in registers: one pass over x serves the token amax and the expansion
   const int nblk = KB1 * 16;                 // blocks over the padded K (KB1 * 256 values); nblk <= 256
   uint4 raw[2][2];
@@ -106,24 +105,21 @@ __global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* __res
   for (int j = 0; j < 2; ++j) {
     const int b = tid + 128 * j;
     if (b >= nblk) break;
-    uint2 codes[kTerms];
-    uint8_t sf[kTerms];
+    const int kb = b >> 4, chunk = (b & 15) >> 1, half = b & 1;   // 8 code bytes = half a 16-byte chunk
+    const bool scales = (b >> 2) < (H / 16 + 3) / 4;
+    auto put = [&](int t, uint2 codes, uint8_t sf) {
+      const int n = tok * kTerms + t;
+      *reinterpret_cast<uint2*>(xb + ((long long)kb * N + n) * 128 + ((chunk ^ (n & 7)) << 4) + half * 8) = codes;
+      if (scales) xsf[(long long)(b >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (b & 3)] = sf;
+    };
     if (tok < M && b * 16 < H) {
       float r[16];
       const uint32_t w[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) { r[2 * i] = __uint_as_float(w[i] << 16); r[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
-      expand_block16(r, g1, codes, sf);
+      expand_block16<false>(r, g1, put);
     } else {
-#pragma unroll
-      for (int t = 0; t < kTerms; ++t) { codes[t] = make_uint2(0u, 0u); sf[t] = 0; }
-    }
-    const int kb = b >> 4, chunk = (b & 15) >> 1, half = b & 1;   // 8 code bytes = half a 16-byte chunk
-#pragma unroll
-    for (int t = 0; t < kTerms; ++t) {
-      const int n = tok * kTerms + t;
-      *reinterpret_cast<uint2*>(xb + ((long long)kb * N + n) * 128 + ((chunk ^ (n & 7)) << 4) + half * 8) = codes[t];
-      if ((b >> 2) < (H / 16 + 3) / 4) xsf[(long long)(b >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (b & 3)] = sf[t];
+      for (int t = 0; t < kTerms; ++t) put(t, make_uint2(0u, 0u), 0);
     }
   }
 }
@@ -669,15 +665,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
               float r[16];
 #pragma unroll
               for (int i = 0; i < 16; ++i) r[i] = s_ex[blk * 16 + i][tk];
-              uint2 codes[kTerms];
-              uint8_t sf[kTerms];
-              if (expand_block16(r, P.act_g1, codes, sf)) P.status[1] = 1;   // beyond the range of the fixed activation scale
-#pragma unroll
-              for (int t = 0; t < kTerms; ++t) {
+              const bool clipped = expand_block16<false>(r, P.act_g1, [&](int t, uint2 codes, uint8_t sf) {
                 const int n = tk * kTerms + t;
-                *reinterpret_cast<uint2*>(slab + n * 128 + ((chunk ^ (n & 7)) << 4) + (blk & 1) * 8) = codes[t];
-                sfp[(n & 31) * 16 + (n >> 5) * 4] = sf[t];
-              }
+                *reinterpret_cast<uint2*>(slab + n * 128 + ((chunk ^ (n & 7)) << 4) + (blk & 1) * 8) = codes;
+                sfp[(n & 31) * 16 + (n >> 5) * 4] = sf;
+              });
+              if (clipped) P.status[1] = 1;   // beyond the range of the fixed activation scale
             } else {
 #pragma unroll
               for (int t = 0; t < kTerms; ++t) {

@@ -35,10 +35,14 @@ __device__ __forceinline__ uint32_t cvt_f32x8_e2m1(const float* v) {
 // next term.
 // Returns true when the block's maximum lies beyond what the first term can hold (its scale clamps at 448, i.e. values
 // above 2688 / g1): the later terms, with their larger global scales, cannot absorb the clipped part.
-__device__ __forceinline__ bool expand_block16(float (&r)[16], float g1, uint2 (&codes)[kTerms], uint8_t (&sf)[kTerms]) {
+// Each term is handed to `put(t, codes, scale byte)` as it is formed. kLoop: the terms as a loop of about a hundred instructions
+// rather than four copies of it, for kernels that run through their code only a few times per launch - an instruction line
+// that is not yet in the SM's cache costs more than the loop does.
+template <bool kLoop, class F>
+__device__ __forceinline__ bool expand_block16(float (&r)[16], float g1, F&& put) {
   float g = g1, ginv = __frcp_rn(g1);
   bool clipped = false;
-#pragma unroll
+#pragma unroll(kLoop ? 1 : kTerms)
   for (int t = 0; t < kTerms; ++t) {
     float m[8];
 #pragma unroll
@@ -67,8 +71,7 @@ __device__ __forceinline__ bool expand_block16(float (&r)[16], float g1, uint2 (
       r[8 + 2 * i] -= b.x * back;
       r[8 + 2 * i + 1] -= b.y * back;
     }
-    codes[t] = make_uint2(lo, hi);
-    sf[t] = sb;
+    put(t, make_uint2(lo, hi), sb);
     g *= 6.0f;
     ginv *= (1.0f / 6.0f);
   }

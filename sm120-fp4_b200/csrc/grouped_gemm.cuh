@@ -1,0 +1,511 @@
+// Ragged grouped GEMM on tcgen05.mma kind::mxf4nvf4: row tiles of gathered tokens (up to 128 rows of one expert) times the
+// expert's weight records. Four forms share the main loop:
+//   PHASE 1  W4A4 FC1:  128 rows x [64 up | 64 gate] columns, epilogue SiLU*mul + NVFP4 re-quantisation into FC2's records
+//   PHASE 2  W4A4 FC2:  128 rows x 128 columns, epilogue alpha * routing weight -> bf16 rows per (token, expert)
+//   PHASE 3  W4A16 FC1: 64 rows (16 pairs x four NVFP4 terms), epilogue term sum + SiLU*mul + four-term re-expansion
+//   PHASE 4  W4A16 FC2: the same rows, epilogue term sum + alpha * routing weight -> fp32 rows
+//
+// What bounds it. Per weight record (128 columns x 256 K values, 18 KB) the tensor core needs 4 x 64 cycles (measured:
+// 128 x 128 x 64 in 64 cycles) plus 8 cycles per tcgen05.cp of a 512-byte scale tile; an SM takes in 63 bytes per cycle from
+// L2 (17.3 TB/s over the chip, from four 18 KB copies in flight on), i.e. 288 cycles per record; HBM delivers a record per
+// SM every ~700 cycles (7.1 TB/s). A batch that touches every expert with few rows is bound by HBM, a large one by the MMAs
+// and the L2 port together. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies
+// its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
+// warp to warp between a record's arrival and its math. (Before, four warps moved the scales through registers and handed every
+// record to the MMA warp over a barrier: 870 cycles a record at 8192 tokens.)
+//
+// A CTA keeps the records of the first NR K boxes of its row tile resident for all column blocks of the tile; boxes beyond NR
+// come through the ring with the weights (gg_plan).
+#pragma once
+#include "common.cuh"
+#include "tcgen05.cuh"
+#include "nvfp4_math.cuh"
+#include "expand.cuh"
+
+namespace b200 {
+
+constexpr int kRec = 18432;          // one tile record: 16 KB codes image + 4 x 512 B scale tiles
+// W4A16 phases: the operand tile holds 64 rows (16 token-expert pairs x four terms) in 10 KB records (8 KB codes image +
+// four 512-byte scale tiles whose row groups 2 and 3 stay zero). The MMA still spans 128 rows: rows 64..127 read whatever
+// follows the record in shared memory, with zero scales, and their accumulator rows are ignored.
+constexpr int kMidRec = 8192 + 2048;
+
+constexpr int kGgThreads = 12 * 32;  // warps 0-7 epilogue (two groups of four), 8 row-tile producer, 9-10 ring producers, 11 MMA issuer
+constexpr int kGgMaxRing = 12;
+constexpr int kGgSmem = 227 * 1024 - 1024;   // dynamic shared memory of a CTA (1 KB is left to the static part)
+
+// byte offset inside a tile record of 8 consecutive code bytes (one 16-value block) of row r, K block b16 (0..15)
+__device__ __forceinline__ int rec_code_offset(int r, int b16) { return r * 128 + ((((b16 >> 1) ^ (r & 7))) << 4) + (b16 & 1) * 8; }
+__device__ __forceinline__ int rec_scale_offset(int r, int b16) { return 16384 + (b16 >> 2) * 512 + (r & 31) * 16 + (r >> 5) * 4 + (b16 & 3); }
+
+struct GroupedParams {
+  const uint8_t* arec;        // operand records [ntiles][KB][kRec or kMidRec]
+  const uint8_t* wrec;        // weight records [E][NBLK][KB][kRec]
+  const int* ntiles;
+  const int* tile_expert;
+  const int* tile_first;      // first and end index of the tile's rows in the router's pair list
+  const int* tile_end;
+  const int* row_pair;        // [ntiles*rows] pair index or -1
+  const float* alpha;         // per-expert weight scale
+  float gs_in;                // PHASE 1/2: global scale the A operand was quantised with
+  float gs_out;               // PHASE 1: global scale for the activation re-quantisation
+  const float* wts;           // PHASE 2/4: routing weights [P]
+  uint8_t* orec;              // PHASE 1/3: FC2 operand records [ntiles][KB2][...]
+  __nv_bfloat16* y;           // PHASE 2: weighted rows [ntiles*128][H]
+  float* yf;                  // PHASE 4: weighted rows [ntiles*16][H] in fp32 (one rounding only, in the combine)
+  int* status;
+  const float* rowscale;      // PHASE 3: 1 / g_t of every term row of the x operand [ntiles*64]
+  float act_g1;               // PHASE 3/4: global scale of the first term of the SiLU*mul activations
+  int NBLK, KB, KT, KB2, H;
+};
+
+struct GgShared {
+  uint64_t a_full[12], a_empty[12];                    // per resident K box
+  uint64_t full[kGgMaxRing], empty[kGgMaxRing];        // per ring slot
+  uint64_t acc_full[2], acc_empty[2];
+  float scale[128];                                    // PHASE 1: gs_out / (E4M3 value), per scale byte
+  uint32_t tmem_base;
+  int max_rows;                                        // most operand rows of any tile this CTA works on
+  volatile int abort_flag;
+};
+
+constexpr int kGgPatch = 32 * 144;   // PHASE 2: one warp's patch for transposed stores (32 rows x 128 bytes, padded)
+
+constexpr int gg_head_bytes(int phase) { return 1024 + (phase == 2 ? 8 * kGgPatch : 0); }   // barriers (+ store patches) ahead of the records
+static_assert(sizeof(GgShared) <= 1024 && (8 * kGgPatch) % 1024 == 0, "the records start on a 1 KB boundary");
+
+// How a CTA divides its shared memory, from the most rows its tiles hold: a resident operand record keeps only those rows (rounded
+// up to 8) and its scale tiles; the rest is the ring. A tile of 64 rows over 8 K boxes takes 80 KB and leaves eight slots,
+// one of 128 rows 144 KB and four. Depth matters when the weights come from HBM: four 18 KB records in flight are worth about
+// 1.7 us of an SM's share, less than HBM latency plus the hand-offs. NR boxes stay resident; if not all of them do, the
+// ring carries operand records as well and should hold kGgMinShared slots. TMEM: 256 accumulator columns + 16 per resident box
+// + 64 for the rotating weight scales + 64 more for streamed operand scales.
+constexpr int kGgMinRing = 4, kGgMinShared = 6;
+struct GgPlan { int astride, NR, NS; };
+__host__ __device__ inline GgPlan gg_plan(int phase, int KB, int max_rows) {
+  GgPlan p;
+  const int room = kGgSmem - 1024 - gg_head_bytes(phase);
+  p.astride = ((max_rows + 7) & ~7) * 128 + 2048;
+  p.NR = KB < 12 ? KB : 12;
+  if ((room - p.NR * p.astride) / kRec < kGgMinRing || p.NR < KB) {
+    p.NR = (room - kGgMinShared * kRec) / p.astride;
+    if (p.NR > 8) p.NR = 8;
+  }
+  p.NS = (room - p.NR * p.astride) / kRec;
+  if (p.NS > kGgMaxRing) p.NS = kGgMaxRing;
+  return p;
+}
+
+// A CTA's work: segments (row tile t, column blocks [n0, n1)). Whole tiles are dealt round-robin for as many full rounds as there
+// are (tiles t and t + 1 of one expert then run on neighbouring CTAs at the same time and in the same block order, so the
+// second reader of a weight record finds it in L2); the tiles left over are cut into equal ranges of column blocks so that
+// every CTA gets a share of them.
+struct GgSplit {
+  int G, cta, NBLK, rounds, T0, ra, rb, nseg;
+  struct Segment { int t, n0, n1; };
+  __device__ GgSplit(int NT, int nblk, int g, int c) : G(g), cta(c), NBLK(nblk) {
+    rounds = NT / G, T0 = rounds * G;
+    const int rem = (NT - T0) * NBLK;
+    ra = (int)((long long)rem * cta / G), rb = (int)((long long)rem * (cta + 1) / G);
+    nseg = rounds + (rb > ra ? (rb - 1) / NBLK - ra / NBLK + 1 : 0);
+  }
+  __device__ Segment segment(int ord) const {
+    if (ord < rounds) return {ord * G + cta, 0, NBLK};
+    const int q = ra / NBLK + (ord - rounds);
+    return {T0 + q, ord == rounds ? ra - q * NBLK : 0, min(NBLK, rb - q * NBLK)};
+  }
+};
+
+// What the kernel ahead of FC1 does beside its records (records_aside): `blocks` extra thread blocks in front of its grid.
+constexpr int kGgWarm = 8;   // weight records per GEMM CTA asked into L2 ahead of the GEMM
+struct GgAside {
+  const int *ntiles, *tile_expert, *tile_first, *tile_end;
+  const uint8_t* wrec;       // FC1 weight records
+  int NBLK, KB, gemm_ctas, blocks;
+};
+
+// ---- epilogues: one warp, 32 accumulator rows x 128 columns at taddr (thread = row). `release` frees the accumulator buffer
+// once its values are in registers.
+
+// W4A4 FC1: columns 0..63 = up, 64..127 = gate of intermediate columns 64n..; SiLU*mul, re-quantise four blocks of 16 and store
+// the row's 32 code bytes (two 16-byte chunks of one sector) and four scale bytes into FC2's record `dst`.
+template <class F>
+__device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float gs_out, const float* scale_table, uint8_t* dst, int row, bool store,
+                                                int n, F&& release) {
+  uint32_t sfw = 0;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    uint32_t up[2][16], gt[2][16];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      tmem_ld_32x32b_x16(taddr + 32 * h + 16 * b, up[b]);
+      tmem_ld_32x32b_x16(taddr + 64 + 32 * h + 16 * b, gt[b]);
+    }
+    tmem_ld_wait();
+    if (h == 1) release();
+    uint2 pk[2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      float a[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;
+        a[i] = __fdividef(g, 1.0f + __expf(-g)) * u;
+      }
+      sfw |= (uint32_t)quantize_block16_t(a, gs_out, scale_table, pk[b]) << (16 * h + 8 * b);
+    }
+    if (store) *reinterpret_cast<uint4*>(dst + rec_code_offset(row, 4 * (n & 3) + 2 * h)) = make_uint4(pk[0].x, pk[0].y, pk[1].x, pk[1].y);
+  }
+  if (store) *reinterpret_cast<uint32_t*>(dst + rec_scale_offset(row, 4 * (n & 3))) = sfw;
+}
+
+// W4A4 FC2: scale, round to bf16, transpose through the warp's patch of shared memory so that every store instruction writes
+// whole 128-byte row segments (four rows per instruction). valid: bit l = row l of the warp holds a pair.
+template <class F>
+__device__ __forceinline__ void gg_epilogue_fc2(uint32_t taddr, float s, unsigned valid, uint8_t* patch, __nv_bfloat16* ybase, int H, int lane, F&& release) {
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    uint32_t r[4][16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x16(taddr + 64 * half + 16 * c, r[c]);
+    tmem_ld_wait();
+    if (half == 1) release();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint32_t o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c][2 * i]) * s, __uint_as_float(r[c][2 * i + 1]) * s);
+        o[i] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(patch + lane * 144 + 32 * c) = make_uint4(o[0], o[1], o[2], o[3]);
+      *reinterpret_cast<uint4*>(patch + lane * 144 + 32 * c + 16) = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int rr = 4 * j + (lane >> 3);   // row of the warp's block this lane stores a 16-byte chunk of
+      const uint4 v4 = *reinterpret_cast<const uint4*>(patch + rr * 144 + (lane & 7) * 16);
+      if ((valid >> rr) & 1u) *reinterpret_cast<uint4*>(ybase + (long long)rr * H + 64 * half + (lane & 7) * 8) = v4;
+    }
+    __syncwarp();
+  }
+}
+
+// W4A16 FC1: rows 4p..4p+3 are the four terms of pair p, each scaled by its 1/g_t. A reduce-scatter over the pair's four lanes
+// leaves lane q with the sums of the q-th 16-column block (up, then gate), so that SiLU*mul and the expansion of the activations
+// into four terms run once per block with every lane at work; the lane writes its block of all four term rows of FC2's operand
+// record. (With two blocks at a time and every second lane idle in the expansion an epilogue took 12,500 cycles, more than the
+// eight weight records of a block take to arrive.) Returns whether a block lay beyond the range of the activation scale.
+__device__ __forceinline__ void gg_reduce_scatter16(uint32_t taddr, float rs, int tq, float (&o)[16]) {
+  uint32_t r[4][16];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x16(taddr + 16 * c, r[c]);
+  tmem_ld_wait();
+  const int hi = tq >> 1, lo = tq & 1;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    float k2[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float mine = __uint_as_float(hi ? r[2 + j][i] : r[j][i]) * rs, other = __uint_as_float(hi ? r[j][i] : r[2 + j][i]) * rs;
+      k2[j] = mine + __shfl_xor_sync(0xffffffffu, other, 2);   // the lane two over keeps the other two blocks and sends these
+    }
+    const float keep = lo ? k2[1] : k2[0], send = lo ? k2[0] : k2[1];
+    o[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+  }
+}
+
+template <class F>
+__device__ __forceinline__ bool gg_epilogue_fc1_a16(uint32_t taddr, float s, float rs, float act_g1, uint8_t* dst, int row, bool used, bool store, int n,
+                                                    int lane, F&& release) {
+  const int tq = lane & 3;
+  float up[16], a[16];
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {   // the up columns, then the gate columns
+#pragma unroll
+    for (int i = 0; i < 16; ++i) up[i] = a[i];
+    gg_reduce_scatter16(taddr + 64 * half, rs, tq, a);
+  }
+  release();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float g = a[i] * s, u = up[i] * s;
+    a[i] = __fdividef(g, 1.0f + __expf(-g)) * u;
+  }
+  bool clipped = false;
+  if (used) {
+    const int r0 = row & ~3;
+    clipped = expand_block16<true>(a, act_g1, [&](int q, uint2 codes, uint8_t sf) {
+      if (!store) return;
+      *reinterpret_cast<uint2*>(dst + rec_code_offset(r0 + q, 4 * (n & 3) + tq)) = codes;
+      dst[8192 + (n & 3) * 512 + ((r0 + q) & 31) * 16 + ((r0 + q) >> 5) * 4 + tq] = sf;
+    });
+  }
+  return clipped && store;
+}
+
+// W4A16 FC2: the four term rows of a pair are scaled and added; lane t of the pair stores columns 16t..16t+15 of each 64-column
+// half, so the four lanes write contiguous 256-byte segments of the pair's row.
+template <class F>
+__device__ __forceinline__ void gg_epilogue_fc2_a16(uint32_t taddr, float s, float rs, bool store, float* yrow, int lane, F&& release) {
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    const int tq = lane & 3;
+    float o[16];
+    gg_reduce_scatter16(taddr + 64 * half, rs, tq, o);
+    if (half == 1) release();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o[i] *= s;
+    if (store) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(yrow + 64 * half + 16 * tq + 4 * i) = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+    }
+  }
+}
+
+template <int PHASE>
+__global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_constant__ GroupedParams P) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int kARec = PHASE >= 3 ? kMidRec : kRec;            // bytes of one operand record in global memory
+  constexpr int kACodes = PHASE >= 3 ? 8192 : 16384;            // ... of which codes; the scale tiles follow
+  constexpr int kARows = PHASE >= 3 ? 64 : 128;                 // operand rows per tile
+  constexpr int kRowsPerPair = PHASE >= 3 ? kTerms : 1;
+  const int KB = P.KB, NBLK = P.NBLK;
+  GgShared& S = *reinterpret_cast<GgShared*>(smem);
+  uint8_t* patches = smem + 1024;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // (a value from lane 0 is known to be warp-uniform)
+  grid_launch_dependents();   // the next kernel of the chain may take over SMs as this one's CTAs leave
+  // The tile tables are read here without waiting for the kernel before this one: the tables' own producer is at least two
+  // kernels back, and the kernel in between lets this one start only after it has seen that producer complete.
+  const int NT = __shfl_sync(0xffffffffu, __ldcg(P.ntiles), 0);
+  const GgSplit split(NT, NBLK, (int)gridDim.x, (int)blockIdx.x);
+  const int nseg = split.nseg;
+  auto for_each_segment = [&](auto&& body) {   // body(t, n0, n1, ordinal), one call site: a copy of a role's code per launch is enough
+#pragma unroll 1
+    for (int ord = 0; ord < nseg; ++ord) {
+      const GgSplit::Segment g = split.segment(ord);
+      body(g.t, g.n0, g.n1, ord);
+    }
+  };
+  auto tile_rows = [&](int t) {   // operand rows that hold something, rounded up to the 8-row groups of the record image
+    return min(kARows, ((__ldcg(P.tile_end + t) - __ldcg(P.tile_first + t)) * kRowsPerPair + 7) & ~7);
+  };
+  if (warp == 10) {   // the most rows of this CTA's tiles
+    int m = 8;
+    for (int i = lane; i < nseg; i += 32) m = max(m, tile_rows(split.segment(i).t));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) S.max_rows = m;
+  }
+  if (tid == 0) {
+    for (int k = 0; k < 12; ++k) { mbar_init(&S.a_full[k], 1); mbar_init(&S.a_empty[k], 1); }
+    for (int s = 0; s < kGgMaxRing; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], 4); }
+    S.abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 11) { tmem_alloc(&S.tmem_base, 512); tmem_relinquish(); }
+  if (PHASE == 1) fill_scale_table(S.scale, P.gs_out, tid, kGgThreads);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const GgPlan plan = gg_plan(PHASE, KB, __shfl_sync(0xffffffffu, S.max_rows, 0));
+  const int NR = plan.NR, NS = plan.NS, astride = plan.astride, acodes = astride - 2048;
+  uint8_t* abuf = smem + gg_head_bytes(PHASE);                  // NR records of the current row tile
+  uint8_t* ring = abuf + NR * astride;                          // NS slots
+  const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem_base, 0);
+  const uint32_t tm_acc = tmem, tm_sfa = tmem + 256, tm_sfb = tmem + 256 + 16 * NR, tm_sfs = tm_sfb + 64;   // 2 x 128 | NR x 16 | 4 x 16 | 4 x 16
+  const int nkt_last = P.KT - 4 * (KB - 1);
+
+  if (warp == 8) {
+    // ============================================================== resident operand records: once per segment, box by box
+    if (lane == 0) {
+      grid_dependency_wait();   // the records are written by the kernel before this one
+      for_each_segment([&](int t, int, int, int ord) {
+        const int codes = tile_rows(t) * 128;   // only the rows in use, then the scale tiles
+        for (int kb = 0; kb < NR; ++kb) {
+          if (ord >= 1 && !mbar_wait(&S.a_empty[kb], (uint32_t)((ord - 1) & 1), &S.abort_flag)) *P.status = 2;
+          const uint8_t* src = P.arec + ((long long)t * KB + kb) * kARec;
+          mbar_expect_tx(&S.a_full[kb], codes + 2048);
+          bulk_load(abuf + kb * astride, src, codes, &S.a_full[kb]);
+          bulk_load(abuf + kb * astride + acodes, src + kACodes, 2048, &S.a_full[kb]);
+        }
+      });
+    }
+    __syncwarp();
+  } else if (warp == 9 || warp == 10) {
+    // ============================================================== ring: weight records (and operand records of boxes >= NR).
+    // Two producers walk the same sequence and issue alternate slots: one thread's wait + issue round is ~430 cycles a copy.
+    if (lane == 0) {
+      int slot = 0;
+      uint32_t ph = 1;          // parity that a free slot's `empty` barrier has completed: the first pass finds all slots free
+      bool mine = warp == 9, waited = NR == KB;
+      auto next = [&]() { mine = !mine; if (++slot == NS) { slot = 0; ph ^= 1u; } };
+      auto acquire = [&]() { if (!mbar_wait(&S.empty[slot], ph, &S.abort_flag)) *P.status = 2; };
+      for_each_segment([&](int t, int n0, int n1, int) {
+        const uint8_t* src = P.wrec + ((long long)__ldcg(P.tile_expert + t) * NBLK + n0) * KB * kRec;   // consecutive column blocks are contiguous
+        const uint8_t* asrc = P.arec + (long long)t * KB * kARec;
+        const int codes = NR < KB ? tile_rows(t) * 128 : 0;
+        for (int n = n0; n < n1; ++n)
+          for (int kb = 0; kb < KB; ++kb, src += kRec) {
+            if (kb >= NR) {
+              if (mine) {
+                acquire();
+                if (!waited) { grid_dependency_wait(); waited = true; }
+                mbar_expect_tx(&S.full[slot], codes + 2048);
+                bulk_load(ring + slot * kRec, asrc + (long long)kb * kARec, codes, &S.full[slot]);
+                bulk_load(ring + slot * kRec + kACodes, asrc + (long long)kb * kARec + kACodes, 2048, &S.full[slot]);
+              }
+              next();
+            }
+            if (mine) {
+              acquire();
+              mbar_expect_tx(&S.full[slot], kRec);
+              bulk_load(ring + slot * kRec, src, kRec, &S.full[slot]);
+            }
+            next();
+          }
+      });
+    }
+    __syncwarp();
+  } else if (warp == 11) {
+    // ============================================================== MMA issuer: the warp stays converged (all values are
+    // warp-uniform) and one elected lane issues. Measured per record (wait, 4 scale copies, 4 MMAs, commit; dynamic slots): 320
+    // cycles this way - the MMAs themselves are 256 - against 450 to 620 from inside a branch that a single lane takes.
+    const uint32_t el = elect_one();
+    const uint32_t idesc = idesc_mxf4nvf4(128, 128);
+    const uint32_t a16 = kDescLoSw128 + (smem_u32(abuf) >> 4), r16 = kDescLoSw128 + (smem_u32(ring) >> 4);   // descriptor low words
+    const uint32_t full_u = smem_u32(S.full), empty_u = smem_u32(S.empty), afull_u = smem_u32(S.a_full), aempty_u = smem_u32(S.a_empty);
+    const uint32_t accf_u = smem_u32(S.acc_full), acce_u = smem_u32(S.acc_empty);
+    int slot = 0, seq = 0;
+    uint32_t ph = 0, rot = 0;
+    auto take = [&]() {   // the next ring slot, landed
+      if (!mbar_wait_warp(full_u + 8 * slot, ph, &S.abort_flag)) *P.status = 1;
+      const int s = slot;
+      if (++slot == NS) { slot = 0; ph ^= 1u; }
+      return s;
+    };
+    auto copy_scales = [&](uint32_t dst, uint32_t rec_lo, int codes16) {   // four 512-byte tiles -> 16 TMEM columns
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) tmem_cp_sf_lo(dst + 4 * jj, rec_lo - kDescLoSw128 + codes16 + 32 * jj, el);
+    };
+    for_each_segment([&](int, int n0, int n1, int ord) {
+      for (int n = n0; n < n1; ++n, ++seq) {
+        const int ab = seq & 1;
+        const bool first = n == n0, last = n == n1 - 1;
+        if (seq >= 2 && !mbar_wait_warp(acce_u + 8 * ab, (uint32_t)((seq >> 1) - 1) & 1u, &S.abort_flag)) *P.status = 5;
+        const uint32_t acc = tm_acc + 128 * ab;
+        for (int kb = 0; kb < KB; ++kb) {
+          uint32_t a_lo, sfa;
+          int aslot = -1;
+          if (kb < NR) {
+            a_lo = a16 + kb * (astride >> 4), sfa = tm_sfa + 16 * kb;
+            if (first) {
+              if (!mbar_wait_warp(afull_u + 8 * kb, (uint32_t)(ord & 1), &S.abort_flag)) *P.status = 1;
+              tc_fence_after();
+              copy_scales(sfa, a_lo, acodes >> 4);
+            }
+          } else {
+            aslot = take();
+            a_lo = r16 + aslot * (kRec >> 4), sfa = tm_sfs + 16 * rot;
+            tc_fence_after();
+            copy_scales(sfa, a_lo, kACodes >> 4);
+          }
+          const int bslot = take();
+          const uint32_t b_lo = r16 + bslot * (kRec >> 4), sfb = tm_sfb + 16 * rot;
+          rot = (rot + 1) & 3u;
+          tc_fence_after();
+          copy_scales(sfb, b_lo, 1024);   // a short last box has zero scale tiles behind its last K step: copying them is harmless
+          if (kb < KB - 1 || nkt_last == 4) {
+            umma_mxf4nvf4_lo(acc, a_lo, b_lo, idesc, sfa, sfb, kb != 0 ? 1u : 0u, el);
+#pragma unroll
+            for (int jj = 1; jj < 4; ++jj) umma_mxf4nvf4_lo(acc, a_lo + 2 * jj, b_lo + 2 * jj, idesc, sfa + 4 * jj, sfb + 4 * jj, 1u, el);
+          } else {
+            for (int jj = 0; jj < nkt_last; ++jj)
+              umma_mxf4nvf4_lo(acc, a_lo + 2 * jj, b_lo + 2 * jj, idesc, sfa + 4 * jj, sfb + 4 * jj, kb + jj != 0 ? 1u : 0u, el);
+          }
+          umma_commit_u32(empty_u + 8 * bslot, el);
+          if (aslot >= 0) umma_commit_u32(empty_u + 8 * aslot, el);
+          else if (last) umma_commit_u32(aempty_u + 8 * kb, el);   // the next segment's record of this box may land
+        }
+        umma_commit_u32(accf_u + 8 * ab, el);
+      }
+    });
+    __syncwarp();
+  } else {
+    // ============================================================== epilogue: group g = warps 4g..4g+3 takes every second block
+    // (accumulator buffer g), so a block's epilogue may last as long as two blocks of MMAs; thread = accumulator row.
+    const int grp = warp >> 2, quad = warp & 3;
+    const int row = quad * 32 + lane;
+    int seq = 0;
+    uint32_t aph = 0;
+    // The first pass through a block is a dry one, on whatever the accumulator holds and without storing: it brings the epilogue's
+    // instructions into the SM while the first records are still on their way. (Without it the first block's epilogue
+    // took 16,000 cycles against 3,000 later on, and the MMAs of the third block waited for it.)
+    bool dry = true;
+    for_each_segment([&](int t, int n0, int n1, int) {
+#pragma unroll 1
+     for (int pass = dry ? 0 : 1; pass < 2; ++pass) {
+      if (dry && pass == 1) {
+        dry = false;
+        grid_dependency_wait();   // what is read and written from here on belongs to the kernels before this one until they are complete
+      }
+      const int rows = tile_rows(t);
+      float s = P.alpha[__ldcg(P.tile_expert + t)];
+      if (PHASE <= 2) s /= P.gs_in;
+      int pr = -1;
+      float rs = 0.f;   // W4A16 phases: 1 / g_t of this operand row's term
+      if (PHASE == 2 || (PHASE == 4 && row < kARows)) {   // FC2: times the row's routing weight
+        pr = __ldcg(P.row_pair + (long long)t * kARows + row);
+        s = pr >= 0 ? s * P.wts[pr] : 0.f;
+      }
+      if (PHASE == 3 && row < rows) rs = __ldcg(P.rowscale + (long long)t * kARows + row);
+      if (PHASE == 4) {
+        float g = P.act_g1;
+        for (int q = 0; q < (lane & 3); ++q) g *= 6.0f;
+        rs = 1.0f / g;
+      }
+      const unsigned valid = PHASE == 2 ? __ballot_sync(0xffffffffu, pr >= 0) : 0u;   // bit l: row quad*32 + l holds a pair
+      const bool work = quad * 32 < rows;   // warp-uniform: this quadrant holds rows of the tile
+#pragma unroll 1
+      for (int n = n0; n < n1; ++n, ++seq) {
+        if (!dry) {
+          if ((seq & 1) != grp) continue;
+          if (!mbar_wait(&S.acc_full[grp], aph, &S.abort_flag)) *P.status = 7;
+          aph ^= 1u;
+          tc_fence_after();
+        }
+        const uint32_t taddr = tm_acc + 128 * grp + ((uint32_t)(quad * 32) << 16);
+        auto release = [&]() {   // the accumulator is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0 && !dry) mbar_arrive(&S.acc_empty[grp]);
+        };
+        if (!work && !dry) {
+          release();
+        } else if (PHASE == 1) {
+          gg_epilogue_fc1(taddr, s, P.gs_out, S.scale, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kRec, row, row < rows && !dry, n, release);
+        } else if (PHASE == 2) {
+          gg_epilogue_fc2(taddr, s, dry ? 0u : valid, patches + warp * kGgPatch, P.y + ((long long)t * 128 + quad * 32) * P.H + 128 * n, P.H, lane, release);
+        } else if (PHASE == 3) {
+          if (gg_epilogue_fc1_a16(taddr, s, rs, P.act_g1, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kMidRec, row, row < rows, !dry, n, lane, release))
+            P.status[1] = 1;   // beyond the range of the fixed activation scale
+        } else {
+          gg_epilogue_fc2_a16(taddr, s, rs, pr >= 0 && !dry, P.yf + ((long long)t * 16 + (row >> 2)) * P.H + 128 * n, lane, release);
+        }
+        if (dry) break;
+      }
+     }
+    });
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 11) tmem_dealloc(tmem, 512);
+  if (S.abort_flag)
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
+
+}  // namespace b200

@@ -1,0 +1,173 @@
+// The plan of one grouped layer call in ONE launch: router tables (experts, offsets, pairs - the same as b200moe_route, bit for
+// bit), tile tables and the map between token-expert pairs and operand rows. It replaced five launches (clear, histogram,
+// scan, placement, row map: 35 us of a 127 us call at 1024 tokens, most of it launch gaps).
+//
+// A cluster of up to eight CTAs. Every warp of the cluster owns a contiguous run of pairs and walks it in index order, 32 at a time:
+// pairs of one expert are ranked by lane (match.any) on top of a running count per (warp, expert) in shared memory, so a pair's
+// position is known up to the start of its warp's run. Per expert the counts are then scanned over the warps, over the CTAs
+// (distributed shared memory) and over the experts; no atomic decides a position. Bound by latency (a few dependent passes of
+// a microsecond each), not by bytes: 4 bytes in and 12 out per pair.
+#pragma once
+#include "common.cuh"
+#include "tcgen05.cuh"
+
+namespace b200 {
+
+constexpr int kPlanMaxE = 256;
+
+__device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+// TILE pairs per row tile, ROWS operand rows per pair. row_pair [tiles*TILE*ROWS] = pair of every operand row of a tile (-1: none),
+// dst_row[pair] = tile * TILE + slot (-1: empty slot, or an id >= E). tile_first / tile_end: first and end index into `pairs`.
+struct PlanTables {
+  int *experts, *offsets, *pairs, *ntiles, *tile_expert, *tile_first, *tile_end, *row_pair, *dst_row;
+};
+
+template <int TILE, int ROWS>
+__global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int Umax, int max_tiles, PlanTables T) {
+  __shared__ int wc[32][kPlanMaxE];     // pairs of expert e in warp w's run, then the start of the run in `pairs`
+  __shared__ int tot[kPlanMaxE];        // ... in this CTA (read by the other CTAs)
+  __shared__ int cnt[kPlanMaxE], off[kPlanMaxE], tb[kPlanMaxE];   // all pairs of expert e, its first index in `pairs`, its first tile
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = (int)cluster_ctarank();
+  int C;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
+  for (int i = tid; i < 32 * kPlanMaxE / 4; i += 1024) reinterpret_cast<int4*>(&wc[0][0])[i] = make_int4(0, 0, 0, 0);
+  grid_dependency_wait();      // the ids, and whoever still reads the tables of the previous call
+  grid_launch_dependents();    // from here on everything before this kernel is complete: the next kernel may read the call's inputs at once
+  __syncthreads();
+  const int L = ((P + C * 32 - 1) / (C * 32) + 31) & ~31;   // pairs per warp
+  const int p0 = (rank * 32 + warp) * L, p1 = min(P, p0 + L);
+  // ---- positions inside the warp's run; dst_row holds (expert, position) until the run's start is known
+#pragma unroll 1
+  for (int s = p0; s < p1; s += 128) {   // four steps of 32, their ids in flight together
+    int id[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) id[k] = s + 32 * k + lane < p1 ? __ldcg(ids + s + 32 * k + lane) : -1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (s + 32 * k >= p1) break;
+      const int p = s + 32 * k + lane;
+      const int e = id[k] < 0 || id[k] >= E ? -1 : id[k];
+      const unsigned peers = __match_any_sync(0xffffffffu, e);
+      const int r = __popc(peers & ((1u << lane) - 1u));
+      const int before = e >= 0 ? wc[warp][e] : 0;
+      __syncwarp();
+      if (e >= 0 && r == 0) wc[warp][e] = before + __popc(peers);
+      if (p < p1) __stcg(T.dst_row + p, e >= 0 ? (e << 22) | (before + r) : -1);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  if (tid < kPlanMaxE) {   // thread e: exclusive scan of expert e's counts over the warps of this CTA
+    int c = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) { const int v = wc[w][tid]; wc[w][tid] = c; c += v; }
+    tot[tid] = c;
+  }
+  cluster_sync_all();
+  int mine = 0;            // thread e: pairs of expert e in the CTAs before this one
+  if (tid < kPlanMaxE) {
+    int c = 0;
+    for (int q = 0; q < C; ++q) {
+      const int v = ld_shared_cluster(mapa_shared(smem_u32(&tot[tid]), (uint32_t)q));
+      if (q < rank) mine += v;
+      c += v;
+    }
+    cnt[tid] = c;
+  }
+  cluster_arrive();        // `tot` of every CTA has been read (waited for before exit)
+  __syncthreads();
+  if (warp == 0) {         // scans over the experts, eight per lane: first pair, index among the touched experts, first tile
+    int c[8], sc = 0, su = 0, st = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { c[i] = cnt[lane * 8 + i]; sc += c[i]; su += c[i] > 0; st += (c[i] + TILE - 1) / TILE; }
+    int ic = sc, iu = su, it = st;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, ic, o), b = __shfl_up_sync(0xffffffffu, iu, o), d = __shfl_up_sync(0xffffffffu, it, o);
+      if (lane >= o) { ic += a; iu += b; it += d; }
+    }
+    int rc = ic - sc, ru = iu - su, rt = it - st;
+    const int routed = __shfl_sync(0xffffffffu, ic, 31), U = __shfl_sync(0xffffffffu, iu, 31), NT = min(__shfl_sync(0xffffffffu, it, 31), max_tiles);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = lane * 8 + i;
+      off[e] = rc, tb[e] = rt;
+      if (rank == 0 && c[i] > 0 && ru < Umax) { T.experts[ru] = e; T.offsets[ru] = rc; }
+      ru += c[i] > 0, rc += c[i], rt += (c[i] + TILE - 1) / TILE;
+    }
+    if (rank == 0) {
+      for (int u = U + lane; u < Umax; u += 32) { T.experts[u] = -1; T.offsets[u + 1] = routed; }
+      if (lane == 0) {
+        if (U <= Umax) T.offsets[U] = routed;
+        T.ntiles[0] = NT;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid < kPlanMaxE) {
+    const int o = off[tid] + mine;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) wc[w][tid] += o;
+  }
+  __syncthreads();
+  // ---- the tables of every pair
+#pragma unroll 1
+  for (int s = p0; s < p1; s += 128) {
+    int v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = s + 32 * k + lane < p1 ? __ldcg(T.dst_row + s + 32 * k + lane) : -1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (v[k] < 0) continue;                  // dst_row stays -1
+      const int p = s + 32 * k + lane, e = v[k] >> 22, pos = wc[warp][e] + (v[k] & ((1 << 22) - 1));
+      const int row = tb[e] * TILE + pos - off[e];
+      T.pairs[pos] = p;
+      const bool fits = row < max_tiles * TILE;
+      T.dst_row[p] = fits ? row : -1;
+      if (fits) {
+        if (ROWS == 4) *reinterpret_cast<int4*>(T.row_pair + 4LL * row) = make_int4(p, p, p, p);
+        else T.row_pair[row] = p;
+      }
+    }
+  }
+  // ---- tile tables and the rows that hold no pair: one warp of the cluster per expert
+  for (int e = rank * 32 + warp; e < E; e += C * 32) {
+    const int c = cnt[e], nt = (c + TILE - 1) / TILE;
+    for (int j = lane; j < nt; j += 32) {
+      const int t = tb[e] + j;
+      if (t < max_tiles) { T.tile_expert[t] = e; T.tile_first[t] = off[e] + j * TILE; T.tile_end[t] = off[e] + c; }
+    }
+    for (int r = c + lane; r < nt * TILE; r += 32) {
+      const int row = tb[e] * TILE + r;
+      if (row < max_tiles * TILE) {
+        if (ROWS == 4) *reinterpret_cast<int4*>(T.row_pair + 4LL * row) = make_int4(-1, -1, -1, -1);
+        else T.row_pair[row] = -1;
+      }
+    }
+  }
+  cluster_wait();
+}
+
+// One cluster, as many CTAs as the pairs keep busy: 512 pairs a CTA (two steps of 32 for half of its warps) up to eight CTAs.
+template <int TILE, int ROWS>
+inline int launch_plan(const int* ids, int P, int E, int Umax, int max_tiles, PlanTables T, cudaStream_t st) {
+  const int C = P <= 1024 ? 1 : P <= 2048 ? 2 : P <= 4096 ? 4 : 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C), cfg.blockDim = dim3(1024), cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = 2;
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plan<TILE, ROWS>, ids, P, E, Umax, max_tiles, T));
+  return B200MOE_OK;
+}
+
+}  // namespace b200

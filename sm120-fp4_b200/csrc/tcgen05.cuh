@@ -81,6 +81,28 @@ __device__ __forceinline__ void umma_commit_p(uint64_t* bar, uint32_t pred) {
   asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)), "r"(pred) : "memory");
 }
 
+// The same from 32-bit pieces: descriptors as low words (their high word is a constant of the layout), barriers as shared-memory
+// addresses - fewer registers to move into uniform ones per operation.
+constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);   // high word of smem_desc_sw128_kmajor
+constexpr uint32_t kDescLoSw128 = (16u >> 4) << 16;
+constexpr uint32_t kDescHiSf = (128u >> 4) | (1u << 14);                     // high word of smem_desc_sf_tile
+__device__ __forceinline__ void umma_mxf4nvf4_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem,
+                                                 uint32_t accumulate, uint32_t pred) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %7, 0;\n mov.b64 a, {%1, %8};\n mov.b64 b, {%2, %8};\n"
+      " @q tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a, b, %3, [%5], [%6], p;\n}\n"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem), "r"(pred), "n"(kDescHiSw128)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_cp_sf_lo(uint32_t taddr, uint32_t s_lo, uint32_t pred) {
+  asm volatile(
+      "{\n .reg .pred q;\n .reg .b64 s;\n setp.ne.b32 q, %2, 0;\n mov.b64 s, {%1, %3};\n"
+      " @q tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], s;\n}\n" ::"r"(taddr), "r"(s_lo), "r"(pred), "n"(kDescHiSf) : "memory");
+}
+__device__ __forceinline__ void umma_commit_u32(uint32_t bar, uint32_t pred) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar), "r"(pred) : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------------- accumulator loads
 // 32 lanes (this warp's quadrant) x 32 consecutive fp32 columns -> 32 registers per thread (thread = lane = row).
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {
