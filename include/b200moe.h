@@ -40,12 +40,20 @@ int b200moe_from_128x4(const void* sf_swizzled, void* sf_linear, int batch, int 
  * bytes of device scratch. b200moe_quantize_nvfp4: global_scale holds one value (gs_rows 0) or one per gs_rows
  * destination rows (stacked experts); destination row r quantises source row src_row[r] (null: r; negative:
  * zero codes and scales); packed u8 [rows, K/2]; sf u8 row-major [rows, K/16] (sf_layout 0) or 128x4-swizzled over
- * [rows, K/16] (sf_layout 1; the caller sizes the buffer for the padded extent). Bit-exact with the reference. */
+ * [rows, K/16] (sf_layout 1; the caller sizes the buffer for the padded extent, whose padding is written 0). Bit-exact with the reference. */
 int b200moe_global_scale(const void* x, int dtype, long long n, void* amax_scratch_u32, float* gs_out, void* stream);
 int b200moe_global_scale_grouped(const void* x, int dtype, int groups, long long group_elems, void* amax_scratch_u32,
                                  float* gs_out, void* stream); /* one scale per group (per expert); scratch 4*groups bytes */
 int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int rows, int K, const float* global_scale,
                            int gs_rows, void* packed, void* sf, int sf_layout, void* stream);
+
+/* The same with each group's own global scale, both passes in one launch: x [groups, rows, K] -> gs_out f32 [groups] (2688 / amax,
+ * as b200moe_global_scale), packed u8 [groups, rows, K/2], sf u8 row-major [groups, rows, K/16] (sf_layout 0) or 128x4-swizzled
+ * per group (sf_layout 1: [groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: 8-byte aligned, zeroed once, then only
+ * ever passed to this function (any sizes); calls that may overlap on the GPU need one each. sm120fp4/reference.py:68-90. */
+long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K);
+int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
+                                     int sf_layout, void* workspace, long long workspace_bytes, void* stream);
 
 /* ---- router: sm120fp4/kernels/moe_w4a16.py:85-91 (route; padded form of k_route :48-83) and the torch router of
  * sm120fp4/kernels/fc1_w4a16.py:272-279. ids i32 [P] -> experts i32 [Umax] (ascending, -1 padding), offsets i32

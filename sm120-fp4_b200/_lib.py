@@ -3,9 +3,10 @@ raises, and every non-zero return code raises with the library's own message."""
 from __future__ import annotations
 
 import ctypes as C
+import os
 from pathlib import Path
 
-import os
+import torch
 
 _PKG = Path(__file__).resolve().parent
 # B200MOE_LIB: load another build of the same library (the diagnostic build of `build.py --diag`); default: the product build
@@ -24,6 +25,8 @@ SIGNATURES = {
     "b200moe_global_scale": (_I, [_P, _I, _LL, _P, _P, _P]),
     "b200moe_global_scale_grouped": (_I, [_P, _I, _I, _LL, _P, _P, _P]),
     "b200moe_quantize_nvfp4": (_I, [_P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _P]),
+    "b200moe_quantize_own_scale_workspace_bytes": (_LL, [_I, _I, _I, _I]),
+    "b200moe_quantize_nvfp4_own_scale": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _I, _P, _LL, _P]),
     "b200moe_route_workspace_bytes": (_LL, [_I, _I]),
     "b200moe_route": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _LL, _P]),
     "b200moe_route_status": (_I, [_P, _I, _I, _P]),
@@ -117,5 +120,5 @@ def ptr(t) -> int:
 
 
 def stream_ptr() -> int:
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """cudaStream_t of the current stream of the current device."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

@@ -75,17 +75,20 @@ __global__ void k_global_scale(const unsigned* __restrict__ amax_bits, float* __
 
 // One thread per 16-element block. Destination row r reads source row src_row[r] (or r when src_row is null); a
 // negative source row writes zero codes and zero scales (padding rows of a per-expert segment).
-// sf_layout 0: row-major [rows, K/16]; 1: 128x4 swizzle over [rows, K/16] (rows padded by the caller's buffer).
+// sf_layout 0: row-major [rows, K/16]; 1: 128x4 swizzle over [rows, K/16], padding written 0.
 template <typename T>
 __global__ void __launch_bounds__(256) k_quantize_nvfp4(const T* __restrict__ x, const int* __restrict__ src_row, int rows,
                                                         int K, const float* __restrict__ gs_ptr, int gs_rows,
                                                         uint8_t* __restrict__ packed, uint8_t* __restrict__ sf, int sf_layout) {
   const int bpr = K >> 4;
   const int nkt = (bpr + 3) >> 2;
-  const long long total = (long long)rows * bpr;
+  // 128x4: the padding rows and columns of the swizzled buffer are part of the index space and get zero scales
+  const int prow = sf_layout == 1 ? (rows + 127) & ~127 : rows, pcol = sf_layout == 1 ? 4 * nkt : bpr;
+  const long long total = (long long)prow * pcol;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(i / bpr), b = (int)(i % bpr);
-    const int s = src_row ? src_row[r] : r;
+    const int r = (int)(i / pcol), b = (int)(i % pcol);
+    const bool inside = r < rows && b < bpr;
+    const int s = !inside ? -1 : src_row ? src_row[r] : r;
     uint2 pk = make_uint2(0u, 0u);
     uint8_t sb = 0;
     if (s >= 0) {
@@ -93,7 +96,7 @@ __global__ void __launch_bounds__(256) k_quantize_nvfp4(const T* __restrict__ x,
       load16(x + (long long)s * K + b * 16, v);
       sb = quantize_block16(v, gs_ptr[gs_rows > 0 ? r / gs_rows : 0], pk);   // one global scale per gs_rows destination rows
     }
-    *reinterpret_cast<uint2*>(packed + (long long)r * (K >> 1) + b * 8) = pk;
+    if (inside) *reinterpret_cast<uint2*>(packed + (long long)r * (K >> 1) + b * 8) = pk;
     if (sf_layout == 0) sf[(long long)r * bpr + b] = sb;
     else sf[sf_offset_128x4(r, b, nkt)] = sb;
   }
@@ -189,7 +192,7 @@ extern "C" int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_r
   if (((uintptr_t)x & 15) || ((uintptr_t)packed & 7)) return B200MOE_ERR_ARG;
   if (rows == 0) return B200MOE_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int g = grid_for((long long)rows * (K / 16), 256);
+  const int g = grid_for(sf_layout == 1 ? (rows + 127LL) / 128 * 128 * ((K / 16 + 3) / 4 * 4) : (long long)rows * (K / 16), 256);
   if (dtype == 0)
     k_quantize_nvfp4<<<g, 256, 0, st>>>((const __nv_bfloat16*)x, src_row, rows, K, global_scale, gs_rows, (uint8_t*)packed, (uint8_t*)sf, sf_layout);
   else

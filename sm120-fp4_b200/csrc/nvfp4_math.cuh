@@ -38,11 +38,14 @@ __device__ __forceinline__ void load16(const float* p, float (&v)[16]) {
 // 8 floats -> 8 E2M1 codes in one word (element 2j in the low nibble of byte j). cvt.rn.satfinite.e2m1x2.f32 d, a, b puts
 // a into the high and b into the low nibble of d.
 __device__ __forceinline__ uint32_t e2m1x8_rn(const float* v) {
-  uint32_t b[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    asm("{\n .reg .b8 t;\n cvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\n cvt.u32.u8 %0, t;\n}\n" : "=r"(b[i]) : "f"(v[2 * i + 1]), "f"(v[2 * i]));
-  return (b[0] | (b[1] << 8)) | ((b[2] << 16) | (b[3] << 24));
+  uint32_t r;
+  asm("{\n .reg .b8 b0, b1, b2, b3;\n"
+      " cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n"
+      " cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n"
+      " mov.b32 %0, {b0, b1, b2, b3};\n}\n"
+      : "=r"(r)
+      : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  return r;
 }
 
 // Quantize one 16-element block: returns the E4M3 scale byte, writes 8 packed bytes.
@@ -72,13 +75,7 @@ __device__ __forceinline__ void fill_scale_table(float* table, float gs, int tid
     table[b] = sf_val > 0.f && sf_val == sf_val ? __fdiv_rn(gs, sf_val) : 0.f;
   }
 }
-__device__ __forceinline__ uint8_t quantize_block16_t(const float (&v)[16], float gs, const float* __restrict__ table, uint2& packed) {
-  float m[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) m[i] = fmaxf(fabsf(v[i]), fabsf(v[i + 8]));
-#pragma unroll
-  for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], m[i + 4]);
-  const float amax = fmaxf(fmaxf(m[0], m[2]), fmaxf(m[1], m[3]));
+__device__ __forceinline__ uint8_t quantize_block16_t(const float (&v)[16], float amax, float gs, const float* __restrict__ table, uint2& packed) {
   const float sf_f = fminf(__fmul_rn(__fdiv_rn(amax, 6.0f), gs), 448.0f);
   const __nv_fp8_storage_t sfb = __nv_cvt_float_to_fp8(sf_f, __NV_SATFINITE, __NV_E4M3);
   const float scale = table[sfb & 127];
@@ -87,6 +84,14 @@ __device__ __forceinline__ uint8_t quantize_block16_t(const float (&v)[16], floa
   for (int i = 0; i < 16; ++i) sc[i] = __fmul_rn(v[i], scale);
   packed = make_uint2(e2m1x8_rn(sc), e2m1x8_rn(sc + 8));
   return (uint8_t)sfb;
+}
+__device__ __forceinline__ uint8_t quantize_block16_t(const float (&v)[16], float gs, const float* __restrict__ table, uint2& packed) {
+  float m[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m[i] = fmaxf(fabsf(v[i]), fabsf(v[i + 8]));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = fmaxf(m[i], m[i + 4]);
+  return quantize_block16_t(v, fmaxf(fmaxf(m[0], m[2]), fmaxf(m[1], m[3])), gs, table, packed);
 }
 
 }  // namespace b200

@@ -1,0 +1,394 @@
+// NVFP4 quantisation with the group's own global scale (2688 / amax): the amax pass and the quantising pass in ONE launch. Same
+// bytes as b200moe_global_scale_grouped followed by b200moe_quantize_nvfp4 (sm120fp4/reference.py:68-90).
+//
+// Small inputs (up to 64 rows of 2048) stay in the registers of one thread-block cluster between the two passes: what bounds
+// them is launches and round trips, and this is one launch with one exchange of maxima over distributed shared memory.
+// Large ones are bound by HBM: the input has to be read twice, but the second read of a group comes right after the first, when
+// the group is still in L2. Work units (64 KB of input) are taken round-robin in an order that keeps a window of groups open:
+// amax(0) .. amax(W-1), then amax(g + W), quantise(g) in turn. A quantising unit waits until its group's amax units have
+// published their maxima; they all stand earlier in the order, and every block takes its units in that order.
+#include "common.cuh"
+#include "nvfp4_math.cuh"
+#include "tcgen05.cuh"
+
+namespace b200 {
+
+constexpr int kQThreads = 512;                                   // of the small form
+constexpr int kQgThreads = 256;                                  // of the large form, two blocks per SM (three of 32 KB units: 3 % slower; four, or the next unit's loads ahead of this one's math: 15 % and more)
+constexpr int kQSmallPerThread = 2;                              // 16-value blocks a thread keeps in registers
+constexpr int kQSmallMaxBlocks = 8 * kQThreads * kQSmallPerThread;
+template <typename T> constexpr int kQPerThread = sizeof(T) == 2 ? 8 : 4;   // 16-value blocks a thread takes of one work unit (64 KB of input)
+constexpr long long kQWindowBytes = 20ll << 20;                  // input bytes between a group's two passes: L2 holds about this and what is in flight (40 MB: 5 % slower)
+
+struct QuantGeom {
+  int rows, bpr;           // rows of a group, 16-value blocks per row
+  int layout;              // 0: scales row-major [groups * rows][bpr]; 1: 128x4 swizzle per group, padded to 128 rows x 4 columns
+  long long sf_stride;     // scale bytes of a group
+  int nkt;
+  bool wide;               // x is 32-byte aligned
+  // i / bpr = i * bpr_inv >> bpr_shift with bpr_inv = ceil(2^shift / bpr): exact while i * (bpr_inv * bpr - 2^shift) < 2^shift, which
+  // i < 2^30 and shift = 30 + the bits of bpr grant
+  unsigned long long bpr_inv;
+  int bpr_shift;
+  int step_r, step_c;      // kQgThreads blocks on, as rows and columns
+};
+
+__device__ __forceinline__ long long sf_swizzled(int r, int c, int nkt) {
+  return ((long long)(r >> 7) * nkt + (c >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (c & 3);
+}
+
+// global_scale = reciprocal(max(amax, 1e-12)) * 2688 with the reference's two roundings (see k_global_scale)
+__device__ __forceinline__ float scale_of(float amax) { return __fmul_rn(__frcp_rn(fmaxf(amax, 1e-12f)), 2688.0f); }
+
+// 16 values as loaded
+template <typename T> struct Raw16 { uint4 r[sizeof(T)]; };
+// wide: the address is 32-byte aligned, so that a thread's 32 (64) bytes are one (two) 256-bit loads and every sector is asked for once
+template <typename T> __device__ __forceinline__ void load_raw(const T* p, bool wide, Raw16<T>& v) {
+  if (wide) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T); i += 2)
+      asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(v.r[i].x), "=r"(v.r[i].y), "=r"(v.r[i].z), "=r"(v.r[i].w), "=r"(v.r[i + 1].x), "=r"(v.r[i + 1].y), "=r"(v.r[i + 1].z), "=r"(v.r[i + 1].w)
+                   : "l"(reinterpret_cast<const uint4*>(p) + i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T); ++i) v.r[i] = reinterpret_cast<const uint4*>(p)[i];
+  }
+}
+// largest magnitude of the 16 values (NaNs are passed over, as fmaxf does)
+__device__ __forceinline__ float amax_raw(const Raw16<__nv_bfloat16>& v) {
+  const uint32_t w[8] = {v.r[0].x, v.r[0].y, v.r[0].z, v.r[0].w, v.r[1].x, v.r[1].y, v.r[1].z, v.r[1].w};
+  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+  const uint32_t b = *reinterpret_cast<const uint32_t*>(&m);
+  return fmaxf(fmaxf(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), 0.f);
+}
+__device__ __forceinline__ float amax_raw(const Raw16<float>& v) {
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    m = fmaxf(fmaxf(fmaxf(m, fabsf(__uint_as_float(v.r[i].x))), fmaxf(fabsf(__uint_as_float(v.r[i].y)), fabsf(__uint_as_float(v.r[i].z)))),
+              fabsf(__uint_as_float(v.r[i].w)));
+  return m;
+}
+__device__ __forceinline__ void floats(const Raw16<__nv_bfloat16>& v, float (&f)[16]) {
+  const uint32_t w[8] = {v.r[0].x, v.r[0].y, v.r[0].z, v.r[0].w, v.r[1].x, v.r[1].y, v.r[1].z, v.r[1].w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { f[2 * i] = __uint_as_float(w[i] << 16); f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+}
+__device__ __forceinline__ void floats(const Raw16<float>& v, float (&f)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[4 * i] = __uint_as_float(v.r[i].x), f[4 * i + 1] = __uint_as_float(v.r[i].y), f[4 * i + 2] = __uint_as_float(v.r[i].z), f[4 * i + 3] = __uint_as_float(v.r[i].w);
+  }
+}
+
+__device__ __forceinline__ float amax16(const float (&v)[16]) {
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(v[i]));
+  return m;
+}
+
+// amax / 6 rounded to nearest for a bf16 amax: quotient by the rounded reciprocal, one residual correction (Markstein's division
+// step). Exact for every bf16 value from 2^-100 up; below that the block's scale is zero whatever the quotient (the largest
+// global scale is 2688 / 1e-12), so nothing depends on it. An fp32 amax takes the IEEE division.
+__device__ __forceinline__ float sixth(float amax, __nv_bfloat16) {
+  const float q = __fmul_rn(amax, 1.0f / 6.0f);
+  return __fmaf_rn(__fmaf_rn(-6.0f, q, amax), 1.0f / 6.0f, q);
+}
+__device__ __forceinline__ float sixth(float amax, float) { return __fdiv_rn(amax, 6.0f); }
+
+// quantize_block16 on values as loaded, its second division looked up and two products per instruction
+template <typename T>
+__device__ __forceinline__ uint32_t quantize_raw(const Raw16<T>& v, float gs, const float* table, uint2& packed) {
+  const float sf_f = fminf(__fmul_rn(sixth(amax_raw(v), T()), gs), 448.0f);
+  uint16_t sb;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb) : "f"(0.0f), "f"(sf_f));
+  const float scale = table[sb & 127];
+  float f[16];
+  floats(v, f);
+#pragma unroll
+  for (int i = 0; i < 16; i += 2)
+    asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %2};\n mul.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}\n"
+        : "+f"(f[i]), "+f"(f[i + 1]) : "f"(scale));
+  packed = make_uint2(e2m1x8_rn(f), e2m1x8_rn(f + 8));
+  return sb;
+}
+
+// maximum over the block's threads, in every thread
+__device__ __forceinline__ float block_max(float m, float* wm) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = wm[threadIdx.x & 15];
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return m;
+}
+
+__device__ __forceinline__ void zero_padding(uint8_t* sf, const QuantGeom& q, int first, int step) {   // 128x4: rows and columns beyond the matrix
+  const int prow = (q.rows + 127) & ~127, pcol = q.nkt * 4;
+  const int spare = pcol - q.bpr;
+  for (int i = first; i < (prow - q.rows) * pcol; i += step) sf[sf_swizzled(q.rows + i / pcol, i % pcol, q.nkt)] = 0;
+  if (spare > 0)
+    for (int i = first; i < q.rows * spare; i += step) sf[sf_swizzled(i / spare, q.bpr + i % spare, q.nkt)] = 0;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kQThreads) k_quantize_small(const T* x, QuantGeom q, float* gs_out, uint8_t* packed, uint8_t* sf) {
+  __shared__ float wm[kQThreads / 32];
+  __shared__ int s_max;
+  const int tid = threadIdx.x, rank = (int)cluster_ctarank(), C = (int)gridDim.x, nblk = q.rows * q.bpr;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  float v[kQSmallPerThread][16], m = 0.f;
+#pragma unroll
+  for (int j = 0; j < kQSmallPerThread; ++j) {
+    const int i = rank * kQThreads + tid + j * C * kQThreads;
+    if (i < nblk) {
+      load16(x + (long long)i * 16, v[j]);
+      m = fmaxf(m, amax16(v[j]));
+    }
+  }
+  m = block_max(m, wm);
+  if (tid == 0) s_max = __float_as_int(m);
+  cluster_sync_all();
+  int mb = 0;   // non-negative floats order like their bit patterns
+  for (int c = 0; c < C; ++c) {
+    int o;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(o) : "r"(mapa_shared(smem_u32(&s_max), (uint32_t)c)) : "memory");
+    mb = max(mb, o);
+  }
+  cluster_arrive();
+  const float gs = scale_of(__int_as_float(mb));
+  if (rank == 0 && tid == 0) *gs_out = gs;
+#pragma unroll
+  for (int j = 0; j < kQSmallPerThread; ++j) {
+    const int i = rank * kQThreads + tid + j * C * kQThreads;
+    if (i < nblk) {
+      uint2 pk;
+      const uint8_t sb = quantize_block16(v[j], gs, pk);
+      *reinterpret_cast<uint2*>(packed + (long long)i * 8) = pk;
+      if (q.layout == 0) sf[i] = sb;
+      else sf[sf_swizzled(i / q.bpr, i % q.bpr, q.nkt)] = sb;
+    }
+  }
+  if (q.layout == 1) zero_padding(sf, q, rank * kQThreads + tid, C * kQThreads);
+  cluster_wait();
+}
+
+// scratch: [0] number of the calls that have used it, [1] blocks of this call that have left (zero between calls); then one 8-byte
+// word {call number + 1, bits of the largest magnitude} per amax unit. A word is stored whole, so whoever reads this call's
+// number in it has the maximum: nothing is counted and nothing is fenced, and a unit's only round trip to L2 overlaps its loads.
+// (With a ticket per unit and counters behind a fence: 330 to 400 us for 128 x 1536 x 2048 bf16.)
+__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, int groups, int units, int window, QuantGeom q, float* gs_out,
+                                                                    uint8_t* packed, uint8_t* sf, unsigned* scratch) {
+  constexpr int kWarps = kQgThreads / 32, kPer = kQPerThread<T>;
+  __shared__ float wm[2][kWarps];
+  __shared__ float s_table[128];
+  __shared__ int3 s_next[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nblk = q.rows * q.bpr;             // 16-value blocks of a group
+  const unsigned total = 2u * (unsigned)groups * (unsigned)units;
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(scratch + 2);
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const unsigned call = __ldcg(scratch) + 1u;   // nobody advances it before every block of this call has left
+  float gs_table = -1.f;                        // the global scale s_table was filled for
+  int k = 0;
+  // maximum over the block, one barrier (the buffer of the unit before may still be read)
+  auto unit_max = [&](float m) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) wm[k][warp] = m;
+    __syncthreads();
+    m = wm[k][lane & (kWarps - 1)];
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    k ^= 1;
+    return m;
+  };
+  // place t in the order -> (group, unit, pass). One thread works it out for the next unit while the block is at the current one.
+  auto place = [&](unsigned t) {
+    const unsigned head = (unsigned)window * (unsigned)units, n = (unsigned)units;
+    if (t >= total) return make_int3(-1, 0, 0);
+    if (t < head) return make_int3((int)(t / n), (int)(t % n), 0);
+    const unsigned r = t - head, pairs = (unsigned)(groups - window);
+    if (r < pairs * 2u * n) {
+      const unsigned p = r / (2u * n), o = r - p * 2u * n;
+      return o < n ? make_int3((int)p + window, (int)o, 0) : make_int3((int)p, (int)(o - n), 1);
+    }
+    const unsigned o = r - pairs * 2u * n;
+    return make_int3((int)(pairs + o / n), (int)(o % n), 1);
+  };
+  if (tid == 0) s_next[0] = place(blockIdx.x);
+  __syncthreads();
+  unsigned t1 = blockIdx.x + gridDim.x;        // the place that is worked out next
+  auto load = [&](const int3& at, Raw16<T> (&v)[kPer]) {
+    if (at.x < 0) return;
+    const int i0 = at.y * (kPer * kQgThreads), left = nblk - i0 - tid;   // this thread's blocks: i0 + tid + j * threads while j * threads < left
+    const T* src = x + ((long long)at.x * nblk + i0 + tid) * 16;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (j * kQgThreads < left) load_raw(src + j * kQgThreads * 16, q.wide, v[j]);
+  };
+  auto process = [&](const int3& at, const Raw16<T> (&v)[kPer]) {
+    const int g = at.x, u = at.y;
+    const bool second = at.z != 0;
+    unsigned long long* gw = words + (long long)g * units;
+    const int i0 = u * (kPer * kQgThreads), left = nblk - i0 - tid;
+    const long long first = (long long)g * nblk + i0 + tid;
+    if (!second) {
+      float m = 0.f;
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (j * kQgThreads < left) m = fmaxf(m, amax_raw(v[j]));
+      m = unit_max(m);
+      if (tid == 0) __stcg(gw + u, ((unsigned long long)call << 32) | __float_as_uint(m));
+      return;
+    }
+    float m = 0.f;
+    for (int w = tid; w < units; w += kQgThreads) {
+      unsigned long long word = 0;
+      bool ok = false;
+      for (int it = 0; it < (1 << 22); ++it) {
+        word = ld_relaxed_gpu_u64(gw + w);
+        ok = (unsigned)(word >> 32) == call;
+        if (ok) break;
+        __nanosleep(100);
+      }
+      // a wait that ran out (a block of this grid was held up for seconds): take that unit's maximum here
+      if (!ok) {
+        float mm = 0.f;
+        Raw16<T> raw;
+        for (int i = w * (kPer * kQgThreads); i < min(nblk, (w + 1) * (kPer * kQgThreads)); ++i) { load_raw(x + ((long long)g * nblk + i) * 16, q.wide, raw); mm = fmaxf(mm, amax_raw(raw)); }
+        word = __float_as_uint(mm);
+      }
+      m = fmaxf(m, __uint_as_float((unsigned)word));
+    }
+    const float gs = scale_of(unit_max(m));
+    if (gs != gs_table) {
+      fill_scale_table(s_table, gs, tid, kQgThreads);
+      gs_table = gs;
+      __syncthreads();
+    }
+    uint8_t* sfg = sf + (long long)g * q.sf_stride;
+    uint2* codes = reinterpret_cast<uint2*>(packed) + first;
+    uint8_t* sfl = sfg + i0 + tid;                                    // row-major place
+    int r = 0, c = 0;                                                 // 128x4: (row, scale column) of the block
+    if (q.layout == 1) {
+      r = (int)(((unsigned long long)(unsigned)(i0 + tid) * q.bpr_inv) >> q.bpr_shift);
+      c = i0 + tid - r * q.bpr;
+    }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (j * kQgThreads < left) {
+        uint2 pk;
+        const uint32_t sb = quantize_raw(v[j], gs, s_table, pk);
+        __stcg(codes + j * kQgThreads, pk);
+        if (q.layout == 0) {
+          sfl[j * kQgThreads] = (uint8_t)sb;
+        } else {
+          sfg[((r >> 7) * q.nkt + (c >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (c & 3)] = (uint8_t)sb;
+          r += q.step_r, c += q.step_c;
+          if (c >= q.bpr) { c -= q.bpr; ++r; }
+        }
+      }
+    }
+    if (u == 0) {
+      if (tid == 0) gs_out[g] = gs;
+      if (q.layout == 1) zero_padding(sfg, q, tid, kQgThreads);
+    }
+  };
+  for (;;) {
+    const int3 at = s_next[k];
+    if (at.x < 0) break;
+    if (tid == kQgThreads - 1) s_next[k ^ 1] = place(t1);   // read behind this unit's barrier
+    t1 += gridDim.x;
+    Raw16<T> v[kPer];
+    load(at, v);
+    process(at, v);
+  }
+  __syncthreads();
+  if (tid == 0 && atomicAdd(scratch + 1, 1u) == gridDim.x - 1u) { scratch[1] = 0u; scratch[0] = call; }
+}
+
+}  // namespace b200
+
+using namespace b200;
+
+static int quant_units(int dtype, int rows, int K) {
+  const long long nblk = (long long)rows * (K / 16), unit = kQgThreads * (dtype == 0 ? kQPerThread<__nv_bfloat16> : kQPerThread<float>);
+  return (int)((nblk + unit - 1) / unit);
+}
+
+extern "C" long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K) {
+  if (groups <= 0 || rows < 0 || K <= 0 || (dtype != 0 && dtype != 1)) return B200MOE_ERR_ARG;
+  return 8 + 8LL * groups * quant_units(dtype, rows, K);
+}
+
+// x [groups, rows, K] (dtype 0 bf16, 1 f32) -> gs_out f32 [groups], packed u8 [groups, rows, K/2], sf u8: sf_layout 0 row-major
+// [groups, rows, K/16], 1 the 128x4 swizzle per group ([groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: zeroed once,
+// then only ever passed to this function; two calls that may overlap on the GPU need one each.
+extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
+                                                void* workspace, long long workspace_bytes, void* stream) {
+  if (!x || !gs_out || !packed || !sf || !workspace || groups <= 0 || rows < 0) return B200MOE_ERR_ARG;
+  if (K <= 0 || K % 16) return B200MOE_ERR_SHAPE;
+  if ((dtype != 0 && dtype != 1) || (sf_layout != 0 && sf_layout != 1)) return B200MOE_ERR_ARG;
+  if (((uintptr_t)x & 15) || ((uintptr_t)packed & 7) || ((uintptr_t)workspace & 7)) return B200MOE_ERR_ARG;
+  if (workspace_bytes < b200moe_quantize_own_scale_workspace_bytes(dtype, groups, rows, K)) return B200MOE_ERR_WORKSPACE;
+  if (rows == 0) return B200MOE_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  QuantGeom q;
+  q.rows = rows, q.bpr = K / 16, q.layout = sf_layout, q.nkt = (q.bpr + 3) / 4;
+  q.sf_stride = sf_layout == 0 ? (long long)rows * q.bpr : ((rows + 127LL) / 128 * 128) * q.nkt * 4;
+  q.wide = ((uintptr_t)x & 31) == 0;
+  q.bpr_shift = 30;
+  for (int b = q.bpr; b; b >>= 1) ++q.bpr_shift;
+  q.bpr_inv = ((1ULL << q.bpr_shift) + q.bpr - 1) / q.bpr;
+  q.step_r = kQgThreads / q.bpr, q.step_c = kQgThreads % q.bpr;
+  const long long nblk = (long long)rows * q.bpr;
+  if (q.sf_stride > 0x7fffffffLL) return B200MOE_ERR_LIMIT;
+  if (nblk > (1LL << 30)) return B200MOE_ERR_LIMIT;
+  unsigned* scratch = (unsigned*)workspace;
+  if (groups == 1 && nblk <= kQSmallMaxBlocks) {
+    int C = 1;   // CTAs: one block per thread, then two
+    while (C < 8 && C * kQThreads < nblk) C *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C), cfg.blockDim = dim3(kQThreads), cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr, cfg.numAttrs = 2;
+    if (dtype == 0) B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_quantize_small<__nv_bfloat16>, (const __nv_bfloat16*)x, q, gs_out, (uint8_t*)packed, (uint8_t*)sf));
+    else B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_quantize_small<float>, (const float*)x, q, gs_out, (uint8_t*)packed, (uint8_t*)sf));
+    return B200MOE_OK;
+  }
+  const int units = quant_units(dtype, rows, K);
+  if (2LL * groups * units > 0x7fffffffLL) return B200MOE_ERR_LIMIT;
+  long long w = kQWindowBytes / (nblk * (dtype == 0 ? 32 : 64));
+  const int window = (int)(w < 1 ? 1 : w > groups ? groups : w);
+  static int sms = 0;   // of the first device used: all devices of a machine are alike, and any grid size is correct
+  if (!sms) {
+    int dev = 0, n = 0;
+    B200_CUDA_TRY(cudaGetDevice(&dev));
+    B200_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    sms = n;
+  }
+  const long long most = 2LL * groups * units;
+  const int grid = (int)(most < 2LL * sms ? most : 2LL * sms);
+  void* args[] = {(void*)&x, (void*)&groups, (void*)&units, (void*)&window, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch};
+  return launch_kernel(dtype == 0 ? (const void*)k_quantize_grouped<__nv_bfloat16> : (const void*)k_quantize_grouped<float>, grid, kQgThreads, 0, true, args, st);
+}

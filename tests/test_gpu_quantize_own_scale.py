@@ -1,0 +1,56 @@
+"""The one-launch quantiser (amax, scale and codes in one kernel) byte for byte against the oracle, at the sizes where its two
+forms and their work units meet: one cluster up to 8192 blocks of 16 values, work units of 2048 (bf16) or 1024 (f32) blocks above."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import nvfp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,k", [(1, 16), (31, 272), (64, 2048), (65, 2032), (64, 2064), (257, 1040), (1024, 2048)])
+def test_single_matrix(rows, k, dtype):
+    import sm120fp4_b200 as pkg
+    x = (torch.randn(rows, k, generator=torch.Generator().manual_seed(rows * 7 + k)) * 3).to(dtype)
+    x[rows // 2, k // 3] = 77.0
+    wq, wsf, wgs = O.quantize_nvfp4(x.float().numpy(), None)
+    for _ in range(2):      # the second call finds the workspace as the first left it
+        q, sf, gs = pkg.quantize_nvfp4(x.cuda())
+        assert np.array_equal(gs.cpu().numpy().view(np.uint32), wgs.view(np.uint32))
+        assert np.array_equal(q.cpu().numpy(), wq) and np.array_equal(sf.cpu().numpy(), wsf)
+    q, sw, _ = pkg.quantize_nvfp4_128x4(x.cuda(), gs)
+    assert np.array_equal(q.cpu().numpy(), wq) and np.array_equal(sw.cpu().numpy(), O.to_128x4(wsf))
+
+
+@pytest.mark.parametrize("swizzle", [False, True])
+@pytest.mark.parametrize("groups,rows,k", [(1, 64, 64), (3, 100, 80), (5, 129, 1040), (40, 192, 512)])
+def test_stacked_matrices(groups, rows, k, swizzle):
+    import sm120fp4_b200 as pkg
+    scale = torch.linspace(0.01, 9.0, groups)[:, None, None]
+    w = (torch.randn(groups, rows, k, generator=torch.Generator().manual_seed(groups)) * scale).to(torch.bfloat16)
+    q, sf, gs = pkg.quantize_nvfp4_experts(w.cuda(), swizzle=swizzle)
+    for g in range(groups):
+        wq, wsf, wgs = O.quantize_nvfp4(w[g].float().numpy(), None)
+        assert np.array_equal(gs[g:g + 1].cpu().numpy().view(np.uint32), wgs.view(np.uint32))
+        assert np.array_equal(q[g].cpu().numpy(), wq)
+        assert np.array_equal(sf[g].cpu().numpy(), O.to_128x4(wsf) if swizzle else wsf)
+
+
+def test_every_bf16_amax():
+    """Every positive bf16 value up to 2^60 as a block's largest magnitude, in matrices whose global scale makes the block scales
+    land on all of E4M3's range: the block scale's division has a form of its own for bf16 inputs."""
+    import sm120fp4_b200 as pkg
+    bits = torch.arange(1, (127 + 60) << 7, dtype=torch.int32).to(torch.int16)
+    for top in (2.0 ** 60, 2.0 ** 20, 1.0, 2.0 ** -20):
+        v = bits.view(torch.bfloat16)
+        v = v[v.float() <= top]
+        x = torch.zeros(v.numel(), 16, dtype=torch.bfloat16)
+        x[:, 5] = v
+        x = x[-(-x.shape[0] // 2):] if x.shape[0] > 1 << 16 else x
+        for rows in (x, x[-8000:]):          # the large and the small form
+            wq, wsf, wgs = O.quantize_nvfp4(rows.float().numpy(), None)
+            q, sf, gs = pkg.quantize_nvfp4(rows.contiguous().cuda())
+            assert np.array_equal(gs.cpu().numpy().view(np.uint32), wgs.view(np.uint32))
+            assert np.array_equal(sf.cpu().numpy(), wsf) and np.array_equal(q.cpu().numpy(), wq), top
