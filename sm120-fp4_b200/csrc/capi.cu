@@ -208,11 +208,23 @@ extern "C" int b200moe_layer_set_act_scale(b200moe_layer* L, float g1) {
   return B200MOE_OK;
 }
 
+// Ring slots of the tcgen05 decode kernel beside the x operand (FC1) or the activation slabs (FC2) that share `region` bytes; 0 when
+// fewer than three fit (hidden sizes near 4096 at more than eight tokens).
+static int decode_tc_ring(const b200moe_layer* L, int N, int* region) {
+  const int xb = L->KB1 * N * 128 + L->KT1 * 512, slab = N * 128 + 2048;
+  for (int NS = 12; NS >= 3; --NS) {
+    *region = (int)align_up(xb > NS * slab ? xb : NS * slab, 1024);
+    if (b200_decode_tc_smem_bytes(NS, *region) <= 227 * 1024 - 6144) return NS;   // room for static shared memory
+  }
+  return 0;
+}
+
+static int decode_tc_columns(int M) { return M <= 4 ? 16 : M <= 8 ? 32 : 64; }   // of the B operand: four terms per token
+
 static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, void* stream) {
   uint8_t* w = (uint8_t*)ws;
   cudaStream_t st = (cudaStream_t)stream;
-  const int nbv = M <= 4 ? 0 : M <= 8 ? 1 : 2;
-  const int N = 16 << nbv;
+  const int N = decode_tc_columns(M);
   int rc = b200_expand_x_launch(x, M, L->H, N, L->KB1, w + L->off_xb, (float*)(w + L->off_xscale), chained, st);
   if (rc != B200MOE_OK) return rc;
   DecodeTcParams p;
@@ -233,14 +245,10 @@ static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const floa
   p.M = M, p.E = L->E, p.H = L->H, p.I = L->I, p.top_k = L->top_k;
   p.Umax = L->E < M * L->top_k ? L->E : M * L->top_k;
   p.KB1 = L->KB1, p.KB2 = L->KB2, p.CB1 = L->CB1, p.NB2 = L->NB2, p.KT1 = L->KT1, p.KT2 = L->KT2;
-  const int xb = L->KB1 * N * 128 + L->KT1 * 512, slab = N * 128 + 2048;
-  int NS = 12;
-  for (; NS >= 2; --NS) {
-    const int region = (int)align_up(xb > NS * slab ? xb : NS * slab, 1024);
-    if (b200_decode_tc_smem_bytes(NS, region) <= 227 * 1024 - 6144) { p.region_bytes = region; break; }   // room for static shared memory
-  }
-  if (NS < 2) return B200MOE_ERR_SHAPE;
-  p.NS = NS;
+  int region = 0;
+  const int NS = decode_tc_ring(L, N, &region);
+  if (NS == 0) return B200MOE_ERR_SHAPE;
+  p.NS = NS, p.region_bytes = region;
   return b200_decode_tc_launch(p, L->sms, b200_decode_tc_smem_bytes(NS, p.region_bytes), chained, st);
 }
 
@@ -301,9 +309,10 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
 // flags bit 0 (B200MOE_ORDERED): both kernels of the call are ordinary stream-ordered launches.
 extern "C" int b200moe_decode_forward_ex(const b200moe_layer* L, const void* x_bf16, const int* topk_ids, const float* topk_weights,
                                          int M, void* out_bf16, void* workspace, long long workspace_bytes, int flags, void* stream) {
-  // the tcgen05 kernel whenever the tile records exist and the shape fits it: x scale tiles of <= 12 K boxes in TMEM, one
-  // worker group per 128-row output block
-  if (L && L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 12 && L->NB2 <= L->sms) {
+  // the tcgen05 kernel whenever the tile records exist and the shape fits it: x scale tiles of <= 16 K boxes in TMEM, one
+  // worker group per 128-row output block, and a ring of at least three records beside the x operand
+  int region;
+  if (L && L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 16 && L->NB2 <= L->sms && decode_tc_ring(L, decode_tc_columns(M), &region) > 0) {
     if (!x_bf16 || !topk_ids || !topk_weights || !out_bf16 || !workspace || M < 0) return B200MOE_ERR_ARG;
     if (M > 16) return B200MOE_ERR_LIMIT;
     if (workspace_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;

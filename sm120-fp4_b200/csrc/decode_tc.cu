@@ -11,13 +11,15 @@
 // 1/g_t. Four terms carry more mantissa than bf16 for the values that decide a dot product and keep the layer's error
 // against the fp32 oracle below the bf16 output rounding.
 //
-// Structure: one CTA per SM = one stream-K worker. Warps 0-3: epilogue (tcgen05.ld of a double-buffered TMEM accumulator,
-// term sums, SiLU*mul, re-expansion of the activations for FC2, fixed-order reduction of split units). Warps 4-7: scale
-// warps, one per TMEM lane quadrant (scale tiles of a landed stage shared memory -> registers -> TMEM). Warp 8: MMA issuer
-// (converged warp, one elected lane: four K=64 MMAs per 256-code tile, tcgen05.commit frees the ring stage). Warps 9-10:
-// TMA producers (one bulk copy per 18 KB tile record into a shared-memory ring, FC2 tiles prefetched across the
-// FC1->FC2 grid barrier). The per-tile loops of the single-thread roles are kept free of divisions: at 148 tiles per
-// microsecond per GPU a role has only a few hundred cycles per tile.
+// Structure: one CTA per SM = one worker. Warps 0-3: epilogue (tcgen05.ld of a double-buffered TMEM accumulator, term sums,
+// SiLU*mul, re-expansion of the activations for FC2, fixed-order reduction of partials). Warp 4: MMA issuer - converged, one
+// elected lane; it waits for a record, copies its scale tiles into TMEM (tcgen05.cp), issues the four K=64 MMAs and commits
+// the ring slot: operations of one lane execute in order, so a record passes from the producer to the tensor core
+// in one hand-off. Warps 5-6: producers (one bulk copy per 18 KB record into the ring, FC2 records prefetched across the gates).
+// Warp 7: routing tables. What bounds it: at 16 tokens the weight stream (an SM's share of HBM is a record per ~740 cycles, the
+// issuer needs ~300 for one), at 1 token a chain of latencies: launch, routing tables, first record, eight
+// records of a unit, gate, three records of FC2, reduction. (With four warps that moved the scales through registers, and
+// an issuer whose lanes left their waits one by one, a record took about 1,000 cycles of issue alone.)
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "decode_params.h"
@@ -27,8 +29,9 @@
 
 namespace b200 {
 
-constexpr int kTcProducers = 2;    // TMA producer warps: one thread issues only ~2.5 M bulk operations per second
-constexpr int kTcThreads = (4 + 4 + 1 + kTcProducers) * 32;   // epilogue warps 0-3, scale warps 4-7, MMA warp 8, producers 9..
+constexpr int kTcMmaWarp = 4, kTcProd0 = 5, kTcTablesWarp = 7;
+constexpr int kTcProducers = 2;    // producer warps: one thread's wait + issue round is ~430 cycles
+constexpr int kTcThreads = 8 * 32;
 constexpr int kTcStage = 18432;   // 16 KB codes + 2 KB scale tiles
 constexpr int kTcMaxE = 256, kTcMaxP = 256;
 
@@ -43,7 +46,7 @@ struct TcTables {
   volatile int abort_flag;
   int last_flag;
   uint32_t tmem_base;
-  uint64_t full[12], empty[12], sfr[12];   // stage landed / stage consumed / scale tiles of the stage are in TMEM
+  uint64_t full[12], empty[12];   // stage landed / stage consumed
   uint64_t acc_full[2], acc_empty[2];
   uint64_t xb_full, fc1_done;   // x operand landed / this worker's FC1 MMAs are complete
 };
@@ -176,7 +179,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   uint8_t* region = smem + NS * kTcStage;                 // FC1: resident x operand [KB1][N x 128 B] then its scale tiles;
                                                           // FC2: NS activation slabs
   TcTables& T = *reinterpret_cast<TcTables*>(region + P.region_bytes);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (a value from lane 0 is known to be warp-uniform)
 #ifdef B200_TIMERS
   if (tid == 0 && P.debug) { unsigned long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); P.debug[blockIdx.x * 16 + 13] = (long long)g; }
 #endif
@@ -198,10 +202,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   // gates of the launch before it on this workspace have opened: whatever this thread reads, rounding down to a multiple of
   // V gives the count before this launch (other workers of this launch may have arrived already).
   unsigned long long my_gate = 0;
-  if (tid == 9 * 32) my_gate = ld_acquire_gpu_u64(P.gates);
-  if (tid == 10 * 32) my_gate = ld_acquire_gpu_u64(P.gates + 1);
+  if (tid == kTcProd0 * 32) my_gate = ld_acquire_gpu_u64(P.gates);
+  if (tid == (kTcProd0 + 1) * 32) my_gate = ld_acquire_gpu_u64(P.gates + 1);
   if (tid == 0) {
-    for (int s = 0; s < NS; ++s) { mbar_init(&T.full[s], 1); mbar_init(&T.empty[s], 1); mbar_init(&T.sfr[s], 4); }
+    for (int s = 0; s < NS; ++s) { mbar_init(&T.full[s], 1); mbar_init(&T.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&T.acc_full[b], 1); mbar_init(&T.acc_empty[b], 4); }
     mbar_init(&T.xb_full, 1);
     mbar_init(&T.fc1_done, 1);
@@ -209,7 +213,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     T.last_flag = 0;
     fence_mbar_init();
   }
-  if (warp == 8) {                       // the MMA warp owns the TMEM allocation (all 512 columns: one CTA per SM)
+  if (warp == kTcMmaWarp) {              // the MMA warp owns the TMEM allocation (all 512 columns: one CTA per SM)
     tmem_alloc(&T.tmem_base, 512);
     tmem_relinquish();
   }
@@ -241,15 +245,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     if (lane == 31) T.U = iff;
   }
   __syncthreads();
-  const int U = T.U;
+  const int U = __shfl_sync(0xffffffffu, T.U, 0);
   if (tid < P.E && T.cnt[tid] > 0) {   // thread e: expert e is touched -> its slot in the tables of touched experts
     const int u = T.uidx[tid] - 1;
     T.experts[u] = tid;
     T.a1[u] = ex_a1;
     T.a2n[u] = ex_a2 * a2inv;
   }
-  if (tid == 9 * 32) T.gate0[0] = my_gate - my_gate % (unsigned long long)V;
-  if (tid == 10 * 32) T.gate0[1] = my_gate - my_gate % (unsigned long long)V;
+  if (tid == kTcProd0 * 32) T.gate0[0] = my_gate - my_gate % (unsigned long long)V;
+  if (tid == (kTcProd0 + 1) * 32) T.gate0[1] = my_gate - my_gate % (unsigned long long)V;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -286,16 +290,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   if (tid == 0 && P.debug) { unsigned long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); P.debug[blockIdx.x * 16 + 15] = (long long)g;
     unsigned sm; asm volatile("mov.u32 %0, %%smid;" : "=r"(sm)); P.debug[blockIdx.x * 16 + 11] = sm; }
 #endif
-  const uint32_t tmem = T.tmem_base;
-  const uint32_t tm_acc = tmem, tm_sfa = tmem + 128, tm_sfb = tmem + 320;   // accumulators 2 x 64 | weight scales NS x 16 (<= 192) | operand scales (<= 192)
+  const uint32_t tmem = __shfl_sync(0xffffffffu, T.tmem_base, 0);
+  // accumulators 2 x 64 | weight scales, 4 x 16 in rotation | scales of the resident x operand, 16 per K box (<= 16 boxes) | of FC2's slabs, 4 x 16
+  const uint32_t tm_acc = tmem, tm_sfa = tmem + 128, tm_sfx = tmem + 192, tm_sfs = tmem + 448;
   uint8_t* xb_sf = region + KB1 * (N * 128);   // scale tiles of the resident x operand (same bulk copy)
 
-  if (warp >= 9) {
+  if (warp == kTcProd0 || warp == kTcProd0 + 1) {
     // ============================================================== TMA producers (one thread each)
     // Both producers walk the worker's whole tile sequence with incremental indices (no divisions in the loop) and
     // issue the tiles whose position is theirs (position mod kTcProducers).
     if (lane == 0) {
-      const int pw = warp - 9;
+      const int pw = warp - kTcProd0;
       const uint64_t pol = policy_evict_first();
       // (The resident B operand of FC1 is fetched by an epilogue thread: it has to wait for the expansion kernel, and a
       // producer that waited with it would leave half of the ring empty while the weights could already be streaming.)
@@ -397,61 +402,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
 #endif
     }
     __syncwarp();
-  } else if (warp >= 4 && warp < 8) {
-    // ============================================================== scale warps: one per TMEM lane quadrant
-    // The E4M3 scale tiles of a landed stage go shared memory -> registers -> TMEM (tcgen05.st): lane l of every quadrant
-    // holds row l of each 512-byte tile (16 bytes = 4 columns). Four warps in parallel replace the 4-8 tcgen05.cp per
-    // tile that a single thread would have to issue one after the other.
-    const uint32_t lane_base = (uint32_t)((warp - 4) * 32) << 16;
-    const uint32_t ring_u = smem_u32(ring) + 16384 + lane * 16, region_u = smem_u32(region);
-    const uint32_t xsf_u = smem_u32(xb_sf) + lane * 16;
-    int si = 0;
-    uint32_t ph = 0;
-    auto put = [&](uint32_t src, uint32_t dst_col, int ntiles) {   // up to four consecutive 512-byte tiles -> 16 columns
-      uint32_t r[16];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint4 t4 = make_uint4(0u, 0u, 0u, 0u);
-        if (j < ntiles) t4 = lds128(src + j * 512);
-        r[4 * j] = t4.x, r[4 * j + 1] = t4.y, r[4 * j + 2] = t4.z, r[4 * j + 3] = t4.w;
-      }
-      tmem_st_32x32b_x16(dst_col + lane_base, r);
-    };
-    auto publish_sf = [&]() {
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&T.sfr[si]);
-      if (++si == NS) { si = 0; ph ^= 1u; }
-    };
-    if (n1 > 0 && !mbar_wait(&T.xb_full, 0, &T.abort_flag)) *P.status = 6;
-    for (int j = 0, kb = 0; j < n1; ++j) {
-      if (!mbar_wait(&T.full[si], ph, &T.abort_flag)) *P.status = 1;
-      TC_TRACE(j, 1);
-      put(ring_u + si * kTcStage, tm_sfa + 16 * si, 4);
-      if (j < KB1) put(xsf_u + kb * 2048, tm_sfb + 16 * kb, min(4, P.KT1 - 4 * kb));   // the x operand's scales: once per K box
-      publish_sf();
-      TC_TRACE(j, 2);
-      if (++kb == KB1) kb = 0;
-    }
-    for (int j = 0; j < n2; ++j) {
-      if (!mbar_wait(&T.full[si], ph, &T.abort_flag)) *P.status = 1;
-      TC_TRACE(n1 + j, 1);
-      put(ring_u + si * kTcStage, tm_sfa + 16 * si, 4);
-      put(region_u + si * kSlab + N * 128 + lane * 16, tm_sfb + 16 * si, 4);
-      publish_sf();
-      TC_TRACE(n1 + j, 2);
-    }
-    // The routing tables in the router's padded form, for callers that ask for them: written by these four warps of the
-    // last worker (the one with the least FC1 work) once their tiles are through, off every critical path.
+  } else if (warp == kTcTablesWarp) {
+    // The routing tables in the router's padded form, for callers that ask for them: written by this warp of the
+    // last worker (the one with the least FC1 work), off every critical path.
     if (blockIdx.x == V - 1 && P.experts_out) {
       grid_dependency_wait();   // the tables of the previous call on this workspace may still be read by its tail
-      const int t4 = tid - 128;
-      for (int e = t4; e < P.E; e += 128)
+      const int t4 = lane;
+      for (int e = t4; e < P.E; e += 32)
         if (T.cnt[e] > 0) { P.experts_out[T.uidx[e] - 1] = e; P.offsets_out[T.uidx[e] - 1] = T.base[e] - T.cnt[e]; }
-      for (int u = U + t4; u < P.Umax; u += 128) { P.experts_out[u] = -1; P.offsets_out[u + 1] = T.base[kTcMaxE - 1]; }
+      for (int u = U + t4; u < P.Umax; u += 32) { P.experts_out[u] = -1; P.offsets_out[u + 1] = T.base[kTcMaxE - 1]; }
       if (t4 == 0) P.offsets_out[U] = T.base[kTcMaxE - 1];
-      for (int p = t4; p < npairs; p += 128) {
+      for (int p = t4; p < npairs; p += 32) {
         const int e = T.ids[p];
         if (e < 0) continue;
         int r = 0;
@@ -459,57 +420,68 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
         P.pairs_out[T.base[e] - T.cnt[e] + r] = p;
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == kTcMmaWarp) {
     // ============================================================== MMA issuer: the whole warp stays converged
-    // Every lane runs the loop with warp-uniform values and one elected lane issues, so descriptors and TMEM addresses
-    // can live in uniform registers (issuing from a single diverged lane costs about twice as many cycles per operation).
     const uint32_t el = elect_one();
     const uint32_t idesc = idesc_mxf4nvf4(128, N);
-    const uint64_t desc0 = smem_desc_sw128_kmajor(0);
-    const uint32_t ring16 = smem_u32(ring) >> 4, region16 = smem_u32(region) >> 4;
+    const uint32_t r16 = kDescLoSw128 + (smem_u32(ring) >> 4), g16 = kDescLoSw128 + (smem_u32(region) >> 4);   // descriptor low words
+    const uint32_t xsf16 = smem_u32(xb_sf) >> 4;
+    const uint32_t full_u = smem_u32(T.full), empty_u = smem_u32(T.empty), accf_u = smem_u32(T.acc_full), acce_u = smem_u32(T.acc_empty);
     const int nkt_last1 = P.KT1 - 4 * (KB1 - 1), nkt_last2 = P.KT2 - 4 * (KB2 - 1);
-    int si = 0, ab = 0, pieces = 0;
-    uint32_t ph = 0;
-    uint32_t aph[2] = {0, 0};
-    auto issue = [&](uint32_t b16, uint32_t sfb, int nkt, bool fresh) {   // the MMAs of the tile in ring slot si
-      if (!mbar_wait(&T.sfr[si], ph, &T.abort_flag)) *P.status = 8;     // scale warps arrive after they saw the stage land
+    int si = 0, piece = 0;
+    uint32_t ph = 0, rot = 0;
+    auto take = [&]() {   // the record in ring slot si has landed
+      if (!mbar_wait_warp(full_u + 8 * si, ph, &T.abort_flag)) *P.status = 1;
       tc_fence_after();
-      const uint64_t ad = desc0 | (uint64_t)(ring16 + si * (kTcStage >> 4)), bd = desc0 | (uint64_t)b16;
-      const uint32_t acc = tm_acc + 64 * ab, sfa = tm_sfa + 16 * si;
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
-        if (jj < nkt) umma_mxf4nvf4_p(acc, ad + 2 * jj, bd + 2 * jj, idesc, sfa + 4 * jj, sfb + 4 * jj, (fresh && jj == 0) ? 0u : 1u, el);
-      umma_commit_p(&T.empty[si], el);
     };
-    auto open_piece = [&]() {   // first tile of a piece: the epilogue must have drained this accumulator buffer
-      if (pieces >= 2 && !mbar_wait(&T.acc_empty[ab], aph[ab] ^ 1u, &T.abort_flag)) *P.status = 5;
+    auto copy_scales = [&](uint32_t dst, uint32_t src16) {   // four 512-byte tiles -> 16 TMEM columns
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) tmem_cp_sf_lo(dst + 4 * jj, src16 + 32 * jj, el);
+    };
+    auto issue = [&](uint32_t acc, uint32_t b_lo, uint32_t sfb, int nkt, bool fresh) {   // scales and MMAs of the record in slot si
+      const uint32_t a_lo = r16 + si * (kTcStage >> 4), sfa = tm_sfa + 16 * rot;
+      copy_scales(sfa, a_lo - kDescLoSw128 + 1024);
+      if (nkt == 4) {
+        umma_mxf4nvf4_lo(acc, a_lo, b_lo, idesc, sfa, sfb, fresh ? 0u : 1u, el);
+#pragma unroll
+        for (int jj = 1; jj < 4; ++jj) umma_mxf4nvf4_lo(acc, a_lo + 2 * jj, b_lo + 2 * jj, idesc, sfa + 4 * jj, sfb + 4 * jj, 1u, el);
+      } else {
+        for (int jj = 0; jj < nkt; ++jj) umma_mxf4nvf4_lo(acc, a_lo + 2 * jj, b_lo + 2 * jj, idesc, sfa + 4 * jj, sfb + 4 * jj, fresh && jj == 0 ? 0u : 1u, el);
+      }
+      umma_commit_u32(empty_u + 8 * si, el);
+      rot = (rot + 1) & 3u;
+      if (++si == NS) { si = 0; ph ^= 1u; }
+    };
+    auto open_piece = [&]() {   // first record of a piece: the epilogue must have drained this accumulator buffer
+      if (piece >= 2 && !mbar_wait_warp(acce_u + 8 * (piece & 1), (uint32_t)((piece >> 1) - 1) & 1u, &T.abort_flag)) *P.status = 5;
+      return tm_acc + 64 * (piece & 1);
     };
     auto close_piece = [&]() {
-      umma_commit_p(&T.acc_full[ab], el);
-      aph[ab] ^= 1u;
-      ab ^= 1;
-      ++pieces;
+      umma_commit_u32(accf_u + 8 * (piece & 1), el);
+      ++piece;
     };
-    if (n1 > 0) {
-      if (!mbar_wait(&T.xb_full, 0, &T.abort_flag)) *P.status = 6;
-      tc_fence_after();
+    if (n1 > 0 && !mbar_wait_warp(smem_u32(&T.xb_full), 0, &T.abort_flag)) *P.status = 6;
+    for (int t = 0; t < nu1; ++t) {   // units: K boxes 0..KB1-1 into one accumulator
+      const uint32_t acc = open_piece();
+      for (int kb = 0; kb < KB1; ++kb) {
+        take();
+        // the scales of the resident x operand: once per K box (a short last box copies what follows its tiles; no MMA reads it)
+        if (t == 0) copy_scales(tm_sfx + 16 * kb, xsf16 + 128 * kb);
+        issue(acc, g16 + kb * ((N * 128) >> 4), tm_sfx + 16 * kb, kb == KB1 - 1 ? nkt_last1 : 4, kb == 0);
+      }
+      close_piece();
     }
-    for (int j = 0, kb = 0; j < n1; ++j) {
-      if (kb == 0) open_piece();
-      issue(region16 + kb * ((N * 128) >> 4), tm_sfb + 16 * kb, kb == KB1 - 1 ? nkt_last1 : 4, kb == 0);
-      TC_TRACE(j, 4);
-      if (++kb == KB1) { kb = 0; close_piece(); }
-      if (++si == NS) { si = 0; ph ^= 1u; }
-    }
-    if (n1 > 0) umma_commit_p(&T.fc1_done, el);   // the x operand's shared memory and scale columns may be reused from here on
+    if (n1 > 0) umma_commit_p(&T.fc1_done, el);   // the x operand's shared memory may be reused from here on
     if (n2 > 0) {   // one piece: all of this worker's items of output block nb2 go into one accumulator
-      open_piece();
-      for (int j = 0, kb = r2 % KB2; j < n2; ++j) {
-        issue(region16 + si * (kSlab >> 4), tm_sfb + 16 * si, kb == KB2 - 1 ? nkt_last2 : 4, j == 0);
-        TC_TRACE(n1 + j, 4);
+      const uint32_t acc = open_piece();
+      int kb = r2 % KB2;
+      for (int j = 0; j < n2; ++j) {
+        take();
+        const uint32_t b_lo = g16 + si * (kSlab >> 4), sfb = tm_sfs + 16 * rot;
+        copy_scales(sfb, b_lo - kDescLoSw128 + ((N * 128) >> 4));
+        issue(acc, b_lo, sfb, kb == KB2 - 1 ? nkt_last2 : 4, j == 0);
         kb += dK2;
         if (kb >= KB2) kb -= KB2;
-        if (++si == NS) { si = 0; ph ^= 1u; }
       }
       close_piece();
     }
@@ -545,7 +517,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     uint32_t aph[2] = {0, 0};
     auto load_terms = [&](float (&val)[16], const float* cs, bool per_column) {   // sum the four term columns of every token
       TC_T0(t0);
-      if (!mbar_wait(&T.acc_full[ab], aph[ab], &T.abort_flag)) *P.status = 7;
+      if (!mbar_wait_warp(smem_u32(&T.acc_full[ab]), aph[ab], &T.abort_flag)) *P.status = 7;
       TC_ADD(tm_a, t0);
 #ifdef B200_TIMERS
       if (tm_d == 0) tm_d = clock64() - tm_begin;   // first accumulator ready
@@ -718,7 +690,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
 #ifdef B200_TIMERS
   if (tid == 0 && P.debug) { unsigned long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); P.debug[blockIdx.x * 16 + 14] = (long long)g; }
 #endif
-  if (warp == 8) tmem_dealloc(tmem, 512);
+  if (warp == kTcMmaWarp) tmem_dealloc(tmem, 512);
   if (T.abort_flag)
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
 }
