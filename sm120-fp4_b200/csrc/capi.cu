@@ -221,11 +221,18 @@ static int decode_tc_ring(const b200moe_layer* L, int N, int* region) {
 
 static int decode_tc_columns(int M) { return M <= 4 ? 16 : M <= 8 ? 32 : 64; }   // of the B operand: four terms per token
 
-static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, void* stream) {
+// the tcgen05 kernel runs whenever the tile records exist and the shape fits it: x scale tiles of <= 16 K boxes in TMEM, one
+// worker group per 128-row output block, and a ring of at least three records beside the x operand
+static bool decode_tc_fits(const b200moe_layer* L, int M) {
+  int region;
+  return L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 16 && L->NB2 <= L->sms && decode_tc_ring(L, decode_tc_columns(M), &region) > 0;
+}
+
+static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, const HostRouting* host, void* stream) {
   uint8_t* w = (uint8_t*)ws;
   cudaStream_t st = (cudaStream_t)stream;
   const int N = decode_tc_columns(M);
-  int rc = b200_expand_x_launch(x, M, L->H, N, L->KB1, w + L->off_xb, (float*)(w + L->off_xscale), chained, st);
+  int rc = b200_expand_x_launch(x, M, L->H, N, L->KB1, w + L->off_xb, (float*)(w + L->off_xscale), host, chained, st);
   if (rc != B200MOE_OK) return rc;
   DecodeTcParams p;
   memset(&p, 0, sizeof(p));
@@ -309,16 +316,13 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
 // flags bit 0 (B200MOE_ORDERED): both kernels of the call are ordinary stream-ordered launches.
 extern "C" int b200moe_decode_forward_ex(const b200moe_layer* L, const void* x_bf16, const int* topk_ids, const float* topk_weights,
                                          int M, void* out_bf16, void* workspace, long long workspace_bytes, int flags, void* stream) {
-  // the tcgen05 kernel whenever the tile records exist and the shape fits it: x scale tiles of <= 16 K boxes in TMEM, one
-  // worker group per 128-row output block, and a ring of at least three records beside the x operand
-  int region;
-  if (L && L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 16 && L->NB2 <= L->sms && decode_tc_ring(L, decode_tc_columns(M), &region) > 0) {
+  if (L && decode_tc_fits(L, M)) {
     if (!x_bf16 || !topk_ids || !topk_weights || !out_bf16 || !workspace || M < 0) return B200MOE_ERR_ARG;
     if (M > 16) return B200MOE_ERR_LIMIT;
     if (workspace_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;
     if (((uintptr_t)workspace & 255) || ((uintptr_t)x_bf16 & 15)) return B200MOE_ERR_ARG;
     if (M == 0) return B200MOE_OK;
-    return decode_tc(const_cast<b200moe_layer*>(L), x_bf16, topk_ids, topk_weights, M, out_bf16, workspace, !(flags & 1), stream);
+    return decode_tc(const_cast<b200moe_layer*>(L), x_bf16, topk_ids, topk_weights, M, out_bf16, workspace, !(flags & 1), nullptr, stream);
   }
   return decode_common(L, x_bf16, topk_ids, topk_weights, M, out_bf16, nullptr, 3, 1, workspace, workspace_bytes, stream);
 }
@@ -329,9 +333,10 @@ extern "C" int b200moe_decode_forward(const b200moe_layer* L, const void* x_bf16
 }
 
 // The same call for a host that keeps its tensors in host memory. Page-locked buffers (cudaHostAlloc, cudaHostRegister,
-// torch's pin_memory) are addressable from the device: the kernels then read x, ids and weights and write the output
-// straight across the host link - no copy is enqueued and the transfer overlaps the layer's own work. Pageable buffers are
-// copied through staging buffers inside the workspace. Everything is enqueued on `stream`; nothing synchronises.
+// torch's pin_memory) are addressable from the device: the expansion kernel reads x across the host link and brings ids and
+// weights into device memory (all 148 workers of the layer kernel need those at their entry), and the layer kernel writes the
+// output straight across the link. Pageable buffers are copied through staging buffers inside the workspace. Everything
+// is enqueued on `stream`; nothing synchronises.
 static void* device_view(const void* host_ptr) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, host_ptr) != cudaSuccess) { cudaGetLastError(); return nullptr; }
@@ -350,26 +355,25 @@ extern "C" int b200moe_decode_forward_host(const b200moe_layer* L, const void* x
     explicit DeviceGuard(int want) { if (cudaGetDevice(&prev) == cudaSuccess && prev != want) cudaSetDevice(want); else prev = -1; }
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
   } guard(L->device);
-  // Page-locked host buffers can be used by the kernels directly across the host link. For the OUTPUT that is a stream of
-  // posted writes and saves a copy after the kernel; for the INPUTS it means that all 148 workers fetch the ids and weights
-  // from host memory in their prologue, one round trip over the link each, which measures slower than three small copies
-  // ahead of the kernel (1.2 TB/s against 0.8 TB/s on the decode sweep). So by default the inputs are staged and the output
-  // is written in place; B200MOE_HOST_IN_PLACE=1 uses all four buffers in place, =0 stages all four.
-  static const int mode = [] { const char* c = getenv("B200MOE_HOST_IN_PLACE"); return !c ? 2 : c[0] == '0' ? 0 : c[0] == '1' ? 1 : 2; }();
-  void* vo = mode != 0 ? device_view(out_host) : nullptr;
-  if (mode == 1 && vo) {
-    void* vx = device_view(x_host);
-    void* vi = device_view(ids_host);
-    void* vw = device_view(wts_host);
-    if (vx && vi && vw && !((uintptr_t)vx & 15))
-      return b200moe_decode_forward(L, vx, (const int*)vi, (const float*)vw, M, vo, workspace, workspace_bytes, stream);
-  }
   uint8_t* w = (uint8_t*)workspace;
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* dx = w + L->off_hstage;
   uint8_t* dout = dx + 16LL * L->H * 2;
   int* dids = (int*)(dout + 16LL * L->H * 2);
   float* dwts = (float*)(dids + 16 * L->top_k);
+  static const bool in_place = [] { const char* e = getenv("B200MOE_HOST_IN_PLACE"); return !(e && e[0] == '0'); }();
+  void* vo = in_place ? device_view(out_host) : nullptr;
+  void* vx = vo ? device_view(x_host) : nullptr;
+  void* vi = vx ? device_view(ids_host) : nullptr;
+  void* vw = vi ? device_view(wts_host) : nullptr;
+  if (vw && !(((uintptr_t)vx | (uintptr_t)vo) & 15)) {
+    if ((uintptr_t)workspace & 255) return B200MOE_ERR_ARG;
+    const HostRouting h = {(const int*)vi, (const float*)vw, M * L->top_k, dids, dwts};
+    if (decode_tc_fits(L, M)) return decode_tc(const_cast<b200moe_layer*>(L), vx, dids, dwts, M, vo, workspace, true, &h, stream);
+    const int rc = b200_host_stage_launch(vx, M * L->H / 8, h, dx, st);
+    if (rc != B200MOE_OK) return rc;
+    return b200moe_decode_forward(L, dx, dids, dwts, M, vo, workspace, workspace_bytes, stream);
+  }
   B200_CUDA_TRY(cudaMemcpyAsync(dx, x_host, (size_t)M * L->H * 2, cudaMemcpyHostToDevice, st));
   B200_CUDA_TRY(cudaMemcpyAsync(dids, ids_host, (size_t)M * L->top_k * 4, cudaMemcpyHostToDevice, st));
   B200_CUDA_TRY(cudaMemcpyAsync(dwts, wts_host, (size_t)M * L->top_k * 4, cudaMemcpyHostToDevice, st));

@@ -72,7 +72,10 @@ struct DecodeTcParams {
 }  // namespace b200
 
 int b200_decode_tc_smem_bytes(int NS, int region_bytes);
-int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, bool chained, cudaStream_t st);
+// routing inputs in page-locked host memory and the device copies that a kernel is to make of them
+struct HostRouting { const int* ids_h; const float* wts_h; int npairs; int* ids_d; float* wts_d; };
+int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, const HostRouting* host, bool chained, cudaStream_t st);
+int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, cudaStream_t st);   // n16: 16-byte words of x
 int b200_pack_tiles_launch(const void* q, const void* sf, void* out, int E, int rows_per_expert, int row_bytes, int blocks, int KB, int KT,
                            int fc1, int I, long long sf_stride, cudaStream_t st);
 int b200_decode_tc_launch(const b200::DecodeTcParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);

@@ -69,12 +69,17 @@ __device__ __forceinline__ float tc_silu_mul(float gate, float up) { return __fd
 // xb: the FC1 B operand exactly as the kernel wants it in shared memory, so that ONE bulk copy brings it in:
 //   [KB1 boxes][N rows (token*4 + term)][128 B] in the 128-byte-swizzle image (16-byte chunk c of row n sits at chunk
 //   c ^ (n & 7)), followed by KT1 scale tiles of 512 B (128x4 order, rows >= N zero). colscale f32 [N] = 1/g_t.
-__global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* __restrict__ x, int M, int H, int N, int KB1, uint8_t* __restrict__ xb,
-                                                  float* __restrict__ colscale) {
+// kHost: x, ids and weights are in page-locked host memory. This kernel reads x across the host link itself and its block 0 brings the
+// routing inputs into device memory (ids_d, wts_d) before it lets the layer kernel start, which reads them at its entry: one
+// kernel instead of three copies that wait for one another and for the link (13 us a call).
+template <bool kHost>
+__global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* x, int M, int H, int N, int KB1, uint8_t* xb, float* colscale,
+                                                      const int* ids_h, const float* wts_h, int npairs, int* ids_d, float* wts_d) {
   const int tok = blockIdx.x, tid = threadIdx.x;
-  grid_launch_dependents();   // the layer kernel may start its prologue and weight prefetch now; it waits before reading xb
+  if (!kHost) grid_launch_dependents();   // the layer kernel may start its prologue and weight prefetch now; it waits before reading xb
   grid_dependency_wait();     // this kernel is itself launched programmatically: x (and the workspace it writes) belong to
                               // whatever ran before it in the stream until that has completed
+  if (kHost && tok != 0) grid_launch_dependents();
   uint8_t* xsf = xb + (long long)KB1 * N * 128;
   __shared__ float wm[4];
   // each thread keeps its (at most two) 16-value blocks in registers: one pass over x serves the token amax and the expansion
@@ -86,8 +91,23 @@ __global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* __res
     const int b = tid + 128 * j;
     raw[j][0] = raw[j][1] = make_uint4(0u, 0u, 0u, 0u);
     if (tok < M && b < nblk && b * 16 < H) {
-      raw[j][0] = *reinterpret_cast<const uint4*>(x + (long long)tok * H + b * 16);
-      raw[j][1] = *reinterpret_cast<const uint4*>(x + (long long)tok * H + b * 16 + 8);
+      const uint4* src = reinterpret_cast<const uint4*>(x + (long long)tok * H + b * 16);
+      raw[j][0] = kHost ? __ldcv(src) : src[0];
+      raw[j][1] = kHost ? __ldcv(src + 1) : src[1];
+    }
+  }
+  if (kHost && tok == 0) {   // (x is in flight)
+    for (int p = tid; p < npairs; p += 128) {
+      __stcg(ids_d + p, __ldcv(ids_h + p));
+      __stcg(wts_d + p, __ldcv(wts_h + p));
+    }
+    __threadfence();
+    __syncthreads();
+    grid_launch_dependents();
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    {
       const uint32_t w[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
 #pragma unroll
       for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
@@ -193,7 +213,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   // one another and the barrier / TMEM set-up: pair p is thread p's (npairs <= 256 < threads).
   int my_e = -1;
   float my_w = 0.f;
-  if (tid < npairs) { my_e = P.ids[tid]; my_w = P.wts[tid]; }
+  if (tid < npairs) { my_e = __ldcg(P.ids + tid); my_w = __ldcg(P.wts + tid); }
   // the per-expert scales of ALL experts come in with the ids (no load depends on another): thread e holds expert e's
   float ex_a1 = 0.f, ex_a2 = 0.f;
   if (tid < P.E) { ex_a1 = P.alpha1[tid]; ex_a2 = P.alpha2[tid]; }
@@ -706,20 +726,26 @@ static bool pdl_chain_enabled() {   // B200MOE_PDL_CHAIN=0: launch the expansion
   return on;
 }
 
-int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, bool chained, cudaStream_t st) {
+int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, const HostRouting* host, bool chained, cudaStream_t st) {
   // programmatic launch: the blocks may be scheduled while the previous kernel of the stream drains (if that kernel
   // allows it, as this library's layer kernel does); griddepcontrol.wait at their top keeps stream order for all data
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(N / kTerms), cfg.blockDim = dim3(128), cfg.dynamicSmemBytes = 0, cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = chained && pdl_chain_enabled() ? 1 : 0;
-  const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
-  uint8_t* xbp = (uint8_t*)xb;
-  void* args[] = {(void*)&xp, (void*)&M, (void*)&H, (void*)&N, (void*)&KB1, (void*)&xbp, (void*)&colscale};
-  B200_CUDA_TRY(cudaLaunchKernelExC(&cfg, (const void*)k_expand_x, args));
+  const HostRouting h = host ? *host : HostRouting{nullptr, nullptr, 0, nullptr, nullptr};
+  void* args[] = {(void*)&x, (void*)&M, (void*)&H, (void*)&N, (void*)&KB1, (void*)&xb, (void*)&colscale,
+                  (void*)&h.ids_h, (void*)&h.wts_h, (void*)&h.npairs, (void*)&h.ids_d, (void*)&h.wts_d};
+  return launch_kernel(host ? (const void*)k_expand_x<true> : (const void*)k_expand_x<false>, N / kTerms, 128, 0, chained && pdl_chain_enabled(), args, st);
+}
+
+// x, ids and weights of a call from page-locked host memory into device memory, for the kernel that does not take them from there
+__global__ void __launch_bounds__(256) k_host_stage(const uint4* x, int n16, const int* ids_h, const float* wts_h, int npairs, uint4* x_d, int* ids_d, float* wts_d) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n16) x_d[i] = __ldcv(x + i);
+  if (i < npairs) { ids_d[i] = __ldcv(ids_h + i); wts_d[i] = __ldcv(wts_h + i); }
+}
+
+int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, cudaStream_t st) {
+  const int n = n16 > h.npairs ? n16 : h.npairs;
+  k_host_stage<<<(n + 255) / 256, 256, 0, st>>>((const uint4*)x, n16, h.ids_h, h.wts_h, h.npairs, (uint4*)x_d, h.ids_d, h.wts_d);
+  B200_LAUNCH_CHECK();
   return B200MOE_OK;
 }
 
@@ -745,13 +771,5 @@ int b200_decode_tc_launch(const DecodeTcParams& p, int grid, int smem_bytes, boo
     configured[which] = smem_bytes;
   }
   // programmatic dependent launch: this kernel's prologue and weight prefetch overlap the activation-expansion kernel
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(grid), cfg.blockDim = dim3(kTcThreads), cfg.dynamicSmemBytes = (size_t)smem_bytes, cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = chained ? 1 : 0;
-  B200_CUDA_TRY(cudaLaunchKernelExC(&cfg, fn, args));
-  return B200MOE_OK;
+  return launch_kernel(fn, grid, kTcThreads, smem_bytes, chained, args, st);
 }
