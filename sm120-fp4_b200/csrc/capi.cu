@@ -57,7 +57,7 @@ struct b200moe_layer {
   long long s1_stride, s2_stride;
   // workspace layout (byte offsets)
   long long off_status, off_cnt1, off_cnt2, off_scratch, off_actfrag, off_tables, off_actbf16, off_debug, off_hstage, ws_bytes;
-  long long off_xb, off_xscale, off_aslab;   // operands of the tcgen05 decode kernel
+  long long off_xb, off_xscale, off_aslab, off_partials;   // operands of the tcgen05 decode kernel
   int umax_cap;
   // tcgen05 decode path: composed FC1 scale tiles + alpha2 reference in a caller-owned buffer (b200moe_layer_prepack)
   const uint8_t* w1t;
@@ -133,6 +133,7 @@ extern "C" int b200moe_layer_create(b200moe_layer** out, int E, int H, int I, in
   L->off_xscale = o, o += 256;
   L->off_aslab = o, o = align_up(o + (long long)L->umax_cap * L->KB2 * (64 * 128 + 2048), 256);
   L->off_hstage = o, o = align_up(o + 2LL * 16 * H * 2 + 2LL * 16 * top_k * 4, 256);   // device copies of host-side inputs / output
+  L->off_partials = o, o = align_up(o + (long long)L->sms * 8 * 128 * 16, 256);
   L->ws_bytes = o;
   L->prepack_bytes = (long long)E * ((long long)L->CB1 * L->KB1 + (long long)L->NB2 * L->KB2) * 18432 + 256;
   L->act_g1 = 8.0f;
@@ -232,16 +233,23 @@ static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const floa
   uint8_t* w = (uint8_t*)ws;
   cudaStream_t st = (cudaStream_t)stream;
   const int N = decode_tc_columns(M);
-  int rc = b200_expand_x_launch(x, M, L->H, N, L->KB1, w + L->off_xb, (float*)(w + L->off_xscale), host, chained, st);
-  if (rc != B200MOE_OK) return rc;
+  const bool self = b200_decode_self_expand(M, L->H);
+  if (!self) {
+    const int rc = b200_expand_x_launch(x, M, L->H, N, L->KB1, w + L->off_xb, (float*)(w + L->off_xscale), host, chained, st);
+    if (rc != B200MOE_OK) return rc;
+  } else if (host) {   // every worker reads x, so it comes across the link once, ahead of the layer kernel
+    void* dx = w + L->off_hstage;
+    const int rc = b200_host_stage_launch(x, M * L->H / 8, *host, dx, chained, st);
+    if (rc != B200MOE_OK) return rc;
+    x = dx;
+  }
   DecodeTcParams p;
   memset(&p, 0, sizeof(p));
   p.w1t = L->w1t, p.w2t = L->w2t, p.alpha1 = L->alpha1, p.alpha2 = L->alpha2, p.alpha2_ref = L->alpha2_ref;
-  p.xb = w + L->off_xb, p.xscale = (const float*)(w + L->off_xscale);
+  p.x = (const __nv_bfloat16*)x, p.xb = w + L->off_xb, p.xscale = (float*)(w + L->off_xscale);
   p.aslab = w + L->off_aslab;
   p.ids = ids, p.wts = wts, p.out = (__nv_bfloat16*)out;
-  p.scratch = (float*)(w + L->off_scratch);
-  p.cnt1 = (unsigned*)(w + L->off_cnt1), p.cnt2 = (unsigned*)(w + L->off_cnt2);
+  p.partials = (uint4*)(w + L->off_partials);
   p.status = (int*)(w + L->off_status);
   p.gates = (unsigned long long*)(w + L->off_status + 128);
   p.experts_out = (int*)(w + L->off_tables);
@@ -255,7 +263,7 @@ static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const floa
   int region = 0;
   const int NS = decode_tc_ring(L, N, &region);
   if (NS == 0) return B200MOE_ERR_SHAPE;
-  p.NS = NS, p.region_bytes = region;
+  p.NS = NS, p.region_bytes = region, p.self = self;
   return b200_decode_tc_launch(p, L->sms, b200_decode_tc_smem_bytes(NS, p.region_bytes), chained, st);
 }
 
@@ -370,7 +378,7 @@ extern "C" int b200moe_decode_forward_host(const b200moe_layer* L, const void* x
     if ((uintptr_t)workspace & 255) return B200MOE_ERR_ARG;
     const HostRouting h = {(const int*)vi, (const float*)vw, M * L->top_k, dids, dwts};
     if (decode_tc_fits(L, M)) return decode_tc(const_cast<b200moe_layer*>(L), vx, dids, dwts, M, vo, workspace, true, &h, stream);
-    const int rc = b200_host_stage_launch(vx, M * L->H / 8, h, dx, st);
+    const int rc = b200_host_stage_launch(vx, M * L->H / 8, h, dx, false, st);
     if (rc != B200MOE_OK) return rc;
     return b200moe_decode_forward(L, dx, dids, dwts, M, vo, workspace, workspace_bytes, stream);
   }

@@ -47,15 +47,14 @@ struct DecodeTcParams {
   const float* alpha1;
   const float* alpha2;
   const float* alpha2_ref;   // [0] = max over experts of alpha2, [1] = its reciprocal
-  const uint8_t* xb;         // expanded x operand: [KB1][N][128 B] images then [KT1][512] scale tiles
-  const float* xscale;       // 1 / g_t per column of the x operand [N]
+  const __nv_bfloat16* x;    // [M, H]
+  uint8_t* xb;               // expanded x operand: [KB1][N][128 B] images then [KT1][512] scale tiles; written by the expansion
+  float* xscale;             // kernel, or (self) by the layer kernel for read-back only; 1 / g_t per column of it [N]
   uint8_t* aslab;            // expanded activations (FC2 operand): [Umax][KB2] slabs of N*128 + 2048 bytes
   const int* ids;
   const float* wts;
   __nv_bfloat16* out;
-  float* scratch;
-  unsigned* cnt1;
-  unsigned* cnt2;
+  uint4* partials;           // workspace: partial sums as flagged words, [workers][8 token pairs][128 rows]
   unsigned long long* gates; // workspace: arrival counters of the two FC1 gates; only ever incremented, V per launch and gate
   int* status;               // workspace: [0] code of the first bounded wait that ran out / bad expert id, [1] activation range
                              // exceeded, [2] routing inputs changed under the call
@@ -67,6 +66,7 @@ struct DecodeTcParams {
   int M, E, H, I, top_k, Umax;
   int NS, region_bytes;
   int KB1, KB2, CB1, NB2, KT1, KT2;
+  int self;                  // the workers expand x themselves
 };
 
 }  // namespace b200
@@ -75,7 +75,9 @@ int b200_decode_tc_smem_bytes(int NS, int region_bytes);
 // routing inputs in page-locked host memory and the device copies that a kernel is to make of them
 struct HostRouting { const int* ids_h; const float* wts_h; int npairs; int* ids_d; float* wts_d; };
 int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, const HostRouting* host, bool chained, cudaStream_t st);
-int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, cudaStream_t st);   // n16: 16-byte words of x
+int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, bool chained, cudaStream_t st);   // n16: 16-byte words of x
+// whether the layer kernel expands x itself (see expand_x_here)
+inline bool b200_decode_self_expand(int M, int H) { return M <= 8 && (long long)M * H <= 16 * 1024; }
 int b200_pack_tiles_launch(const void* q, const void* sf, void* out, int E, int rows_per_expert, int row_bytes, int blocks, int KB, int KT,
                            int fc1, int I, long long sf_stride, cudaStream_t st);
 int b200_decode_tc_launch(const b200::DecodeTcParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);

@@ -16,7 +16,7 @@
 // elected lane; it waits for a record, copies its scale tiles into TMEM (tcgen05.cp), issues the four K=64 MMAs and commits
 // the ring slot: operations of one lane execute in order, so a record passes from the producer to the tensor core
 // in one hand-off. Warps 5-6: producers (one bulk copy per 18 KB record into the ring, FC2 records prefetched across the gates).
-// Warp 7: routing tables. What bounds it: at 16 tokens the weight stream (an SM's share of HBM is a record per ~740 cycles, the
+// Warp 7: arrivals at the gates, warp 8: routing tables. What bounds it: at 16 tokens the weight stream (an SM's share of HBM is a record per ~740 cycles, the
 // issuer needs ~300 for one), at 1 token a chain of latencies: launch, routing tables, first record, eight
 // records of a unit, gate, three records of FC2, reduction. (With four warps that moved the scales through registers, and
 // an issuer whose lanes left their waits one by one, a record took about 1,000 cycles of issue alone.)
@@ -24,27 +24,33 @@
 #include "tcgen05.cuh"
 #include "decode_params.h"
 #include "expand.cuh"
+#include "nvfp4_math.cuh"
 #include <string.h>
+#include <type_traits>
 #include <stdlib.h>
 
 namespace b200 {
 
-constexpr int kTcMmaWarp = 4, kTcProd0 = 5, kTcTablesWarp = 7;
+constexpr int kTcMmaWarp = 4, kTcProd0 = 5, kTcUnitsWarp = 7, kTcTablesWarp = 8;
 constexpr int kTcProducers = 2;    // producer warps: one thread's wait + issue round is ~430 cycles
-constexpr int kTcThreads = 8 * 32;
+constexpr int kTcThreads = 9 * 32;
 constexpr int kTcStage = 18432;   // 16 KB codes + 2 KB scale tiles
 constexpr int kTcMaxE = 256, kTcMaxP = 256;
+constexpr int kTcPause = 100;
+constexpr int kTcPace = 700, kTcAhead = 24;   // see ask_ahead
 
 struct TcTables {
   int ids[kTcMaxP];
   float wts[kTcMaxP];
   int cnt[kTcMaxE], base[kTcMaxE], uidx[kTcMaxE], experts[kTcMaxE];
+  unsigned xmax[16];           // amax bits of every token
+  float xg1[16];
   float colscale[64];          // 1 / g_t of every B column of the FC1 operand (token-major, four terms per token)
   float a1[kTcMaxE], a2n[kTcMaxE];   // per touched expert (unit index): alpha1, alpha2 relative to the layer's largest alpha2
   int U;
+  volatile int units_done;       // FC1 units whose activations the epilogue has written
   unsigned long long gate0[2];   // arrival counts of the two FC1 gates before this launch (a multiple of the worker count)
   volatile int abort_flag;
-  int last_flag;
   uint32_t tmem_base;
   uint64_t full[12], empty[12];   // stage landed / stage consumed
   uint64_t acc_full[2], acc_empty[2];
@@ -187,10 +193,94 @@ __global__ void __launch_bounds__(256) k_pack_tiles(const uint8_t* __restrict__ 
   }
 }
 
+// ------------------------------------------------------------------------------------------------ x -> B operand, inside the layer kernel
+// Small operands (P.self: up to 1024 blocks of 16 values, e.g. eight tokens of 2048) every worker expands by itself, with its 128
+// epilogue threads, straight into shared memory. As a kernel of its own (16 blocks) the expansion costs a launch, and its
+// result has to travel: from the completion of the kernel before to the operand's arrival 4.3 us at one token of 2048 values
+// and 5.7 us at four of 2816, against 2.7 and 5.8 us here. The work in a worker grows with the tokens (0.35 us per 128 blocks),
+// so beyond 1024 blocks the separate kernel is ahead.
+__device__ __forceinline__ void zero_scales(uint8_t* xsf, int KT1, int et) {   // rows that hold no token keep zero scales
+  for (int i = et; i < KT1 * 32; i += 128) reinterpret_cast<uint4*>(xsf)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+template <int N>
+__device__ __forceinline__ void expand_x_here(const DecodeTcParams& P, uint8_t* region, float* colscale, unsigned* amax, float* g1s, int et) {
+  constexpr int kTok = N / kTerms, kMost = 8;   // blocks per thread
+  const int nb = P.H >> 4, lane = et & 31, total = P.M * nb;
+  uint8_t* xsf = region + P.KB1 * (N * 128);
+  // this thread's blocks: et, et + 128, ...; all of x is loaded at once and stays in registers (a load takes 1 to 2 us here, while the
+  // weight stream fills the memory system's queues)
+  uint4 raw[kMost][2];
+#pragma unroll
+  for (int j = 0; j < kMost; ++j) {
+    raw[j][0] = raw[j][1] = make_uint4(0u, 0u, 0u, 0u);
+    if (et + 128 * j < total) {   // x is [M, H] without gaps: block i of the batch starts at value 16 i
+      const uint4* src = reinterpret_cast<const uint4*>(P.x + (long long)(et + 128 * j) * 16);
+      raw[j][0] = src[0], raw[j][1] = src[1];
+    }
+  }
+  int tok0 = 0, b0 = et;
+  while (b0 >= nb) b0 -= nb, ++tok0;
+  {
+    int tok = tok0, b = b0;
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+      if (128 * j >= total) break;
+      const uint32_t w[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
+      __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
+#pragma unroll
+      for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+      const uint32_t bits = *reinterpret_cast<const uint32_t*>(&m);
+      const unsigned mine = max(bits << 16, bits & 0xffff0000u);   // non-negative floats order like their bits
+      const int first = __shfl_sync(0xffffffffu, tok, 0), last = __shfl_sync(0xffffffffu, tok, 31);
+      for (int t = first; t <= last && t < P.M; ++t) {             // the tokens this warp's 32 blocks belong to
+        const unsigned wm = __reduce_max_sync(0xffffffffu, tok == t ? mine : 0u);
+        if (lane == 0) atomicMax(amax + t, wm);
+      }
+      b += 128;
+      while (b >= nb) b -= nb, ++tok;
+    }
+  }
+  named_bar_sync(1, 128);
+  if (et < kTok) g1s[et] = 2688.0f / fmaxf(__uint_as_float(amax[et]), 1e-30f);
+  named_bar_sync(1, 128);
+  if (et < N) {
+    float g = g1s[et >> 2];
+    for (int q = 0; q < (et & 3); ++q) g *= 6.0f;
+    colscale[et] = (et >> 2) < P.M ? 1.0f / g : 0.f;
+  }
+  int left = (total - et + 127) >> 7, tok = tok0, b = b0;
+  auto expand = [&](auto two) {
+    constexpr int K = decltype(two)::value;
+    int tk[K], bb[K];
+    float r[K][16], g[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      tk[k] = tok, bb[k] = b, g[k] = g1s[tok];
+      const uint32_t w[8] = {raw[k][0].x, raw[k][0].y, raw[k][0].z, raw[k][0].w, raw[k][1].x, raw[k][1].y, raw[k][1].z, raw[k][1].w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r[k][2 * i] = __uint_as_float(w[i] << 16), r[k][2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      b += 128;
+      while (b >= nb) b -= nb, ++tok;
+    }
+    expand_blocks16<true, K>(r, g, [&](int k, int t, uint2 codes, uint8_t sf) {
+      const int n = tk[k] * kTerms + t, c = bb[k];   // 8 code bytes = half a 16-byte chunk
+      *reinterpret_cast<uint2*>(region + (c >> 4) * (N * 128) + n * 128 + ((((c & 15) >> 1) ^ (n & 7)) << 4) + (c & 1) * 8) = codes;
+      xsf[(c >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (c & 3)] = sf;
+    });
+#pragma unroll
+    for (int j = 0; j + K < kMost; ++j) raw[j][0] = raw[j + K][0], raw[j][1] = raw[j + K][1];
+  };
+#pragma unroll 1
+  for (; left >= 2; left -= 2) expand(std::integral_constant<int, 2>());
+  if (left > 0) expand(std::integral_constant<int, 1>());
+}
+
 // ------------------------------------------------------------------------------------------------ the layer kernel
 template <int NB>   // N = 16 * NB columns of the B operand (tokens x four terms): NB = 1 (M<=4), 2 (M<=8), 4 (M<=16)
 __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_constant__ DecodeTcParams P) {
   constexpr int N = 16 * NB;
+  const bool self = NB <= 2 && P.self != 0;   // the worker expands x itself
   constexpr int kSlab = N * 128 + 2048;     // FC2 activation slab of one tile: N rows x 128 B codes + 4 scale tiles
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -218,7 +308,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   float ex_a1 = 0.f, ex_a2 = 0.f;
   if (tid < P.E) { ex_a1 = P.alpha1[tid]; ex_a2 = P.alpha2[tid]; }
   const float a2inv = P.alpha2_ref[1];
-  // The gate counters are only ever incremented, by exactly V arrivals per launch and gate, and a launch starts after the
+  // The gate counters are only ever incremented, by exactly V arrivals per launch and gate (so their quotient numbers the
+  // launches: what the flagged words of the partial sums carry), and a launch starts after the
   // gates of the launch before it on this workspace have opened: whatever this thread reads, rounding down to a multiple of
   // V gives the count before this launch (other workers of this launch may have arrived already).
   unsigned long long my_gate = 0;
@@ -228,9 +319,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     for (int s = 0; s < NS; ++s) { mbar_init(&T.full[s], 1); mbar_init(&T.empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&T.acc_full[b], 1); mbar_init(&T.acc_empty[b], 4); }
     mbar_init(&T.xb_full, 1);
-    mbar_init(&T.fc1_done, 1);
     T.abort_flag = 0;
-    T.last_flag = 0;
+    T.units_done = 0;
     fence_mbar_init();
   }
   if (warp == kTcMmaWarp) {              // the MMA warp owns the TMEM allocation (all 512 columns: one CTA per SM)
@@ -238,6 +328,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     tmem_relinquish();
   }
   for (int i = tid; i < kTcMaxE; i += kTcThreads) T.cnt[i] = 0;
+  if (tid < 16) T.xmax[tid] = 0u;
   if (tid < npairs) {   // a negative id marks an empty slot (expert-parallel shards mask the experts they do not own)
     if (my_e >= P.E) { *P.status = 4; my_e = -1; }
     if (my_e < 0) my_e = -1;
@@ -272,6 +363,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     T.a1[u] = ex_a1;
     T.a2n[u] = ex_a2 * a2inv;
   }
+  // One worker leaves the x operand it expanded in the workspace, for tools and tests that read it back: the last one, which has the
+  // least FC1 work (at one token none: it then expands x for this alone). Its fc1_done is complete when the copy has read the
+  // operand, too. (On the first worker the copy's 32 KB held up the release of its unit, and with it everybody, by 3 us.)
+  const bool x_out = self && blockIdx.x == V - 1 && U > 0;
+  if (tid == 0) { mbar_init(&T.fc1_done, (blockIdx.x < U * CB1 ? 1 : 0) + (x_out ? 1 : 0) > 1 ? 2 : 1); fence_mbar_init(); }
   if (tid == kTcProd0 * 32) T.gate0[0] = my_gate - my_gate % (unsigned long long)V;
   if (tid == (kTcProd0 + 1) * 32) T.gate0[1] = my_gate - my_gate % (unsigned long long)V;
   tc_fence_before();
@@ -284,8 +380,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   // has finished its units of group A, gate B when all of FC1 is done; a worker's FC2 items of group A keep it busy
   // while gate B and the last slabs are still on their way.
   // FC2: the workers are split into NB2 groups, one per 128-row output block; inside a group, worker r takes the items
-  // i = (u, kb) = r, r + W, ... in ascending order, accumulates them in one TMEM accumulator, and the group's partials are
-  // added in worker order by whoever arrives last. A worker's first items belong to group A: they run while the tail of
+  // i = (u, kb) = r, r + W, ... in ascending order, accumulates them in one TMEM accumulator, and the group's partials
+  // travel as flagged words and are added in worker order by its first workers. A worker's first items belong to group A: they run while the tail of
   // FC1, gate B and the fetch of the remaining activation slabs are still in flight elsewhere.
   const int v = blockIdx.x;
   const int Q1 = U * CB1;
@@ -310,6 +406,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
   if (tid == 0 && P.debug) { unsigned long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); P.debug[blockIdx.x * 16 + 15] = (long long)g;
     unsigned sm; asm volatile("mov.u32 %0, %%smid;" : "=r"(sm)); P.debug[blockIdx.x * 16 + 11] = sm; }
 #endif
+  const unsigned call = (unsigned)(T.gate0[1] / (unsigned long long)V) + 1u;   // number of this launch on the workspace, from 1
   const uint32_t tmem = __shfl_sync(0xffffffffu, T.tmem_base, 0);
   // accumulators 2 x 64 | weight scales, 4 x 16 in rotation | scales of the resident x operand, 16 per K box (<= 16 boxes) | of FC2's slabs, 4 x 16
   const uint32_t tm_acc = tmem, tm_sfa = tmem + 128, tm_sfx = tmem + 192, tm_sfs = tmem + 448;
@@ -333,11 +430,34 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
       // An activation slab may land only when (a) the gate of its expert group is open and (b) this worker's own FC1 MMAs
       // are complete: the slabs share their shared memory with the resident x operand, and their scale columns in TMEM
       // with the x operand's. Weight tiles of FC2 are prefetched regardless; only the slab loads wait.
-      bool local_ok = n1 == 0;
+      bool local_ok = n1 == 0 && !x_out;
       auto flush = [&]() {   // issue the parked slab loads whose conditions hold now
         while (pend_head < npend && local_ok && passed[pend_g[pend_head & 15]]) { load_slab(pend_slot[pend_head & 15], pend_idx[pend_head & 15]); ++pend_head; }
       };
-      auto open_gate = [&](int g) {   // blocking: wait for (b) and for gate g and every gate before it; issue what waited for them
+      // While this worker can issue nothing - the x operand comes from another kernel and is not there yet, or activations are
+      // awaited, and the ring is full - its next records are asked into L2, one per kTcPace cycles, about the rate at which HBM
+      // delivers them: HBM would be idle meanwhile. (Not while the worker expands x itself: that waits for loads of its own,
+      // which the stream delays. 16 tokens: 48 -> 46 us a layer with it; 4 tokens, asking during the expansion: 29 -> 31.)
+      int pf_next = 0;          // position of the next record to ask for
+      long long pf_last = 0;
+      auto record_at = [&](int j) {   // the weight record of position j of this worker's sequence
+        if (j < n1) {
+          const int t = j / KB1, q = v + t * V, u = q / CB1;
+          return P.w1t + (((long long)T.experts[u] * CB1 + (q - u * CB1)) * KB1 + (j - t * KB1)) * kTcStage;
+        }
+        const int i = r2 + (j - n1) * W2, u = i / KB2;
+        return P.w2t + (((long long)T.experts[u] * NB2 + nb2) * KB2 + (i - u * KB2)) * kTcStage;
+      };
+      auto ask_ahead = [&](int pos) {   // pos: the position this producer will issue next
+        const long long now = clock64();
+        if (now - pf_last < kTcProducers * kTcPace) return;
+        if (pf_next < pos) pf_next = pos;
+        if (pf_next >= n1 + n2 || pf_next > pos + kTcAhead) return;
+        l2_prefetch(record_at(pf_next), kTcStage);
+        pf_next += kTcProducers;
+        pf_last = now;
+      };
+      auto open_gate = [&](int g, int pos) {   // blocking: wait for (b) and for gate g and every gate before it; issue what waited for them
         if (!local_ok) {
           if (!mbar_wait(&T.fc1_done, 0, &T.abort_flag)) *P.status = 9;
           local_ok = true;
@@ -348,6 +468,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
           for (uint32_t it = 0; it < (1u << 24); ++it) {
             if (ld_acquire_gpu_u64(P.gates + gg) - T.gate0[gg] >= (unsigned long long)V) { ok = true; break; }
             if (T.abort_flag) break;
+            ask_ahead(pos);
+            __nanosleep(kTcPause);   // 296 threads that spin on one line hold up the arrivals they wait for
           }
           if (!ok) { T.abort_flag = 1; *P.status = 3; }
           passed[gg] = true;
@@ -363,9 +485,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
         flush();
       };
       int slot = 0, use = 0, mine = pw == 0 ? 0 : kTcProducers - pw;   // `mine` counts down to this producer's next tile
-      auto acquire = [&](int gate) {   // the ring slot of the current position, free of its previous occupant
+      bool x_there = n1 == 0;
+      auto acquire = [&](int gate, int pos) {   // the ring slot of the current position, free of its previous occupant
         if (use >= 1) {
-          if (gate >= 0) open_gate(gate);   // that occupant may be an FC2 tile still waiting for its activations
+          if (!x_there) {
+            for (uint32_t it = 0; it < (1u << 22) && !self && !mbar_test_wait(&T.xb_full, 0) && !T.abort_flag; ++it) ask_ahead(pos);
+            x_there = true;
+          }
+          if (gate >= 0) open_gate(gate, pos);   // that occupant may be an FC2 tile still waiting for its activations
           if (!mbar_wait(&T.empty[slot], (use - 1) & 1, &T.abort_flag)) *P.status = 2;
         }
       };
@@ -379,7 +506,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
         const uint8_t* src = P.w1t + ((long long)T.experts[u] * CB1 + cb) * KB1 * kTcStage;
         for (int kb = 0; kb < KB1; ++kb, ++j) {
           if (mine == 0) {
-            acquire(-1);
+            acquire(-1, j);
             TC_TRACE(j, 0);
             mbar_expect_tx(&T.full[slot], kTcStage);
             bulk_load_hint(ring + slot * kTcStage, src + (long long)kb * kTcStage, kTcStage, &T.full[slot], pol);
@@ -395,7 +522,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
           const int prev_g = j >= NS ? slot_g[slot] : -1;   // gate of the FC2 tile that holds this slot now, if any
           slot_g[slot] = g;
           if (mine == 0) {
-            acquire(prev_g);
+            acquire(prev_g, n1 + j);
             TC_TRACE(n1 + j, 0);
             mbar_expect_tx(&T.full[slot], kTcStage + kSlab);
             bulk_load_hint(ring + slot * kTcStage, P.w2t + (((long long)T.experts[u] * NB2 + nb2) * KB2 + kb) * kTcStage, kTcStage, &T.full[slot], pol);
@@ -408,13 +535,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
           advance();
         }
       }
-      if (pend_head < npend) open_gate(1);
+      if (pend_head < npend) open_gate(1, n1 + n2);
       if (pw == 0) {
         // The kernel after this one in the stream, if it was launched programmatically (the activation expansion of the
         // next layer call is), may be scheduled once every worker has seen gate B open: its blocks start as SMs free up
         // and wait for this grid's completion before they touch any data. Not earlier: a next call on the same workspace
         // reads the gate words at its entry, and they are final only when the last gate of this launch has opened.
-        open_gate(1);
+        open_gate(1, n1 + n2);
         grid_launch_dependents();
       }
 #ifdef B200_TIMERS
@@ -422,7 +549,32 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
 #endif
     }
     __syncwarp();
+  } else if (warp == kTcUnitsWarp) {
+    // ============================================================== arrivals at the gates of FC1
+    // Everything this worker wrote for the experts of the gate's group is visible to the bulk loads of every worker that sees the
+    // gate open (the producers are the only waiters, and they fence the proxies). A warp of its own does it, so that nobody in
+    // the epilogue waits for the stores to be acknowledged (1 to 2 us while the weight stream runs).
+    if (lane == 0) {
+      auto arrive = [&](int g, int units) {   // when that many units are done
+        for (uint32_t it = 0; T.units_done < units && !T.abort_flag; ++it)
+          if (it > 64) __nanosleep(20);
+        __threadfence_block();
+        red_add_release_gpu_u64(P.gates + g, 1ull);   // nothing to wait for: the gate is open when V have arrived
+      };
+      if (use_gate_a) arrive(0, nuA);
+      arrive(1, nu1);
+    }
+    __syncwarp();
   } else if (warp == kTcTablesWarp) {
+    // ============================================================== x operand copies, routing tables
+    if (x_out) {
+      if (!mbar_wait_warp(smem_u32(&T.xb_full), 0, &T.abort_flag)) *P.status = 6;
+      if (lane == 0) {
+        bulk_store(P.xb, region, KB1 * (N * 128) + P.KT1 * 512);
+        mbar_arrive(&T.fc1_done);   // the store has read the region
+      }
+      __syncwarp();
+    }
     // The routing tables in the router's padded form, for callers that ask for them: written by this warp of the
     // last worker (the one with the least FC1 work), off every critical path.
     if (blockIdx.x == V - 1 && P.experts_out) {
@@ -513,16 +665,27 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
     const int et = tid;                            // 0..127
     const int quad = warp;                     // TMEM lane quadrant this warp may read
     const int row = quad * 32 + lane;              // accumulator row (MMA M index)
-    __shared__ float s_ex[64][17];                 // gate values / activations of one unit: [column][token]
+    __shared__ float s_up[N / 4][68], s_gate[N / 4][68];   // one unit's FC1 sums: [token][intermediate column]
     __shared__ float s_w[16];
+    __shared__ unsigned s_mask;
+    __shared__ int s_tok[16];                      // the routed tokens
+    if (self && (n1 > 0 || x_out)) zero_scales(region + KB1 * (N * 128), P.KT1, et);
     grid_dependency_wait();   // everything before this kernel in the stream is complete and visible from here on
-    if (et == 0 && n1 > 0) {
+    if (self) {
+      if (n1 > 0 || x_out) {
+        if constexpr (NB <= 2) expand_x_here<N>(P, region, T.colscale, T.xmax, T.xg1, et);
+        fence_proxy_async();
+        named_bar_sync(1, 128);
+        if (et == 0) mbar_arrive(&T.xb_full);
+        if (x_out && et < N) P.xscale[et] = T.colscale[et];
+      }
+    } else if (et == 0 && n1 > 0) {
       // the resident B operand of FC1 (x expanded into NVFP4 terms by the kernel launched just before this one) and its
       // scale tiles: one bulk copy
       mbar_expect_tx(&T.xb_full, KB1 * (N * 128) + P.KT1 * 512);
       bulk_load(region, P.xb, KB1 * (N * 128) + P.KT1 * 512, &T.xb_full);
     }
-    if (et < N) T.colscale[et] = P.xscale[et];
+    if (!self && et < N) T.colscale[et] = __ldcg(P.xscale + et);
     // The routing inputs were read at entry, before the wait above, so that the weight stream could start early. If they
     // were still being written then (a producer kernel that lets its successors start before it has written them), the
     // copies used here are stale: say so instead of returning a wrong result silently.
@@ -564,118 +727,65 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
       aph[ab] ^= 1u;
       ab ^= 1;
     };
-    // Sum of the partials of workers vlo..vhi in worker order (a fixed order: bit-identical from call to call). A partial
-    // holds N/4 floats per row; kRedBatch workers are loaded at once so that the L2 round trips overlap.
-    constexpr int kRedBatch = NB == 4 ? 6 : 12;
-    auto reduce = [&](int vlo, int nlive, float (&val)[16]) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) val[i] = 0.f;
-      for (int p0 = 0; p0 < nlive; p0 += kRedBatch) {
-        float4 tmp[kRedBatch][NB];
-#pragma unroll
-        for (int b = 0; b < kRedBatch; ++b) {
-          const bool live = p0 + b < nlive;
-          const float* src = P.scratch + ((long long)((vlo + (live ? p0 + b : 0)) * 2) * 128 + et) * 16;
-#pragma unroll
-          for (int i = 0; i < NB; ++i) tmp[b][i] = live ? __ldcg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int b = 0; b < kRedBatch; ++b)
-          if (p0 + b < nlive) {
-#pragma unroll
-            for (int i = 0; i < NB; ++i) { val[4 * i] += tmp[b][i].x; val[4 * i + 1] += tmp[b][i].y; val[4 * i + 2] += tmp[b][i].z; val[4 * i + 3] += tmp[b][i].w; }
-          }
-      }
-    };
-    // publish this worker's partial of its output block and learn whether it arrived last of the `nlive` holders
-    auto publish = [&](const float (&val)[16], unsigned* counter, int nlive) -> bool {
-      float* mine = P.scratch + ((long long)(v * 2) * 128 + et) * 16;
-#pragma unroll
-      for (int i = 0; i < NB; ++i) *reinterpret_cast<float4*>(mine + 4 * i) = make_float4(val[4 * i], val[4 * i + 1], val[4 * i + 2], val[4 * i + 3]);
-      named_bar_sync(1, 128);
-      if (et == 0) {
-        const unsigned old = atom_add_acq_rel_gpu(counter, 1u);   // releases the partial (barrier above), acquires the others'
-        const int last = old + 1u == (unsigned)nlive;
-        if (last) *counter = 0;   // nobody touches the counter again before the next launch
-        T.last_flag = last;
-      }
-      named_bar_sync(1, 128);
-      return T.last_flag != 0;   // the next write of last_flag is behind at least one more barrier of these 128 threads
-    };
-    // arrive at gate g of FC1: everything this worker wrote for the experts of the gate's group is visible to the TMA
-    // loads of every worker that sees the gate open (the producers are the only waiters)
-    auto arrive_gate = [&](int g) {
-      fence_proxy_async();
-      named_bar_sync(1, 128);
-      if (et == 0) red_add_release_gpu_u64(P.gates + g, 1ull);   // nothing to wait for: the gate is open when V have arrived
-    };
-
     // ---- FC1 pieces
     {
-      if (use_gate_a && nuA == 0) arrive_gate(0);
-      if (nu1 == 0) arrive_gate(1);
       for (int t = 0; t < nu1; ++t) {
         const int q = v + t * V, u = q / CB1, cb = q - u * CB1;   // a whole unit: K boxes 0..KB1-1 of (expert u, block cb)
         const int e = T.experts[u];
+        // s_w[tk]: routing weight of token tk on this expert folded with alpha2 (relative to the layer's largest), 0 when the
+        // token is not routed here - only routed tokens cost any arithmetic below (bit tk of s_mask).
+        if (warp == 0) {
+          float wsum = 0.f;
+          if (lane < P.M)
+            for (int sidx = 0; sidx < P.top_k; ++sidx)
+              if (T.ids[lane * P.top_k + sidx] == e) wsum += T.wts[lane * P.top_k + sidx];
+          wsum *= T.a2n[u];
+          const unsigned mask = __ballot_sync(0xffffffffu, wsum != 0.f);
+          if (lane < 16) s_w[lane] = wsum;
+          if (wsum != 0.f) s_tok[__popc(mask & ((1u << lane) - 1u))] = lane;
+          if (lane == 0) s_mask = mask;
+        }
         float val[16];
         load_terms(val, T.colscale, true);
         TC_T0(tfix);
         {
-          // rows 0..63 hold the up columns 64cb.., rows 64..127 the gate columns: exchange through shared memory.
-          // s_w[tk]: routing weight of token tk on this expert folded with alpha2 (relative to the layer's largest), 0 when
-          // the token is not routed here - only routed tokens cost any arithmetic below.
+          // rows 0..63 hold the up columns 64cb.., rows 64..127 the gate columns: exchange through shared memory
           const float alpha = T.a1[u];
-          if (et < 16) {
-            float wsum = 0.f;
-            if (et < P.M)
-              for (int sidx = 0; sidx < P.top_k; ++sidx)
-                if (T.ids[et * P.top_k + sidx] == e) wsum += T.wts[et * P.top_k + sidx];
-            s_w[et] = wsum * T.a2n[u];
-          }
-          if (row >= 64) {
+          float* mine = row < 64 ? &s_up[0][row] : &s_gate[0][row - 64];
 #pragma unroll
-            for (int tk = 0; tk < 16; ++tk) s_ex[row - 64][tk] = val[tk] * alpha;
-          }
+          for (int tk = 0; tk < N / 4; ++tk) mine[tk * 68] = val[tk] * alpha;
           named_bar_sync(1, 128);
-          if (row < 64) {
-#pragma unroll
-            for (int tk = 0; tk < 16; ++tk) {
-              const float wf = s_w[tk];
-              s_ex[row][tk] = wf != 0.f ? tc_silu_mul(s_ex[row][tk], val[tk] * alpha) * wf : 0.f;   // only this thread reads that gate value
-            }
-          }
-          named_bar_sync(1, 128);
-          // re-expand: thread (token, 16-column block) -> four NVFP4 terms of the FC2 operand; a token that is not routed
-          // here only gets zero scale bytes (a zero scale silences whatever codes the row holds). (Spreading a block over
-          // four lanes - expand_block16_quad - was measured: no gain at any batch size, the expansion is off the critical path.)
-          if (et < N) {
-            const int tk = et >> 2, blk = et & 3;
-            uint8_t* slab = P.aslab + ((long long)u * KB2 + (cb >> 2)) * kSlab;   // slab of K box cb/4
-            uint8_t* sfp = slab + N * 128 + (cb & 3) * 512 + blk;
+          const unsigned mask = s_mask;
+          const int cnt = __popc(mask);
+          uint8_t* slab = P.aslab + ((long long)u * KB2 + (cb >> 2)) * kSlab;   // slab of K box cb/4
+          uint8_t* sfp = slab + N * 128 + (cb & 3) * 512;
+          // a token that is not routed here only gets zero scale bytes (a zero scale silences whatever codes the row holds)
+          if (et < N && !((mask >> (et >> 2)) & 1u)) *reinterpret_cast<uint32_t*>(sfp + (et & 31) * 16 + (et >> 5) * 4) = 0u;
+          // SiLU*mul and re-expansion, four lanes per (routed token, 16-column block): four NVFP4 terms of the FC2 operand. (With a
+          // thread per block, in two passes through shared memory, a unit's epilogue took 2.4 us; several of them stand between
+          // FC1's last MMA and its gate.)
+#pragma unroll 1
+          for (int i0 = warp * 8; i0 < 4 * cnt; i0 += 32) {
+            const int i = i0 + (lane >> 2), blk = i & 3;
+            const bool live = i < 4 * cnt;
+            const int tk = live ? s_tok[i >> 2] : 0;
+            const int col = blk * 16 + 4 * (lane & 3);
+            const float4 up = *reinterpret_cast<const float4*>(&s_up[tk][col]), gt = *reinterpret_cast<const float4*>(&s_gate[tk][col]);
+            const float wf = s_w[tk];
+            float r[4] = {tc_silu_mul(gt.x, up.x) * wf, tc_silu_mul(gt.y, up.y) * wf, tc_silu_mul(gt.z, up.z) * wf, tc_silu_mul(gt.w, up.w) * wf};
             const int chunk = 2 * (cb & 3) + (blk >> 1);                        // 16-byte chunk of the row's 128 bytes
-            if (s_w[tk] != 0.f) {
-              float r[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) r[i] = s_ex[blk * 16 + i][tk];
-              const bool clipped = expand_block16<false>(r, P.act_g1, [&](int t, uint2 codes, uint8_t sf) {
-                const int n = tk * kTerms + t;
-                *reinterpret_cast<uint2*>(slab + n * 128 + ((chunk ^ (n & 7)) << 4) + (blk & 1) * 8) = codes;
-                sfp[(n & 31) * 16 + (n >> 5) * 4] = sf;
-              });
-              if (clipped) P.status[1] = 1;   // beyond the range of the fixed activation scale
-            } else {
-#pragma unroll
-              for (int t = 0; t < kTerms; ++t) {
-                const int n = tk * kTerms + t;
-                sfp[(n & 31) * 16 + (n >> 5) * 4] = 0;
-              }
-            }
+            const bool clipped = expand_quad(r, P.act_g1, [&](int t, uint16_t codes, uint8_t sf) {
+              const int n = tk * kTerms + t;
+              if (!live) return;
+              *reinterpret_cast<uint16_t*>(slab + n * 128 + ((chunk ^ (n & 7)) << 4) + (blk & 1) * 8 + 2 * (lane & 3)) = codes;
+              if ((lane & 3) == 0) sfp[(n & 31) * 16 + (n >> 5) * 4 + blk] = sf;
+            });
+            if (clipped && live) P.status[1] = 1;   // beyond the range of the fixed activation scale
           }
           named_bar_sync(1, 128);
+          if (et == 0) { __threadfence_block(); T.units_done = t + 1; }
         }
         TC_ADD(tm_b, tfix);
-        if (use_gate_a && t == nuA - 1) arrive_gate(0);
-        if (t == nu1 - 1) arrive_gate(1);
       }
 #ifdef B200_TIMERS
       tm_c = clock64() - tm_begin;
@@ -692,11 +802,41 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_moe_decode_tc(const __grid_co
       }
       float val[16];
       load_terms(val, cs, false);
-      if (publish(val, P.cnt2 + nb2, live2)) {
-        reduce(vlo2, live2, val);
+      // Publish the partial as flagged words ([worker][token pair][row], 16 bytes each); the first workers of the group add the
+      // block's outputs, in worker order. Nothing is fenced or counted: a word that carries this launch's number has its value.
+      // One adder per two token pairs, and the others leave at once, so that the next launch's blocks can start on their SMs.
+      // (With a counter whose last arriver adds: 0.9 us more for its round trip, and nobody leaves before it. With every worker of
+      // the group adding a share: all leave 2 us later, 12 % more per layer at one token.)
+      const int tpairs = (P.M + 1) >> 1;
+      uint4* words = reinterpret_cast<uint4*>(P.partials);
 #pragma unroll
-        for (int tk = 0; tk < 16; ++tk)
-          if (tk < P.M) P.out[(long long)tk * P.H + 128 * nb2 + row] = __float2bfloat16_rn(val[tk]);
+      for (int tp = 0; tp < N / 8; ++tp)
+        if (tp < tpairs) st_flagged2(words + ((long long)v * 8 + tp) * 128 + row, val[2 * tp], val[2 * tp + 1], call);
+      const int tasks = 128 * tpairs, adders = min(live2, (tpairs + 1) >> 1);
+      const int first = r2 < adders ? tasks * r2 / adders : 0, last = r2 < adders ? tasks * (r2 + 1) / adders : 0;
+      for (int i = first + et; i < last; i += 128) {
+        const uint4* src = words + (long long)vlo2 * 1024 + i;
+        float s0 = 0.f, s1 = 0.f;
+        constexpr int kBatch = 8;
+        for (int p0 = 0; p0 < live2; p0 += kBatch) {
+          float a[kBatch], b[kBatch];
+          for (uint32_t it = 0;; ++it) {
+            bool ok = true;
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
+              if (p0 + k < live2) ok &= ld_flagged2(src + (long long)(p0 + k) * 1024, call, a[k], b[k]);
+            if (ok) break;
+            if (T.abort_flag || it >= (1u << 22)) { T.abort_flag = 1; *P.status = 10; break; }
+            __nanosleep(50);
+          }
+#pragma unroll
+          for (int k = 0; k < kBatch; ++k)
+            if (p0 + k < live2) s0 += a[k], s1 += b[k];
+        }
+        const int tk = 2 * (i >> 7);
+        __nv_bfloat16* dst = P.out + (long long)tk * P.H + 128 * nb2 + (i & 127);
+        dst[0] = __float2bfloat16_rn(s0);
+        if (tk + 1 < P.M) dst[P.H] = __float2bfloat16_rn(s1);
       }
     } else if (I2 == 0 && r2 == 0) {   // every slot of the batch is empty: the layer's output is zero
       for (int tk = 0; tk < P.M; ++tk) P.out[(long long)tk * P.H + 128 * nb2 + row] = __float2bfloat16_rn(0.f);
@@ -735,18 +875,33 @@ int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, 
   return launch_kernel(host ? (const void*)k_expand_x<true> : (const void*)k_expand_x<false>, N / kTerms, 128, 0, chained && pdl_chain_enabled(), args, st);
 }
 
-// x, ids and weights of a call from page-locked host memory into device memory, for the kernel that does not take them from there
-__global__ void __launch_bounds__(256) k_host_stage(const uint4* x, int n16, const int* ids_h, const float* wts_h, int npairs, uint4* x_d, int* ids_d, float* wts_d) {
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i < n16) x_d[i] = __ldcv(x + i);
-  if (i < npairs) { ids_d[i] = __ldcv(ids_h + i); wts_d[i] = __ldcv(wts_h + i); }
+// x, ids and weights of a call from page-locked host memory into device memory. Block 0 brings the routing inputs, which the
+// layer kernel reads at its entry, before it lets that kernel start; the others bring x.
+__global__ void __launch_bounds__(128) k_host_stage(const uint4* x, int n16, const int* ids_h, const float* wts_h, int npairs, uint4* x_d, int* ids_d, float* wts_d) {
+  const int tid = threadIdx.x;
+  grid_dependency_wait();   // a kernel before this one may still read the copies it replaces
+  if (blockIdx.x != 0) {
+    grid_launch_dependents();
+    const int i = (blockIdx.x - 1) * 128 + tid;
+    if (i < n16) __stcg(x_d + i, __ldcv(x + i));
+    return;
+  }
+  int id[2];
+  float wt[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (tid + 128 * j < npairs) { id[j] = __ldcv(ids_h + tid + 128 * j); wt[j] = __ldcv(wts_h + tid + 128 * j); }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (tid + 128 * j < npairs) { __stcg(ids_d + tid + 128 * j, id[j]); __stcg(wts_d + tid + 128 * j, wt[j]); }
+  __threadfence();
+  __syncthreads();
+  grid_launch_dependents();
 }
 
-int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, cudaStream_t st) {
-  const int n = n16 > h.npairs ? n16 : h.npairs;
-  k_host_stage<<<(n + 255) / 256, 256, 0, st>>>((const uint4*)x, n16, h.ids_h, h.wts_h, h.npairs, (uint4*)x_d, h.ids_d, h.wts_d);
-  B200_LAUNCH_CHECK();
-  return B200MOE_OK;
+int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, bool chained, cudaStream_t st) {
+  void* args[] = {(void*)&x, (void*)&n16, (void*)&h.ids_h, (void*)&h.wts_h, (void*)&h.npairs, (void*)&x_d, (void*)&h.ids_d, (void*)&h.wts_d};
+  return launch_kernel((const void*)k_host_stage, 1 + (n16 + 127) / 128, 128, 0, chained && pdl_chain_enabled(), args, st);
 }
 
 // q u8 [E, rows, row_bytes], sf = 128x4-swizzled scales per expert -> tile records (see k_pack_tiles)

@@ -99,6 +99,11 @@ __device__ __forceinline__ void bulk_load_hint(void* dst, const void* src, uint3
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
                : "memory");
 }
+// 1-D bulk copy shared -> global; returns when the shared memory has been read
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n cp.async.bulk.commit_group;\n cp.async.bulk.wait_group.read 0;"
+               ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
 // ask for `bytes` (a multiple of 16) of global memory to be brought into L2
 __device__ __forceinline__ void l2_prefetch(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
@@ -198,6 +203,24 @@ __device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned 
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+
+__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// Flagged words: two 8-byte words {value, flag} per 16-byte access; each word is stored and loaded whole, so whoever finds the flag in a
+// word has its value.
+__device__ __forceinline__ void st_flagged2(void* p, float a, float b, unsigned flag) {
+  const unsigned long long w0 = ((unsigned long long)flag << 32) | __float_as_uint(a), w1 = ((unsigned long long)flag << 32) | __float_as_uint(b);
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(w0), "l"(w1) : "memory");
+}
+__device__ __forceinline__ bool ld_flagged2(const void* p, unsigned flag, float& a, float& b) {
+  unsigned long long w0, w1;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p) : "memory");
+  a = __uint_as_float((unsigned)w0), b = __uint_as_float((unsigned)w1);
+  return (unsigned)(w0 >> 32) == flag && (unsigned)(w1 >> 32) == flag;
 }
 
 }  // namespace b200

@@ -184,12 +184,6 @@ __global__ void __launch_bounds__(kQThreads) k_quantize_small(const T* x, QuantG
 // word {call number + 1, bits of the largest magnitude} per amax unit. A word is stored whole, so whoever reads this call's
 // number in it has the maximum: nothing is counted and nothing is fenced, and a unit's only round trip to L2 overlaps its loads.
 // (With a ticket per unit and counters behind a fence: 330 to 400 us for 128 x 1536 x 2048 bf16.)
-__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, int groups, int units, int window, QuantGeom q, float* gs_out,
                                                                     uint8_t* packed, uint8_t* sf, unsigned* scratch) {
