@@ -70,8 +70,11 @@ struct TcTables {
 __device__ __forceinline__ float tc_silu_mul(float gate, float up) { return __fdividef(gate, 1.0f + __expf(-gate)) * up; }
 
 // ------------------------------------------------------------------------------------------------ x -> B operand
-// One block of 128 threads per token slot (N/4 slots): token amax, then every 16-value block expanded into four NVFP4
-// terms. The block is small enough (registers, shared memory) to be resident next to a block of the layer kernel.
+// One block of 256 threads per token slot (N/4 slots), a thread per 16-value block: token amax, then the block expanded into four
+// NVFP4 terms. The block is small enough (registers, shared memory) to be resident next to a block of the layer kernel.
+// What bounds it is latency: it starts when the kernel before it has completed and the layer kernel waits for it. So it goes
+// through its code once before that, on zeros and without storing: a launch finds none of its instructions in the SM's cache, and
+// fetching them took 2 of the 3 us it needed.
 // xb: the FC1 B operand exactly as the kernel wants it in shared memory, so that ONE bulk copy brings it in:
 //   [KB1 boxes][N rows (token*4 + term)][128 B] in the 128-byte-swizzle image (16-byte chunk c of row n sits at chunk
 //   c ^ (n & 7)), followed by KT1 scale tiles of 512 B (128x4 order, rows >= N zero). colscale f32 [N] = 1/g_t.
@@ -79,77 +82,64 @@ __device__ __forceinline__ float tc_silu_mul(float gate, float up) { return __fd
 // routing inputs into device memory (ids_d, wts_d) before it lets the layer kernel start, which reads them at its entry: one
 // kernel instead of three copies that wait for one another and for the link (13 us a call).
 template <bool kHost>
-__global__ void __launch_bounds__(128, 10) k_expand_x(const __nv_bfloat16* x, int M, int H, int N, int KB1, uint8_t* xb, float* colscale,
-                                                      const int* ids_h, const float* wts_h, int npairs, int* ids_d, float* wts_d) {
-  const int tok = blockIdx.x, tid = threadIdx.x;
+__global__ void __launch_bounds__(256, 4) k_expand_x(const __nv_bfloat16* x, int M, int H, int N, int KB1, uint8_t* xb, float* colscale,
+                                                     const int* ids_h, const float* wts_h, int npairs, int* ids_d, float* wts_d) {
+  const int tok = blockIdx.x, tid = threadIdx.x, b = tid;
   if (!kHost) grid_launch_dependents();   // the layer kernel may start its prologue and weight prefetch now; it waits before reading xb
-  grid_dependency_wait();     // this kernel is itself launched programmatically: x (and the workspace it writes) belong to
-                              // whatever ran before it in the stream until that has completed
-  if (kHost && tok != 0) grid_launch_dependents();
   uint8_t* xsf = xb + (long long)KB1 * N * 128;
-  __shared__ float wm[4];
-  // each thread keeps its (at most two) 16-value blocks in registers: one pass over x serves the token amax and the expansion
-  const int nblk = KB1 * 16;                 // blocks over the padded K (KB1 * 256 values); nblk <= 256
-  uint4 raw[2][2];
-  float m = 0.f;
+  __shared__ unsigned wm[8];
+  const bool live = tok < M && b * 16 < H;
+  const int kb = b >> 4, chunk = (b & 15) >> 1, half = b & 1;   // 8 code bytes = half a 16-byte chunk
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    uint4 u = make_uint4(0u, 0u, 0u, 0u), v = u;
+    if (pass == 1) {
+      grid_dependency_wait();     // this kernel is itself launched programmatically: x (and the workspace it writes) belong to
+                                  // whatever ran before it in the stream until that has completed
+      if (kHost && tok != 0) grid_launch_dependents();
+      if (live) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + (long long)tok * H + b * 16);
+        u = kHost ? __ldcv(src) : src[0];
+        v = kHost ? __ldcv(src + 1) : src[1];
+      }
+      if (kHost && tok == 0) {   // (x is in flight)
+        if (tid < npairs) {
+          __stcg(ids_d + tid, __ldcv(ids_h + tid));
+          __stcg(wts_d + tid, __ldcv(wts_h + tid));
+        }
+        __threadfence();
+        __syncthreads();
+        grid_launch_dependents();
+      }
+    }
+    const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    __nv_bfloat162 m2 = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int b = tid + 128 * j;
-    raw[j][0] = raw[j][1] = make_uint4(0u, 0u, 0u, 0u);
-    if (tok < M && b < nblk && b * 16 < H) {
-      const uint4* src = reinterpret_cast<const uint4*>(x + (long long)tok * H + b * 16);
-      raw[j][0] = kHost ? __ldcv(src) : src[0];
-      raw[j][1] = kHost ? __ldcv(src + 1) : src[1];
-    }
-  }
-  if (kHost && tok == 0) {   // (x is in flight)
-    for (int p = tid; p < npairs; p += 128) {
-      __stcg(ids_d + p, __ldcv(ids_h + p));
-      __stcg(wts_d + p, __ldcv(wts_h + p));
-    }
-    __threadfence();
+    for (int i = 1; i < 8; ++i) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+    const uint32_t bits = *reinterpret_cast<const uint32_t*>(&m2);
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, max(bits << 16, bits & 0xffff0000u));   // non-negative floats order like their bits
+    if ((tid & 31) == 0) wm[tid >> 5] = wmax;
     __syncthreads();
-    grid_launch_dependents();
-  }
+    unsigned mb = 0;
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    {
-      const uint32_t w[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(fabsf(__uint_as_float(w[i] << 16)), fabsf(__uint_as_float(w[i] & 0xffff0000u))));
+    for (int i = 0; i < 8; ++i) mb = max(mb, wm[i]);
+    const float g1 = 2688.0f / fmaxf(__uint_as_float(mb), 1e-30f);
+    if (tid < kTerms) {
+      float g = g1;
+      for (int t = 0; t < tid; ++t) g *= 6.0f;
+      if (pass == 1) colscale[tok * kTerms + tid] = tok < M ? 1.0f / g : 0.f;
     }
-  }
+    float r[16];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((tid & 31) == 0) wm[tid >> 5] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
-  const float g1 = 2688.0f / fmaxf(m, 1e-30f);
-  if (tid < kTerms) {
-    float g = g1;
-    for (int t = 0; t < tid; ++t) g *= 6.0f;
-    colscale[tok * kTerms + tid] = tok < M ? 1.0f / g : 0.f;
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int b = tid + 128 * j;
-    if (b >= nblk) break;
-    const int kb = b >> 4, chunk = (b & 15) >> 1, half = b & 1;   // 8 code bytes = half a 16-byte chunk
-    const bool scales = (b >> 2) < (H / 16 + 3) / 4;
-    auto put = [&](int t, uint2 codes, uint8_t sf) {
+    for (int i = 0; i < 8; ++i) { r[2 * i] = __uint_as_float(w[i] << 16); r[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    // (a block beyond the batch or the row is all zeros, and so are its codes and scales)
+    expand_block16<true>(r, g1, [&](int t, uint2 codes, uint8_t sf) {
+      if (pass == 0 || b >= KB1 * 16) return;
       const int n = tok * kTerms + t;
       *reinterpret_cast<uint2*>(xb + ((long long)kb * N + n) * 128 + ((chunk ^ (n & 7)) << 4) + half * 8) = codes;
-      if (scales) xsf[(long long)(b >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (b & 3)] = sf;
-    };
-    if (tok < M && b * 16 < H) {
-      float r[16];
-      const uint32_t w[8] = {raw[j][0].x, raw[j][0].y, raw[j][0].z, raw[j][0].w, raw[j][1].x, raw[j][1].y, raw[j][1].z, raw[j][1].w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { r[2 * i] = __uint_as_float(w[i] << 16); r[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
-      expand_block16<false>(r, g1, put);
-    } else {
-      for (int t = 0; t < kTerms; ++t) put(t, make_uint2(0u, 0u), 0);
-    }
+      if ((b >> 2) < (H / 16 + 3) / 4) xsf[(long long)(b >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (b & 3)] = sf;
+    });
+    __syncthreads();   // wm is free again
   }
 }
 
@@ -194,18 +184,18 @@ __global__ void __launch_bounds__(256) k_pack_tiles(const uint8_t* __restrict__ 
 }
 
 // ------------------------------------------------------------------------------------------------ x -> B operand, inside the layer kernel
-// Small operands (P.self: up to 1024 blocks of 16 values, e.g. eight tokens of 2048) every worker expands by itself, with its 128
-// epilogue threads, straight into shared memory. As a kernel of its own (16 blocks) the expansion costs a launch, and its
-// result has to travel: from the completion of the kernel before to the operand's arrival 4.3 us at one token of 2048 values
-// and 5.7 us at four of 2816, against 2.7 and 5.8 us here. The work in a worker grows with the tokens (0.35 us per 128 blocks),
-// so beyond 1024 blocks the separate kernel is ahead.
+// Small operands (P.self: up to 256 blocks of 16 values, e.g. two tokens of 2048) every worker expands by itself, with its 128
+// epilogue threads, straight into shared memory: a launch less, and nothing has to travel (one token of 2048 values: 2.7 us from
+// the completion of the kernel before to the operand, against 3.5 to 4.3 with the kernel above; a layer 12.2 us against 13.5).
+// Beyond that the kernel's 16 blocks are ahead: four tokens of 2816 values take 6 us here, where loads wait behind the weight
+// stream and the work per thread grows (a layer 27.3 us against 26.0).
 __device__ __forceinline__ void zero_scales(uint8_t* xsf, int KT1, int et) {   // rows that hold no token keep zero scales
   for (int i = et; i < KT1 * 32; i += 128) reinterpret_cast<uint4*>(xsf)[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int N>
 __device__ __forceinline__ void expand_x_here(const DecodeTcParams& P, uint8_t* region, float* colscale, unsigned* amax, float* g1s, int et) {
-  constexpr int kTok = N / kTerms, kMost = 8;   // blocks per thread
+  constexpr int kTok = N / kTerms, kMost = 2;   // blocks per thread
   const int nb = P.H >> 4, lane = et & 31, total = P.M * nb;
   uint8_t* xsf = region + P.KB1 * (N * 128);
   // this thread's blocks: et, et + 128, ...; all of x is loaded at once and stays in registers (a load takes 1 to 2 us here, while the
@@ -249,7 +239,7 @@ __device__ __forceinline__ void expand_x_here(const DecodeTcParams& P, uint8_t* 
     for (int q = 0; q < (et & 3); ++q) g *= 6.0f;
     colscale[et] = (et >> 2) < P.M ? 1.0f / g : 0.f;
   }
-  int left = (total - et + 127) >> 7, tok = tok0, b = b0;
+  int tok = tok0, b = b0;
   auto expand = [&](auto two) {
     constexpr int K = decltype(two)::value;
     int tk[K], bb[K];
@@ -268,12 +258,10 @@ __device__ __forceinline__ void expand_x_here(const DecodeTcParams& P, uint8_t* 
       *reinterpret_cast<uint2*>(region + (c >> 4) * (N * 128) + n * 128 + ((((c & 15) >> 1) ^ (n & 7)) << 4) + (c & 1) * 8) = codes;
       xsf[(c >> 2) * 512 + (n & 31) * 16 + (n >> 5) * 4 + (c & 3)] = sf;
     });
-#pragma unroll
-    for (int j = 0; j + K < kMost; ++j) raw[j][0] = raw[j + K][0], raw[j][1] = raw[j + K][1];
   };
-#pragma unroll 1
-  for (; left >= 2; left -= 2) expand(std::integral_constant<int, 2>());
-  if (left > 0) expand(std::integral_constant<int, 1>());
+  const int mine = (total - et + 127) >> 7;
+  if (mine == 2) expand(std::integral_constant<int, 2>());
+  else if (mine == 1) expand(std::integral_constant<int, 1>());
 }
 
 // ------------------------------------------------------------------------------------------------ the layer kernel
@@ -872,7 +860,7 @@ int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, 
   const HostRouting h = host ? *host : HostRouting{nullptr, nullptr, 0, nullptr, nullptr};
   void* args[] = {(void*)&x, (void*)&M, (void*)&H, (void*)&N, (void*)&KB1, (void*)&xb, (void*)&colscale,
                   (void*)&h.ids_h, (void*)&h.wts_h, (void*)&h.npairs, (void*)&h.ids_d, (void*)&h.wts_d};
-  return launch_kernel(host ? (const void*)k_expand_x<true> : (const void*)k_expand_x<false>, N / kTerms, 128, 0, chained && pdl_chain_enabled(), args, st);
+  return launch_kernel(host ? (const void*)k_expand_x<true> : (const void*)k_expand_x<false>, N / kTerms, 256, 0, chained && pdl_chain_enabled(), args, st);
 }
 
 // x, ids and weights of a call from page-locked host memory into device memory. Block 0 brings the routing inputs, which the
