@@ -215,7 +215,7 @@ static int decode_tc_ring(const b200moe_layer* L, int N, int* region) {
   const int xb = L->KB1 * N * 128 + L->KT1 * 512, slab = N * 128 + 2048;
   for (int NS = 12; NS >= 3; --NS) {
     *region = (int)align_up(xb > NS * slab ? xb : NS * slab, 1024);
-    if (b200_decode_tc_smem_bytes(NS, *region) <= 227 * 1024 - 6144) return NS;   // room for static shared memory
+    if (b200_decode_tc_smem_bytes(NS, *region) + b200_decode_tc_static_bytes(N) <= 227 * 1024) return NS;
   }
   return 0;
 }

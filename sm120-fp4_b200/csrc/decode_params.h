@@ -72,6 +72,7 @@ struct DecodeTcParams {
 }  // namespace b200
 
 int b200_decode_tc_smem_bytes(int NS, int region_bytes);
+int b200_decode_tc_static_bytes(int N);
 // routing inputs in page-locked host memory and the device copies that a kernel is to make of them
 struct HostRouting { const int* ids_h; const float* wts_h; int npairs; int* ids_d; float* wts_d; };
 int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, const HostRouting* host, bool chained, cudaStream_t st);

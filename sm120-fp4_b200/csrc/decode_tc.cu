@@ -849,6 +849,9 @@ using namespace b200;
 
 int b200_decode_tc_smem_bytes(int NS, int region_bytes) { return 1024 + NS * kTcStage + region_bytes + (int)sizeof(TcTables); }
 
+// static shared memory of the kernel for N operand columns: FC1's sums [N / 4][68] of up and of gate, and a few words
+int b200_decode_tc_static_bytes(int N) { return 2 * (N / 4) * 68 * 4 + 256; }
+
 static bool pdl_chain_enabled() {   // B200MOE_PDL_CHAIN=0: launch the expansion kernel as an ordinary stream-ordered kernel
   static const bool on = [] { const char* c = getenv("B200MOE_PDL_CHAIN"); return !(c && c[0] == '0'); }();
   return on;

@@ -1,0 +1,40 @@
+"""Sizes at which the decode call changes its way: hidden sizes above 3072 (the tcgen05 kernel takes them up to 4096; with more than
+eight tokens some of them fall to the mma.sync kernel), x expanded by every worker itself up to 256 blocks of 16 values and eight
+tokens, and the same boundaries for tensors in page-locked host memory."""
+import pytest
+import torch
+
+from helpers import check_layer_output, make_layer
+from oracle import nvfp4_oracle as O
+from test_gpu_decode import inputs, run
+
+pytestmark = pytest.mark.gpu
+
+_layers = {}
+
+
+def edge_layer(hidden, inter=192):
+    cfg = dict(experts=16, hidden=hidden, inter=inter, top_k=4)
+    if (hidden, inter) not in _layers:
+        _layers.clear()
+        _layers[hidden, inter] = make_layer(**cfg, seed=9)
+    return cfg, *_layers[hidden, inter]
+
+
+# 512: 8 tokens are the last, 256 blocks; 4096: one token is; 2048 x 2; 3200 = 12.5 K boxes
+@pytest.mark.parametrize("hidden,m", [(512, 8), (512, 9), (2048, 2), (2048, 3), (3072, 1), (3072, 16), (3200, 1), (3200, 8), (3200, 9), (3200, 16),
+                                      (4096, 1), (4096, 2), (4096, 8), (4096, 9), (4096, 16)])
+def test_hidden_sizes_and_batches(hidden, m):
+    cfg, w, ow = edge_layer(hidden)
+    x, ids, wts = inputs(cfg, m, 40 + m)
+    out = run(w, x, ids, wts).clone()
+    check_layer_output(out, O.moe_reference(x.float().numpy(), ow, ids.numpy(), wts.numpy()), f"hidden {hidden}, {m} tokens")
+    pinned = [t.pin_memory() for t in (x, ids, wts)]
+    host = torch.empty_like(x).pin_memory()
+    for _ in range(2):
+        host.zero_()
+        torch.cuda.synchronize()
+        w.forward_host(*pinned, host)
+        torch.cuda.synchronize()
+        assert torch.equal(host, out.cpu())
+    w.status()
