@@ -6,7 +6,9 @@
 // pairs of one expert are ranked by lane (match.any) on top of a running count per (warp, expert) in shared memory, so a pair's
 // position is known up to the start of its warp's run. Per expert the counts are then scanned over the warps, over the CTAs
 // (distributed shared memory) and over the experts; no atomic decides a position. Bound by latency (a few dependent passes of
-// a microsecond each), not by bytes: 4 bytes in and 12 out per pair.
+// a microsecond each). What is scattered by row (`pairs`, `row_pair`) is written by the kernel behind this one (put_pair, one thread
+// per pair on every SM): eight SMs take one 32-byte sector a cycle each, and with those stores in here a plan of
+// 65536 pairs took 27 us instead of 16. A warp keeps its run's positions in registers between the two passes, up to 256 pairs.
 #pragma once
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -21,14 +23,27 @@ __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
   return v;
 }
 
-// TILE pairs per row tile, ROWS operand rows per pair. row_pair [tiles*TILE*ROWS] = pair of every operand row of a tile (-1: none),
+// TILE pairs per row tile (at most P / TILE + Umax tiles: the tables have room for them), ROWS operand rows per pair. row_pair
+// [tiles*TILE*ROWS] = pair of every operand row of a tile (-1: none),
 // dst_row[pair] = tile * TILE + slot (-1: empty slot, or an id >= E). tile_first / tile_end: first and end index into `pairs`.
 struct PlanTables {
-  int *experts, *offsets, *pairs, *ntiles, *tile_expert, *tile_first, *tile_end, *row_pair, *dst_row;
+  int *experts, *offsets, *ntiles, *tile_expert, *tile_first, *tile_end, *dst_row;
 };
 
+// The scattered tables, written behind the plan kernel. `first` = tile_first of the pair's tile (read ahead by the caller).
+struct PairTables {
+  const int* tile_first;
+  int *pairs, *row_pair;
+};
 template <int TILE, int ROWS>
-__global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int Umax, int max_tiles, PlanTables T) {
+__device__ __forceinline__ void put_pair(const PairTables& T, int pair, int row, int first) {
+  T.pairs[first + row % TILE] = pair;
+  if (ROWS == 4) *reinterpret_cast<int4*>(T.row_pair + 4LL * row) = make_int4(pair, pair, pair, pair);
+  else T.row_pair[row] = pair;
+}
+
+template <int TILE>
+__global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int Umax, PlanTables T) {
   __shared__ int wc[32][kPlanMaxE];     // pairs of expert e in warp w's run, then the start of the run in `pairs`
   __shared__ int tot[kPlanMaxE];        // ... in this CTA (read by the other CTAs)
   __shared__ int cnt[kPlanMaxE], off[kPlanMaxE], tb[kPlanMaxE];   // all pairs of expert e, its first index in `pairs`, its first tile
@@ -42,23 +57,27 @@ __global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int
   __syncthreads();
   const int L = ((P + C * 32 - 1) / (C * 32) + 31) & ~31;   // pairs per warp
   const int p0 = (rank * 32 + warp) * L, p1 = min(P, p0 + L);
-  // ---- positions inside the warp's run; dst_row holds (expert, position) until the run's start is known
+  // ---- positions inside the warp's run. (expert, position) is kept in `held` until the run's start is known, or in dst_row by runs that do
+  // not fit
+  constexpr int kHeld = 8;
+  const bool fits = L <= 32 * kHeld;
+  int held[kHeld];
 #pragma unroll 1
-  for (int s = p0; s < p1; s += 128) {   // four steps of 32, their ids in flight together
-    int id[4];
+  for (int s = p0; s < p1; s += 32 * kHeld) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) id[k] = s + 32 * k + lane < p1 ? __ldcg(ids + s + 32 * k + lane) : -1;
+    for (int k = 0; k < kHeld; ++k) held[k] = s + 32 * k + lane < p1 ? __ldcg(ids + s + 32 * k + lane) : -1;   // in flight together
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < kHeld; ++k) {
       if (s + 32 * k >= p1) break;
-      const int p = s + 32 * k + lane;
-      const int e = id[k] < 0 || id[k] >= E ? -1 : id[k];
+      const int e = held[k] < 0 || held[k] >= E ? -1 : held[k];
       const unsigned peers = __match_any_sync(0xffffffffu, e);
       const int r = __popc(peers & ((1u << lane) - 1u));
       const int before = e >= 0 ? wc[warp][e] : 0;
       __syncwarp();
       if (e >= 0 && r == 0) wc[warp][e] = before + __popc(peers);
-      if (p < p1) __stcg(T.dst_row + p, e >= 0 ? (e << 22) | (before + r) : -1);
+      held[k] = e >= 0 ? (e << 22) | (before + r) : -1;
+      const int p = s + 32 * k + lane;
+      if (!fits && p < p1) __stcg(T.dst_row + p, held[k]);
       __syncwarp();
     }
   }
@@ -93,7 +112,7 @@ __global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int
       if (lane >= o) { ic += a; iu += b; it += d; }
     }
     int rc = ic - sc, ru = iu - su, rt = it - st;
-    const int routed = __shfl_sync(0xffffffffu, ic, 31), U = __shfl_sync(0xffffffffu, iu, 31), NT = min(__shfl_sync(0xffffffffu, it, 31), max_tiles);
+    const int routed = __shfl_sync(0xffffffffu, ic, 31), U = __shfl_sync(0xffffffffu, iu, 31), NT = __shfl_sync(0xffffffffu, it, 31);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int e = lane * 8 + i;
@@ -111,52 +130,38 @@ __global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int
   }
   __syncthreads();
   if (tid < kPlanMaxE) {
-    const int o = off[tid] + mine;
+    const int o = tb[tid] * TILE + mine;   // from here on: operand row (TILE per tile) of the first pair of expert e in warp w's run
 #pragma unroll 8
     for (int w = 0; w < 32; ++w) wc[w][tid] += o;
   }
   __syncthreads();
-  // ---- the tables of every pair
+  // ---- the row of every pair
 #pragma unroll 1
-  for (int s = p0; s < p1; s += 128) {
-    int v[4];
+  for (int s = p0; s < p1; s += 32 * kHeld) {
+    if (!fits) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = s + 32 * k + lane < p1 ? __ldcg(T.dst_row + s + 32 * k + lane) : -1;
+      for (int k = 0; k < kHeld; ++k) held[k] = s + 32 * k + lane < p1 ? __ldcg(T.dst_row + s + 32 * k + lane) : -1;
+    }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (v[k] < 0) continue;                  // dst_row stays -1
-      const int p = s + 32 * k + lane, e = v[k] >> 22, pos = wc[warp][e] + (v[k] & ((1 << 22) - 1));
-      const int row = tb[e] * TILE + pos - off[e];
-      T.pairs[pos] = p;
-      const bool fits = row < max_tiles * TILE;
-      T.dst_row[p] = fits ? row : -1;
-      if (fits) {
-        if (ROWS == 4) *reinterpret_cast<int4*>(T.row_pair + 4LL * row) = make_int4(p, p, p, p);
-        else T.row_pair[row] = p;
-      }
+    for (int k = 0; k < kHeld; ++k) {
+      const int p = s + 32 * k + lane;
+      if (p < p1) T.dst_row[p] = held[k] < 0 ? -1 : wc[warp][held[k] >> 22] + (held[k] & ((1 << 22) - 1));
     }
   }
-  // ---- tile tables and the rows that hold no pair: one warp of the cluster per expert
+  // ---- tile tables: one warp of the cluster per expert
   for (int e = rank * 32 + warp; e < E; e += C * 32) {
     const int c = cnt[e], nt = (c + TILE - 1) / TILE;
     for (int j = lane; j < nt; j += 32) {
       const int t = tb[e] + j;
-      if (t < max_tiles) { T.tile_expert[t] = e; T.tile_first[t] = off[e] + j * TILE; T.tile_end[t] = off[e] + c; }
-    }
-    for (int r = c + lane; r < nt * TILE; r += 32) {
-      const int row = tb[e] * TILE + r;
-      if (row < max_tiles * TILE) {
-        if (ROWS == 4) *reinterpret_cast<int4*>(T.row_pair + 4LL * row) = make_int4(-1, -1, -1, -1);
-        else T.row_pair[row] = -1;
-      }
+      T.tile_expert[t] = e, T.tile_first[t] = off[e] + j * TILE, T.tile_end[t] = off[e] + c;
     }
   }
   cluster_wait();
 }
 
 // One cluster, as many CTAs as the pairs keep busy: 512 pairs a CTA (two steps of 32 for half of its warps) up to eight CTAs.
-template <int TILE, int ROWS>
-inline int launch_plan(const int* ids, int P, int E, int Umax, int max_tiles, PlanTables T, cudaStream_t st) {
+template <int TILE>
+inline int launch_plan(const int* ids, int P, int E, int Umax, PlanTables T, cudaStream_t st) {
   const int C = P <= 1024 ? 1 : P <= 2048 ? 2 : P <= 4096 ? 4 : 8;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C), cfg.blockDim = dim3(1024), cfg.stream = st;
@@ -166,7 +171,7 @@ inline int launch_plan(const int* ids, int P, int E, int Umax, int max_tiles, Pl
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = 2;
-  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plan<TILE, ROWS>, ids, P, E, Umax, max_tiles, T));
+  B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plan<TILE>, ids, P, E, Umax, T));
   return B200MOE_OK;
 }
 

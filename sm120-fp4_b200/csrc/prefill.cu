@@ -25,10 +25,10 @@ namespace b200 {
 
 // ------------------------------------------------------------------------------------------------ x -> records
 // Blocks [0, aside) do what else the records and the GEMM behind this kernel need: block i zeroes the scale bytes of the rows of
-// tile i that hold no pair (a zero scale silences whatever codes a row holds, so their codes are never written) and asks
-// the first weight records of GEMM CTA i into L2, which is idle meanwhile.
+// tile i that hold no pair (a zero scale silences whatever codes a row holds, so their codes are never written), marks these rows
+// in row_pair and asks the first weight records of GEMM CTA i into L2, which is idle meanwhile.
 template <int ARows, int Rec>
-__device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, int tid, int nthreads) {
+__device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, int* row_pair, int tid, int nthreads) {
   const int NT = __ldcg(A.ntiles), i = blockIdx.x;
   if (i < NT) {
     constexpr int kPer = ARows == 64 ? kTerms : 1;
@@ -37,6 +37,7 @@ __device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, in
       const int r = used + j % spare, q = j / spare;   // scale word q & 3 of K box q >> 2
       *reinterpret_cast<uint32_t*>(rec + ((long long)i * A.KB + (q >> 2)) * Rec + (Rec - 2048) + (q & 3) * 512 + (r & 31) * 16 + (r >> 5) * 4) = 0u;
     }
+    for (int r = used + tid; r < ARows; r += nthreads) row_pair[(long long)i * ARows + r] = -1;
   }
   if (i < A.gemm_ctas && tid < kGgWarm) {
     const GgSplit s(NT, A.NBLK, A.gemm_ctas, i);
@@ -52,11 +53,11 @@ __device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, in
 // running, and its codes and scale bytes are then stored into the record rows of each of its top_k pairs (dst_row, -1 = empty
 // slot). rec [ntiles][KB][18432]; blocks beyond H inside the last K box are written as zero codes and zero scales.
 __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* __restrict__ x, const int* dst_row, int H, int KB, int top_k, float gs,
-                                                          uint8_t* rec, GgAside A) {
+                                                          uint8_t* rec, GgAside A, PairTables T) {
   if ((int)blockIdx.x < A.blocks) {
     grid_dependency_wait();
     grid_launch_dependents();
-    records_aside<128, kRec>(A, rec, threadIdx.x, 128);
+    records_aside<128, kRec>(A, rec, T.row_pair, threadIdx.x, 128);
     return;
   }
   __shared__ float s_scale[128];   // gs / (E4M3 value) for every scale byte: one division per table entry instead of one per block
@@ -66,6 +67,8 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
   __syncthreads();
   const int nblk = KB * 16;
   bool waited = false;
+  const int slot = threadIdx.x - 96;   // warp 3: this token's entries of the pair tables
+  int my_row = -1, my_first = 0;
 #pragma unroll 1
   for (int b = threadIdx.x; b < ((nblk + 127) & ~127); b += 128) {   // whole warps stay in the loop: the shuffles below need them
     uint2 pk = make_uint2(0u, 0u);
@@ -83,7 +86,11 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
       waited = true;
       grid_dependency_wait();
       grid_launch_dependents();
-      if (threadIdx.x < top_k) s_row[threadIdx.x] = __ldcg(dst_row + tok * top_k + threadIdx.x);
+      if (slot >= 0 && slot < top_k) {
+        my_row = __ldcg(dst_row + tok * top_k + slot);
+        s_row[slot] = my_row;
+        if (my_row >= 0) my_first = __ldcg(T.tile_first + (my_row >> 7));
+      }
       __syncthreads();
     }
     if (b >= nblk) continue;
@@ -97,6 +104,7 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
       if ((b & 3) == 0) *reinterpret_cast<uint32_t*>(dst + rec_scale_offset(r, b16)) = sf4;
     }
   }
+  if (my_row >= 0) put_pair<128, 1>(T, tok * top_k + slot, my_row, my_first);
 }
 
 // ------------------------------------------------------------------------------------------------ x -> W4A16 records
@@ -109,12 +117,12 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
 // write the rows' 1 / g_t.
 // The row's amax is taken while the plan kernel is still running. Blocks [0, aside): see records_aside.
 __global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __restrict__ x, const int* dst_row, int H, int KB, int top_k, uint8_t* rec,
-                                                        float* rowscale, GgAside A) {
+                                                        float* rowscale, GgAside A, PairTables T) {
   const int tid = threadIdx.x;
   if ((int)blockIdx.x < A.blocks) {
     grid_dependency_wait();
     grid_launch_dependents();
-    records_aside<64, kMidRec>(A, rec, tid, 128);
+    records_aside<64, kMidRec>(A, rec, T.row_pair, tid, 128);
     return;
   }
   __shared__ float wm[4];
@@ -132,7 +140,13 @@ __global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __r
   if ((tid & 31) == 0) wm[tid >> 5] = m;
   grid_dependency_wait();
   grid_launch_dependents();
-  if (tid < top_k) s_row[tid] = __ldcg(dst_row + tok * top_k + tid);
+  const int slot = tid - 96;   // warp 3: this token's entries of the pair tables
+  int my_row = -1, my_first = 0;
+  if (slot >= 0 && slot < top_k) {
+    my_row = __ldcg(dst_row + tok * top_k + slot);
+    s_row[slot] = my_row;
+    if (my_row >= 0) my_first = __ldcg(T.tile_first + (my_row >> 4));
+  }
   __syncthreads();
   m = fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
   const float g1 = 2688.0f / fmaxf(m, 1e-30f);
@@ -164,6 +178,7 @@ __global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __r
       for (int q = 0; q < kTerms; ++q) put(q, make_uint2(0u, 0u), 0);
     }
   }
+  if (my_row >= 0) put_pair<16, kTerms>(T, tok * top_k + slot, my_row, my_first);
 }
 
 // ------------------------------------------------------------------------------------------------ combine
@@ -312,14 +327,15 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   int* status = (int*)(w + L.status);
   if (Umax > 256) return B200MOE_ERR_LIMIT;
   const int max_tiles = P / 128 + Umax;   // tiles this batch can need (<= the workspace's capacity)
-  const PlanTables tab = {experts, offsets, pairs, ntiles, tile_expert, tile_first, tile_end, row_pair, dst_row};
-  int rc = launch_plan<128, 1>(ids, P, E, Umax, max_tiles, tab, st);
+  const PlanTables tab = {experts, offsets, ntiles, tile_expert, tile_first, tile_end, dst_row};
+  const PairTables ptab = {tile_first, pairs, row_pair};
+  int rc = launch_plan<128>(ids, P, E, Umax, tab, st);
   if (rc != B200MOE_OK) return rc;
   {
     const GgAside aside = {ntiles, tile_expert, tile_first, tile_end, w1t, I / 64, KB1, sms, max_tiles > sms ? max_tiles : sms};
     const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
     uint8_t* rec = w + L.xrec;
-    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&gs_x, (void*)&rec, (void*)&aside};
+    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&gs_x, (void*)&rec, (void*)&aside, (void*)&ptab};
     rc = launch_kernel((const void*)k_quantize_scatter, aside.blocks + M, 128, 0, true, args, st);
     if (rc != B200MOE_OK) return rc;
   }
@@ -406,14 +422,15 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   int* dst_row = (int*)(w + L.dst_row);
   const int max_tiles = P / 16 + Umax;
   int* tile_end = tile_first + max_tiles;
-  const PlanTables tab = {experts, offsets, pairs, ntiles, tile_expert, tile_first, tile_end, row_pair, dst_row};
-  int rc = launch_plan<16, kTerms>(ids, P, E, Umax, max_tiles, tab, st);
+  const PlanTables tab = {experts, offsets, ntiles, tile_expert, tile_first, tile_end, dst_row};
+  const PairTables ptab = {tile_first, pairs, row_pair};
+  int rc = launch_plan<16>(ids, P, E, Umax, tab, st);
   if (rc != B200MOE_OK) return rc;
   {
     const GgAside aside = {ntiles, tile_expert, tile_first, tile_end, w1t, I / 64, KB1, sms, max_tiles > sms ? max_tiles : sms};
     const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
     uint8_t* rec = w + L.xrec;
-    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&rec, (void*)&rowscale, (void*)&aside};
+    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&rec, (void*)&rowscale, (void*)&aside, (void*)&ptab};
     rc = launch_kernel((const void*)k_expand_scatter, aside.blocks + M, 128, 0, true, args, st);
     if (rc != B200MOE_OK) return rc;
   }

@@ -1,0 +1,53 @@
+"""Sizes at which the plan kernel and the grouped GEMM of a W4A4 layer call change their split: one, two, four and eight CTAs in the
+plan's cluster (1024, 2048 and 4096 pairs are the last sizes of one, two and four), runs of pairs too long for a warp's registers
+(more than 65536 pairs), operand boxes streamed through the ring because a tile's records do not fit (13 boxes of 128 rows).
+
+A token's result does not depend on the batch around it: its rows are quantised on their own, accumulated in the same K order in
+whatever tile they sit, and summed in slot order. So a call must equal the same tokens in calls of at most 64 bit for bit, and calls of
+that size are checked against the oracle stage by stage (test_gpu_prefill; the streamed operand here)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import _i32, check_prefill_call, make_layer, prefill_map
+from test_gpu_decode import inputs
+from test_gpu_prefill import run_prefill, sample
+
+pytestmark = pytest.mark.gpu
+
+MOST = 4097
+
+
+def in_parts(w, x, ids, wts, most):
+    n = -(-x.shape[0] // 64)
+    return torch.cat([run_prefill(w, a, b, c, most).clone() for a, b, c in zip(*(torch.tensor_split(t, n) for t in (x, ids, wts)))])
+
+
+@pytest.mark.parametrize("top_k,m", [(8, 128), (8, 129), (8, 256), (8, 257), (8, 512), (8, 513), (16, 4096), (16, MOST)])
+def test_plan_sizes(top_k, m):
+    cfg = dict(experts=24, hidden=256, inter=64, top_k=top_k)
+    w, _ = make_layer(**cfg, seed=8)
+    x, ids, wts = inputs(cfg, m, 50 + m)
+    ids, wts = ids.clone(), wts.clone()
+    ids[m // 2, 1], wts[m // 2, 1] = -1, 0          # an empty slot
+    parts = in_parts(w, x, ids, wts, MOST)
+    out = run_prefill(w, x, ids, wts, MOST)
+    assert torch.equal(out, parts)
+    flat = ids.reshape(-1).numpy()
+    order = np.argsort(np.where(flat < 0, 1 << 20, flat), kind="stable")[: (flat >= 0).sum()]
+    mp, ws = prefill_map(w, MOST), w.prefill.workspace
+    assert np.array_equal(_i32(ws, mp["pairs"], flat.size)[: order.size], order)
+    rows = _i32(ws, mp["dst_row"], flat.size)
+    row_pair = _i32(ws, mp["row_pair"], 128 * int(_i32(ws, mp["ntiles"], 1)[0]))
+    assert np.array_equal(row_pair[rows[order]], order) and (row_pair >= 0).sum() == order.size and rows[flat < 0].max() == -1
+
+
+@pytest.mark.parametrize("m", [40, 150])
+def test_streamed_operand_boxes(m):
+    cfg = dict(experts=4, hidden=3328, inter=192, top_k=2)
+    w, ow = make_layer(**cfg, seed=5)
+    x, ids, wts = inputs(cfg, m, 6)
+    ids = ids.clone()
+    ids[:, 1] = 1 + ids[:, 1] % 3
+    ids[:, 0] = 0                                   # one expert of many rows; the others' records fit
+    check_prefill_call(w, ow, x, ids, wts, run_prefill(w, x, ids, wts), 512, sample_tokens=sample(ids, 8, 1), what=f"13 K boxes, {m} tokens")
