@@ -119,11 +119,11 @@ int b200moe_prefill_status(const b200moe_layer* layer, const void* workspace, in
  * (r&31)*16 + (r>>5)*4 + (b&3) - i.e. four 128x4 scale tiles. */
 int b200moe_prefill_workspace_map(const b200moe_layer* layer, int max_tokens, long long* out14);
 
-/* forward: x bf16 [M, H], topk_ids i32 [M, top_k], topk_weights f32 [M, top_k] -> out bf16 [M, H]; one launch
- * (routing + FC1 + SiLU*mul + FC2 + weighted combine). Replaces Weights._slice, sm120fp4/vllm_backend.py:174-190. */
+/* forward: x bf16 [M, H], topk_ids i32 [M, top_k], topk_weights f32 [M, top_k] -> out bf16 [M, H]; one layer kernel
+ * (routing + FC1 + SiLU*mul + FC2 + weighted combine), behind a small one that expands x above 8 tokens or 4096 values of x. Replaces Weights._slice, sm120fp4/vllm_backend.py:174-190. */
 int b200moe_decode_forward(const b200moe_layer* layer, const void* x_bf16, const int* topk_ids, const float* topk_weights,
                            int M, void* out_bf16, void* workspace, long long workspace_bytes, void* stream);
-/* The same with flags. B200MOE_ORDERED: the two kernels of the call are ordinary stream-ordered launches. By default they are
+/* The same with flags. B200MOE_ORDERED: the kernels of the call are ordinary stream-ordered launches. By default they are
  * launched programmatically, so that the call's prologue and weight stream overlap the tail of whatever precedes it in
  * the stream, and topk_ids / topk_weights are read at kernel entry: they must be complete when the kernel BEFORE this call
  * starts (true for any producer that does not itself release its successors early, or that releases them only after these

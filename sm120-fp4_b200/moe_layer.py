@@ -4,10 +4,10 @@ The reference picks, per batch size and shape, between CUDA-core and mma.sync ke
 its three launches are chained programmatically. Here the same three functions state the rule THIS library runs - they are
 what `Weights.forward` consults, not a description beside it:
 
-  tokens 1..16     one fused launch (routing + FC1 + SiLU*mul + FC2 + combine). The tcgen05 kernel ("tcgen05_fused": FP4
+  tokens 1..16     one fused layer kernel (routing + FC1 + SiLU*mul + FC2 + combine). The tcgen05 kernel ("tcgen05_fused": FP4
                    weights straight into kind::mxf4nvf4 MMAs) whenever the hidden size is at most 3072 (its x scale tiles
                    stay resident in TMEM: 12 K boxes of 256) and there is a worker per 128-row output block; otherwise the
-                   mma.sync kernel ("mma_sync_fused"). Both BASELINE shapes (2048 x 768 and 2816 x 704) take the tcgen05 kernel
+                   mma.sync kernel ("mma_sync_fused"). The shapes 2048 x 768 and 2816 x 704 take the tcgen05 kernel
                    at every batch size: on B200 there is no CUDA-core / tensor-core crossover inside the decode regime.
   tokens 17 and up "prefill_w4a4" when activation scales were given (`Weights.enable_prefill`): the reference's rule for
                    every batch above 16 tokens (sm120fp4/vllm_backend.py:161-168). Otherwise "mid_w4a16" (one W4A16 grouped
