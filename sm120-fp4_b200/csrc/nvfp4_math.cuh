@@ -11,13 +11,6 @@
 
 namespace b200 {
 
-__device__ __forceinline__ uint32_t e2m1_code(float v) {
-  // round to nearest, ties to the even code, saturate at 6, sign bit kept on zero (sm120fp4/reference.py:28-44)
-  const float m = fabsf(v);
-  uint32_t c = (m > 0.25f) + (m >= 0.75f) + (m > 1.25f) + (m >= 1.75f) + (m > 2.5f) + (m >= 3.5f) + (m > 5.0f);
-  return c | ((__float_as_uint(v) >> 31) << 3);
-}
-
 __device__ __forceinline__ void load16(const __nv_bfloat16* p, float (&v)[16]) {
   const uint4 a = reinterpret_cast<const uint4*>(p)[0], b = reinterpret_cast<const uint4*>(p)[1];
   const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
