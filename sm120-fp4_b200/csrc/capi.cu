@@ -210,7 +210,7 @@ extern "C" int b200moe_layer_set_act_scale(b200moe_layer* L, float g1) {
 }
 
 // Ring slots of the tcgen05 decode kernel beside the x operand (FC1) or the activation slabs (FC2) that share `region` bytes; 0 when
-// fewer than three fit (hidden sizes near 4096 at more than eight tokens).
+// fewer than three fit (none of the hidden sizes up to 3072).
 static int decode_tc_ring(const b200moe_layer* L, int N, int* region) {
   const int xb = L->KB1 * N * 128 + L->KT1 * 512, slab = N * 128 + 2048;
   for (int NS = 12; NS >= 3; --NS) {
@@ -222,12 +222,11 @@ static int decode_tc_ring(const b200moe_layer* L, int N, int* region) {
 
 static int decode_tc_columns(int M) { return M <= 4 ? 16 : M <= 8 ? 32 : 64; }   // of the B operand: four terms per token
 
-// the tcgen05 kernel runs whenever the tile records exist and the shape fits it: x scale tiles of <= 16 K boxes in TMEM, one
-// worker group per 128-row output block, and a ring of at least three records beside the x operand
-static bool decode_tc_fits(const b200moe_layer* L, int M) {
-  int region;
-  return L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 16 && L->NB2 <= L->sms && decode_tc_ring(L, decode_tc_columns(M), &region) > 0;
-}
+// The tcgen05 kernel runs whenever the tile records exist, the hidden size is at most 3072 (12 K boxes) and there is a worker for every
+// 128-row output block. Wider layers decode on the mma.sync kernel at every batch size: its f16 activations hold magnitudes up to 65504
+// and keep 11 bits, where four FP4 terms under the fixed activation scale clip a block beyond 336 and keep about 10. (Two layer calls
+// of 8 tokens at 4096 x 1536 would take 187 us instead of 261.)
+static bool decode_tc_fits(const b200moe_layer* L) { return L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 12 && L->NB2 <= L->sms; }
 
 static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, const HostRouting* host, void* stream) {
   uint8_t* w = (uint8_t*)ws;
@@ -324,7 +323,7 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
 // flags bit 0 (B200MOE_ORDERED): both kernels of the call are ordinary stream-ordered launches.
 extern "C" int b200moe_decode_forward_ex(const b200moe_layer* L, const void* x_bf16, const int* topk_ids, const float* topk_weights,
                                          int M, void* out_bf16, void* workspace, long long workspace_bytes, int flags, void* stream) {
-  if (L && decode_tc_fits(L, M)) {
+  if (L && decode_tc_fits(L)) {
     if (!x_bf16 || !topk_ids || !topk_weights || !out_bf16 || !workspace || M < 0) return B200MOE_ERR_ARG;
     if (M > 16) return B200MOE_ERR_LIMIT;
     if (workspace_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;
@@ -377,7 +376,7 @@ extern "C" int b200moe_decode_forward_host(const b200moe_layer* L, const void* x
   if (vw && !(((uintptr_t)vx | (uintptr_t)vo) & 15)) {
     if ((uintptr_t)workspace & 255) return B200MOE_ERR_ARG;
     const HostRouting h = {(const int*)vi, (const float*)vw, M * L->top_k, dids, dwts};
-    if (decode_tc_fits(L, M)) return decode_tc(const_cast<b200moe_layer*>(L), vx, dids, dwts, M, vo, workspace, true, &h, stream);
+    if (decode_tc_fits(L)) return decode_tc(const_cast<b200moe_layer*>(L), vx, dids, dwts, M, vo, workspace, true, &h, stream);
     const int rc = b200_host_stage_launch(vx, M * L->H / 8, h, dx, false, st);
     if (rc != B200MOE_OK) return rc;
     return b200moe_decode_forward(L, dx, dids, dwts, M, vo, workspace, workspace_bytes, stream);

@@ -25,8 +25,7 @@ MID_MIN_TOKENS = 33
 
 
 def decode_kernel(hidden: int = 2048, inter: int = 768, sm_count: int = 148, prepacked: bool = True) -> str:
-    """The kernel that serves every decode batch of this shape. (Between 3072 and 4096 the call itself takes the tcgen05 kernel for
-    the batches whose x operand leaves room for a ring of weight records beside it: up to 8 tokens at 4096.)"""
+    """The kernel that serves every decode batch of this shape."""
     if hidden % 128 or inter % 64:
         raise ValueError(f"the kernels take a hidden size that is a multiple of 128 and an intermediate size that is a multiple of 64, not {hidden}/{inter}")
     if prepacked and hidden <= TCGEN05_MAX_HIDDEN and hidden // 128 <= sm_count <= 256:

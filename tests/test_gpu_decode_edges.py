@@ -1,6 +1,5 @@
-"""Sizes at which the decode call changes its way: hidden sizes above 3072 (the tcgen05 kernel takes them up to 4096; with more than
-eight tokens some of them fall to the mma.sync kernel), x expanded by every worker itself up to 256 blocks of 16 values and eight
-tokens, and the same boundaries for tensors in page-locked host memory."""
+"""Sizes at which the decode call changes its way: hidden sizes above 3072 (mma.sync kernel), x expanded by every worker itself up to
+256 blocks of 16 values and eight tokens, and the same boundaries for tensors in page-locked host memory."""
 import pytest
 import torch
 
@@ -38,3 +37,15 @@ def test_hidden_sizes_and_batches(hidden, m):
         torch.cuda.synchronize()
         assert torch.equal(host, out.cpu())
     w.status()
+
+
+# Activations far beyond what the tcgen05 kernel's fixed activation scale holds (336 by default): the layers above 3072 compute with
+# f16 activations, whatever the batch size.
+@pytest.mark.parametrize("hidden,m", [(3200, 2), (4096, 1), (4096, 8), (4096, 9)])
+def test_wide_layers_hold_large_activations(hidden, m):
+    cfg, w, ow = edge_layer(hidden)
+    x, ids, wts = inputs(cfg, m, 70 + m)
+    x = (x.float() * 20).to(torch.bfloat16)
+    out = run(w, x, ids, wts)
+    w.status()
+    check_layer_output(out, O.moe_reference(x.float().numpy(), ow, ids.numpy(), wts.numpy()), f"hidden {hidden}, {m} tokens, x * 20")
