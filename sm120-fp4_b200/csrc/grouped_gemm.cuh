@@ -124,12 +124,17 @@ struct GgAside {
   int NBLK, KB, gemm_ctas, blocks;
 };
 
+// W4A4 FC1 divides with IEEE rounding where the operand has more than nine K boxes (hidden sizes above 2304): the results of these
+// layers were defined that way, and an approximate quotient moves an activation on the edge of two FP4 codes to the other one (1.4e-4
+// of a layer's output at 4096 x 1536). Up to nine boxes it has always been the approximate one.
+inline bool gg_ieee_silu(int KB1) { return KB1 > 9; }
+
 // ---- epilogues: one warp, 32 accumulator rows x 128 columns at taddr (thread = row). `release` frees the accumulator buffer
 // once its values are in registers.
 
 // W4A4 FC1: columns 0..63 = up, 64..127 = gate of intermediate columns 64n..; SiLU*mul, re-quantise four blocks of 16 and store
 // the row's 32 code bytes (two 16-byte chunks of one sector) and four scale bytes into FC2's record `dst`.
-template <class F>
+template <bool Ieee, class F>
 __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float gs_out, const float* scale_table, uint8_t* dst, int row, bool store,
                                                 int n, F&& release) {
   uint32_t sfw = 0;
@@ -150,7 +155,8 @@ __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float g
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;
-        a[i] = __fdividef(g, 1.0f + __expf(-g)) * u;
+        const float d = 1.0f + __expf(-g);
+        a[i] = (Ieee ? __fdiv_rn(g, d) : __fdividef(g, d)) * u;
       }
       sfw |= (uint32_t)quantize_block16_t(a, gs_out, scale_table, pk[b]) << (16 * h + 8 * b);
     }
@@ -265,7 +271,8 @@ __device__ __forceinline__ void gg_epilogue_fc2_a16(uint32_t taddr, float s, flo
   }
 }
 
-template <int PHASE>
+// Ieee (PHASE 1): SiLU divides with IEEE rounding instead of __fdividef; see gg_ieee_silu.
+template <int PHASE, bool Ieee = false>
 __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_constant__ GroupedParams P) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -487,7 +494,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
         if (!work && !dry) {
           release();
         } else if (PHASE == 1) {
-          gg_epilogue_fc1(taddr, s, P.gs_out, S.scale, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kRec, row, row < rows && !dry, n, release);
+          gg_epilogue_fc1<Ieee>(taddr, s, P.gs_out, S.scale, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kRec, row, row < rows && !dry, n, release);
         } else if (PHASE == 2) {
           gg_epilogue_fc2(taddr, s, dry ? 0u : valid, patches + warp * kGgPatch, P.y + ((long long)t * 128 + quad * 32) * P.H + 128 * n, P.H, lane, release);
         } else if (PHASE == 3) {

@@ -291,14 +291,16 @@ void b200_prefill_workspace_map(int E, int H, int I, int top_k, int max_tokens, 
 // One launch of the grouped GEMM (grouped_gemm.cuh): one persistent CTA per SM, programmatically behind the kernel before it so
 // that its set-up and the first weight records overlap that kernel's tail.
 static int launch_gemm(GroupedParams p, int phase, int sms, cudaStream_t st) {
-  const void* fn = phase == 1 ? (const void*)k_grouped_gemm<1> : phase == 2 ? (const void*)k_grouped_gemm<2>
-                 : phase == 3 ? (const void*)k_grouped_gemm<3> : (const void*)k_grouped_gemm<4>;
-  static thread_local unsigned configured[4] = {0, 0, 0, 0};   // bit d: device d has the attribute
+  static const void* const kernels[5] = {(const void*)k_grouped_gemm<1>, (const void*)k_grouped_gemm<2>, (const void*)k_grouped_gemm<3>,
+                                         (const void*)k_grouped_gemm<4>, (const void*)k_grouped_gemm<1, true>};
+  const int which = phase == 1 && gg_ieee_silu(p.KB) ? 4 : phase - 1;
+  const void* fn = kernels[which];
+  static thread_local unsigned configured[5] = {0, 0, 0, 0, 0};   // bit d: device d has the attribute
   int dev = 0;
   B200_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev > 31 || !((configured[phase - 1] >> dev) & 1u)) {
+  if (dev > 31 || !((configured[which] >> dev) & 1u)) {
     B200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGgSmem));
-    if (dev <= 31) configured[phase - 1] |= 1u << dev;
+    if (dev <= 31) configured[which] |= 1u << dev;
   }
   void* args[] = {(void*)&p};
   return launch_kernel(fn, sms, kGgThreads, kGgSmem, true, args, st);

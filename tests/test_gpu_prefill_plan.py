@@ -51,3 +51,26 @@ def test_streamed_operand_boxes(m):
     ids[:, 1] = 1 + ids[:, 1] % 3
     ids[:, 0] = 0                                   # one expert of many rows; the others' records fit
     check_prefill_call(w, ow, x, ids, wts, run_prefill(w, x, ids, wts), 512, sample_tokens=sample(ids, 8, 1), what=f"13 K boxes, {m} tokens")
+
+
+@pytest.mark.parametrize("hidden", [2560, 4096])
+def test_silu_division_of_wide_layers(hidden):
+    """Above nine K boxes FC1's SiLU divides with IEEE rounding. A gate of -88 shows it: 1 + exp(88) lies between 2^126 and 2^128, where
+    the approximate division returns zero. The up value and the activation scale (1e28) bring the quotient (-5e-37) back into range.
+    Every value of a block is the same, so its code is exact and the error is that of the E4M3 scale (2^-4) and of the output's bf16."""
+    from sm120fp4_b200.vllm_backend import Weights
+    inter, m = 64, 20
+    q1 = torch.zeros(1, 2 * inter, hidden // 2, dtype=torch.uint8, device="cuda")
+    s1 = torch.full((1, 2 * inter, hidden // 16), 0x38, dtype=torch.uint8, device="cuda")        # 1.0
+    q1[:, :inter], s1[:, :inter] = 0x77, 0x7e                                                    # up: 6 x 448 everywhere
+    q1[:, inter:, 0] = 0x0a                                                                      # gate: -1 at the first value
+    q2 = torch.full((1, hidden, inter // 2), 0x22, dtype=torch.uint8, device="cuda")             # 1.0
+    s2 = torch.full((1, hidden, inter // 16), 0x38, dtype=torch.uint8, device="cuda")
+    xq = 6 * 0.171875                                                                            # what x = 1 becomes in NVFP4 (scale E4M3(1/6))
+    a1, a2 = 88.0 / xq, 1e28
+    w = Weights(q1, s1, torch.tensor([a1], device="cuda"), q2, s2, torch.tensor([a2], device="cuda"), 1)
+    w.enable_prefill(a2_scale=1e-28, max_tokens=m)
+    out = w.forward(torch.ones(m, hidden, dtype=torch.bfloat16, device="cuda"), torch.zeros(m, 1, dtype=torch.int32, device="cuda"),
+                    torch.ones(m, 1, device="cuda")).double()
+    want = -88.0 / (1.0 + np.exp(88.0)) * (hidden * 6 * 448 * xq * a1) * inter * a2
+    assert (out / want - 1).abs().max() < 2.0 ** -4 + 2.0 ** -7, (out.flatten()[:4], want)
