@@ -69,6 +69,12 @@ struct TcTables {
 
 __device__ __forceinline__ float tc_silu_mul(float gate, float up) { return __fdividef(gate, 1.0f + __expf(-gate)) * up; }
 
+// The larger of two non-negative bf16 values in one word, as the bits of a float (which order like the values). A NaN, which is what the
+// packed maximum leaves where all values were NaN, counts as zero: it would pass for the largest value of the row.
+__device__ __forceinline__ unsigned pair_max_bits(uint32_t w) {
+  return __float_as_uint(fmaxf(fmaxf(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), 0.f));
+}
+
 // ------------------------------------------------------------------------------------------------ x -> B operand
 // One block of 256 threads per token slot (N/4 slots), a thread per 16-value block: token amax, then the block expanded into four
 // NVFP4 terms. The block is small enough (registers, shared memory) to be resident next to a block of the layer kernel.
@@ -117,7 +123,7 @@ __global__ void __launch_bounds__(256, 4) k_expand_x(const __nv_bfloat16* x, int
 #pragma unroll
     for (int i = 1; i < 8; ++i) m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
     const uint32_t bits = *reinterpret_cast<const uint32_t*>(&m2);
-    const unsigned wmax = __reduce_max_sync(0xffffffffu, max(bits << 16, bits & 0xffff0000u));   // non-negative floats order like their bits
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, pair_max_bits(bits));
     if ((tid & 31) == 0) wm[tid >> 5] = wmax;
     __syncthreads();
     unsigned mb = 0;
@@ -221,7 +227,7 @@ __device__ __forceinline__ void expand_x_here(const DecodeTcParams& P, uint8_t* 
 #pragma unroll
       for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
       const uint32_t bits = *reinterpret_cast<const uint32_t*>(&m);
-      const unsigned mine = max(bits << 16, bits & 0xffff0000u);   // non-negative floats order like their bits
+      const unsigned mine = pair_max_bits(bits);
       const int first = __shfl_sync(0xffffffffu, tok, 0), last = __shfl_sync(0xffffffffu, tok, 31);
       for (int t = first; t <= last && t < P.M; ++t) {             // the tokens this warp's 32 blocks belong to
         const unsigned wm = __reduce_max_sync(0xffffffffu, tok == t ? mine : 0u);

@@ -1,9 +1,10 @@
 """Sizes at which the decode call changes its way: hidden sizes above 3072 (mma.sync kernel), x expanded by every worker itself up to
 256 blocks of 16 values and eight tokens, and the same boundaries for tensors in page-locked host memory."""
+import numpy as np
 import pytest
 import torch
 
-from helpers import check_layer_output, make_layer
+from helpers import check_layer_output, decode_map, make_layer
 from oracle import nvfp4_oracle as O
 from test_gpu_decode import inputs, run
 
@@ -49,3 +50,19 @@ def test_wide_layers_hold_large_activations(hidden, m):
     out = run(w, x, ids, wts)
     w.status()
     check_layer_output(out, O.moe_reference(x.float().numpy(), ow, ids.numpy(), wts.numpy()), f"hidden {hidden}, {m} tokens, x * 20")
+
+
+# A row's scale comes from its finite values: NaNs are passed over, also where they fill a block of 16 or every second value of one
+# (two values are compared at a time). Expanded by the workers (1 and 2 tokens of 2048) and by the kernel ahead of them (9).
+@pytest.mark.parametrize("which", [slice(32, 48), slice(32, 48, 2), slice(33, 48, 2)])
+@pytest.mark.parametrize("m", [1, 2, 9])
+def test_nan_values_do_not_set_the_row_scale(m, which):
+    cfg, w, _ = edge_layer(2048)
+    x, ids, wts = inputs(cfg, m, 90 + m)
+    x = x.clone()
+    x[0, which] = float("nan")
+    run(w, x, ids, wts)
+    amax = x[0].float()[~x[0].isnan()].abs().max().numpy()
+    at = decode_map(w)["xscale"]
+    got = w.workspace[at:at + 4].view(torch.float32).cpu().numpy()[0]
+    assert got == np.float32(1) / (np.float32(2688) / amax)
