@@ -55,22 +55,23 @@ template <typename T> __device__ __forceinline__ void load_raw(const T* p, bool 
     for (int i = 0; i < (int)sizeof(T); ++i) v.r[i] = reinterpret_cast<const uint4*>(p)[i];
   }
 }
-// largest magnitude of the 16 values (NaNs are passed over, as fmaxf does)
+// largest magnitude of the 16 values; NaNs are passed over, as fmaxf does, unless there is nothing else (a block of NaNs then gets the
+// largest block scale, as quantize_block16 gives it)
 __device__ __forceinline__ float amax_raw(const Raw16<__nv_bfloat16>& v) {
   const uint32_t w[8] = {v.r[0].x, v.r[0].y, v.r[0].z, v.r[0].w, v.r[1].x, v.r[1].y, v.r[1].z, v.r[1].w};
   __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
 #pragma unroll
   for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
   const uint32_t b = *reinterpret_cast<const uint32_t*>(&m);
-  return fmaxf(fmaxf(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)), 0.f);
+  return fmaxf(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
 }
 __device__ __forceinline__ float amax_raw(const Raw16<float>& v) {
-  float m = 0.f;
+  float m[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    m = fmaxf(fmaxf(fmaxf(m, fabsf(__uint_as_float(v.r[i].x))), fmaxf(fabsf(__uint_as_float(v.r[i].y)), fabsf(__uint_as_float(v.r[i].z)))),
-              fabsf(__uint_as_float(v.r[i].w)));
-  return m;
+    m[i] = fmaxf(fmaxf(fabsf(__uint_as_float(v.r[i].x)), fabsf(__uint_as_float(v.r[i].y))),
+                 fmaxf(fabsf(__uint_as_float(v.r[i].z)), fabsf(__uint_as_float(v.r[i].w))));
+  return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
 }
 __device__ __forceinline__ void floats(const Raw16<__nv_bfloat16>& v, float (&f)[16]) {
   const uint32_t w[8] = {v.r[0].x, v.r[0].y, v.r[0].z, v.r[0].w, v.r[1].x, v.r[1].y, v.r[1].z, v.r[1].w};

@@ -54,3 +54,21 @@ def test_every_bf16_amax():
             q, sf, gs = pkg.quantize_nvfp4(rows.contiguous().cuda())
             assert np.array_equal(gs.cpu().numpy().view(np.uint32), wgs.view(np.uint32))
             assert np.array_equal(sf.cpu().numpy(), wsf) and np.array_equal(q.cpu().numpy(), wq), top
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [8, 300])
+def test_nan_and_infinite_values(rows, dtype):
+    """A block of NaNs, single NaNs and infinities: the same bytes as amax, scale and codes in separate launches."""
+    import sm120fp4_b200 as pkg
+    base = torch.randn(rows, 1040, generator=torch.Generator().manual_seed(rows)).to(dtype)
+    for where, value in (((3, slice(32, 48)), "nan"), ((5, 7), "nan"), ((6, slice(16, 32, 2)), "nan"), ((0, 9), "inf"), ((0, 9), "-inf")):
+        x = base.clone()
+        x[where] = float(value)
+        x = x.cuda()
+        q, sf, gs = pkg.quantize_nvfp4(x)
+        assert torch.equal(gs, pkg.quant.global_scale_for(x))
+        wq, wsf, _ = pkg.quantize_nvfp4(x, gs)
+        assert torch.equal(q, wq) and torch.equal(sf, wsf)
+        qe, se, ge = pkg.quantize_nvfp4_experts(torch.stack([x, x]))
+        assert torch.equal(ge, gs.expand(2)) and torch.equal(qe, wq.expand(2, -1, -1)) and torch.equal(se, wsf.expand(2, -1, -1))
