@@ -50,7 +50,8 @@ int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int row
 /* The same with each group's own global scale, both passes in one launch: x [groups, rows, K] -> gs_out f32 [groups] (2688 / amax,
  * as b200moe_global_scale), packed u8 [groups, rows, K/2], sf u8 row-major [groups, rows, K/16] (sf_layout 0) or 128x4-swizzled
  * per group (sf_layout 1: [groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: 8-byte aligned, zeroed once, then only
- * ever passed to this function (any sizes); calls that may overlap on the GPU need one each. sm120fp4/reference.py:68-90. */
+ * ever passed to this function (any sizes); calls that may overlap on the GPU need one each, and a captured call is in flight whenever
+ * its graph is. Where the size is 0 (one matrix of up to 8192 blocks of 16) it may be null. sm120fp4/reference.py:68-90. */
 long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K);
 int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
                                      int sf_layout, void* workspace, long long workspace_bytes, void* stream);

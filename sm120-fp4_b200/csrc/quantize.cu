@@ -327,20 +327,25 @@ static int quant_units(int dtype, int rows, int K) {
   return (int)((nblk + unit - 1) / unit);
 }
 
+static bool quant_one_cluster(int groups, int rows, int K) { return groups == 1 && (long long)rows * (K / 16) <= kQSmallMaxBlocks; }
+
 extern "C" long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K) {
   if (groups <= 0 || rows < 0 || K <= 0 || (dtype != 0 && dtype != 1)) return B200MOE_ERR_ARG;
+  if (quant_one_cluster(groups, rows, K)) return 0;
   return 8 + 8LL * groups * quant_units(dtype, rows, K);
 }
 
 // x [groups, rows, K] (dtype 0 bf16, 1 f32) -> gs_out f32 [groups], packed u8 [groups, rows, K/2], sf u8: sf_layout 0 row-major
 // [groups, rows, K/16], 1 the 128x4 swizzle per group ([groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: zeroed once,
-// then only ever passed to this function; two calls that may overlap on the GPU need one each.
+// then only ever passed to this function; two calls that may overlap on the GPU (a replay of a captured call is one) need one each.
+// Null where b200moe_quantize_own_scale_workspace_bytes says 0.
 extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
                                                 void* workspace, long long workspace_bytes, void* stream) {
-  if (!x || !gs_out || !packed || !sf || !workspace || groups <= 0 || rows < 0) return B200MOE_ERR_ARG;
+  if (!x || !gs_out || !packed || !sf || groups <= 0 || rows < 0) return B200MOE_ERR_ARG;
   if (K <= 0 || K % 16) return B200MOE_ERR_SHAPE;
   if ((dtype != 0 && dtype != 1) || (sf_layout != 0 && sf_layout != 1)) return B200MOE_ERR_ARG;
   if (((uintptr_t)x & 15) || ((uintptr_t)packed & 7) || ((uintptr_t)workspace & 7)) return B200MOE_ERR_ARG;
+  if (!workspace && !quant_one_cluster(groups, rows, K)) return B200MOE_ERR_ARG;
   if (workspace_bytes < b200moe_quantize_own_scale_workspace_bytes(dtype, groups, rows, K)) return B200MOE_ERR_WORKSPACE;
   if (rows == 0) return B200MOE_OK;
   cudaStream_t st = (cudaStream_t)stream;
@@ -356,7 +361,7 @@ extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int gr
   if (q.sf_stride > 0x7fffffffLL) return B200MOE_ERR_LIMIT;
   if (nblk > (1LL << 30)) return B200MOE_ERR_LIMIT;
   unsigned* scratch = (unsigned*)workspace;
-  if (groups == 1 && nblk <= kQSmallMaxBlocks) {
+  if (quant_one_cluster(groups, rows, K)) {
     int C = 1;   // CTAs: one block per thread, then two
     while (C < 8 && C * kQThreads < nblk) C *= 2;
     cudaLaunchConfig_t cfg = {};

@@ -36,16 +36,20 @@ def _check_2d(x: torch.Tensor) -> None:
         raise RuntimeError("quantize_nvfp4 runs on the GPU; there is no CPU path in this package")
 
 
-_WS: dict = {}   # (device index, stream) -> zeroed workspace of the one-launch quantiser, grown on demand
+_ONE_CLUSTER = 8192 * BLOCK   # values of one matrix up to which the quantiser keeps them in registers and takes no workspace
+_WS: dict = {}                # (device index, stream) -> zeroed workspace of eager calls, grown on demand
 
 
 def _workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
-    """Zeroed once; calls on different streams do not share one."""
+    """Zeroed once and kept for the eager calls of one stream, which the stream runs one after the other. A captured call is replayed
+    on any stream at any later time, and its zeroing runs with the replay: it gets a workspace of its own, from the graph's memory."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.zeros(nbytes, dtype=torch.uint8, device=device)
     key = (device.index, stream)
     ws = _WS.get(key)
     if ws is None or ws.numel() < nbytes:
         if len(_WS) >= 64:     # streams come and go: the memory of those of long ago goes back to torch's allocator
-            _WS.pop(next(iter(_WS)))
+            _WS.pop(next(iter(_WS)), None)
         ws = _WS[key] = torch.zeros(max(nbytes, 4096), dtype=torch.uint8, device=device)
     return ws
 
@@ -60,11 +64,12 @@ def _own_scale(x: torch.Tensor, groups: int, rows: int, k: int, gs, packed, sf, 
     h = _lib.lib()
     st = _lib.stream_ptr()
     dt = 0 if x.dtype == torch.bfloat16 else 1
-    # one 8-byte word per unit of at least 1024 blocks of 16 values: these calls fit the smallest workspace there is
-    nbytes = 4096 if groups * rows * k <= 1 << 20 and groups <= 64 else h.b200moe_quantize_own_scale_workspace_bytes(dt, groups, rows, k)
-    ws = _workspace(x.device, st, nbytes)
+    ws, nbytes = None, 0
+    if groups > 1 or rows * k > _ONE_CLUSTER:
+        nbytes = h.b200moe_quantize_own_scale_workspace_bytes(dt, groups, rows, k)
+        ws = _workspace(x.device, st, nbytes)
     rc = h.b200moe_quantize_nvfp4_own_scale(x.data_ptr(), dt, groups, rows, k, gs.data_ptr(), packed.data_ptr(),
-                                            sf.data_ptr(), layout, ws.data_ptr(), ws.numel(), st)
+                                            sf.data_ptr(), layout, _lib.ptr(ws), nbytes, st)
     if rc:
         _lib.check(rc, what)
 

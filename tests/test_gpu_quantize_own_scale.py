@@ -72,3 +72,69 @@ def test_nan_and_infinite_values(rows, dtype):
         assert torch.equal(q, wq) and torch.equal(sf, wsf)
         qe, se, ge = pkg.quantize_nvfp4_experts(torch.stack([x, x]))
         assert torch.equal(ge, gs.expand(2)) and torch.equal(qe, wq.expand(2, -1, -1)) and torch.equal(se, wsf.expand(2, -1, -1))
+
+
+def _expect(x, got):
+    wq, wsf, wgs = O.quantize_nvfp4(x.float().cpu().numpy(), None)
+    q, sf, gs = got
+    assert np.array_equal(gs.cpu().numpy().view(np.uint32), wgs.view(np.uint32))
+    assert np.array_equal(q.cpu().numpy(), wq) and np.array_equal(sf.cpu().numpy(), wsf)
+
+
+def _captured(x, stream):
+    import sm120fp4_b200 as pkg
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        out = pkg.quantize_nvfp4(x)
+    return graph, out
+
+
+def _randn(rows, k, seed):
+    return torch.randn(rows, k, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
+
+
+def test_captured_call_keeps_its_workspace():
+    """A larger eager call on the stream of a captured one, and whatever it lets the allocator hand out, touch nothing that a replay uses."""
+    import sm120fp4_b200 as pkg
+    stream = torch.cuda.Stream()
+    x = _randn(1024, 2048, 1)
+    pkg.quantize_nvfp4(x)
+    torch.cuda.synchronize()
+    graph, out = _captured(x, stream)
+    with torch.cuda.stream(stream):
+        big = _randn(4096, 2048, 2)
+        _expect(big, pkg.quantize_nvfp4(big))
+        filled = [torch.full((4096,), 0x5a, dtype=torch.uint8, device="cuda") for _ in range(256)]
+    torch.cuda.synchronize()
+    for seed in (3, 4):
+        x.copy_(_randn(1024, 2048, seed) * seed)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        _expect(x, out)
+    assert all(bool((t == 0x5a).all()) for t in filled)
+
+
+def test_two_graphs_of_one_stream():
+    """Captured on one stream before any eager call on it; the second alone, then an eager call, then each on either stream."""
+    import sm120fp4_b200 as pkg
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    xs = [_randn(1024, 2048, 5), _randn(640, 4096, 6)]
+    torch.cuda.synchronize()
+    (g0, out0), (g1, out1) = (_captured(x, stream) for x in xs)
+    for seed in (7, 8):
+        xs[1].copy_(_randn(640, 4096, seed) * seed)
+        torch.cuda.synchronize()
+        g1.replay()
+        torch.cuda.synchronize()
+        _expect(xs[1], out1)
+    with torch.cuda.stream(stream):
+        e = _randn(300, 2048, 9)
+        _expect(e, pkg.quantize_nvfp4(e))
+    torch.cuda.synchronize()
+    for g, s in ((g0, stream), (g1, other), (g0, other)):
+        with torch.cuda.stream(s):
+            g.replay()
+        torch.cuda.synchronize()
+    _expect(xs[0], out0)
+    _expect(xs[1], out1)
