@@ -48,7 +48,7 @@ int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int row
                            int gs_rows, void* packed, void* sf, int sf_layout, void* stream);
 
 /* The same with each group's own global scale, both passes in one launch: x [groups, rows, K] -> gs_out f32 [groups] (2688 / amax,
- * as b200moe_global_scale), packed u8 [groups, rows, K/2], sf u8 row-major [groups, rows, K/16] (sf_layout 0) or 128x4-swizzled
+ * as b200moe_global_scale; at most 65535 groups), packed u8 [groups, rows, K/2], sf u8 row-major [groups, rows, K/16] (sf_layout 0) or 128x4-swizzled
  * per group (sf_layout 1: [groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: 8-byte aligned, zeroed once, then only
  * ever passed to this function (any sizes); calls that may overlap on the GPU need one each, and a captured call is in flight whenever
  * its graph is. Where the size is 0 (one matrix of up to 8192 blocks of 16) it may be null. sm120fp4/reference.py:68-90. */

@@ -322,6 +322,10 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 
 using namespace b200;
 
+extern "C" int b200moe_global_scale(const void* x, int dtype, long long n, void* amax_scratch_u32, float* gs_out, void* stream);
+extern "C" int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int rows, int K, const float* global_scale, int gs_rows, void* packed,
+                                      void* sf, int sf_layout, void* stream);
+
 static int quant_units(int dtype, int rows, int K) {
   const long long nblk = (long long)rows * (K / 16), unit = kQgThreads * (dtype == 0 ? kQPerThread<__nv_bfloat16> : kQPerThread<float>);
   return (int)((nblk + unit - 1) / unit);
@@ -335,13 +339,26 @@ extern "C" long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int g
   return 8 + 8LL * groups * quant_units(dtype, rows, K);
 }
 
+// Matrices beyond what the one launch can index: amax, scale and codes of one group after the other, in launches of their own.
+static int quant_separate(const void* x, int dtype, int groups, int rows, int K, float* gs_out, uint8_t* packed, uint8_t* sf, int sf_layout,
+                          long long sf_stride, unsigned* word, void* stream) {
+  const long long n = (long long)rows * K;
+  for (int g = 0; g < groups; ++g) {
+    const void* xg = (const uint8_t*)x + g * n * (dtype == 0 ? 2 : 4);
+    int rc = b200moe_global_scale(xg, dtype, n, word, gs_out + g, stream);
+    if (rc == B200MOE_OK) rc = b200moe_quantize_nvfp4(xg, dtype, nullptr, rows, K, gs_out + g, 0, packed + g * (n / 2), sf + g * sf_stride, sf_layout, stream);
+    if (rc != B200MOE_OK) return rc;
+  }
+  return B200MOE_OK;
+}
+
 // x [groups, rows, K] (dtype 0 bf16, 1 f32) -> gs_out f32 [groups], packed u8 [groups, rows, K/2], sf u8: sf_layout 0 row-major
 // [groups, rows, K/16], 1 the 128x4 swizzle per group ([groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: zeroed once,
 // then only ever passed to this function; two calls that may overlap on the GPU (a replay of a captured call is one) need one each.
 // Null where b200moe_quantize_own_scale_workspace_bytes says 0.
 extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
                                                 void* workspace, long long workspace_bytes, void* stream) {
-  if (!x || !gs_out || !packed || !sf || groups <= 0 || rows < 0) return B200MOE_ERR_ARG;
+  if (!x || !gs_out || !packed || !sf || groups <= 0 || groups > 65535 || rows < 0) return B200MOE_ERR_ARG;
   if (K <= 0 || K % 16) return B200MOE_ERR_SHAPE;
   if ((dtype != 0 && dtype != 1) || (sf_layout != 0 && sf_layout != 1)) return B200MOE_ERR_ARG;
   if (((uintptr_t)x & 15) || ((uintptr_t)packed & 7) || ((uintptr_t)workspace & 7)) return B200MOE_ERR_ARG;
@@ -358,9 +375,11 @@ extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int gr
   q.bpr_inv = ((1ULL << q.bpr_shift) + q.bpr - 1) / q.bpr;
   q.step_r = kQgThreads / q.bpr, q.step_c = kQgThreads % q.bpr;
   const long long nblk = (long long)rows * q.bpr;
-  if (q.sf_stride > 0x7fffffffLL) return B200MOE_ERR_LIMIT;
-  if (nblk > (1LL << 30)) return B200MOE_ERR_LIMIT;
   unsigned* scratch = (unsigned*)workspace;
+  // 2^30 blocks a group and 2 GB of scales are what the kernels' 32-bit offsets hold. (The word lent here is a unit's: its flag half
+  // stays as it is, so no later call takes the value for a maximum of its own.)
+  if (q.sf_stride > 0x7fffffffLL || nblk > (1LL << 30))
+    return quant_separate(x, dtype, groups, rows, K, gs_out, (uint8_t*)packed, (uint8_t*)sf, sf_layout, q.sf_stride, scratch + 2, stream);
   if (quant_one_cluster(groups, rows, K)) {
     int C = 1;   // CTAs: one block per thread, then two
     while (C < 8 && C * kQThreads < nblk) C *= 2;

@@ -74,6 +74,28 @@ def test_nan_and_infinite_values(rows, dtype):
         assert torch.equal(ge, gs.expand(2)) and torch.equal(qe, wq.expand(2, -1, -1)) and torch.equal(se, wsf.expand(2, -1, -1))
 
 
+def test_scales_beyond_two_gigabytes():
+    """One row of 2^28 values: its padded 128x4 scales take 2 GB, more than the one launch indexes."""
+    import sm120fp4_b200 as pkg
+    k = 1 << 28
+    x = torch.randn(1, k, generator=torch.Generator(device="cuda").manual_seed(1), dtype=torch.bfloat16, device="cuda")
+    q, sf, gs = pkg.quantize_nvfp4(x)
+    qe, se, ge = pkg.quantize_nvfp4_experts(x[None], swizzle=True)
+    assert torch.equal(ge, gs) and torch.equal(qe[0], q)
+    tiles = se.view(-1, 512)
+    assert torch.equal(tiles[:, :4].reshape(1, -1), sf) and not tiles[:, 4:].any()
+
+
+def test_more_groups_than_a_grid_holds_are_refused():
+    import sm120fp4_b200 as pkg
+    from sm120fp4_b200._lib import ERR_ARG, B200MoEError
+    with pytest.raises(B200MoEError) as e:
+        pkg.quantize_nvfp4_experts(torch.ones(65536, 1, 16, dtype=torch.bfloat16, device="cuda"))
+    assert e.value.code == ERR_ARG
+    q, _, _ = pkg.quantize_nvfp4_experts(torch.ones(65535, 1, 16, dtype=torch.bfloat16, device="cuda"))
+    assert bool((q == 0x77).all())
+
+
 def _expect(x, got):
     wq, wsf, wgs = O.quantize_nvfp4(x.float().cpu().numpy(), None)
     q, sf, gs = got
