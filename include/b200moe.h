@@ -55,6 +55,10 @@ int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int row
 long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K);
 int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
                                      int sf_layout, void* workspace, long long workspace_bytes, void* stream);
+/* For tests: the same call with the number of looks at a work unit's maximum after which a block that needs it works it out itself
+ * (blocks of a grid that is not resident as a whole wait for one another at most that long, about 1.5 ms in the call above). */
+int b200moe_quantize_own_scale_probe(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
+                                     int sf_layout, void* workspace, long long workspace_bytes, int polls, void* stream);
 
 /* ---- router: sm120fp4/kernels/moe_w4a16.py:85-91 (route; padded form of k_route :48-83) and the torch router of
  * sm120fp4/kernels/fc1_w4a16.py:272-279. ids i32 [P] -> experts i32 [Umax] (ascending, -1 padding), offsets i32

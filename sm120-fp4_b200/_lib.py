@@ -27,6 +27,7 @@ SIGNATURES = {
     "b200moe_quantize_nvfp4": (_I, [_P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _P]),
     "b200moe_quantize_own_scale_workspace_bytes": (_LL, [_I, _I, _I, _I]),
     "b200moe_quantize_nvfp4_own_scale": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _I, _P, _LL, _P]),
+    "b200moe_quantize_own_scale_probe": (_I, [_P, _I, _I, _I, _I, _P, _P, _P, _I, _P, _LL, _I, _P]),
     "b200moe_route_workspace_bytes": (_LL, [_I, _I]),
     "b200moe_route": (_I, [_P, _I, _I, _I, _P, _P, _P, _P, _LL, _P]),
     "b200moe_route_status": (_I, [_P, _I, _I, _P]),

@@ -184,12 +184,13 @@ __global__ void __launch_bounds__(kQThreads) k_quantize_small(const T* x, QuantG
 // scratch: [0] number of the calls that have used it, [1] blocks of this call that have left (zero between calls); then one 8-byte
 // word {call number + 1, bits of the largest magnitude} per amax unit. A word is stored whole, so whoever reads this call's
 // number in it has the maximum: nothing is counted and nothing is fenced, and a unit's only round trip to L2 overlaps its loads.
+// A quantising unit looks `polls` times for the words of its group; then its block works out what is missing by itself.
 // (With a ticket per unit and counters behind a fence: 330 to 400 us for 128 x 1536 x 2048 bf16.)
 template <typename T>
 __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, int groups, int units, int window, QuantGeom q, float* gs_out,
-                                                                    uint8_t* packed, uint8_t* sf, unsigned* scratch) {
+                                                                    uint8_t* packed, uint8_t* sf, unsigned* scratch, int polls) {
   constexpr int kWarps = kQgThreads / 32, kPer = kQPerThread<T>;
-  __shared__ float wm[2][kWarps];
+  __shared__ unsigned wm[2][kWarps], late[kWarps];
   __shared__ float s_table[128];
   __shared__ int3 s_next[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -202,14 +203,11 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
   float gs_table = -1.f;                        // the global scale s_table was filled for
   int k = 0;
   // maximum over the block, one barrier (the buffer of the unit before may still be read)
-  auto unit_max = [&](float m) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  auto unit_max = [&](unsigned m) {
+    m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0) wm[k][warp] = m;
     __syncthreads();
-    m = wm[k][lane & (kWarps - 1)];
-#pragma unroll
-    for (int o = kWarps / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    m = __reduce_max_sync(0xffffffffu, wm[k][lane & (kWarps - 1)]);
     k ^= 1;
     return m;
   };
@@ -237,7 +235,34 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
     for (int j = 0; j < kPer; ++j)
       if (j * kQgThreads < left) load_raw(src + j * kQgThreads * 16, q.wide, v[j]);
   };
-  auto process = [&](const int3& at, const Raw16<T> (&v)[kPer]) {
+  // The maximum of group g by this block alone, for units whose blocks have not run for a long time (another kernel holds their SMs:
+  // nothing says that the grid is resident as a whole). What it finds out it publishes, so that others need not.
+  constexpr unsigned kMissing = ~0u;   // above the bits of every magnitude
+  auto group_max = [&](int g) {
+    unsigned all = 0u;
+#pragma unroll 1
+    for (int w = 0; w < units; ++w) {
+      unsigned long long* at = words + (long long)g * units + w;
+      const unsigned long long word = ld_relaxed_gpu_u64(at);
+      if (__syncthreads_and((unsigned)(word >> 32) == call)) { all = max(all, (unsigned)word); continue; }
+      float m = 0.f;
+      const int i1 = min(nblk, (w + 1) * (kPer * kQgThreads));
+#pragma unroll 1
+      for (int i = w * (kPer * kQgThreads) + tid; i < i1; i += kQgThreads) {
+        Raw16<T> raw;
+        load_raw(x + ((long long)g * nblk + i) * 16, q.wide, raw);
+        m = fmaxf(m, amax_raw(raw));
+      }
+      unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+      if (lane == 0) late[warp] = mb;      // (read before the next round's barrier)
+      __syncthreads();
+      mb = __reduce_max_sync(0xffffffffu, late[lane & (kWarps - 1)]);
+      if (tid == 0) __stcg(at, ((unsigned long long)call << 32) | mb);
+      all = max(all, mb);
+    }
+    return all;
+  };
+  auto process = [&](const int3& at, Raw16<T> (&v)[kPer]) {
     const int g = at.x, u = at.y;
     const bool second = at.z != 0;
     unsigned long long* gw = words + (long long)g * units;
@@ -248,30 +273,28 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 #pragma unroll
       for (int j = 0; j < kPer; ++j)
         if (j * kQgThreads < left) m = fmaxf(m, amax_raw(v[j]));
-      m = unit_max(m);
-      if (tid == 0) __stcg(gw + u, ((unsigned long long)call << 32) | __float_as_uint(m));
+      const unsigned mb = unit_max(__float_as_uint(m));
+      if (tid == 0) __stcg(gw + u, ((unsigned long long)call << 32) | mb);
       return;
     }
-    float m = 0.f;
+    unsigned m = 0u;
+    int looks = polls;
     for (int w = tid; w < units; w += kQgThreads) {
-      unsigned long long word = 0;
       bool ok = false;
-      for (int it = 0; it < (1 << 22); ++it) {
-        word = ld_relaxed_gpu_u64(gw + w);
+      for (; looks > 0; --looks) {
+        const unsigned long long word = ld_relaxed_gpu_u64(gw + w);
         ok = (unsigned)(word >> 32) == call;
-        if (ok) break;
+        if (ok) { m = max(m, (unsigned)word); break; }
         __nanosleep(100);
       }
-      // a wait that ran out (a block of this grid was held up for seconds): take that unit's maximum here
-      if (!ok) {
-        float mm = 0.f;
-        Raw16<T> raw;
-        for (int i = w * (kPer * kQgThreads); i < min(nblk, (w + 1) * (kPer * kQgThreads)); ++i) { load_raw(x + ((long long)g * nblk + i) * 16, q.wide, raw); mm = fmaxf(mm, amax_raw(raw)); }
-        word = __float_as_uint(mm);
-      }
-      m = fmaxf(m, __uint_as_float((unsigned)word));
+      if (!ok) { m = kMissing; break; }
     }
-    const float gs = scale_of(unit_max(m));
+    m = unit_max(m);
+    if (m == kMissing) {
+      m = group_max(g);
+      load(at, v);
+    }
+    const float gs = scale_of(__uint_as_float(m));
     if (gs != gs_table) {
       fill_scale_table(s_table, gs, tid, kQgThreads);
       gs_table = gs;
@@ -331,6 +354,8 @@ static int quant_units(int dtype, int rows, int K) {
   return (int)((nblk + unit - 1) / unit);
 }
 
+constexpr int kQPolls = 2048;   // looks of ~0.7 us: a unit takes 5 to 10 us, so the words are there long before unless the grid is held up
+
 static bool quant_one_cluster(int groups, int rows, int K) { return groups == 1 && (long long)rows * (K / 16) <= kQSmallMaxBlocks; }
 
 extern "C" long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K) {
@@ -356,8 +381,8 @@ static int quant_separate(const void* x, int dtype, int groups, int rows, int K,
 // [groups, rows, K/16], 1 the 128x4 swizzle per group ([groups, pad128(rows) * pad4(K/16)], padding written 0). workspace: zeroed once,
 // then only ever passed to this function; two calls that may overlap on the GPU (a replay of a captured call is one) need one each.
 // Null where b200moe_quantize_own_scale_workspace_bytes says 0.
-extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
-                                                void* workspace, long long workspace_bytes, void* stream) {
+static int quantize_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout, void* workspace,
+                              long long workspace_bytes, int polls, void* stream) {
   if (!x || !gs_out || !packed || !sf || groups <= 0 || groups > 65535 || rows < 0) return B200MOE_ERR_ARG;
   if (K <= 0 || K % 16) return B200MOE_ERR_SHAPE;
   if ((dtype != 0 && dtype != 1) || (sf_layout != 0 && sf_layout != 1)) return B200MOE_ERR_ARG;
@@ -408,6 +433,17 @@ extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int gr
   }
   const long long most = 2LL * groups * units;
   const int grid = (int)(most < 2LL * sms ? most : 2LL * sms);
-  void* args[] = {(void*)&x, (void*)&groups, (void*)&units, (void*)&window, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch};
+  void* args[] = {(void*)&x, (void*)&groups, (void*)&units, (void*)&window, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&polls};
   return launch_kernel(dtype == 0 ? (const void*)k_quantize_grouped<__nv_bfloat16> : (const void*)k_quantize_grouped<float>, grid, kQgThreads, 0, true, args, st);
+}
+
+extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
+                                                void* workspace, long long workspace_bytes, void* stream) {
+  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, kQPolls, stream);
+}
+
+// The same call that looks `polls` times for a unit's maximum before it works it out again (0: never waits), for tests of that way.
+extern "C" int b200moe_quantize_own_scale_probe(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
+                                                void* workspace, long long workspace_bytes, int polls, void* stream) {
+  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, polls, stream);
 }

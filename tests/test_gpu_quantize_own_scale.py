@@ -115,6 +115,40 @@ def _randn(rows, k, seed):
     return torch.randn(rows, k, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
 
 
+@pytest.mark.parametrize("polls", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("groups,rows,k", [(1, 257, 1040), (3, 300, 2048), (40, 192, 512), (6, 1536, 2048)])
+def test_blocks_that_do_not_wait(groups, rows, k, dtype, polls):
+    """A block that gives up waiting for other blocks' maxima works them out itself: the same bytes, twice on one workspace."""
+    import sm120fp4_b200 as pkg
+    import sm120fp4_b200._lib as L
+    w = torch.randn(groups, rows, k, generator=torch.Generator().manual_seed(rows)).to(dtype).cuda() * torch.arange(1, groups + 1, device="cuda").to(dtype)[:, None, None]
+    want = pkg.quantize_nvfp4_experts(w)
+    dt = 0 if dtype == torch.bfloat16 else 1
+    ws = torch.zeros(L.lib().b200moe_quantize_own_scale_workspace_bytes(dt, groups, rows, k), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        got = [torch.empty_like(t) for t in want]
+        L.check(L.lib().b200moe_quantize_own_scale_probe(L.ptr(w), dt, groups, rows, k, L.ptr(got[2]), L.ptr(got[0]), L.ptr(got[1]), 0, L.ptr(ws),
+                                                         ws.numel(), polls, L.stream_ptr()), "probe")
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_two_calls_at_once():
+    """Two large calls on two streams share the GPU's SMs in whatever way they are scheduled."""
+    import sm120fp4_b200 as pkg
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    ws = [torch.randn(24, 768, 2048, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda", dtype=torch.float32) for i in range(2)]
+    want = [pkg.quantize_nvfp4_experts(w) for w in ws]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(6):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(pkg.quantize_nvfp4_experts(ws[i]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for i in range(2) for o in got[i] for a, b in zip(o, want[i]))
+
+
 def test_captured_call_keeps_its_workspace():
     """A larger eager call on the stream of a captured one, and whatever it lets the allocator hand out, touch nothing that a replay uses."""
     import sm120fp4_b200 as pkg
