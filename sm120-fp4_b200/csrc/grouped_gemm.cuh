@@ -465,11 +465,13 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
       if (PHASE <= 2) s /= P.gs_in;
       int pr = -1;
       float rs = 0.f;   // W4A16 phases: 1 / g_t of this operand row's term
-      if (PHASE == 2 || (PHASE == 4 && row < kARows)) {   // FC2: times the row's routing weight
+      // (not in the dry pass: the kernel that writes row_pair and rowscale may still be running, and what an earlier, larger call left in
+      // row_pair would index beyond this call's weights)
+      if (!dry && (PHASE == 2 || (PHASE == 4 && row < kARows))) {   // FC2: times the row's routing weight
         pr = __ldcg(P.row_pair + (long long)t * kARows + row);
         s = pr >= 0 ? s * P.wts[pr] : 0.f;
       }
-      if (PHASE == 3 && row < rows) rs = __ldcg(P.rowscale + (long long)t * kARows + row);
+      if (PHASE == 3 && !dry && row < rows) rs = __ldcg(P.rowscale + (long long)t * kARows + row);
       if (PHASE == 4) {
         float g = P.act_g1;
         for (int q = 0; q < (lane & 3); ++q) g *= 6.0f;

@@ -42,6 +42,26 @@ def test_plan_sizes(top_k, m):
     assert np.array_equal(row_pair[rows[order]], order) and (row_pair >= 0).sum() == order.size and rows[flat < 0].max() == -1
 
 
+@pytest.mark.parametrize("m", [17, 40])
+def test_small_call_after_a_large_one(m):
+    """The tables that a large call left in the workspace index beyond a small call's tensors: nothing of them may be used."""
+    cfg = dict(experts=24, hidden=1024, inter=128, top_k=8)
+    w, _ = make_layer(**cfg, seed=3)
+    big = [t.cuda() for t in inputs(cfg, 2000, 1)]
+    x, ids, wts = (t.cuda() for t in inputs(cfg, m, 2))
+    w.enable_prefill(max_tokens=2000)
+    first = w.forward(x, ids, wts).clone()
+    w.forward(*big)
+    assert torch.equal(w.forward(x, ids, wts), first)
+    w.prefill_status()
+    w.prefill = None
+    w.enable_mid(max_tokens=2000, min_tokens=17)
+    first = w.forward(x, ids, wts).clone()
+    w.forward(*big)
+    assert torch.equal(w.forward(x, ids, wts), first)
+    w.mid_status()
+
+
 @pytest.mark.parametrize("m", [40, 150])
 def test_streamed_operand_boxes(m):
     cfg = dict(experts=4, hidden=3328, inter=192, top_k=2)
