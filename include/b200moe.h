@@ -123,6 +123,8 @@ int b200moe_prefill_status(const b200moe_layer* layer, const void* workspace, in
  * row r, 16-value block b at r*128 + (((b>>1) ^ (r&7)) << 4) + (b&1)*8 (8 code bytes), its scale byte at 16384 + (b>>2)*512 +
  * (r&31)*16 + (r>>5)*4 + (b&3) - i.e. four 128x4 scale tiles. */
 int b200moe_prefill_workspace_map(const b200moe_layer* layer, int max_tokens, long long* out14);
+/* For tests: out[i] = a[i] / b[i] as the W4A4 FC1 epilogue of hidden sizes above 2304 divides (IEEE rounding). */
+int b200moe_quotient_probe(const float* a, const float* b, float* out, int n, void* stream);
 
 /* forward: x bf16 [M, H], topk_ids i32 [M, top_k], topk_weights f32 [M, top_k] -> out bf16 [M, H]; one layer kernel
  * (routing + FC1 + SiLU*mul + FC2 + weighted combine), behind a small one that expands x above 8 tokens or 4096 values of x. Replaces Weights._slice, sm120fp4/vllm_backend.py:174-190. */

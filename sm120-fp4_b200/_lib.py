@@ -48,6 +48,7 @@ SIGNATURES = {
     "b200moe_prefill_forward": (_I, [_P, _P, _P, _P, _I, _P, _P, _LL, _I, C.c_float, C.c_float, _P]),
     "b200moe_prefill_status": (_I, [_P, _P, _I, _P]),
     "b200moe_prefill_workspace_map": (_I, [_P, _I, _P]),
+    "b200moe_quotient_probe": (_I, [_P, _P, _P, _I, _P]),
     "b200moe_decode_forward": (_I, [_P, _P, _P, _P, _I, _P, _P, _LL, _P]),
     "b200moe_decode_forward_ex": (_I, [_P, _P, _P, _P, _I, _P, _P, _LL, _I, _P]),
     "b200moe_decode_forward_host": (_I, [_P, _P, _P, _P, _I, _P, _P, _LL, _P]),

@@ -128,6 +128,18 @@ struct GgAside {
 // layers were defined that way, and an approximate quotient moves an activation on the edge of two FP4 codes to the other one (1.4e-4
 // of a layer's output at 4096 x 1536). Up to nine boxes it has always been the approximate one.
 inline bool gg_ieee_silu(int KB1) { return KB1 > 9; }
+// g / d rounded to nearest, d in [1, 2^64]: Markstein's method (IBM J. Res. Dev. 34, 1990) - the approximate reciprocal, one Newton
+// step, the quotient and one correction by its exact residual. Magnitudes of g between 2^-64 and 2^64 keep every step in the normal
+// range; a zero keeps its sign. Anything else sets `odd` and goes through __fdiv_rn. (333 tokens of 2816 x 704: 79 us, 77 with the
+// approximate quotient. With __fdiv_rn throughout 103: an empty row of a tile holds zeros, and a zero numerator takes its special path.)
+__device__ __forceinline__ float gg_quotient(float g, float d, bool& odd) {
+  float y = rcp_approx(d);
+  y = __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
+  const float q = __fmul_rn(g, y);
+  const float m = fabsf(g);
+  odd |= !(m <= 0x1p64f && d <= 0x1p64f && (m >= 0x1p-64f || m == 0.f));
+  return m == 0.f ? g : __fmaf_rn(__fmaf_rn(-d, q, g), y, q);
+}
 
 // ---- epilogues: one warp, 32 accumulator rows x 128 columns at taddr (thread = row). `release` frees the accumulator buffer
 // once its values are in registers.
@@ -152,11 +164,19 @@ __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float g
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       float a[16];
+      bool odd = false;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;
         const float d = 1.0f + __expf(-g);
-        a[i] = (Ieee ? __fdiv_rn(g, d) : __fdividef(g, d)) * u;
+        a[i] = (Ieee ? gg_quotient(g, d, odd) : __fdividef(g, d)) * u;
+      }
+      if (Ieee && odd) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;
+          a[i] = __fdiv_rn(g, 1.0f + __expf(-g)) * u;
+        }
       }
       sfw |= (uint32_t)quantize_block16_t(a, gs_out, scale_table, pk[b]) << (16 * h + 8 * b);
     }

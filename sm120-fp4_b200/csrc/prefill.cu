@@ -455,3 +455,20 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   void* args[] = {(void*)&y, (void*)&dst_row, (void*)&M, (void*)&top_k, (void*)&H, (void*)&out};
   return launch_kernel((const void*)k_combine<true>, sms * 4, 256, 0, true, args, st);
 }
+
+// out[i] = a[i] / b[i] as FC1's epilogue divides in wide layers (gg_quotient), for tests.
+static __global__ void __launch_bounds__(256) k_quotient(const float* a, const float* b, float* out, int n) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  bool odd = false;
+  const float q = gg_quotient(a[i], b[i], odd);
+  out[i] = odd ? __fdiv_rn(a[i], b[i]) : q;
+}
+
+extern "C" int b200moe_quotient_probe(const float* a, const float* b, float* out, int n, void* stream) {
+  if (!a || !b || !out || n < 0) return B200MOE_ERR_ARG;
+  if (n == 0) return B200MOE_OK;
+  k_quotient<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(a, b, out, n);
+  B200_LAUNCH_CHECK();
+  return B200MOE_OK;
+}
