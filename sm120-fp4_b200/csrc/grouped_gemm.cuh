@@ -223,6 +223,9 @@ __device__ __forceinline__ void gg_epilogue_fc2(uint32_t taddr, float s, unsigne
 // into four terms run once per block with every lane at work; the lane writes its block of all four term rows of FC2's operand
 // record. (With two blocks at a time and every second lane idle in the expansion an epilogue took 12,500 cycles, more than the
 // eight weight records of a block take to arrive.) Returns whether a block lay beyond the range of the activation scale.
+// Fused: whether the lane's own product is rounded before the add. Which of the two a phase does is part of its results: a bf16 output
+// in a few thousand moves by one step with the other.
+template <bool Fused>
 __device__ __forceinline__ void gg_reduce_scatter16(uint32_t taddr, float rs, int tq, float (&o)[16]) {
   uint32_t r[4][16];
 #pragma unroll
@@ -234,8 +237,9 @@ __device__ __forceinline__ void gg_reduce_scatter16(uint32_t taddr, float rs, in
     float k2[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const float mine = __uint_as_float(hi ? r[2 + j][i] : r[j][i]) * rs, other = __uint_as_float(hi ? r[j][i] : r[2 + j][i]) * rs;
-      k2[j] = mine + __shfl_xor_sync(0xffffffffu, other, 2);   // the lane two over keeps the other two blocks and sends these
+      const float mine = __uint_as_float(hi ? r[2 + j][i] : r[j][i]), other = __fmul_rn(__uint_as_float(hi ? r[j][i] : r[2 + j][i]), rs);
+      const float got = __shfl_xor_sync(0xffffffffu, other, 2);   // the lane two over keeps the other two blocks and sends these
+      k2[j] = Fused ? __fmaf_rn(mine, rs, got) : __fadd_rn(__fmul_rn(mine, rs), got);
     }
     const float keep = lo ? k2[1] : k2[0], send = lo ? k2[0] : k2[1];
     o[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
@@ -251,7 +255,7 @@ __device__ __forceinline__ bool gg_epilogue_fc1_a16(uint32_t taddr, float s, flo
   for (int half = 0; half < 2; ++half) {   // the up columns, then the gate columns
 #pragma unroll
     for (int i = 0; i < 16; ++i) up[i] = a[i];
-    gg_reduce_scatter16(taddr + 64 * half, rs, tq, a);
+    gg_reduce_scatter16<false>(taddr + 64 * half, rs, tq, a);
   }
   release();
 #pragma unroll
@@ -279,7 +283,7 @@ __device__ __forceinline__ void gg_epilogue_fc2_a16(uint32_t taddr, float s, flo
   for (int half = 0; half < 2; ++half) {
     const int tq = lane & 3;
     float o[16];
-    gg_reduce_scatter16(taddr + 64 * half, rs, tq, o);
+    gg_reduce_scatter16<true>(taddr + 64 * half, rs, tq, o);
     if (half == 1) release();
 #pragma unroll
     for (int i = 0; i < 16; ++i) o[i] *= s;

@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from helpers import check_layer_output
+from helpers import check_layer_output, make_layer
 from oracle import nvfp4_oracle as O
 from test_gpu_decode import inputs, layer
 
@@ -56,3 +56,14 @@ def test_qwen_shape_mid_batches():
         x, ids, wts = inputs(cfg, m, 8100 + m)
         out = run_mid(w, x, ids, wts)
         check_layer_output(out, O.moe_reference(x.float().numpy(), ow, ids.numpy(), wts.numpy()), f"mid qwen m={m}")
+
+
+# Outputs (bf16 bits) that move by one step when the order of roundings in a term sum changes - FC1 rounds a term's product before it
+# adds it, FC2 does not - as this path has computed them from its first form on.
+@pytest.mark.parametrize("m,want", [(40, {(1, 238): -17320, (1, 426): 15468, (1, 440): -18272, (1, 498): -17332, (6, 166): 14253}),
+                                    (90, {(7, 11): 14738, (7, 133): 15404, (7, 157): -17462, (7, 354): -17398, (7, 482): -17682, (8, 86): -17929})])
+def test_mid_roundings_are_pinned(m, want):
+    cfg = dict(experts=12, hidden=512, inter=640, top_k=4)
+    w, _ = make_layer(**cfg, seed=1)
+    bits = run_mid(w, *inputs(cfg, m, 900 + m)).cpu().view(torch.int16)
+    assert {at: int(bits[at]) for at in want} == want
