@@ -256,7 +256,7 @@ static PrefillLayout prefill_layout(int E, int H, int I, int top_k, int max_toke
   PrefillLayout L;
   const long long P = (long long)max_tokens * top_k;
   const int KB1 = (H + 255) / 256, KB2 = (I + 255) / 256;
-  L.max_tiles = (int)(P / 128 + 2 * E);   // every expert may end in a partly filled tile, plus one empty tile to make its count even
+  L.max_tiles = (int)(P / 128 + E);   // every expert may end in a partly filled tile
   long long o = 0;
   L.experts = o, o = pf_align(o + 4LL * E);
   L.offsets = o, o = pf_align(o + 4LL * (E + 1));
@@ -368,7 +368,7 @@ int b200_prefill_status_offset(int E, int H, int I, int top_k, int max_tokens, l
 // ---------------------------------------------------------------------------------------------------------------------
 // W4A16 layer call for mid-sized batches (the decode path's arithmetic, one pass over the touched experts' weights).
 struct MidLayout {
-  long long experts, offsets, pairs, ntiles, tile_expert, tile_tab, row_pair, rowscale, dst_row, tok_amax, status, xrec, arec, y, total;
+  long long experts, offsets, pairs, ntiles, tile_expert, tile_tab, row_pair, rowscale, dst_row, status, xrec, arec, y, total;
   int max_tiles;
 };
 
@@ -387,7 +387,6 @@ static MidLayout mid_layout(int E, int H, int I, int top_k, int max_tokens) {
   L.row_pair = o, o = pf_align(o + 4LL * L.max_tiles * 64);
   L.rowscale = o, o = pf_align(o + 4LL * L.max_tiles * 64);
   L.dst_row = o, o = pf_align(o + 4 * P);
-  L.tok_amax = o, o = pf_align(o + 4LL * max_tokens);
   L.status = o, o += 256;
   L.xrec = o, o = pf_align(o + (long long)L.max_tiles * KB1 * kMidRec);
   L.arec = o, o = pf_align(o + (long long)L.max_tiles * KB2 * kMidRec);

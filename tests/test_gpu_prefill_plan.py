@@ -42,6 +42,25 @@ def test_plan_sizes(top_k, m):
     assert np.array_equal(row_pair[rows[order]], order) and (row_pair >= 0).sum() == order.size and rows[flat < 0].max() == -1
 
 
+def test_workspace_holds_the_most_tiles_there_can_be():
+    """Every expert ends in a tile of one row at the very number of tokens the workspace was sized for: all of its tiles are in use, and
+    nothing is written behind it."""
+    cfg = dict(experts=16, hidden=512, inter=128, top_k=8)
+    w, _ = make_layer(**cfg, seed=4)
+    m = 16 * 129 // 8
+    x, _, wts = inputs(cfg, m, 3)
+    ids = (torch.arange(m * 8, dtype=torch.int32) % 16).reshape(m, 8)
+    nbytes = w.prefill_workspace_bytes(m)
+    ws = torch.zeros(nbytes + (1 << 20), dtype=torch.uint8, device="cuda")
+    ws[nbytes:] = 0x5a
+    w.enable_prefill(max_tokens=m, workspace=ws)
+    out = run_prefill(w, x, ids, wts, m).clone()
+    mp = prefill_map(w, m)
+    assert mp["max_tiles"] == 32 == int(_i32(ws, mp["ntiles"], 1)[0])
+    assert bool((ws[nbytes:] == 0x5a).all())
+    assert torch.equal(out, in_parts(w, x, ids, wts, 1000))
+
+
 @pytest.mark.parametrize("m", [17, 40])
 def test_small_call_after_a_large_one(m):
     """The tables that a large call left in the workspace index beyond a small call's tensors: nothing of them may be used."""
