@@ -38,6 +38,28 @@ def test_stacked_matrices(groups, rows, k, swizzle):
         assert np.array_equal(sf[g].cpu().numpy(), O.to_128x4(wsf) if swizzle else wsf)
 
 
+# More than 20 MB in all: the passes of different groups alternate (10 and 5 groups apart here, the last unit of each ragged); a group
+# above 20 MB: its two passes follow one another.
+@pytest.mark.parametrize("dtype,groups,rows,k", [(torch.bfloat16, 16, 1000, 1040), (torch.float32, 12, 1000, 1040), (torch.bfloat16, 2, 6400, 2048)])
+def test_groups_in_alternating_order(dtype, groups, rows, k):
+    import sm120fp4_b200 as pkg
+    scale = torch.linspace(0.01, 9.0, groups, device="cuda")[:, None, None]
+    w = (torch.randn(groups, rows, k, generator=torch.Generator(device="cuda").manual_seed(groups), device="cuda") * scale).to(dtype)
+    want = [O.quantize_nvfp4(w[g].float().cpu().numpy(), None) for g in range(groups)]
+    small = torch.randn(3, 100, 80, generator=torch.Generator().manual_seed(1)).to(dtype).cuda()
+    for swizzle in (False, True):
+        q, sf, gs = pkg.quantize_nvfp4_experts(w, swizzle=swizzle)
+        pkg.quantize_nvfp4_experts(small)            # a smaller call in between, on the same workspace
+        for g, (wq, wsf, wgs) in enumerate(want):
+            assert np.array_equal(gs[g:g + 1].cpu().numpy().view(np.uint32), wgs.view(np.uint32))
+            assert np.array_equal(q[g].cpu().numpy(), wq)
+            assert np.array_equal(sf[g].cpu().numpy(), O.to_128x4(wsf) if swizzle else wsf)
+    got = pkg.quantize_nvfp4_experts(small)
+    for g in range(3):
+        wq, wsf, wgs = O.quantize_nvfp4(small[g].float().cpu().numpy(), None)
+        assert np.array_equal(got[0][g].cpu().numpy(), wq) and np.array_equal(got[1][g].cpu().numpy(), wsf)
+
+
 def test_every_bf16_amax():
     """Every positive bf16 value up to 2^60 as a block's largest magnitude, in matrices whose global scale makes the block scales
     land on all of E4M3's range: the block scale's division has a form of its own for bf16 inputs."""
