@@ -123,8 +123,9 @@ int b200moe_prefill_status(const b200moe_layer* layer, const void* workspace, in
  * row r, 16-value block b at r*128 + (((b>>1) ^ (r&7)) << 4) + (b&1)*8 (8 code bytes), its scale byte at 16384 + (b>>2)*512 +
  * (r&31)*16 + (r>>5)*4 + (b&3) - i.e. four 128x4 scale tiles. */
 int b200moe_prefill_workspace_map(const b200moe_layer* layer, int max_tokens, long long* out14);
-/* For tests: out[i] = a[i] / b[i] as the W4A4 FC1 epilogue of hidden sizes above 2304 divides (IEEE rounding). */
-int b200moe_quotient_probe(const float* a, const float* b, float* out, int n, void* stream);
+/* For tests: out[i] = gate[i] / den[i], den[i] = 1 + exp(-gate[i]), as the W4A4 FC1 epilogue of hidden sizes above 2304 divides (IEEE
+ * rounding). */
+int b200moe_quotient_probe(const float* gate, float* den, float* out, int n, void* stream);
 
 /* forward: x bf16 [M, H], topk_ids i32 [M, top_k], topk_weights f32 [M, top_k] -> out bf16 [M, H]; one layer kernel
  * (routing + FC1 + SiLU*mul + FC2 + weighted combine), behind a small one that expands x above 8 tokens or 4096 values of x. Replaces Weights._slice, sm120fp4/vllm_backend.py:174-190. */
@@ -141,9 +142,10 @@ int b200moe_decode_forward(const b200moe_layer* layer, const void* x_bf16, const
 int b200moe_decode_forward_ex(const b200moe_layer* layer, const void* x_bf16, const int* topk_ids, const float* topk_weights,
                               int M, void* out_bf16, void* workspace, long long workspace_bytes, int flags, void* stream);
 /* b200moe_decode_forward for a caller whose tensors live in host memory: x bf16 [M, H], ids int32 [M, top_k], weights f32
- * [M, top_k] in, out bf16 [M, H] back. The inputs go through staging buffers inside the workspace (three small copies on
- * `stream`); a page-locked output buffer is written by the kernel directly across the host link, a pageable one is copied
- * back. Everything is enqueued on `stream`, nothing synchronises. M <= 16. Replaces the same call
+ * [M, top_k] in, out bf16 [M, H] back. Where all four buffers are page-locked and x and out 16-byte aligned, kernels read the inputs
+ * and write the output across the host link; otherwise the inputs are copied through staging buffers inside the workspace, and an
+ * output that is not page-locked is copied back. Everything is enqueued on `stream`, nothing synchronises: the buffers are read
+ * and written while the stream runs the call. M <= 16. Replaces the same call
  * site as b200moe_decode_forward (sm120fp4/vllm_backend.py:174-190) for hosts that do not hold device tensors. */
 int b200moe_decode_forward_host(const b200moe_layer* layer, const void* x_host, const int* ids_host, const float* wts_host, int M,
                                 void* out_host, void* workspace, long long workspace_bytes, void* stream);

@@ -8,8 +8,9 @@
 // What bounds it. Per weight record (128 columns x 256 K values, 18 KB) the tensor core needs 4 x 64 cycles (measured:
 // 128 x 128 x 64 in 64 cycles) plus 8 cycles per tcgen05.cp of a 512-byte scale tile; an SM takes in 63 bytes per cycle from
 // L2 (17.3 TB/s over the chip, from four 18 KB copies in flight on), i.e. 288 cycles per record; HBM delivers a record per
-// SM every ~700 cycles (7.1 TB/s). A batch that touches every expert with few rows is bound by HBM, a large one by the MMAs
-// and the L2 port together. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies
+// SM every ~700 cycles (7.1 TB/s). A batch that touches every expert with few rows is bound by HBM. In a large one no unit is
+// near its peak over the whole kernel (FC1 of 8192 tokens: tensor pipe 48 %, shared memory 51 %, L2 24 %, HBM 30 %; about 530
+// cycles a record): what a record waits for beside its MMAs has not been separated. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies
 // its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
 // warp to warp between a record's arrival and its math. (Before, four warps moved the scales through registers and handed every
 // record to the MMA warp over a barrier: 870 cycles a record at 8192 tokens.)
@@ -128,18 +129,18 @@ struct GgAside {
 // layers were defined that way, and an approximate quotient moves an activation on the edge of two FP4 codes to the other one (1.4e-4
 // of a layer's output at 4096 x 1536). Up to nine boxes it has always been the approximate one.
 inline bool gg_ieee_silu(int KB1) { return KB1 > 9; }
-// g / d rounded to nearest, d in [1, 2^64]: Markstein's method (IBM J. Res. Dev. 34, 1990) - the approximate reciprocal, one Newton
-// step, the quotient and one correction by its exact residual. Magnitudes of g between 2^-64 and 2^64 keep every step in the normal
-// range; a zero keeps its sign. Anything else sets `odd` and goes through __fdiv_rn. (333 tokens of 2816 x 704: 79 us, 77 with the
-// approximate quotient. With __fdiv_rn throughout 103: an empty row of a tile holds zeros, and a zero numerator takes its special path.)
-__device__ __forceinline__ float gg_quotient(float g, float d, bool& odd) {
+// g / d rounded to nearest for d = 1 + exp(-g) and -44 <= g <= 2^64: Markstein's method (IBM J. Res. Dev. 34, 1990) - the approximate
+// reciprocal, one Newton step, the quotient and one correction by its exact residual. In that range d is below 2^64 and no step leaves
+// the normal numbers (below 2^-24 d is exactly 2); a zero keeps its sign. The caller takes __fdiv_rn elsewhere. (333 tokens of 2816 x
+// 704: 76 us, 74 with the approximate quotient. With __fdiv_rn throughout 103: an empty row of a tile holds zeros, and a zero
+// numerator takes its special path.)
+__device__ __forceinline__ float gg_quotient(float g, float d) {
   float y = rcp_approx(d);
   y = __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
   const float q = __fmul_rn(g, y);
-  const float m = fabsf(g);
-  odd |= !(m <= 0x1p64f && d <= 0x1p64f && (m >= 0x1p-64f || m == 0.f));
-  return m == 0.f ? g : __fmaf_rn(__fmaf_rn(-d, q, g), y, q);
+  return g == 0.f ? g : __fmaf_rn(__fmaf_rn(-d, q, g), y, q);
 }
+constexpr float kGgQuotLo = -44.f, kGgQuotHi = 0x1p64f;   // (a NaN may go either way)
 
 // ---- epilogues: one warp, 32 accumulator rows x 128 columns at taddr (thread = row). `release` frees the accumulator buffer
 // once its values are in registers.
@@ -164,14 +165,15 @@ __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float g
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       float a[16];
-      bool odd = false;
+      float lo = 0.f, hi = 0.f;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;
         const float d = 1.0f + __expf(-g);
-        a[i] = (Ieee ? gg_quotient(g, d, odd) : __fdividef(g, d)) * u;
+        if (Ieee) lo = fminf(lo, g), hi = fmaxf(hi, g);
+        a[i] = (Ieee ? gg_quotient(g, d) : __fdividef(g, d)) * u;
       }
-      if (Ieee && odd) {
+      if (Ieee && (lo < kGgQuotLo || hi > kGgQuotHi) && store) {   // (not in the dry pass, on whatever the accumulator holds)
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float g = __uint_as_float(gt[b][i]) * s, u = __uint_as_float(up[b][i]) * s;

@@ -455,19 +455,19 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   return launch_kernel((const void*)k_combine<true>, sms * 4, 256, 0, true, args, st);
 }
 
-// out[i] = a[i] / b[i] as FC1's epilogue divides in wide layers (gg_quotient), for tests.
-static __global__ void __launch_bounds__(256) k_quotient(const float* a, const float* b, float* out, int n) {
+// out[i] = g[i] / den[i], den[i] = 1 + exp(-g[i]), as FC1's epilogue divides in wide layers (gg_quotient), for tests.
+static __global__ void __launch_bounds__(256) k_quotient(const float* gate, float* den, float* out, int n) {
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
-  bool odd = false;
-  const float q = gg_quotient(a[i], b[i], odd);
-  out[i] = odd ? __fdiv_rn(a[i], b[i]) : q;
+  const float g = gate[i], d = 1.0f + __expf(-g);
+  den[i] = d;
+  out[i] = g < kGgQuotLo || g > kGgQuotHi ? __fdiv_rn(g, d) : gg_quotient(g, d);
 }
 
-extern "C" int b200moe_quotient_probe(const float* a, const float* b, float* out, int n, void* stream) {
-  if (!a || !b || !out || n < 0) return B200MOE_ERR_ARG;
+extern "C" int b200moe_quotient_probe(const float* gate, float* den, float* out, int n, void* stream) {
+  if (!gate || !den || !out || n < 0) return B200MOE_ERR_ARG;
   if (n == 0) return B200MOE_OK;
-  k_quotient<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(a, b, out, n);
+  k_quotient<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(gate, den, out, n);
   B200_LAUNCH_CHECK();
   return B200MOE_OK;
 }
