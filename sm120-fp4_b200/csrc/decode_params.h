@@ -77,7 +77,8 @@ int b200_decode_tc_static_bytes(int N);
 struct HostRouting { const int* ids_h; const float* wts_h; int npairs; int* ids_d; float* wts_d; };
 int b200_expand_x_launch(const void* x, int M, int H, int N, int KB1, void* xb, float* colscale, const HostRouting* host, bool chained, cudaStream_t st);
 int b200_host_stage_launch(const void* x, int n16, const HostRouting& h, void* x_d, bool chained, cudaStream_t st);   // n16: 16-byte words of x
-// whether the layer kernel expands x itself (see expand_x_here)
+// whether the layer kernel expands x itself: up to 256 blocks of 16 values, two for each of its 128 threads (measured on both sides of the
+// line: see expand_x_here)
 inline bool b200_decode_self_expand(int M, int H) { return M <= 8 && M * H <= 16 * 256; }
 int b200_pack_tiles_launch(const void* q, const void* sf, void* out, int E, int rows_per_expert, int row_bytes, int blocks, int KB, int KT,
                            int fc1, int I, long long sf_stride, cudaStream_t st);

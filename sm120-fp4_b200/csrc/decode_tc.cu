@@ -193,8 +193,9 @@ __global__ void __launch_bounds__(256) k_pack_tiles(const uint8_t* __restrict__ 
 // Small operands (P.self: up to 256 blocks of 16 values, e.g. two tokens of 2048) every worker expands by itself, with its 128
 // epilogue threads, straight into shared memory: a launch less, and nothing has to travel (one token of 2048 values: 2.7 us from
 // the completion of the kernel before to the operand, against 3.5 to 4.3 with the kernel above; a layer 12.2 us against 13.5).
-// Beyond that the kernel's 16 blocks are ahead: four tokens of 2816 values take 6 us here, where loads wait behind the weight
-// stream and the work per thread grows (a layer 27.3 us against 26.0).
+// Beyond that the kernel's 16 blocks are ahead: loads wait behind the weight stream here and the work per thread grows. With four blocks
+// a thread a layer of 352 blocks takes 17.4 us against 16.9 with the kernel, 384 blocks 19.2 against 17.8, 512 21.6 against 20.5, and the
+// longer code costs the calls of up to 256 blocks 0.3 to 0.5 us; 704 blocks, with six a thread, 27.3 against 26.0.
 __device__ __forceinline__ void zero_scales(uint8_t* xsf, int KT1, int et) {   // rows that hold no token keep zero scales
   for (int i = et; i < KT1 * 32; i += 128) reinterpret_cast<uint4*>(xsf)[i] = make_uint4(0u, 0u, 0u, 0u);
 }

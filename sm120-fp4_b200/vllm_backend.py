@@ -220,8 +220,8 @@ class Weights:
     def forward(self, x: torch.Tensor, topk_ids: torch.Tensor, topk_weights: torch.Tensor, out: torch.Tensor | None = None,
                 pdl: bool | None = None) -> torch.Tensor:
         """The MoE forward for a batch of any size (sm120fp4/vllm_backend.py:147-172). `pdl` (the reference's per-call
-        switch for programmatic dependent launch): None or True - the two launches of a decode call are programmatic, so the
-        call overlaps the tail of its predecessor in the stream and reads topk_ids / topk_weights at kernel entry (they must
+        switch for programmatic dependent launch): None or True - the launches of a decode call (the layer kernel, above 8 tokens or
+        4096 values of x behind one that expands x) are programmatic, so the call overlaps the tail of its predecessor in the stream and reads topk_ids / topk_weights at kernel entry (they must
         be complete when the kernel before this call starts; a violation is reported by `status()`); False - ordinary
         stream-ordered launches, no such requirement."""
         if x.dtype != torch.bfloat16 or x.dim() != 2 or x.shape[1] != self.H:
@@ -263,7 +263,7 @@ class Weights:
     def forward_host(self, x: torch.Tensor, topk_ids: torch.Tensor, topk_weights: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """The forward for tensors in host memory: x bf16 [tokens, H], ids int32 and weights f32 [tokens, top_k], out bf16
         [tokens, H], all on the CPU. One library call per 16 tokens enqueues everything on the current stream of the layer's
-        device (the inputs are staged by three small copies, a page-locked `out` is written by the kernel directly); nothing
+        device (page-locked tensors are read and written by the kernels across the host link, others are copied); nothing
         synchronises - read `out` after synchronising the stream. A set of tensors is validated once and then recognised by
         its addresses, so that a serving loop that reuses its buffers pays for one foreign-function call only."""
         m = x.shape[0]
