@@ -118,7 +118,7 @@ extern "C" int b200moe_layer_create(b200moe_layer** out, int E, int H, int I, in
   if (rc == B200MOE_OK) rc = make_codes_map(&L->tm2, q2, (long long)E * H, I / 2, 128);
   if (rc != B200MOE_OK) { delete L; return rc; }
   // workspace
-  const int V = 2 * L->sms;
+  const int V = 3 * L->sms;   // workers of the mma.sync kernel
   L->umax_cap = E < 16 * top_k ? E : 16 * top_k;
   long long o = 0;
   L->off_status = o, o += 256;                                               // status + grid barrier words
@@ -267,7 +267,7 @@ static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const floa
 }
 
 static int decode_common(const b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* act_bf16,
-                         int phases, int write_tables, void* ws, long long ws_bytes, void* stream) {
+                         int phases, int write_tables, void* ws, long long ws_bytes, bool chained, void* stream) {
   if (!L || !ids || !wts || !ws) return B200MOE_ERR_ARG;
   if (!L->q1) return B200MOE_ERR_ARG;   // the mma.sync kernel reads the checkpoint layout, which the caller released
   if ((phases & 1) && !x) return B200MOE_ERR_ARG;
@@ -277,11 +277,12 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   if (ws_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;
   if (((uintptr_t)ws & 255) || ((uintptr_t)x & 15)) return B200MOE_ERR_ARG;
   if (M == 0) return B200MOE_OK;
-  if (2 * L->sms > 512) return B200MOE_ERR_DEVICE;   // share tables of the kernel hold 512 workers
+  if (3 * L->sms > 512) return B200MOE_ERR_DEVICE;   // share tables of the kernel hold 512 workers
   uint8_t* w = (uint8_t*)ws;
   DecodeParams p;
   memset(&p, 0, sizeof(p));
   p.tm1 = L->tm1, p.tm2 = L->tm2;
+  p.w1t = L->w1t, p.w2t = L->w2t;
   p.s1 = (const uint8_t*)L->s1, p.s2 = (const uint8_t*)L->s2;
   p.alpha1 = L->alpha1, p.alpha2 = L->alpha2;
   p.x = (const __nv_bfloat16*)x, p.ids = ids, p.wts = wts, p.out = (__nv_bfloat16*)out;
@@ -308,14 +309,16 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   const int nb8 = M <= 8 ? 1 : 2;
   const int slab = nb8 * 4096;
   const int limit = 227 * 1024;
-  int NS = 8;
-  for (; NS >= 2; NS -= 2) {
+  p.slot_bytes = b200_decode_slot_bytes(p.w1t != nullptr);
+  const int groups = b200_decode_groups(M);
+  int NS = 9 / groups * groups;
+  for (; NS >= groups; NS -= groups) {
     const int region = (L->KB1 * slab > NS * slab) ? L->KB1 * slab : NS * slab;
-    if (b200_decode_smem_bytes(NS, region) <= limit) { p.region_bytes = region; break; }
+    if (b200_decode_smem_bytes(NS, p.slot_bytes, region) <= limit) { p.region_bytes = region; break; }
   }
-  if (NS < 2) return B200MOE_ERR_SHAPE;
+  if (NS < groups) return B200MOE_ERR_SHAPE;
   p.NS = NS;
-  return b200_decode_launch(p, L->sms, b200_decode_smem_bytes(NS, p.region_bytes), (cudaStream_t)stream);
+  return b200_decode_launch(p, L->sms, b200_decode_smem_bytes(NS, p.slot_bytes, p.region_bytes), chained, (cudaStream_t)stream);
 }
 
 // The whole decode layer: out[M, H] (bf16) = sum_j w[t,j] * FC2_e(silu(gate) * up), e = ids[t,j]. M <= 16.
@@ -331,7 +334,7 @@ extern "C" int b200moe_decode_forward_ex(const b200moe_layer* L, const void* x_b
     if (M == 0) return B200MOE_OK;
     return decode_tc(const_cast<b200moe_layer*>(L), x_bf16, topk_ids, topk_weights, M, out_bf16, workspace, !(flags & 1), nullptr, stream);
   }
-  return decode_common(L, x_bf16, topk_ids, topk_weights, M, out_bf16, nullptr, 3, 1, workspace, workspace_bytes, stream);
+  return decode_common(L, x_bf16, topk_ids, topk_weights, M, out_bf16, nullptr, 3, 1, workspace, workspace_bytes, !(flags & 1), stream);
 }
 
 extern "C" int b200moe_decode_forward(const b200moe_layer* L, const void* x_bf16, const int* topk_ids, const float* topk_weights,
@@ -395,7 +398,7 @@ extern "C" int b200moe_decode_forward_host(const b200moe_layer* L, const void* x
 extern "C" int b200moe_decode_fc1(const b200moe_layer* L, const void* x_bf16, const int* topk_ids, const float* topk_weights, int M,
                                   void* act_bf16, void* workspace, long long workspace_bytes, void* stream) {
   if (!act_bf16) return B200MOE_ERR_ARG;
-  return decode_common(L, x_bf16, topk_ids, topk_weights, M, nullptr, act_bf16, 1, 1, workspace, workspace_bytes, stream);
+  return decode_common(L, x_bf16, topk_ids, topk_weights, M, nullptr, act_bf16, 1, 1, workspace, workspace_bytes, false, stream);
 }
 
 // FC2 alone (sm120fp4/kernels/fc2_w4a16.py:276-279, fc2_mma_pf.py:403-421): consumes act[M*top_k, I] bf16.
@@ -407,14 +410,14 @@ extern "C" int b200moe_decode_fc2(const b200moe_layer* L, const void* act_bf16, 
   if (workspace_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;
   if (M == 0) return B200MOE_OK;
   // routing tables first (phase mask 0 runs only the prologue), then the fragment-ordered copy of the activations
-  int rc = decode_common(L, nullptr, topk_ids, topk_weights, M, nullptr, nullptr, 0, 1, workspace, workspace_bytes, stream);
+  int rc = decode_common(L, nullptr, topk_ids, topk_weights, M, nullptr, nullptr, 0, 1, workspace, workspace_bytes, false, stream);
   if (rc != B200MOE_OK) return rc;
   uint8_t* w = (uint8_t*)workspace;
   const int umax = L->E < M * L->top_k ? L->E : M * L->top_k;
   rc = b200_act_to_frag_launch(act_bf16, topk_ids, (const int*)(w + L->off_tables), umax, M, L->top_k, L->I, L->KB2,
                                w + L->off_actfrag, (cudaStream_t)stream);
   if (rc != B200MOE_OK) return rc;
-  return decode_common(L, nullptr, topk_ids, topk_weights, M, out_bf16, nullptr, 2, 0, workspace, workspace_bytes, stream);
+  return decode_common(L, nullptr, topk_ids, topk_weights, M, out_bf16, nullptr, 2, 0, workspace, workspace_bytes, false, stream);
 }
 
 // Copy out the routing tables the last decode call wrote: experts [Umax], offsets [Umax+1], pairs [M*top_k] (device to

@@ -4,11 +4,12 @@
 // (FP4 code x E4M3 block scale, fp32 accumulation, alpha applied in fp32, __expf SiLU, one rounding of the output).
 //
 // Structure (B200-first, memory-bound):
-//  * one CTA per SM; warps 0-3 and 4-7 are two consumer groups ("workers"), warps 8 and 9 their TMA producers.
-//  * the work is a flat list of weight tiles: FC1 tile = 64 up rows + 64 gate rows x 256 K-codes (two 8 KB TMA boxes,
-//    128B swizzle) + their 128x4 scale runs; FC2 tile = 128 output rows x 256 K-codes + scale run + the activation slab
-//    of that expert / K-box. Every worker owns a contiguous, equal share of the flat list (stream-K), so any number of
-//    touched experts balances over the 2 x #SM workers.
+//  * one CTA per SM; three (above 8 tokens two) consumer groups of four warps are its "workers", each with a TMA producer warp.
+//  * the work is a flat list of weight tiles: FC1 tile = 64 up rows + 64 gate rows x 256 K-codes + their scales; FC2 tile = 128
+//    output rows x 256 K-codes + their scales + the activation slab of that expert / K-box. Where the layer has been prepacked a
+//    tile is one 18 KB record (one bulk copy; two layers of 4096 x 1536 at 8 tokens, two groups: 254 us, together with the overlapped
+//    launch, against 269), else boxes and scale runs of the checkpoint layout (three to four copies). Every worker owns a contiguous, equal share of the flat list (stream-K), so any number of
+//    touched experts balances over the workers.
 //  * tiles land in a ring of shared-memory stages guarded by full/empty mbarriers; the producer runs ahead of the math by
 //    the ring depth and, across the FC1->FC2 dependency, prefetches FC2 weight tiles before the grid-wide barrier opens.
 //  * math: codes -> f16 with cvt.rn.f16x2.e2m1x2, times the E4M3 scale (exact in f16), mma.sync m16n8k16 f16 with fp32
@@ -22,13 +23,19 @@
 
 namespace b200 {
 
-constexpr int kConsumerWarps = 8;
 constexpr int kGroupThreads = 128;
-constexpr int kThreads = (kConsumerWarps + 2) * 32;   // + one TMA producer warp per consumer group
-constexpr int kSlotBytes = 20480;      // 16 KB codes + 4 KB scales
+// Consumer groups of a CTA, each a worker with a producer warp of its own. A worker's chain - wait for a tile, its math, the end of a
+// piece - is serial, so more of them keep the pipes busy: two layers of 8 tokens at 4096 x 1536 take 234 us with three groups, 254 with
+// two and 253 with four (whose pieces are smaller: one token 78 against 72). Above 8 tokens the x operand leaves four ring stages at
+// that size, which two groups can share. (Eight warps a tile, each with half of its K codes: 257.)
+constexpr int kMostGroups = 3;
+constexpr int decode_groups(int nb8) { return nb8 == 1 ? 3 : 2; }
+constexpr int decode_threads(int groups) { return groups * (kGroupThreads + 32); }
 constexpr int kCodesBytes = 16384;
+constexpr int kRecordBytes = kCodesBytes + 2048;     // a tile record: codes and four scale tiles
+constexpr int kCheckpointSlot = kCodesBytes + 4096;  // from the checkpoint layout FC1 needs the scale runs of its up and of its gate rows
 constexpr int kMaxE = 256, kMaxP = 256;
-constexpr int kMaxWorkers = 512;       // 2 x SM count
+constexpr int kMaxWorkers = 512;       // up to three per SM
 
 enum { ST_OK = 0, ST_TIMEOUT_FULL = 1, ST_TIMEOUT_EMPTY = 2, ST_TIMEOUT_GRID = 3, ST_BAD_ID = 4 };
 
@@ -45,9 +52,9 @@ struct Tables {
   int U;
   unsigned gen0;       // grid-barrier generation at kernel start
   volatile int abort_flag;
-  int last_flag[2];
-  uint64_t full[8];
-  uint64_t empty[8];
+  int last_flag[kMostGroups];
+  uint64_t full[9];
+  uint64_t empty[9];
 };
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }
@@ -158,17 +165,19 @@ __device__ __forceinline__ void reduce_pieces(const float* __restrict__ scratch,
 }
 
 template <int NB8>
-__global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constant__ DecodeParams P) {
+__global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_decode(const __grid_constant__ DecodeParams P) {
+  constexpr int kGroups = decode_groups(NB8), kConsumerWarps = 4 * kGroups, kThreads = decode_threads(kGroups);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int NS = P.NS;                          // ring stages (even); worker g uses slots 2*i+g
+  const int NS = P.NS;                          // ring stages, a multiple of the groups; worker g uses slots kGroups*i+g
   uint8_t* ring = smem;
-  uint8_t* region = smem + NS * kSlotBytes;     // FC1: x in fragment order (f16); FC2: activation slabs per ring slot
+  const int slot_bytes = P.slot_bytes;
+  uint8_t* region = smem + NS * slot_bytes;     // FC1: x in fragment order (f16); FC2: activation slabs per ring slot
   Tables& T = *reinterpret_cast<Tables*>(region + P.region_bytes);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int npairs = P.M * P.top_k;
-  const int V = 2 * gridDim.x;
+  const int V = kGroups * gridDim.x;
 
   // ---------------------------------------------------------------- prologue: barriers + routing tables (every CTA)
   if (tid == 0) {
@@ -177,12 +186,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
       mbar_init(&T.empty[s], 4);
     }
     T.abort_flag = 0;
-    T.last_flag[0] = T.last_flag[1] = 0;
-    // read before any group of this CTA can arrive, so the generation cannot have advanced yet
-    T.gen0 = ld_acquire_gpu(P.gridbar + 1);
+    for (int g = 0; g < kGroups; ++g) T.last_flag[g] = 0;
     fence_mbar_init();
   }
   if (tid < kMaxE) T.cnt[tid] = 0;
+  grid_dependency_wait();   // launched programmatically: no data is touched before all that stands ahead in the stream is complete
+  if (tid == 0) T.gen0 = ld_acquire_gpu(P.gridbar + 1);   // before any group of this CTA can arrive, so the generation cannot have advanced yet
   __syncthreads();
   for (int p = tid; p < npairs; p += kThreads) {
     int e = P.ids[p];   // a negative id marks an empty slot (expert-parallel shards mask the experts they do not own)
@@ -260,17 +269,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
   }
 
   const int slab_bytes = NB8 * 4096;
-  const int per = NS / 2;
+  const int per = NS / kGroups;
+  const bool records = P.w1t != nullptr;
 #ifdef B200_TIMERS
   long long tm_wait = 0, tm_mma = 0, tm_fix = 0, tm_pwait = 0, tm_pgrid = 0;
   const long long tm_begin = clock64();
 #endif
 
   if (warp >= kConsumerWarps) {
-    // ============================================================== producers: warp 8 feeds group 0, warp 9 group 1
+    // ============================================================== producers: one warp per group
     if (lane == 0) {
       const int grp = warp - kConsumerWarps;
-      const int v = 2 * blockIdx.x + grp;
+      const int v = kGroups * blockIdx.x + grp;
       prefetch_tensormap(&P.tm1);
       prefetch_tensormap(&P.tm2);
       const uint64_t pol = policy_evict_first();
@@ -295,13 +305,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
           bulk_load(region + pend_slot[i] * slab_bytes, pend_src[i], slab_bytes, &T.full[pend_slot[i]]);
         npend = 0;
         passed = true;
+        // The next kernel of the stream may be scheduled as this one's blocks leave: it waits for this grid's completion. Not
+        // earlier: every worker has arrived by now, so a next call on this workspace reads a generation that stays.
+        grid_launch_dependents();
         TIMER_ADD(tm_pgrid, t0);
       };
       int si = 0;           // ring position of this group (0..per-1)
       uint32_t ph = 0;      // parity of the current pass over the ring
       int j = 0;            // tiles issued
       auto claim_slot = [&](bool prev_was_fc2_pending) -> int {
-        const int slot = 2 * si + grp;
+        const int slot = kGroups * si + grp;
         if (j >= per) {
           if (prev_was_fc2_pending) wait_grid();   // the previous occupant still waits for its activations: open the gate first
           TIMER_START(t0);
@@ -320,8 +333,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
         int kb = f0 % KB1, q = f0 / KB1, cb = q % CB1, u = q / CB1;
         for (int i = 0; i < n1; ++i) {
           const int slot = claim_slot(false);
-          uint8_t* st = ring + slot * kSlotBytes;
+          uint8_t* st = ring + slot * slot_bytes;
           const int e = T.experts[u];
+          if (records) {
+            mbar_expect_tx(&T.full[slot], kRecordBytes);
+            bulk_load_hint(st, P.w1t + (((long long)e * CB1 + cb) * KB1 + kb) * kRecordBytes, kRecordBytes, &T.full[slot], pol);
+            advance();
+            if (++kb == KB1) { kb = 0; if (++cb == CB1) { cb = 0; ++u; } }
+            continue;
+          }
           const int nkt = min(4, P.KT1 - 4 * kb);
           const int up_row = 64 * cb, gate_row = P.I + 64 * cb;
           mbar_expect_tx(&T.full[slot], kCodesBytes + 2 * nkt * 512);
@@ -340,13 +360,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
         int kb = f0 % KB2, q = f0 / KB2, u = q % U, nb = q / U;
         for (int i = 0; i < n2; ++i) {
           const int slot = claim_slot(!passed && (j - per) >= n1);
-          uint8_t* st = ring + slot * kSlotBytes;
+          uint8_t* st = ring + slot * slot_bytes;
           const int e = T.experts[u];
-          const int nkt = min(4, P.KT2 - 4 * kb);
-          mbar_expect_tx(&T.full[slot], kCodesBytes + nkt * 512 + slab_bytes);
-          tma_load_2d_hint(st, &P.tm2, 128 * kb, e * P.H + 128 * nb, &T.full[slot], pol);
-          bulk_load_hint(st + kCodesBytes, P.s2 + (long long)e * P.s2_expert_stride + ((long long)nb * P.KT2 + 4 * kb) * 512,
-                         nkt * 512, &T.full[slot], pol);
+          if (records) {
+            mbar_expect_tx(&T.full[slot], kRecordBytes + slab_bytes);
+            bulk_load_hint(st, P.w2t + (((long long)e * NB2 + nb) * KB2 + kb) * kRecordBytes, kRecordBytes, &T.full[slot], pol);
+          } else {
+            const int nkt = min(4, P.KT2 - 4 * kb);
+            mbar_expect_tx(&T.full[slot], kCodesBytes + nkt * 512 + slab_bytes);
+            tma_load_2d_hint(st, &P.tm2, 128 * kb, e * P.H + 128 * nb, &T.full[slot], pol);
+            bulk_load_hint(st + kCodesBytes, P.s2 + (long long)e * P.s2_expert_stride + ((long long)nb * P.KT2 + 4 * kb) * 512,
+                           nkt * 512, &T.full[slot], pol);
+          }
           const uint8_t* src = reinterpret_cast<const uint8_t*>(P.actfrag) + ((long long)u * KB2 + kb) * slab_bytes;
           if (passed) bulk_load(region + slot * slab_bytes, src, slab_bytes, &T.full[slot]);
           else { pend_slot[npend] = slot; pend_src[npend] = src; ++npend; }
@@ -361,9 +386,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
     }
     __syncwarp();
   } else {
-    // ============================================================== consumers: two groups of four warps
+    // ============================================================== consumers: groups of four warps
     const int grp = warp >> 2, w = warp & 3;
-    const int v = 2 * blockIdx.x + grp;
+    const int v = kGroups * blockIdx.x + grp;
     const int gtid = tid & (kGroupThreads - 1);
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring_a = smem_u32(ring), region_a = smem_u32(region);
@@ -390,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
         }
         *reinterpret_cast<uint4*>(region + frag_index<NB8>(k, tok) * 2) = outv;
       }
-      named_bar_sync(3, kConsumerWarps * 32);
+      named_bar_sync(1 + kMostGroups, kConsumerWarps * 32);
 
       // ---- FC1 pieces of this worker
       const int fs = T.sb1[v], fe = T.sb1[v + 1];
@@ -408,16 +433,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
             for (int n = 0; n < NB8; ++n)
 #pragma unroll
               for (int i = 0; i < 4; ++i) acc[pa][a][n][i] = 0.f;
-        const int rt_up = ((64 * cb) & 127) + 16 * w, rt_gate = ((P.I + 64 * cb) & 127) + 16 * w;
+        // scale rows of this warp's up and gate rows: inside the record's tiles, or inside the two 128-row runs of the checkpoint layout
+        const int rt_up = (records ? 0 : (64 * cb) & 127) + 16 * w, rt_gate = (records ? 64 : (P.I + 64 * cb) & 127) + 16 * w;
+        const int gate_scales = kCodesBytes + (records ? 0 : 2048);
         const unsigned octets = NB8 == 1 ? 1u : T.omask[u];
         for (int kb = k0; kb < k1; ++kb) {
-          const int slot = 2 * si + grp;
+          const int slot = kGroups * si + grp;
           TIMER_START(t0);
           if (!mbar_wait(&T.full[slot], ph, &T.abort_flag)) *P.status = ST_TIMEOUT_FULL;
           TIMER_ADD(tm_wait, t0);
           TIMER_START(t1);
-          const uint32_t st = ring_a + slot * kSlotBytes;
-          mma_tile<NB8>(st, 16 * w, 64 + 16 * w, st + kCodesBytes, rt_up, st + kCodesBytes + 2048, rt_gate,
+          const uint32_t st = ring_a + slot * slot_bytes;
+          mma_tile<NB8>(st, 16 * w, 64 + 16 * w, st + kCodesBytes, rt_up, st + gate_scales, rt_gate,
                         4 * kb + t < P.KT1, region_a + kb * (NB8 * 4096), lane, octets, acc);
           __syncwarp();
           if (lane == 0) mbar_arrive(&T.empty[slot]);
@@ -538,12 +565,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_moe_decode(const __grid_constan
           f += k1 - kb;
           const unsigned octets = NB8 == 1 ? 1u : T.omask[u];
           for (; kb < k1; ++kb) {
-            const int slot = 2 * si + grp;
+            const int slot = kGroups * si + grp;
             TIMER_START(t0);
             if (!mbar_wait(&T.full[slot], ph, &T.abort_flag)) *P.status = ST_TIMEOUT_FULL;
             TIMER_ADD(tm_wait, t0);
             TIMER_START(t1);
-            const uint32_t st = ring_a + slot * kSlotBytes;
+            const uint32_t st = ring_a + slot * slot_bytes;
             mma_tile<NB8>(st, 32 * w, 32 * w + 16, st + kCodesBytes, 32 * w, st + kCodesBytes, 32 * w + 16,
                           4 * kb + t < P.KT2, region_a + slot * slab_bytes, lane, octets, acc);
             __syncwarp();
@@ -650,11 +677,16 @@ __global__ void __launch_bounds__(256) k_act_to_frag(const __nv_bfloat16* __rest
 
 using namespace b200;
 
-int b200_decode_smem_bytes(int NS, int region_bytes) { return 1024 + NS * kSlotBytes + region_bytes + (int)sizeof(Tables); }
+int b200_decode_groups(int M) { return decode_groups(M <= 8 ? 1 : 2); }
 
-int b200_decode_launch(const DecodeParams& p, int grid, int smem_bytes, cudaStream_t st) {
+int b200_decode_slot_bytes(bool records) { return records ? kRecordBytes : kCheckpointSlot; }
+
+int b200_decode_smem_bytes(int NS, int slot_bytes, int region_bytes) { return 1024 + NS * slot_bytes + region_bytes + (int)sizeof(Tables); }
+
+int b200_decode_launch(const DecodeParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st) {
   void* args[] = {(void*)&p};
   const void* fn = p.M <= 8 ? (const void*)k_moe_decode<1> : (const void*)k_moe_decode<2>;
+  const int threads = decode_threads(decode_groups(p.M <= 8 ? 1 : 2));
   static thread_local int configured[2] = {0, 0};
   const int which = p.M <= 8 ? 0 : 1;
   if (configured[which] < smem_bytes) {
@@ -665,11 +697,10 @@ int b200_decode_launch(const DecodeParams& p, int grid, int smem_bytes, cudaStre
   // grid-wide barrier inside the kernel can complete; its waits are bounded either way. A cooperative launch makes
   // co-residency a launch-time guarantee at the price of a few microseconds between back-to-back launches.
   if (p.cooperative) {
-    B200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, (size_t)smem_bytes, st));
-  } else {
-    B200_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, (size_t)smem_bytes, st));
+    B200_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, (size_t)smem_bytes, st));
+    return B200MOE_OK;
   }
-  return B200MOE_OK;
+  return launch_kernel(fn, grid, threads, smem_bytes, chained, args, st);
 }
 
 int b200_act_to_frag_launch(const void* act, const int* ids, const int* experts, int Umax, int M, int top_k, int I, int KB2,

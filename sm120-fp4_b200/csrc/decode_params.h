@@ -12,6 +12,8 @@ struct DecodeParams {
   CUtensorMap tm2;   // FC2 codes viewed u8 [E*H rows, I/2 bytes], box 128 B x 128 rows, 128B swizzle
   const uint8_t* s1;  // FC1 block scales, 128x4 swizzle per expert
   const uint8_t* s2;  // FC2 block scales, 128x4 swizzle per expert
+  const uint8_t* w1t; // the tile records of k_pack_tiles (as in DecodeTcParams), or null: the kernel then reads the checkpoint layout above
+  const uint8_t* w2t;
   const float* alpha1;
   const float* alpha2;
   const __nv_bfloat16* x;   // [M, H]
@@ -33,7 +35,7 @@ struct DecodeParams {
   int M, E, H, I, top_k, Umax;
   int phases;               // bit 0: FC1, bit 1: FC2
   int cooperative;          // launch with cudaLaunchCooperativeKernel
-  int NS;                   // ring stages (even)
+  int NS, slot_bytes;       // ring stages (a multiple of the kernel's groups) and their size
   int region_bytes;         // shared-memory region for x fragments / activation slabs
   int KB1, KB2;             // 256-code K boxes of FC1 (over H) and FC2 (over I)
   int CB1, NB2;             // 64-column blocks of FC1, 128-row blocks of FC2
@@ -83,7 +85,9 @@ inline bool b200_decode_self_expand(int M, int H) { return M <= 8 && M * H <= 16
 int b200_pack_tiles_launch(const void* q, const void* sf, void* out, int E, int rows_per_expert, int row_bytes, int blocks, int KB, int KT,
                            int fc1, int I, long long sf_stride, cudaStream_t st);
 int b200_decode_tc_launch(const b200::DecodeTcParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);
-int b200_decode_smem_bytes(int NS, int region_bytes);
-int b200_decode_launch(const b200::DecodeParams& p, int grid, int smem_bytes, cudaStream_t st);
+int b200_decode_groups(int M);   // consumer groups of a block, which its ring stages are dealt to
+int b200_decode_slot_bytes(bool records);
+int b200_decode_smem_bytes(int NS, int slot_bytes, int region_bytes);
+int b200_decode_launch(const b200::DecodeParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);
 int b200_act_to_frag_launch(const void* act, const int* ids, const int* experts, int Umax, int M, int top_k, int I, int KB2,
                             void* actfrag, cudaStream_t st);

@@ -66,3 +66,55 @@ def test_nan_values_do_not_set_the_row_scale(m, which):
     at = decode_map(w)["xscale"]
     got = w.workspace[at:at + 4].view(torch.float32).cpu().numpy()[0]
     assert got == np.float32(1) / (np.float32(2688) / amax)
+
+
+# The mma.sync kernel on a layer that has not been prepacked reads the checkpoint layout instead of the tile records: the same tiles in
+# the same order, so the same bits. Three groups of workers up to 8 tokens, two above; intermediate sizes with a whole and a part
+# 128-row scale run and K box.
+@pytest.mark.parametrize("hidden,inter", [(256, 64), (640, 192), (3200, 192), (4096, 320)])
+def test_tile_records_and_checkpoint_layout_agree(hidden, inter):
+    import ctypes as C
+    from sm120fp4_b200 import _lib
+    cfg, w, _ = edge_layer(hidden, inter)
+    h, bare = _lib.lib(), C.c_void_p()
+    _lib.check(h.b200moe_layer_create(C.byref(bare), w.E, w.H, w.I, w.k, _lib.ptr(w.q1), _lib.ptr(w.s1), _lib.ptr(w.alpha1), _lib.ptr(w.q2),
+                                      _lib.ptr(w.s2), _lib.ptr(w.alpha2)), "create")
+    ws = torch.zeros_like(w.workspace)
+    w.set_decode_impl("mma")
+    try:
+        for m in (1, 8, 9, 16):
+            x, ids, wts = (t.cuda() for t in inputs(cfg, m, 50 + m))
+            out = torch.empty_like(x)
+            _lib.check(h.b200moe_decode_forward(bare, _lib.ptr(x), _lib.ptr(ids), _lib.ptr(wts), m, _lib.ptr(out), _lib.ptr(ws), ws.numel(),
+                                                _lib.stream_ptr()), "decode")
+            assert torch.equal(out, w.forward(x, ids, wts)), m
+        w.status()
+    finally:
+        w.set_decode_impl("auto")
+        torch.cuda.synchronize()
+        h.b200moe_layer_destroy(bare)
+
+
+# Calls of a wide layer overlap their launches: a chain of them, each on the output of the one before, gives what the calls give one by one.
+def test_chained_wide_calls():
+    cfg, w, _ = edge_layer(3200)
+    for m in (2, 9):
+        x, ids, wts = (t.cuda() for t in inputs(cfg, m, 60 + m))
+        want = []
+        y = x
+        for _ in range(6):
+            y = w.forward(y, ids, wts)
+            torch.cuda.synchronize()
+            want.append(y.clone())
+            y = (y.float() / y.float().abs().amax()).to(torch.bfloat16)
+        ys = [x]
+        outs = []
+        for _ in range(6):
+            outs.append(w.forward(ys[-1], ids, wts))
+            ys.append((outs[-1].float() / outs[-1].float().abs().amax()).to(torch.bfloat16))
+        for _ in range(20):
+            back_to_back = [w.forward(v, ids, wts) for v in ys[:6]]
+        torch.cuda.synchronize()
+        for a, b, c in zip(want, outs, back_to_back):
+            assert torch.equal(a, b) and torch.equal(a, c)
+    w.status()
