@@ -306,6 +306,11 @@ static int launch_gemm(GroupedParams p, int phase, int sms, cudaStream_t st) {
   return launch_kernel(fn, sms, kGgThreads, kGgSmem, true, args, st);
 }
 
+// whether both projections' tile records together are more than L2 holds (126 MB)
+static bool gg_stream_weights(int E, int H, int I) {
+  return (long long)E * ((long long)(I / 64) * ((H + 255) / 256) + (long long)(H / 128) * ((I + 255) / 256)) * kRec > (126LL << 20);
+}
+
 // w1t / w2t: the weight tile records of b200moe_layer_prepack. gs_x / gs_a: global scales of the two activation quantisations.
 // Launches: plan -> token-major quantiser -> FC1 GEMM -> FC2 GEMM -> combine.
 int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const uint8_t* w2t, const float* alpha1, const float* alpha2,
@@ -344,6 +349,7 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   GroupedParams p;
   memset(&p, 0, sizeof(p));
   p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = status, p.H = H;
+  p.stream = gg_stream_weights(E, H, I);
   // FC1
   p.arec = w + L.xrec, p.wrec = w1t, p.alpha = alpha1, p.gs_in = gs_x, p.gs_out = gs_a, p.orec = w + L.arec;
   p.NBLK = I / 64, p.KB = KB1, p.KT = KT1, p.KB2 = KB2;
@@ -438,6 +444,7 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   GroupedParams p;
   memset(&p, 0, sizeof(p));
   p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = (int*)(w + L.status), p.H = H;
+  p.stream = gg_stream_weights(E, H, I);
   p.rowscale = rowscale, p.act_g1 = act_g1;
   // FC1
   p.arec = w + L.xrec, p.wrec = w1t, p.alpha = alpha1, p.orec = w + L.arec;
