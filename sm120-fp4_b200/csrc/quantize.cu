@@ -355,6 +355,211 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
   if (tid == 0 && atomicAdd(scratch + 1, 1u) == gridDim.x - 1u) { scratch[1] = 0u; scratch[0] = call; }
 }
 
+// The same for bf16 groups of which the shared memory of all SMs holds more than one (one block per SM, 32 KB units taken round-robin): a
+// unit is copied into shared memory once, its maximum is published, and it is quantised from there one unit of its worker later,
+// when the maxima of its group have normally all been published. A block is three workers of eight warps, a copying warp and one that
+// looks for the maxima. The kernel above reads every value twice into registers and is held up by latency with the 16 warps an SM that
+// its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 190 instructions per 16 values (66 %
+// busy). 128 x 1536 x 2048 bf16: 216 us, 243 above; with two workers 245. (fp32 has half the arithmetic per byte, and its 64-byte blocks
+// meet a quarter of the banks: 60 x 1024 x 1536 take 96 us either way, or 115 here without instructions that avoid the conflicts.)
+constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
+constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
+constexpr int kQcLooks = 8;        // maxima that may wait for their worker
+constexpr int kQcBlocks = kQcUnit / 32;   // 16-value blocks of a unit
+struct QcShared {
+  uint64_t full[kQcSlots], empty[kQcSlots], known[kQcLooks], taken[kQcLooks];
+  unsigned gmax[kQcLooks];
+  float table[kQcWorkers][128];
+  unsigned wm[kQcWorkers][2][8], late[kQcWorkers][8];
+  int abort_flag;
+};
+constexpr int kQcSmem = kQcSlots * kQcUnit + (int)sizeof(QcShared) + 128;
+
+// 16 values of a thread from shared memory. (Neighbouring threads' blocks are 32 bytes apart, so eight of them share half of the banks:
+// that time is there. Reading the halves in turn and putting them in order takes as long.)
+__device__ __forceinline__ void load_shared(uint32_t at, Raw16<__nv_bfloat16>& v) { v.r[0] = lds128(at), v.r[1] = lds128(at + 16); }
+
+__global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_bfloat16* x, int groups, int units, QuantGeom q, float* gs_out, uint8_t* packed, uint8_t* sf,
+                                                                     unsigned* scratch, int polls) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+  QcShared& S = *reinterpret_cast<QcShared*>(smem + kQcSlots * kQcUnit);
+  constexpr int kUnitBlocks = kQcBlocks, kPer = kUnitBlocks / kQcWorkerThreads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int nblk = q.rows * q.bpr;             // 16-value blocks of a group
+  const unsigned total = (unsigned)groups * (unsigned)units, G = gridDim.x;
+  const int n = (int)((total - blockIdx.x + G - 1u) / G);   // this block's units: places blockIdx.x + k * G in the order (group, unit)
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(scratch + 2);
+  if (tid == 0) {
+    for (int s = 0; s < kQcSlots; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 8); }
+    for (int s = 0; s < kQcLooks; ++s) { mbar_init(&S.known[s], 1); mbar_init(&S.taken[s], 1); }
+    S.abort_flag = 0;
+    fence_mbar_init();
+  }
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const unsigned call = __ldcg(scratch) + 1u;   // nobody advances it before every block of this call has left
+  __syncthreads();
+  constexpr unsigned kMissing = ~0u;            // above the bits of every magnitude
+  auto place = [&](int k) { const unsigned p = blockIdx.x + (unsigned)k * G; return make_int2((int)(p / (unsigned)units), (int)(p % (unsigned)units)); };
+  if (warp == 8 * kQcWorkers) {
+    // ============================================================== copies
+    if (lane == 0) {
+      const uint64_t once = policy_evict_first();
+      int slot = 0;
+      uint32_t ph = 1;   // parity that a free slot's barrier has completed: the first pass finds all slots free
+      for (int k = 0; k < n; ++k) {
+        const int2 at = place(k);
+        const int i0 = at.y * kUnitBlocks, bytes = min(kUnitBlocks, nblk - i0) * 32;
+        mbar_wait(&S.empty[slot], ph, &S.abort_flag);
+        mbar_expect_tx(&S.full[slot], bytes);
+        bulk_load_hint(smem + slot * kQcUnit, x + ((long long)at.x * nblk + i0) * 16, bytes, &S.full[slot], once);
+        if (++slot == kQcSlots) { slot = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 8 * kQcWorkers + 1) {
+    // ============================================================== the maximum of each unit's group, looked at `polls` times
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+      const unsigned long long* gw = words + (long long)place(k).x * units;
+      unsigned m = 0u;
+      bool ok = false;
+      int looks = polls;
+#pragma unroll 1
+      for (;;) {
+        m = 0u, ok = looks > 0;
+#pragma unroll 4
+        for (int w = lane; w < units; w += 32) {
+          const unsigned long long word = ld_relaxed_gpu_u64(gw + w);
+          ok &= (unsigned)(word >> 32) == call;
+          m = max(m, (unsigned)word);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok || looks <= 0) break;
+        --looks;
+        __nanosleep(50);
+      }
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (k >= kQcLooks) mbar_wait_warp(smem_u32(&S.taken[k % kQcLooks]), (uint32_t)((k / kQcLooks - 1) & 1), &S.abort_flag);
+      if (lane == 0) {
+        S.gmax[k % kQcLooks] = ok ? m : kMissing;
+        mbar_arrive(&S.known[k % kQcLooks]);
+      }
+      __syncwarp();
+    }
+  } else {
+    // ============================================================== workers: unit k belongs to worker k % kQcWorkers
+    const int grp = warp >> 3, wt = tid & (kQcWorkerThreads - 1), ww = wt >> 5;
+    auto sync = [&]() { named_bar_sync(1 + grp, kQcWorkerThreads); };
+    const uint64_t once = policy_evict_first();
+    const uint32_t ring = smem_u32(smem);
+    float gs_table = -1.f;
+    // The maximum of group g by this worker alone, for units whose blocks have not run for a long time (another kernel holds their
+    // SMs: nothing says that the grid is resident as a whole). What it finds out it publishes, so that others need not.
+    auto group_max = [&](int g) {
+      unsigned all = 0u;
+#pragma unroll 1
+      for (int w = 0; w < units; ++w) {
+        unsigned long long* at = words + (long long)g * units + w;
+        const unsigned long long word = ld_relaxed_gpu_u64(at);
+        const bool there = (unsigned)(word >> 32) == call;   // (threads may see it differently: they agree below)
+        float m = 0.f;
+        const int i1 = min(nblk, (w + 1) * kUnitBlocks);
+        if (!there) {
+#pragma unroll 1
+          for (int i = w * kUnitBlocks + wt; i < i1; i += kQcWorkerThreads) {
+            Raw16<__nv_bfloat16> raw;
+            load_raw(x + ((long long)g * nblk + i) * 16, q.wide, false, raw);
+            m = fmaxf(m, amax_raw(raw));
+          }
+        }
+        unsigned mb = there ? (unsigned)word : __float_as_uint(m);   // the larger of a published maximum and a part of it is the maximum
+        mb = __reduce_max_sync(0xffffffffu, mb);
+        if (lane == 0) S.late[grp][ww] = mb;
+        sync();
+        mb = __reduce_max_sync(0xffffffffu, S.late[grp][lane & 7]);
+        sync();
+        if (wt == 0) __stcg(at, ((unsigned long long)call << 32) | mb);
+        all = max(all, mb);
+      }
+      return all;
+    };
+    int buf = 0;
+#pragma unroll 1
+    for (int k = grp; k < n + kQcWorkers; k += kQcWorkers) {
+      if (k < n) {
+        const int2 at = place(k);
+        const int slot = k % kQcSlots, left = nblk - at.y * kUnitBlocks - wt;
+        mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag);
+        float m = 0.f;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          if (j * kQcWorkerThreads < left) {
+            Raw16<__nv_bfloat16> v;
+            load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
+            m = fmaxf(m, amax_raw(v));
+          }
+        }
+        __syncwarp();
+        unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if (lane == 0) S.wm[grp][buf][ww] = mb;
+        sync();
+        if (ww == 0) {
+          mb = __reduce_max_sync(0xffffffffu, S.wm[grp][buf][lane & 7]);
+          if (lane == 0) __stcg(words + (long long)at.x * units + at.y, ((unsigned long long)call << 32) | mb);
+        }
+        buf ^= 1;
+      }
+      const int kq = k - kQcWorkers;
+      if (kq < 0) continue;
+      const int2 at = place(kq);
+      const int g = at.x, u = at.y, slot = kq % kQcSlots, i0 = u * kUnitBlocks, left = nblk - i0 - wt;
+      mbar_wait_warp(smem_u32(&S.known[kq % kQcLooks]), (uint32_t)((kq / kQcLooks) & 1), &S.abort_flag);
+      unsigned m = S.gmax[kq % kQcLooks];
+      if (m == kMissing) m = group_max(g);
+      const float gs = scale_of(__uint_as_float(m));
+      sync();                                     // nobody is at the table any more, and all have the maximum
+      if (wt == 0) mbar_arrive(&S.taken[kq % kQcLooks]);
+      if (gs != gs_table) fill_scale_table(S.table[grp], gs, wt, kQcWorkerThreads);
+      gs_table = gs;
+      sync();
+      uint8_t* sfg = sf + (long long)g * q.sf_stride;
+      uint2* codes = reinterpret_cast<uint2*>(packed) + (long long)g * nblk + i0 + wt;
+      uint8_t* sfl = sfg + i0 + wt;                                    // row-major place
+      int r = 0, c = 0;                                                // 128x4: (row, scale column) of the block
+      if (q.layout == 1) {
+        r = (int)(((unsigned long long)(unsigned)(i0 + wt) * q.bpr_inv) >> q.bpr_shift);
+        c = i0 + wt - r * q.bpr;
+      }
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) {
+        if (j * kQcWorkerThreads < left) {
+          Raw16<__nv_bfloat16> v;
+          load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
+          uint2 pk;
+          const uint32_t sb = quantize_raw(v, gs, S.table[grp], pk);
+          st_policy(codes + j * kQcWorkerThreads, pk, once);
+          if (q.layout == 0) {
+            sfl[j * kQcWorkerThreads] = (uint8_t)sb;
+          } else {
+            sfg[((r >> 7) * q.nkt + (c >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (c & 3)] = (uint8_t)sb;
+            r += q.step_r, c += q.step_c;
+            if (c >= q.bpr) { c -= q.bpr; ++r; }
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.empty[slot]);
+      if (u == 0) {
+        if (wt == 0) gs_out[g] = gs;
+        if (q.layout == 1) zero_padding(sfg, q, wt, kQcWorkerThreads);
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0 && atomicAdd(scratch + 1, 1u) == G - 1u) { scratch[1] = 0u; scratch[0] = call; }
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -363,11 +568,18 @@ extern "C" int b200moe_global_scale(const void* x, int dtype, long long n, void*
 extern "C" int b200moe_quantize_nvfp4(const void* x, int dtype, const int* src_row, int rows, int K, const float* global_scale, int gs_rows, void* packed,
                                       void* sf, int sf_layout, void* stream);
 
+static int quant_resident_units(int dtype, int rows, int K) {
+  return dtype == 0 ? (int)(((long long)rows * (K / 16) + kQcBlocks - 1) / kQcBlocks) : 0;
+}
+
 static int quant_units(int dtype, int rows, int K) {
   const long long nblk = (long long)rows * (K / 16), unit = kQgThreads * (dtype == 0 ? kQPerThread<__nv_bfloat16> : kQPerThread<float>);
   return (int)((nblk + unit - 1) / unit);
 }
 
+// Inputs beyond L2 take the resident form. Below, latency is not what the other form waits for: 8 x 1536 x 2048 bf16 (50 MB) 21.4 us against
+// 25.0, 60 x 384 x 768 15.2 against 17.6; above, 128 x 1024 x 1024 (268 MB) 83.4 against 75.9.
+constexpr long long kQResidentFrom = 126ll << 20;
 constexpr int kQPolls = 2048;   // looks of ~0.7 us: a unit takes 5 to 10 us, so the words are there long before unless the grid is held up
 
 static bool quant_one_cluster(int groups, int rows, int K) { return groups == 1 && (long long)rows * (K / 16) <= kQSmallMaxBlocks; }
@@ -375,7 +587,8 @@ static bool quant_one_cluster(int groups, int rows, int K) { return groups == 1 
 extern "C" long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int rows, int K) {
   if (groups <= 0 || rows < 0 || K <= 0 || (dtype != 0 && dtype != 1)) return B200MOE_ERR_ARG;
   if (quant_one_cluster(groups, rows, K)) return 0;
-  return 8 + 8LL * groups * quant_units(dtype, rows, K);
+  const int a = quant_units(dtype, rows, K), b = quant_resident_units(dtype, rows, K);
+  return 8 + 8LL * groups * (a > b ? a : b);
 }
 
 // Matrices beyond what the one launch can index: amax, scale and codes of one group after the other, in launches of their own.
@@ -444,6 +657,24 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
     B200_CUDA_TRY(cudaGetDevice(&dev));
     B200_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
     sms = n;
+  }
+  if (dtype == 0 && groups * nblk * 32 > kQResidentFrom) {
+    // The resident form where a group's units are at most 2.4 rounds of the grid: its last maximum is then published by the time that
+    // the first unit's worker, three units on, quantises it. (With two more rounds of lag only one slot would be left to fill.)
+    const int ru = quant_resident_units(dtype, rows, K);
+    const long long all = (long long)groups * ru;
+    const int G = (int)(all < sms ? all : sms);
+    if (5LL * ru <= 12LL * G && all < 0x7fffffffLL) {
+      static thread_local unsigned configured = 0;   // bit d: device d has the attribute
+      int dev = 0;
+      B200_CUDA_TRY(cudaGetDevice(&dev));
+      if (dev > 31 || !((configured >> dev) & 1u)) {
+        B200_CUDA_TRY(cudaFuncSetAttribute((const void*)k_quantize_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, kQcSmem));
+        if (dev <= 31) configured |= 1u << dev;
+      }
+      void* args[] = {(void*)&x, (void*)&groups, (void*)&ru, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&polls};
+      return launch_kernel((const void*)k_quantize_resident, G, kQcThreads, kQcSmem, true, args, st);
+    }
   }
   const long long most = 2LL * groups * units;
   const int grid = (int)(most < 2LL * sms ? most : 2LL * sms);

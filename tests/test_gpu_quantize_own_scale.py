@@ -38,6 +38,26 @@ def test_stacked_matrices(groups, rows, k, swizzle):
         assert np.array_equal(sf[g].cpu().numpy(), O.to_128x4(wsf) if swizzle else wsf)
 
 
+# More than 126 MB of bf16 in groups of up to 11 MB stay in shared memory between the passes, in units of 1024 blocks of 16 values: groups
+# of many units with a ragged last one, of one ragged unit, and the largest that the form takes (2.4 rounds of 148 units) beside the
+# first that it does not. The fp32 copy of the same values goes the other way, and its bytes are the same.
+@pytest.mark.parametrize("groups,rows,k", [(65, 1000, 1040), (8400, 500, 16), (13, 2840, 2048), (13, 2848, 2048)])
+def test_large_inputs_on_chip(groups, rows, k):
+    import sm120fp4_b200 as pkg
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = torch.empty(groups, rows, k, dtype=torch.bfloat16, device="cuda").normal_(generator=g)
+    w *= torch.linspace(0.01, 9.0, groups, device="cuda")[:, None, None].to(torch.bfloat16)
+    w[groups // 2] = 0
+    w[1, 0, :16] = float("nan")
+    for swizzle in (False, True):
+        got = pkg.quantize_nvfp4_experts(w, swizzle=swizzle)
+        want = pkg.quantize_nvfp4_experts(w.float(), swizzle=swizzle)
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+        again = pkg.quantize_nvfp4_experts(w, swizzle=swizzle)
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, again))
+
+
 # More than 20 MB in all: the passes of different groups alternate (10 and 5 groups apart here, the last unit of each ragged); a group
 # above 20 MB: its two passes follow one another.
 @pytest.mark.parametrize("dtype,groups,rows,k", [(torch.bfloat16, 16, 1000, 1040), (torch.float32, 12, 1000, 1040), (torch.bfloat16, 2, 6400, 2048)])
@@ -139,7 +159,7 @@ def _randn(rows, k, seed):
 
 @pytest.mark.parametrize("polls", [0, 1])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("groups,rows,k", [(1, 257, 1040), (3, 300, 2048), (40, 192, 512), (6, 1536, 2048)])
+@pytest.mark.parametrize("groups,rows,k", [(1, 257, 1040), (3, 300, 2048), (40, 192, 512), (6, 1536, 2048), (45, 1530, 1040)])
 def test_blocks_that_do_not_wait(groups, rows, k, dtype, polls):
     """A block that gives up waiting for other blocks' maxima works them out itself: the same bytes, twice on one workspace."""
     import sm120fp4_b200 as pkg
@@ -155,11 +175,12 @@ def test_blocks_that_do_not_wait(groups, rows, k, dtype, polls):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
-def test_two_calls_at_once():
+@pytest.mark.parametrize("dtype,groups", [(torch.float32, 24), (torch.bfloat16, 48)])   # (the second stays in shared memory)
+def test_two_calls_at_once(dtype, groups):
     """Two large calls on two streams share the GPU's SMs in whatever way they are scheduled."""
     import sm120fp4_b200 as pkg
     streams = [torch.cuda.Stream() for _ in range(2)]
-    ws = [torch.randn(24, 768, 2048, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda", dtype=torch.float32) for i in range(2)]
+    ws = [torch.randn(groups, 768, 2048, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda", dtype=dtype) for i in range(2)]
     want = [pkg.quantize_nvfp4_experts(w) for w in ws]
     torch.cuda.synchronize()
     got = [[], []]
