@@ -59,6 +59,7 @@ struct GroupedParams {
   float act_g1;               // PHASE 3/4: global scale of the first term of the SiLU*mul activations
   int NBLK, KB, KT, KB2, H;
   int stream;                 // the layer's weights do not fit in L2
+  int wait_tables;            // the kernel before this one writes the tile tables
 };
 
 struct GgShared {
@@ -312,10 +313,21 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   uint8_t* patches = smem + 1024;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // (a value from lane 0 is known to be warp-uniform)
+  // Without wait_tables the tile tables are read without waiting for the kernel before this one: the tables' own producer is at least
+  // two kernels back, and the kernel in between lets this one start only after it has seen that producer complete.
+  int ntiles = P.wait_tables ? 0 : __ldcg(P.ntiles);
+  if (tid == 0) {
+    for (int k = 0; k < 12; ++k) { mbar_init(&S.a_full[k], 1); mbar_init(&S.a_empty[k], 1); }
+    for (int s = 0; s < kGgMaxRing; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], 4); }
+    S.abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 11) { tmem_alloc(&S.tmem_base, 512); tmem_relinquish(); }
+  if (PHASE == 1) fill_scale_table(S.scale, P.gs_out, tid, kGgThreads);
+  if (P.wait_tables) { grid_dependency_wait(); ntiles = __ldcg(P.ntiles); }
   grid_launch_dependents();   // the next kernel of the chain may take over SMs as this one's CTAs leave
-  // The tile tables are read here without waiting for the kernel before this one: the tables' own producer is at least two
-  // kernels back, and the kernel in between lets this one start only after it has seen that producer complete.
-  const int NT = __shfl_sync(0xffffffffu, __ldcg(P.ntiles), 0);
+  const int NT = __shfl_sync(0xffffffffu, ntiles, 0);
   const GgSplit split(NT, NBLK, (int)gridDim.x, (int)blockIdx.x);
   const int nseg = split.nseg;
   auto for_each_segment = [&](auto&& body) {   // body(t, n0, n1, ordinal), one call site: a copy of a role's code per launch is enough
@@ -334,15 +346,6 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
     m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0) S.max_rows = m;
   }
-  if (tid == 0) {
-    for (int k = 0; k < 12; ++k) { mbar_init(&S.a_full[k], 1); mbar_init(&S.a_empty[k], 1); }
-    for (int s = 0; s < kGgMaxRing; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&S.acc_full[b], 1); mbar_init(&S.acc_empty[b], 4); }
-    S.abort_flag = 0;
-    fence_mbar_init();
-  }
-  if (warp == 11) { tmem_alloc(&S.tmem_base, 512); tmem_relinquish(); }
-  if (PHASE == 1) fill_scale_table(S.scale, P.gs_out, tid, kGgThreads);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

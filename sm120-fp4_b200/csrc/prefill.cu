@@ -5,7 +5,7 @@
 //
 // Pipeline (all on the caller's stream, no host synchronisation):
 //   k_plan:             router tables, per-expert row segments padded to 128-row tiles (the tile plan) and the map between
-//                       token-expert pairs and operand rows (plan.cuh)
+//                       token-expert pairs and operand rows (plan.cuh); for up to 1024 pairs part of the kernel after it
 //   k_quantize_scatter: bf16 x -> NVFP4 "tile records" (128 rows x 256 codes in the 128-byte-swizzle shared-memory image
 //                       + four 512 B scale tiles, 18 KB contiguous): every token row quantised once, stored to its pairs' rows
 //   k_grouped_gemm<1>:  FC1 tiles (128 rows x [64 up | 64 gate] columns), epilogue SiLU*mul + NVFP4 re-quantisation
@@ -13,13 +13,14 @@
 //   k_grouped_gemm<2>:  FC2 tiles (128 rows x 128 columns), epilogue alpha * routing weight -> bf16 rows per (token, expert)
 //   k_combine:          out[token] = sum over its top-k rows, in slot order (deterministic)
 // Both GEMM operands are streamed as 18 KB records with one bulk copy each (weights: the records built by
-// b200moe_layer_prepack), so no tensor map is needed. All five launches are programmatic (each kernel is scheduled while the one
+// b200moe_layer_prepack), so no tensor map is needed. All launches are programmatic (each kernel is scheduled while the one
 // before it drains and waits for its results with grid_dependency_wait); every kernel waits before it touches what an
 // earlier one wrote, except where a comment says why that kernel must already have completed.
 #include "grouped_gemm.cuh"
 #include "plan.cuh"
 #include <string.h>
 #include <stdlib.h>
+#include <type_traits>
 
 namespace b200 {
 
@@ -27,24 +28,58 @@ namespace b200 {
 // Blocks [0, aside) do what else the records and the GEMM behind this kernel need: block i zeroes the scale bytes of the rows of
 // tile i that hold no pair (a zero scale silences whatever codes a row holds, so their codes are never written), marks these rows
 // in row_pair and asks the first weight records of GEMM CTA i into L2, which is idle meanwhile.
-template <int ARows, int Rec>
-__device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, int* row_pair, int tid, int nthreads) {
-  const int NT = __ldcg(A.ntiles), i = blockIdx.x;
+//
+// Planned (both kernels below): there is no plan kernel before this one, every block works the plan out for itself (plan.cuh).
+struct GgPlanning { const int* ids; int P, E, Umax; PlanTables T; };
+template <bool Planned, int ARows, int Rec>
+__device__ __forceinline__ void records_aside(const GgAside& A, const GgPlanning& Q, BlockPlan& B, uint8_t* rec, int* row_pair, int tid, int nthreads) {
+  constexpr int kPer = ARows == 64 ? kTerms : 1, kTile = ARows / kPer;
+  const int i = blockIdx.x;
+  if (Planned) block_plan<kTile>(Q.ids, Q.P, Q.E, Q.Umax, Q.T, i == 0, B);
+  const int NT = Planned ? B.NT : __ldcg(A.ntiles);
+  if (i < A.gemm_ctas) {
+    const GgSplit s(NT, A.NBLK, A.gemm_ctas, i);
+    if (s.nseg > 0) {
+      const GgSplit::Segment g = s.segment(0);
+      const int e = Planned ? block_plan_tile<kTile>(B, g.t).x : __ldcg(A.tile_expert + g.t);
+      if (tid < kGgWarm && tid < (g.n1 - g.n0) * A.KB) l2_prefetch(A.wrec + (((long long)e * A.NBLK + g.n0) * A.KB + tid) * kRec, kRec);
+    }
+  }
   if (i < NT) {
-    constexpr int kPer = ARows == 64 ? kTerms : 1;
-    const int used = min(ARows, (__ldcg(A.tile_end + i) - __ldcg(A.tile_first + i)) * kPer), spare = ARows - used;
+    const int pairs = Planned ? block_plan_tile<kTile>(B, i).y : __ldcg(A.tile_end + i) - __ldcg(A.tile_first + i);
+    const int used = min(ARows, pairs * kPer), spare = ARows - used;
     for (int j = tid; j < spare * 4 * A.KB; j += nthreads) {
       const int r = used + j % spare, q = j / spare;   // scale word q & 3 of K box q >> 2
       *reinterpret_cast<uint32_t*>(rec + ((long long)i * A.KB + (q >> 2)) * Rec + (Rec - 2048) + (q & 3) * 512 + (r & 31) * 16 + (r >> 5) * 4) = 0u;
     }
     for (int r = used + tid; r < ARows; r += nthreads) row_pair[(long long)i * ARows + r] = -1;
   }
-  if (i < A.gemm_ctas && tid < kGgWarm) {
-    const GgSplit s(NT, A.NBLK, A.gemm_ctas, i);
-    if (s.nseg > 0) {
-      const GgSplit::Segment g = s.segment(0);
-      if (tid < (g.n1 - g.n0) * A.KB) l2_prefetch(A.wrec + (((long long)__ldcg(A.tile_expert + g.t) * A.NBLK + g.n0) * A.KB + tid) * kRec, kRec);
+}
+
+// The rows of a token's pairs into s_row, and this thread's (warp 3: slot tid - 96) row and tile_first. The block synchronises.
+template <bool Planned, int TILE>
+__device__ __forceinline__ void token_rows(const GgPlanning& Q, BlockPlan& B, const PairTables& T, int* dst_row, int tok, int top_k, int* s_row, int* s_first,
+                                           int& my_row, int& my_first) {
+  const int tid = threadIdx.x, slot = tid - 96;
+  if (Planned) {
+    block_plan<TILE>(Q.ids, Q.P, Q.E, Q.Umax, Q.T, false, B);
+    for (int j = tid >> 5; j < top_k; j += 4) {
+      int first = 0;
+      const int row = block_plan_row<TILE>(B, tok * top_k + j, &first);
+      if ((tid & 31) == 0) s_row[j] = row, s_first[j] = first;
     }
+    __syncthreads();
+    if (slot >= 0 && slot < top_k) {
+      my_row = s_row[slot], my_first = s_first[slot];
+      dst_row[tok * top_k + slot] = my_row;
+    }
+  } else {
+    if (slot >= 0 && slot < top_k) {
+      my_row = __ldcg(dst_row + tok * top_k + slot);
+      s_row[slot] = my_row;
+      if (my_row >= 0) my_first = __ldcg(T.tile_first + my_row / TILE);
+    }
+    __syncthreads();
   }
 }
 
@@ -52,19 +87,23 @@ __device__ __forceinline__ void records_aside(const GgAside& A, uint8_t* rec, in
 // the token's row is read and quantised ONCE (the reference's block arithmetic, bit-exact), while the plan kernel is still
 // running, and its codes and scale bytes are then stored into the record rows of each of its top_k pairs (dst_row, -1 = empty
 // slot). rec [ntiles][KB][18432]; blocks beyond H inside the last K box are written as zero codes and zero scales.
-__global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* __restrict__ x, const int* dst_row, int H, int KB, int top_k, float gs,
-                                                          uint8_t* rec, GgAside A, PairTables T) {
+template <bool Planned>
+__global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* __restrict__ x, int* dst_row, int H, int KB, int top_k, float gs,
+                                                          uint8_t* rec, GgAside A, PairTables T, GgPlanning Q) {
+  __shared__ typename std::conditional<Planned, BlockPlan, int>::type s_plan;
+  BlockPlan& B = reinterpret_cast<BlockPlan&>(s_plan);
   if ((int)blockIdx.x < A.blocks) {
     grid_dependency_wait();
     grid_launch_dependents();
-    records_aside<128, kRec>(A, rec, T.row_pair, threadIdx.x, 128);
+    records_aside<Planned, 128, kRec>(A, Q, B, rec, T.row_pair, threadIdx.x, 128);
     return;
   }
   __shared__ float s_scale[128];   // gs / (E4M3 value) for every scale byte: one division per table entry instead of one per block
-  __shared__ int s_row[16];
+  __shared__ int s_row[16], s_first[16];
   fill_scale_table(s_scale, gs, threadIdx.x, blockDim.x);
   const int tok = blockIdx.x - A.blocks;
   __syncthreads();
+  if (Planned) grid_dependency_wait();   // x and the ids alike
   const int nblk = KB * 16;
   bool waited = false;
   const int slot = threadIdx.x - 96;   // warp 3: this token's entries of the pair tables
@@ -86,12 +125,7 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
       waited = true;
       grid_dependency_wait();
       grid_launch_dependents();
-      if (slot >= 0 && slot < top_k) {
-        my_row = __ldcg(dst_row + tok * top_k + slot);
-        s_row[slot] = my_row;
-        if (my_row >= 0) my_first = __ldcg(T.tile_first + (my_row >> 7));
-      }
-      __syncthreads();
+      token_rows<Planned, 128>(Q, B, T, dst_row, tok, top_k, s_row, s_first, my_row, my_first);
     }
     if (b >= nblk) continue;
 #pragma unroll 4
@@ -116,17 +150,21 @@ __global__ void __launch_bounds__(128) k_quantize_scatter(const __nv_bfloat16* _
 // into the four term rows of each of the token's pairs (dst_row[pair] = tile * 16 + pair row); the first four threads also
 // write the rows' 1 / g_t.
 // The row's amax is taken while the plan kernel is still running. Blocks [0, aside): see records_aside.
-__global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __restrict__ x, const int* dst_row, int H, int KB, int top_k, uint8_t* rec,
-                                                        float* rowscale, GgAside A, PairTables T) {
+template <bool Planned>
+__global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __restrict__ x, int* dst_row, int H, int KB, int top_k, uint8_t* rec,
+                                                        float* rowscale, GgAside A, PairTables T, GgPlanning Q) {
+  __shared__ typename std::conditional<Planned, BlockPlan, int>::type s_plan;
+  BlockPlan& B = reinterpret_cast<BlockPlan&>(s_plan);
   const int tid = threadIdx.x;
   if ((int)blockIdx.x < A.blocks) {
     grid_dependency_wait();
     grid_launch_dependents();
-    records_aside<64, kMidRec>(A, rec, T.row_pair, tid, 128);
+    records_aside<Planned, 64, kMidRec>(A, Q, B, rec, T.row_pair, tid, 128);
     return;
   }
+  if (Planned) grid_dependency_wait();   // x and the ids alike
   __shared__ float wm[4];
-  __shared__ int s_row[16];
+  __shared__ int s_row[16], s_first[16];
   const int tok = blockIdx.x - A.blocks;
   float m = 0.f;
   for (int i = tid * 8; i < H; i += 128 * 8) {
@@ -142,12 +180,7 @@ __global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __r
   grid_launch_dependents();
   const int slot = tid - 96;   // warp 3: this token's entries of the pair tables
   int my_row = -1, my_first = 0;
-  if (slot >= 0 && slot < top_k) {
-    my_row = __ldcg(dst_row + tok * top_k + slot);
-    s_row[slot] = my_row;
-    if (my_row >= 0) my_first = __ldcg(T.tile_first + (my_row >> 4));
-  }
-  __syncthreads();
+  token_rows<Planned, 16>(Q, B, T, dst_row, tok, top_k, s_row, s_first, my_row, my_first);
   m = fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
   const float g1 = 2688.0f / fmaxf(m, 1e-30f);
   if (tid < kTerms) {
@@ -336,14 +369,16 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   const int max_tiles = P / 128 + Umax;   // tiles this batch can need (<= the workspace's capacity)
   const PlanTables tab = {experts, offsets, ntiles, tile_expert, tile_first, tile_end, dst_row};
   const PairTables ptab = {tile_first, pairs, row_pair};
-  int rc = launch_plan<128>(ids, P, E, Umax, tab, st);
+  const bool planned = P <= kBlockPlanPairs;   // no plan kernel (plan.cuh)
+  int rc = planned ? B200MOE_OK : launch_plan<128>(ids, P, E, Umax, tab, st);
   if (rc != B200MOE_OK) return rc;
   {
     const GgAside aside = {ntiles, tile_expert, tile_first, tile_end, w1t, I / 64, KB1, sms, max_tiles > sms ? max_tiles : sms};
+    const GgPlanning planning = {ids, P, E, Umax, tab};
     const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
     uint8_t* rec = w + L.xrec;
-    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&gs_x, (void*)&rec, (void*)&aside, (void*)&ptab};
-    rc = launch_kernel((const void*)k_quantize_scatter, aside.blocks + M, 128, 0, true, args, st);
+    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&gs_x, (void*)&rec, (void*)&aside, (void*)&ptab, (void*)&planning};
+    rc = launch_kernel(planned ? (const void*)k_quantize_scatter<true> : (const void*)k_quantize_scatter<false>, aside.blocks + M, 128, 0, true, args, st);
     if (rc != B200MOE_OK) return rc;
   }
   GroupedParams p;
@@ -353,12 +388,14 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   // FC1
   p.arec = w + L.xrec, p.wrec = w1t, p.alpha = alpha1, p.gs_in = gs_x, p.gs_out = gs_a, p.orec = w + L.arec;
   p.NBLK = I / 64, p.KB = KB1, p.KT = KT1, p.KB2 = KB2;
+  p.wait_tables = planned;
   rc = launch_gemm(p, 1, sms, st);
   if (rc != B200MOE_OK) return rc;
   // FC2
   p.arec = w + L.arec, p.wrec = w2t, p.alpha = alpha2, p.gs_in = gs_a, p.gs_out = 0.f, p.orec = nullptr;
   p.wts = wts, p.y = (__nv_bfloat16*)(w + L.y);
   p.NBLK = H / 128, p.KB = KB2, p.KT = KT2;
+  p.wait_tables = 0;
   rc = launch_gemm(p, 2, sms, st);
   if (rc != B200MOE_OK) return rc;
   const uint8_t* y = w + L.y;
@@ -431,14 +468,16 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   int* tile_end = tile_first + max_tiles;
   const PlanTables tab = {experts, offsets, ntiles, tile_expert, tile_first, tile_end, dst_row};
   const PairTables ptab = {tile_first, pairs, row_pair};
-  int rc = launch_plan<16>(ids, P, E, Umax, tab, st);
+  const bool planned = P <= kBlockPlanPairs && KB1 <= 8;   // no plan kernel   // no plan kernel
+  int rc = planned ? B200MOE_OK : launch_plan<16>(ids, P, E, Umax, tab, st);
   if (rc != B200MOE_OK) return rc;
   {
     const GgAside aside = {ntiles, tile_expert, tile_first, tile_end, w1t, I / 64, KB1, sms, max_tiles > sms ? max_tiles : sms};
+    const GgPlanning planning = {ids, P, E, Umax, tab};
     const __nv_bfloat16* xp = (const __nv_bfloat16*)x;
     uint8_t* rec = w + L.xrec;
-    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&rec, (void*)&rowscale, (void*)&aside, (void*)&ptab};
-    rc = launch_kernel((const void*)k_expand_scatter, aside.blocks + M, 128, 0, true, args, st);
+    void* args[] = {(void*)&xp, (void*)&dst_row, (void*)&H, (void*)&KB1, (void*)&top_k, (void*)&rec, (void*)&rowscale, (void*)&aside, (void*)&ptab, (void*)&planning};
+    rc = launch_kernel(planned ? (const void*)k_expand_scatter<true> : (const void*)k_expand_scatter<false>, aside.blocks + M, 128, 0, true, args, st);
     if (rc != B200MOE_OK) return rc;
   }
   GroupedParams p;
@@ -449,12 +488,14 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   // FC1
   p.arec = w + L.xrec, p.wrec = w1t, p.alpha = alpha1, p.orec = w + L.arec;
   p.NBLK = I / 64, p.KB = KB1, p.KT = KT1, p.KB2 = KB2;
+  p.wait_tables = planned;
   rc = launch_gemm(p, 3, sms, st);
   if (rc != B200MOE_OK) return rc;
   // FC2
   p.arec = w + L.arec, p.wrec = w2t, p.alpha = alpha2, p.orec = nullptr;
   p.wts = wts, p.yf = (float*)(w + L.y);
   p.NBLK = H / 128, p.KB = KB2, p.KT = KT2;
+  p.wait_tables = 0;
   rc = launch_gemm(p, 4, sms, st);
   if (rc != B200MOE_OK) return rc;
   const uint8_t* y = w + L.y;

@@ -50,6 +50,18 @@ def test_mid_is_deterministic_row_independent_and_close_to_the_slices():
     assert float(out[0].float().abs().max()) == 0.0
 
 
+# Up to 1024 pairs, and hidden sizes up to 2048, there is no plan kernel: the same tokens in a batch beyond that give the same bits.
+@pytest.mark.parametrize("hidden,m,more", [(256, 128, 129), (256, 33, 200), (2048, 100, 140), (2304, 100, 140)])
+def test_mid_batches_on_both_sides_of_the_plan_kernel(hidden, m, more):
+    cfg = dict(experts=24, hidden=hidden, inter=128, top_k=8)
+    w, _ = make_layer(**cfg, seed=6)
+    x, ids, wts = inputs(cfg, more, 60 + m)
+    ids, wts = ids.clone(), wts.clone()
+    ids[m // 2, 1], wts[m // 2, 1] = -1, 0
+    whole = run_mid(w, x, ids, wts).clone()
+    assert torch.equal(run_mid(w, x[:m], ids[:m], wts[:m]), whole[:m])
+
+
 def test_qwen_shape_mid_batches():
     cfg, w, ow = layer("qwen")
     for m in (40, 128):

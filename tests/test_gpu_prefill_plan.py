@@ -42,6 +42,45 @@ def test_plan_sizes(top_k, m):
     assert np.array_equal(row_pair[rows[order]], order) and (row_pair >= 0).sum() == order.size and rows[flat < 0].max() == -1
 
 
+# Up to 1024 pairs every block of the quantising kernel works the plan out for itself, above it is a kernel: all tables against the router's
+# definition on both sides of the line, with empty slots, an id that is no expert, one expert with all pairs, up to 256 experts.
+@pytest.mark.parametrize("experts,top_k,m,same", [(24, 8, 17, False), (24, 8, 128, False), (24, 8, 129, False), (24, 8, 128, True), (256, 6, 170, False),
+                                                  (256, 6, 171, False), (256, 16, 64, False), (2, 1, 1000, False), (2, 2, 512, True)])
+def test_tables_of_small_batches(experts, top_k, m, same):
+    cfg = dict(experts=experts, hidden=128, inter=64, top_k=top_k)
+    w, _ = make_layer(**cfg, seed=8)
+    x, ids, wts = inputs(cfg, m, 90 + m)
+    ids, wts = ids.clone(), wts.clone()
+    if same:
+        ids[:] = torch.arange(top_k, dtype=torch.int32)
+    ids[m // 2, top_k - 1], wts[m // 2, top_k - 1] = -1, 0
+    ids[m // 3, 0], wts[m // 3, 0] = experts, 0
+    run_prefill(w, x, ids, wts, 1024)
+    mp, ws = prefill_map(w, 1024), w.prefill.workspace
+    flat = ids.reshape(-1).numpy()
+    e = np.where((flat < 0) | (flat >= experts), 1 << 20, flat)
+    routed = int((e < experts).sum())
+    order = np.argsort(e, kind="stable")[:routed]
+    cnt = np.bincount(flat[order], minlength=experts)
+    off = np.concatenate([[0], np.cumsum(cnt)])
+    touched = np.nonzero(cnt)[0]
+    tiles = [(q, off[q] + 128 * j, off[q + 1]) for q in touched for j in range(-(-cnt[q] // 128))]
+    umax, nt = min(experts, flat.size), len(tiles)
+    assert int(_i32(ws, mp["ntiles"], 1)[0]) == nt
+    assert np.array_equal(_i32(ws, mp["experts"], umax), np.pad(touched, (0, umax - touched.size), constant_values=-1))
+    assert np.array_equal(_i32(ws, mp["offsets"], umax + 1), np.pad(off[touched], (0, umax + 1 - touched.size), constant_values=routed))
+    assert np.array_equal(_i32(ws, mp["pairs"], routed), order)
+    for i, name in enumerate(("tile_expert", "tile_first", "tile_end")):
+        assert np.array_equal(_i32(ws, mp[name], nt), [t[i] for t in tiles]), name
+    first_tile = np.concatenate([[0], np.cumsum(-(-cnt // 128))])
+    rows = np.full(flat.size, -1)
+    rows[order] = np.concatenate([128 * first_tile[q] + np.arange(cnt[q]) for q in touched])
+    assert np.array_equal(_i32(ws, mp["dst_row"], flat.size), rows)
+    row_pair = np.full(128 * nt, -1)
+    row_pair[rows[order]] = order
+    assert np.array_equal(_i32(ws, mp["row_pair"], 128 * nt), row_pair)
+
+
 def test_workspace_holds_the_most_tiles_there_can_be():
     """Every expert ends in a tile of one row at the very number of tokens the workspace was sized for: all of its tiles are in use, and
     nothing is written behind it."""
