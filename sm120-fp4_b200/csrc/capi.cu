@@ -225,7 +225,7 @@ static int decode_tc_columns(int M) { return M <= 4 ? 16 : M <= 8 ? 32 : 64; }  
 // The tcgen05 kernel runs whenever the tile records exist, the hidden size is at most 3072 (12 K boxes) and there is a worker for every
 // 128-row output block. Wider layers decode on the mma.sync kernel at every batch size: its f16 activations hold magnitudes up to 65504
 // and keep 11 bits, where four FP4 terms under the fixed activation scale clip a block beyond 336 and keep about 10. (Two layer calls
-// of 8 tokens at 4096 x 1536 would take 187 us instead of 261.)
+// of 8 tokens at 4096 x 1536 would take 187 us instead of 234.)
 static bool decode_tc_fits(const b200moe_layer* L) { return L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 12 && L->NB2 <= L->sms; }
 
 static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, const HostRouting* host, void* stream) {

@@ -8,8 +8,8 @@
 //  * the work is a flat list of weight tiles: FC1 tile = 64 up rows + 64 gate rows x 256 K-codes + their scales; FC2 tile = 128
 //    output rows x 256 K-codes + their scales + the activation slab of that expert / K-box. Where the layer has been prepacked a
 //    tile is one 18 KB record (one bulk copy; two layers of 4096 x 1536 at 8 tokens, two groups: 254 us, together with the overlapped
-//    launch, against 269), else boxes and scale runs of the checkpoint layout (three to four copies). Every worker owns a contiguous, equal share of the flat list (stream-K), so any number of
-//    touched experts balances over the workers.
+//    launch, against 269), else boxes and scale runs of the checkpoint layout (three to four copies). Every worker owns a
+//    contiguous, equal share of the flat list (stream-K), so any number of touched experts balances over the workers.
 //  * tiles land in a ring of shared-memory stages guarded by full/empty mbarriers; the producer runs ahead of the math by
 //    the ring depth and, across the FC1->FC2 dependency, prefetches FC2 weight tiles before the grid-wide barrier opens.
 //  * math: codes -> f16 with cvt.rn.f16x2.e2m1x2, times the E4M3 scale (exact in f16), mma.sync m16n8k16 f16 with fp32
