@@ -118,13 +118,13 @@ extern "C" int b200moe_layer_create(b200moe_layer** out, int E, int H, int I, in
   if (rc == B200MOE_OK) rc = make_codes_map(&L->tm2, q2, (long long)E * H, I / 2, 128);
   if (rc != B200MOE_OK) { delete L; return rc; }
   // workspace
-  const int V = 3 * L->sms;   // workers of the mma.sync kernel
+  const int V = 2 * L->sms;   // shares of the mma.sync kernel
   L->umax_cap = E < 16 * top_k ? E : 16 * top_k;
   long long o = 0;
   L->off_status = o, o += 256;                                               // status + grid barrier words
   L->off_cnt1 = o, o = align_up(o + (long long)L->umax_cap * L->CB1 * 4, 256);
   L->off_cnt2 = o, o = align_up(o + (long long)L->NB2 * 4, 256);
-  L->off_scratch = o, o = align_up(o + (long long)V * 2 * 128 * 16 * 4, 256);
+  L->off_scratch = o, o = align_up(o + (long long)V * 3 * 128 * 16 * 4, 256);
   L->off_actfrag = o, o = align_up(o + (long long)L->umax_cap * L->KB2 * 8192, 256);
   L->off_tables = o, o = align_up(o + (long long)(2 * L->umax_cap + 1 + 16 * top_k) * 4, 256);
   L->off_actbf16 = o, o = align_up(o + (long long)16 * top_k * I * 2, 256);
@@ -225,7 +225,7 @@ static int decode_tc_columns(int M) { return M <= 4 ? 16 : M <= 8 ? 32 : 64; }  
 // The tcgen05 kernel runs whenever the tile records exist, the hidden size is at most 3072 (12 K boxes) and there is a worker for every
 // 128-row output block. Wider layers decode on the mma.sync kernel at every batch size: its f16 activations hold magnitudes up to 65504
 // and keep 11 bits, where four FP4 terms under the fixed activation scale clip a block beyond 336 and keep about 10. (Two layer calls
-// of 8 tokens at 4096 x 1536 would take 187 us instead of 234.)
+// of 8 tokens at 4096 x 1536 would take 187 us instead of 232.)
 static bool decode_tc_fits(const b200moe_layer* L) { return L->w1t && L->decode_impl != 1 && L->sms <= 256 && L->KB1 <= 12 && L->NB2 <= L->sms; }
 
 static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* ws, bool chained, const HostRouting* host, void* stream) {
@@ -277,7 +277,7 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   if (ws_bytes < L->ws_bytes) return B200MOE_ERR_WORKSPACE;
   if (((uintptr_t)ws & 255) || ((uintptr_t)x & 15)) return B200MOE_ERR_ARG;
   if (M == 0) return B200MOE_OK;
-  if (3 * L->sms > 512) return B200MOE_ERR_DEVICE;   // share tables of the kernel hold 512 workers
+  if (2 * L->sms > 512) return B200MOE_ERR_DEVICE;   // the kernel's tables hold 512 shares
   uint8_t* w = (uint8_t*)ws;
   DecodeParams p;
   memset(&p, 0, sizeof(p));
@@ -310,7 +310,7 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   const int slab = nb8 * 4096;
   const int limit = 227 * 1024;
   p.slot_bytes = b200_decode_slot_bytes(p.w1t != nullptr);
-  const int groups = b200_decode_groups(M);
+  const int groups = M <= 8 ? 3 : 2;
   int NS = 9 / groups * groups;
   for (; NS >= groups; NS -= groups) {
     const int region = (L->KB1 * slab > NS * slab) ? L->KB1 * slab : NS * slab;
@@ -318,7 +318,7 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   }
   if (NS < groups) return B200MOE_ERR_SHAPE;
   p.NS = NS;
-  return b200_decode_launch(p, L->sms, b200_decode_smem_bytes(NS, p.slot_bytes, p.region_bytes), chained, (cudaStream_t)stream);
+  return b200_decode_launch(p, groups, L->sms, b200_decode_smem_bytes(NS, p.slot_bytes, p.region_bytes), chained, (cudaStream_t)stream);
 }
 
 // The whole decode layer: out[M, H] (bf16) = sum_j w[t,j] * FC2_e(silu(gate) * up), e = ids[t,j]. M <= 16.

@@ -4,19 +4,20 @@
 // (FP4 code x E4M3 block scale, fp32 accumulation, alpha applied in fp32, __expf SiLU, one rounding of the output).
 //
 // Structure (B200-first, memory-bound):
-//  * one CTA per SM; three (above 8 tokens two) consumer groups of four warps are its "workers", each with a TMA producer warp.
+//  * one CTA per SM; its "workers" are two or three consumer groups of four warps, each with a TMA producer warp.
 //  * the work is a flat list of weight tiles: FC1 tile = 64 up rows + 64 gate rows x 256 K-codes + their scales; FC2 tile = 128
 //    output rows x 256 K-codes + their scales + the activation slab of that expert / K-box. Where the layer has been prepacked a
-//    tile is one 18 KB record (one bulk copy; two layers of 4096 x 1536 at 8 tokens, two groups: 254 us, together with the overlapped
-//    launch, against 269), else boxes and scale runs of the checkpoint layout (three to four copies). Every worker owns a
-//    contiguous, equal share of the flat list (stream-K), so any number of touched experts balances over the workers.
+//    tile is one 18 KB record (one bulk copy; two layers of 4096 x 1536 at 8 tokens, two groups: 246 us
+//    against 250), else boxes and scale runs of the checkpoint layout (three to four copies). The list is cut into two
+//    equal contiguous shares per CTA (stream-K), so any number of touched experts balances over the chip. The shares alone say where
+//    K is cut and in which order partial sums are added: the result does not depend on how many workers a CTA has.
 //  * tiles land in a ring of shared-memory stages guarded by full/empty mbarriers; the producer runs ahead of the math by
 //    the ring depth and, across the FC1->FC2 dependency, prefetches FC2 weight tiles before the grid-wide barrier opens.
 //  * math: codes -> f16 with cvt.rn.f16x2.e2m1x2, times the E4M3 scale (exact in f16), mma.sync m16n8k16 f16 with fp32
 //    accumulators, tokens as the N dimension ("global token columns": column j is token j for every expert, so partial
 //    sums of different experts add in registers and the routing weight is applied per expert in fp32).
 //  * a tile range that cuts a unit writes its partial sums to an L2-resident scratch; the last arriver (atomic counter)
-//    adds the pieces in worker order, so the result is bit-identical from call to call.
+//    adds the pieces in share order, so the result is bit-identical from call to call.
 #include "common.cuh"
 #include "ptx.cuh"
 #include "decode_params.h"
@@ -24,18 +25,18 @@
 namespace b200 {
 
 constexpr int kGroupThreads = 128;
-// Consumer groups of a CTA, each a worker with a producer warp of its own. A worker's chain - wait for a tile, its math, the end of a
-// piece - is serial, so more of them keep the pipes busy: two layers of 8 tokens at 4096 x 1536 take 234 us with three groups, 254 with
-// two and 253 with four (whose pieces are smaller: one token 78 against 72). Above 8 tokens the x operand leaves four ring stages at
-// that size, which two groups can share. (Eight warps a tile, each with half of its K codes: 257.)
+// Consumer groups of a CTA, each a worker with a producer warp of its own. Two take a share each. Of three (up to 8 tokens) all have a third
+// of the FC1 tiles of the CTA's two shares and two of them run the FC2 shares, whose sums over the experts are one chain. A worker's own
+// chain - wait for a tile, its math, the end of a piece - is serial, so a third one keeps the pipes busier. Two layers of 4096 x 1536, us with
+// three (two; repeats differ by 0.3): 8 tokens 232.2 (245.8), 4 154.8 (157.0), 2 103.8 (106.8), 1 72.3 (74.4). With whole pieces dealt out
+// instead of thirds 240 and 110 at 8 and 2 tokens. Above 8 tokens x leaves four ring stages at that size, which two groups can share.
 constexpr int kMostGroups = 3;
-constexpr int decode_groups(int nb8) { return nb8 == 1 ? 3 : 2; }
 constexpr int decode_threads(int groups) { return groups * (kGroupThreads + 32); }
 constexpr int kCodesBytes = 16384;
 constexpr int kRecordBytes = kCodesBytes + 2048;     // a tile record: codes and four scale tiles
 constexpr int kCheckpointSlot = kCodesBytes + 4096;  // from the checkpoint layout FC1 needs the scale runs of its up and of its gate rows
 constexpr int kMaxE = 256, kMaxP = 256;
-constexpr int kMaxWorkers = 512;       // up to three per SM
+constexpr int kMaxShares = 512;        // two per SM
 
 enum { ST_OK = 0, ST_TIMEOUT_FULL = 1, ST_TIMEOUT_EMPTY = 2, ST_TIMEOUT_GRID = 3, ST_BAD_ID = 4 };
 
@@ -47,20 +48,22 @@ struct Tables {
   int uidx[kMaxE];     // inclusive scan of touched flags
   int experts[kMaxE];  // touched experts ascending
   unsigned omask[kMaxE];  // per touched expert: bit n set when a token of octet n (tokens 8n..8n+7) is routed to it
-  int sb1[kMaxWorkers + 1];   // first FC1 tile of every worker (stream-K shares); sb1[V] = T1
-  int sb2[kMaxWorkers + 1];   // same for FC2
+  int sb1[kMaxShares + 1];   // first FC1 tile of every share; sb1[V] = T1
+  int sb2[kMaxShares + 1];   // same for FC2
   int U;
   unsigned gen0;       // grid-barrier generation at kernel start
   volatile int abort_flag;
   int last_flag[kMostGroups];
+  uint64_t handed[kMostGroups - 1];
   uint64_t full[9];
   uint64_t empty[9];
 };
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }
 
-// Owner of flat tile f when worker v owns [v*T/V, (v+1)*T/V): ceil((f+1)*V/T) - 1. Products stay below 2^31 (host check).
-__device__ __forceinline__ int worker_of(int f, int T, int V) { return (int)(((unsigned)(f + 1) * (unsigned)V - 1u) / (unsigned)T); }
+// Share of flat tile f when share v is [v*T/V, (v+1)*T/V): ceil((f+1)*V/T) - 1. Products stay below 2^32: at
+// 296 shares that is 14.5 million tiles, 267 GB of weights.
+__device__ __forceinline__ int share_of(int f, int T, int V) { return (int)(((unsigned)(f + 1) * (unsigned)V - 1u) / (unsigned)T); }
 
 #ifdef B200_TIMERS
 #define TIMER_START(var) long long var = clock64()
@@ -133,7 +136,7 @@ __device__ __forceinline__ int frag_index(int k, int tok) {
   return kb * (NB8 * 2048) + ((((h * 4 + jj) * NB8 + (tok >> 3)) * 32 + lane) << 3) + (k & 7);
 }
 
-// Sum the partial results of the workers [vlo, vhi] that own a piece of the unit starting at flat tile `first`, in worker
+// Sum the partial results of the shares [vlo, vhi] that hold a piece of the unit starting at flat tile `first`, in share
 // order (fixed summation order), four pieces' loads in flight at a time. v[] has 8*NB8 floats per thread.
 template <int NB8>
 __device__ __forceinline__ void reduce_pieces(const float* __restrict__ scratch, const int* sb, int first, int vlo, int vhi,
@@ -147,7 +150,7 @@ __device__ __forceinline__ void reduce_pieces(const float* __restrict__ scratch,
     for (int b = 0; b < 4; ++b) {
       const int pv = p0 + b;
       live[b] = pv <= vhi && sb[pv + 1] > sb[pv];
-      const int pslot = (live[b] && sb[pv] < first) ? 1 : 0;   // a piece that starts its worker's share sits in slot 0
+      const int pslot = (live[b] && sb[pv] < first) ? 1 : 0;   // a piece that starts its share sits in slot 0
       const float* src = scratch + ((long long)((live[b] ? pv : vlo) * 2 + pslot) * kGroupThreads + gtid) * 16;
 #pragma unroll
       for (int i = 0; i < 2 * NB8; ++i)
@@ -164,9 +167,65 @@ __device__ __forceinline__ void reduce_pieces(const float* __restrict__ scratch,
   }
 }
 
-template <int NB8>
-__global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_decode(const __grid_constant__ DecodeParams P) {
-  constexpr int kGroups = decode_groups(NB8), kConsumerWarps = 4 * kGroups, kThreads = decode_threads(kGroups);
+// The FC1 tiles of a consumer group in runs, the same walk for the group and for its producer. A piece is a share's tiles of one unit: one
+// chain of MMAs. Two groups have a share each, whose runs are its pieces. Three cut the tiles of both shares into equal thirds. A piece on the line
+// between two thirds is begun by one group, which hands its accumulators on, and continued by the next: the chain stays what it is.
+// What is handed on comes first in a third and what is taken over last, so that hardly anybody waits.
+template <int kGroups>
+struct Fc1Walk {
+  int f, n, q, k0, v;       // first tile and tiles of the run at hand, its unit, K box of its first tile, its share
+  int from, to;             // tiles of its piece
+  bool taken, handed;       // it continues the accumulators of the group before; the next group continues its own
+  int lo, hi, pos, stage;   // the group's tiles [lo, hi); next run of whole pieces; 0: handed on, 1: whole pieces, 2: taken over, 3: end
+  int ql, kl, qp, kp;       // unit and K box of lo and of pos
+  int first, begin, mid, end, KB1;
+  __device__ __forceinline__ int share_begin(int t) const { return t < mid ? begin : mid; }
+  __device__ __forceinline__ int share_end(int t) const { return t < mid ? mid : end; }
+  __device__ __forceinline__ void behind(int t) {   // pos goes on to t, a piece's end
+    kp += t - pos, pos = t;
+    if (kp >= KB1) kp -= KB1, ++qp;
+  }
+  __device__ __forceinline__ Fc1Walk(const Tables& T, int cta, int grp, int kb1) : KB1(kb1) {
+    first = 2 * cta + (kGroups == 2 ? grp : 0);
+    begin = T.sb1[first], mid = T.sb1[first + 1], end = kGroups == 2 ? mid : T.sb1[first + 2];
+    lo = begin + (kGroups == 2 ? 0 : grp * (end - begin) / 3), hi = kGroups == 2 ? end : begin + (grp + 1) * (end - begin) / 3;
+    stage = lo < hi ? 0 : 3;
+    ql = lo / KB1, kl = lo - ql * KB1;
+    pos = lo, qp = ql, kp = kl;
+    if (kGroups > 2 && lo < hi && max(lo - kl, share_begin(lo)) < lo) behind(min(hi, min(lo - kl + KB1, share_end(lo))));   // (taken over)
+  }
+  __device__ __forceinline__ bool run(int f0, int f1, int unit, int k, bool t, bool h) {
+    f = f0, n = f1 - f0, q = unit, k0 = k, taken = t, handed = h, v = first + (kGroups > 2 && f0 >= mid);
+    from = kGroups > 2 ? max(unit * KB1, share_begin(f0)) : f0, to = kGroups > 2 ? min(unit * KB1 + KB1, share_end(f0)) : f1;
+    return true;
+  }
+  __device__ __forceinline__ bool next() {
+    if (kGroups > 2 && stage == 0) {
+      stage = 1;
+      const int unit = (hi - 1) / KB1, b = max(unit * KB1, share_begin(hi - 1));
+      if (min(unit * KB1 + KB1, share_end(hi - 1)) > hi && b >= lo) return run(b, hi, unit, b - unit * KB1, false, true);
+    }
+    if (kGroups == 2 || stage == 1) {
+      const int e = min(pos - kp + KB1, share_end(pos));
+      if (pos < hi && e <= hi) {
+        run(pos, e, qp, kp, false, false);
+        behind(e);
+        return true;
+      }
+      stage = 2;
+    }
+    if (kGroups > 2 && stage == 2) {
+      stage = 3;
+      const int e = min(lo - kl + KB1, share_end(lo));
+      if (max(lo - kl, share_begin(lo)) < lo) return run(lo, min(hi, e), ql, kl, true, e > hi);
+    }
+    return false;
+  }
+};
+
+template <int NB8, int kGroups>
+__global__ void __launch_bounds__(decode_threads(kGroups), 1) k_moe_decode(const __grid_constant__ DecodeParams P) {
+  constexpr int kConsumerWarps = 4 * kGroups, kThreads = decode_threads(kGroups);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int NS = P.NS;                          // ring stages, a multiple of the groups; worker g uses slots kGroups*i+g
@@ -177,7 +236,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int npairs = P.M * P.top_k;
-  const int V = kGroups * gridDim.x;
+  const int V = 2 * gridDim.x;                  // shares
 
   // ---------------------------------------------------------------- prologue: barriers + routing tables (every CTA)
   if (tid == 0) {
@@ -185,6 +244,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
       mbar_init(&T.full[s], 1);
       mbar_init(&T.empty[s], 4);
     }
+    for (int g = 0; g < kMostGroups - 1; ++g) mbar_init(&T.handed[g], 4);
     T.abort_flag = 0;
     for (int g = 0; g < kGroups; ++g) T.last_flag[g] = 0;
     fence_mbar_init();
@@ -241,7 +301,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
         if (T.ids[tok * P.top_k + sidx] == tid) m |= 1u << (tok >> 3);
     T.omask[T.uidx[tid] - 1] = m;
   }
-  for (int v = tid; v <= V; v += kThreads) {   // stream-K shares: worker v owns tiles [sb[v], sb[v+1])
+  for (int v = tid; v <= V; v += kThreads) {   // share v is tiles [sb[v], sb[v+1])
     T.sb1[v] = (int)(((unsigned)v * (unsigned)T1) / (unsigned)V);
     T.sb2[v] = (int)(((unsigned)v * (unsigned)T2) / (unsigned)V);
   }
@@ -280,13 +340,13 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
     // ============================================================== producers: one warp per group
     if (lane == 0) {
       const int grp = warp - kConsumerWarps;
-      const int v = kGroups * blockIdx.x + grp;
+      const int v = 2 * blockIdx.x + grp;      // its FC2 share (a third group has none)
       prefetch_tensormap(&P.tm1);
       prefetch_tensormap(&P.tm2);
       const uint64_t pol = policy_evict_first();
       const unsigned gen0 = T.gen0;
       bool passed = !do1;            // without an FC1 phase the activations are already in place
-      const int n1 = T.sb1[v + 1] - T.sb1[v], n2 = T.sb2[v + 1] - T.sb2[v];
+      const int n2 = grp < 2 ? T.sb2[v + 1] - T.sb2[v] : 0;
       int pend_slot[4];
       const uint8_t* pend_src[4];
       int npend = 0;
@@ -327,11 +387,10 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
         ++j;
         if (++si == per) { si = 0; ph ^= 1u; }
       };
-      // ---- FC1 tiles of this worker, in flat order (expert slot u, column block cb, K box kb)
-      if (n1 > 0) {
-        const int f0 = T.sb1[v];
-        int kb = f0 % KB1, q = f0 / KB1, cb = q % CB1, u = q / CB1;
-        for (int i = 0; i < n1; ++i) {
+      // ---- FC1 tiles of this worker (expert slot u, column block cb, K box kb)
+      for (Fc1Walk<kGroups> at(T, blockIdx.x, grp, KB1); at.next();) {
+        const int cb = at.q % CB1, u = at.q / CB1;
+        for (int kb = at.k0; kb < at.k0 + at.n; ++kb) {
           const int slot = claim_slot(false);
           uint8_t* st = ring + slot * slot_bytes;
           const int e = T.experts[u];
@@ -339,7 +398,6 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
             mbar_expect_tx(&T.full[slot], kRecordBytes);
             bulk_load_hint(st, P.w1t + (((long long)e * CB1 + cb) * KB1 + kb) * kRecordBytes, kRecordBytes, &T.full[slot], pol);
             advance();
-            if (++kb == KB1) { kb = 0; if (++cb == CB1) { cb = 0; ++u; } }
             continue;
           }
           const int nkt = min(4, P.KT1 - 4 * kb);
@@ -351,9 +409,9 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
           bulk_load_hint(st + kCodesBytes, sbase + ((long long)(up_row >> 7) * P.KT1 + 4 * kb) * 512, nkt * 512, &T.full[slot], pol);
           bulk_load_hint(st + kCodesBytes + 2048, sbase + ((long long)(gate_row >> 7) * P.KT1 + 4 * kb) * 512, nkt * 512, &T.full[slot], pol);
           advance();
-          if (++kb == KB1) { kb = 0; if (++cb == CB1) { cb = 0; ++u; } }
         }
       }
+      const int n1 = j;
       // ---- FC2 tiles, in flat order (output block nb, expert slot u, K box kb); weights run ahead of the grid barrier
       if (n2 > 0) {
         const int f0 = T.sb2[v];
@@ -381,14 +439,14 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
       }
       if (npend > 0) wait_grid();
 #ifdef B200_TIMERS
-      if (P.debug) { P.debug[v * 8 + 4] = tm_pwait; P.debug[v * 8 + 5] = tm_pgrid; P.debug[v * 8 + 6] = clock64() - tm_begin; }
+      const int worker = kGroups * blockIdx.x + grp;
+      if (P.debug) { P.debug[worker * 8 + 4] = tm_pwait; P.debug[worker * 8 + 5] = tm_pgrid; P.debug[worker * 8 + 6] = clock64() - tm_begin; }
 #endif
     }
     __syncwarp();
   } else {
     // ============================================================== consumers: groups of four warps
     const int grp = warp >> 2, w = warp & 3;
-    const int v = kGroups * blockIdx.x + grp;
     const int gtid = tid & (kGroupThreads - 1);
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring_a = smem_u32(ring), region_a = smem_u32(region);
@@ -396,7 +454,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
     uint32_t ph = 0;
 
     if (do1) {
-      // ---- stage x as f16 in fragment order (all 256 consumer threads), zero beyond M tokens / H columns
+      // ---- stage x as f16 in fragment order (all consumer threads), zero beyond M tokens / H columns
       const int chunks_per_tok = KB1 * 32;   // 16-byte chunks (8 values) per token over the padded K
       for (int i = tid; i < 8 * NB8 * chunks_per_tok; i += kConsumerWarps * 32) {
         const int tok = i / chunks_per_tok, c8 = i % chunks_per_tok, k = c8 * 8;
@@ -417,22 +475,24 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
       }
       named_bar_sync(1 + kMostGroups, kConsumerWarps * 32);
 
-      // ---- FC1 pieces of this worker
-      const int fs = T.sb1[v], fe = T.sb1[v + 1];
-      int f = fs;
-      while (f < fe) {
-        const int q = f / KB1, cb = q % CB1, u = q / CB1;
-        const int k0 = f % KB1, k1 = min(KB1, k0 + (fe - f));
+      // ---- FC1 tiles of this worker
+      float* handover = P.scratch + (2LL * V + 2 * blockIdx.x) * (kGroupThreads * 16) + gtid * 16;   // of this CTA, group to group
+      for (Fc1Walk<kGroups> at(T, blockIdx.x, grp, KB1); at.next();) {
+        const int v = at.v, q = at.q, cb = q % CB1, u = q / CB1;
+        const int k0 = at.k0, k1 = k0 + at.n;
         const int e = T.experts[u];
         float acc[2][2][NB8][4];
+        const float* from = handover + (grp - 1) * (kGroupThreads * 16);
+        if (kGroups > 2 && at.taken && !mbar_wait(&T.handed[grp - 1], 0u, &T.abort_flag)) *P.status = ST_TIMEOUT_FULL;
 #pragma unroll
         for (int pa = 0; pa < 2; ++pa)
 #pragma unroll
           for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int n = 0; n < NB8; ++n)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) acc[pa][a][n][i] = 0.f;
+            for (int n = 0; n < NB8; ++n) {
+              const float4 c = kGroups > 2 && at.taken ? __ldcg(reinterpret_cast<const float4*>(from) + (pa * 2 + a) * NB8 + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+              acc[pa][a][n][0] = c.x, acc[pa][a][n][1] = c.y, acc[pa][a][n][2] = c.z, acc[pa][a][n][3] = c.w;
+            }
         // scale rows of this warp's up and gate rows: inside the record's tiles, or inside the two 128-row runs of the checkpoint layout
         const int rt_up = (records ? 0 : (64 * cb) & 127) + 16 * w, rt_gate = (records ? 64 : (P.I + 64 * cb) & 127) + 16 * w;
         const int gate_scales = kCodesBytes + (records ? 0 : 2048);
@@ -452,6 +512,20 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
           TIMER_ADD(tm_mma, t1);
         }
         TIMER_START(t2);
+        if (kGroups > 2 && at.handed) {
+          float* to = handover + grp * (kGroupThreads * 16);
+#pragma unroll
+          for (int pa = 0; pa < 2; ++pa)
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+              for (int n = 0; n < NB8; ++n)
+                __stcg(reinterpret_cast<float4*>(to) + (pa * 2 + a) * NB8 + n, make_float4(acc[pa][a][n][0], acc[pa][a][n][1], acc[pa][a][n][2], acc[pa][a][n][3]));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&T.handed[grp]);   // (each thread continues what its counterpart has begun)
+          TIMER_ADD(tm_fix, t2);
+          continue;
+        }
         float r[8 * NB8];   // [rb][n][4]: rb 0 = up, rb 1 = gate
 #pragma unroll
         for (int a = 0; a < 2; ++a)
@@ -459,18 +533,16 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
           for (int n = 0; n < NB8; ++n)
 #pragma unroll
             for (int i = 0; i < 4; ++i) r[(a * NB8 + n) * 4 + i] = acc[0][a][n][i] + acc[1][a][n][i];
-        const int piece_first = f;
-        f += k1 - k0;
         // ---- finish the unit: directly when this piece covers all of K, else through the scratch and a last arriver
         bool finalize = true;
-        if (!(k0 == 0 && k1 == KB1)) {
-          const int slot_id = piece_first == fs ? 0 : 1;
+        if (at.to - at.from < KB1) {
+          const int slot_id = at.from == T.sb1[v] ? 0 : 1;
           float* mine = P.scratch + ((long long)(v * 2 + slot_id) * kGroupThreads + gtid) * 16;
 #pragma unroll
           for (int i = 0; i < 2 * NB8; ++i)
             *reinterpret_cast<float4*>(mine + 4 * i) = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
           named_bar_sync(1 + grp, kGroupThreads);
-          const int vlo = worker_of(q * KB1, T1, V), vhi = worker_of(q * KB1 + KB1 - 1, T1, V);
+          const int vlo = share_of(q * KB1, T1, V), vhi = share_of(q * KB1 + KB1 - 1, T1, V);
           if (gtid == 0) {
             __threadfence();   // cumulative: orders the group's stores (observed through the barrier) before the arrival
             int nlive = 0;
@@ -525,7 +597,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
         if (gtid == 0) {
           __threadfence();
           const unsigned old = atomicAdd(P.gridbar, 1u);
-          if (old == (unsigned)(V - 1)) {
+          if (old == (unsigned)(kGroups * gridDim.x - 1)) {
             P.gridbar[0] = 0;
             __threadfence();
             atomicAdd(P.gridbar + 1, 1u);
@@ -537,8 +609,9 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
     const long long tm_phase1 = clock64() - tm_begin;
 #endif
 
-    if (do2) {
-      // ---- FC2 pieces of this worker: tiles ordered (output block nb, expert u, K box kb)
+    if (do2 && grp < 2) {
+      // ---- FC2 pieces of this worker's share: tiles ordered (output block nb, expert u, K box kb)
+      const int v = 2 * blockIdx.x + grp;
       const int fs = T.sb2[v], fe = T.sb2[v + 1];
       const int per_nb = U * KB2;
       int f = fs;
@@ -598,7 +671,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
             }
           if (kb == KB2) { kb = 0; ++u; }   // u wraps only at a piece boundary, where it is recomputed
         }
-        // ---- every output block is shared by several workers: partial sums to the scratch, last arriver reduces
+        // ---- every output block lies in several shares: partial sums to the scratch, last arriver reduces
         {
           TIMER_START(t2);
           const int slot_id = piece_start == fs ? 0 : 1;
@@ -607,7 +680,7 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
           for (int i = 0; i < 2 * NB8; ++i)
             *reinterpret_cast<float4*>(mine + 4 * i) = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
           named_bar_sync(1 + grp, kGroupThreads);
-          const int vlo = worker_of(nb * per_nb, T2, V), vhi = worker_of((nb + 1) * per_nb - 1, T2, V);
+          const int vlo = share_of(nb * per_nb, T2, V), vhi = share_of((nb + 1) * per_nb - 1, T2, V);
           if (gtid == 0) {
             __threadfence();
             int nlive = 0;
@@ -639,8 +712,9 @@ __global__ void __launch_bounds__(decode_threads(decode_groups(NB8)), 1) k_moe_d
     }
 #ifdef B200_TIMERS
     if (P.debug && gtid == 0) {
-      P.debug[v * 8 + 0] = tm_wait; P.debug[v * 8 + 1] = tm_mma; P.debug[v * 8 + 2] = tm_fix; P.debug[v * 8 + 3] = tm_phase1;
-      P.debug[v * 8 + 7] = clock64() - tm_begin;
+      const int worker = kGroups * blockIdx.x + grp;
+      P.debug[worker * 8 + 0] = tm_wait; P.debug[worker * 8 + 1] = tm_mma; P.debug[worker * 8 + 2] = tm_fix; P.debug[worker * 8 + 3] = tm_phase1;
+      P.debug[worker * 8 + 7] = clock64() - tm_begin;
     }
 #endif
   }
@@ -677,18 +751,16 @@ __global__ void __launch_bounds__(256) k_act_to_frag(const __nv_bfloat16* __rest
 
 using namespace b200;
 
-int b200_decode_groups(int M) { return decode_groups(M <= 8 ? 1 : 2); }
-
 int b200_decode_slot_bytes(bool records) { return records ? kRecordBytes : kCheckpointSlot; }
 
 int b200_decode_smem_bytes(int NS, int slot_bytes, int region_bytes) { return 1024 + NS * slot_bytes + region_bytes + (int)sizeof(Tables); }
 
-int b200_decode_launch(const DecodeParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st) {
+int b200_decode_launch(const DecodeParams& p, int groups, int grid, int smem_bytes, bool chained, cudaStream_t st) {
   void* args[] = {(void*)&p};
-  const void* fn = p.M <= 8 ? (const void*)k_moe_decode<1> : (const void*)k_moe_decode<2>;
-  const int threads = decode_threads(decode_groups(p.M <= 8 ? 1 : 2));
-  static thread_local int configured[2] = {0, 0};
-  const int which = p.M <= 8 ? 0 : 1;
+  const int which = p.M > 8 ? 2 : groups == 3 ? 1 : 0;
+  const void* fn = which == 2 ? (const void*)k_moe_decode<2, 2> : which == 1 ? (const void*)k_moe_decode<1, 3> : (const void*)k_moe_decode<1, 2>;
+  const int threads = decode_threads(which == 1 ? 3 : 2);
+  static thread_local int configured[3] = {0, 0, 0};
   if (configured[which] < smem_bytes) {
     B200_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
     configured[which] = smem_bytes;

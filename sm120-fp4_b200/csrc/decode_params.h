@@ -22,7 +22,7 @@ struct DecodeParams {
   __nv_bfloat16* out;       // [M, H]
   __nv_bfloat16* act_bf16;  // optional [M*top_k, I], row = pair index
   __half* actfrag;          // workspace: FC1 output in the fragment order FC2 streams
-  float* scratch;           // workspace: split-unit partial sums, 2 slots x 128 threads x 16 floats per worker
+  float* scratch;           // workspace, slots of 128 threads x 16 floats: partial sums of split units, 2 per share; then accumulators handed on, 2 per CTA
   unsigned* cnt1;           // workspace: arrival counters per FC1 unit (self-resetting)
   unsigned* cnt2;           // workspace: arrival counters per FC2 output block (self-resetting)
   unsigned* gridbar;        // workspace: [0] arrivals, [1] generation
@@ -85,9 +85,8 @@ inline bool b200_decode_self_expand(int M, int H) { return M <= 8 && M * H <= 16
 int b200_pack_tiles_launch(const void* q, const void* sf, void* out, int E, int rows_per_expert, int row_bytes, int blocks, int KB, int KT,
                            int fc1, int I, long long sf_stride, cudaStream_t st);
 int b200_decode_tc_launch(const b200::DecodeTcParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);
-int b200_decode_groups(int M);   // consumer groups of a block, which its ring stages are dealt to
 int b200_decode_slot_bytes(bool records);
 int b200_decode_smem_bytes(int NS, int slot_bytes, int region_bytes);
-int b200_decode_launch(const b200::DecodeParams& p, int grid, int smem_bytes, bool chained, cudaStream_t st);
+int b200_decode_launch(const b200::DecodeParams& p, int groups, int grid, int smem_bytes, bool chained, cudaStream_t st);
 int b200_act_to_frag_launch(const void* act, const int* ids, const int* experts, int Umax, int M, int top_k, int I, int KB2,
                             void* actfrag, cudaStream_t st);

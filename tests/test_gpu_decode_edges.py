@@ -95,6 +95,21 @@ def test_tile_records_and_checkpoint_layout_agree(hidden, inter):
         h.b200moe_layer_destroy(bare)
 
 
+# Where K is cut and in which order partial sums are added follows from the shares of the tile list alone, not from how many workers deal
+# with it: up to 8 tokens three workers a block have the bits of two, which run batches above 8 (here with a ninth token of empty slots).
+# Few tiles a block (chains over all three workers) up to about 50.
+@pytest.mark.parametrize("hidden,inter", [(3200, 64), (3328, 192), (4096, 320), (4096, 832)])
+def test_sums_do_not_depend_on_the_number_of_workers(hidden, inter):
+    cfg, w, _ = edge_layer(hidden, inter)
+    for m in (1, 2, 5, 8):
+        x, ids, wts = inputs(cfg, m, 30 + m)
+        pad = 9 - m
+        more = run(w, torch.cat([x, torch.zeros(pad, hidden, dtype=x.dtype)]), torch.cat([ids, torch.full((pad, cfg["top_k"]), -1, dtype=ids.dtype)]),
+                   torch.cat([wts, torch.zeros(pad, cfg["top_k"])])).clone()
+        assert torch.equal(run(w, x, ids, wts), more[:m]), m
+    w.status()
+
+
 # Calls of a wide layer overlap their launches: a chain of them, each on the output of the one before, gives what the calls give one by one.
 def test_chained_wide_calls():
     cfg, w, _ = edge_layer(3200)
