@@ -310,15 +310,16 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   const int slab = nb8 * 4096;
   const int limit = 227 * 1024;
   p.slot_bytes = b200_decode_slot_bytes(p.w1t != nullptr);
-  const int groups = M <= 8 ? 3 : 2;
-  int NS = 9 / groups * groups;
-  for (; NS >= groups; NS -= groups) {
-    const int region = (L->KB1 * slab > NS * slab) ? L->KB1 * slab : NS * slab;
-    if (b200_decode_smem_bytes(NS, p.slot_bytes, region) <= limit) { p.region_bytes = region; break; }
-  }
-  if (NS < groups) return B200MOE_ERR_SHAPE;
-  p.NS = NS;
-  return b200_decode_launch(p, groups, L->sms, b200_decode_smem_bytes(NS, p.slot_bytes, p.region_bytes), chained, (cudaStream_t)stream);
+  // Three workers a CTA where the ring has two stages for each of them, else two workers. (At 7168 x 2048, two layers of 8 tokens, three workers
+  // with one stage each take 529 us, two with two 425; 144 and 119 with one token.)
+  int groups = 0;
+  for (int g = M <= 8 ? 3 : 2; g >= 2 && !groups; --g)
+    for (int NS = 9 / g * g; NS >= (g == 3 ? 6 : 2); NS -= g) {
+      const int region = (L->KB1 * slab > NS * slab) ? L->KB1 * slab : NS * slab;
+      if (b200_decode_smem_bytes(NS, p.slot_bytes, region) <= limit) { groups = g, p.NS = NS, p.region_bytes = region; break; }
+    }
+  if (!groups) return B200MOE_ERR_SHAPE;
+  return b200_decode_launch(p, groups, L->sms, b200_decode_smem_bytes(p.NS, p.slot_bytes, p.region_bytes), chained, (cudaStream_t)stream);
 }
 
 // The whole decode layer: out[M, H] (bf16) = sum_j w[t,j] * FC2_e(silu(gate) * up), e = ids[t,j]. M <= 16.

@@ -21,6 +21,25 @@ def edge_layer(hidden, inter=192):
     return cfg, *_layers[hidden, inter]
 
 
+def bare_forward(w, x, ids, wts):
+    """The decode call of a second handle on the same weights that has not been prepacked; None where it refuses the shape."""
+    import ctypes as C
+    from sm120fp4_b200 import _lib
+    h, bare = _lib.lib(), C.c_void_p()
+    _lib.check(h.b200moe_layer_create(C.byref(bare), w.E, w.H, w.I, w.k, _lib.ptr(w.q1), _lib.ptr(w.s1), _lib.ptr(w.alpha1), _lib.ptr(w.q2),
+                                      _lib.ptr(w.s2), _lib.ptr(w.alpha2)), "create")
+    ws = torch.zeros_like(w.workspace)
+    x, ids, wts = x.cuda(), ids.cuda(), wts.cuda()
+    out = torch.empty_like(x)
+    rc = h.b200moe_decode_forward(bare, _lib.ptr(x), _lib.ptr(ids), _lib.ptr(wts), x.shape[0], _lib.ptr(out), _lib.ptr(ws), ws.numel(), _lib.stream_ptr())
+    torch.cuda.synchronize()
+    h.b200moe_layer_destroy(bare)
+    if rc == -2:
+        return None
+    _lib.check(rc, "decode")
+    return out
+
+
 # 512: 8 tokens are the last, 256 blocks; 4096: one token is; 2048 x 2; 3200 = 12.5 K boxes
 @pytest.mark.parametrize("hidden,m", [(512, 8), (512, 9), (2048, 2), (2048, 3), (3072, 1), (3072, 16), (3200, 1), (3200, 8), (3200, 9), (3200, 16),
                                       (4096, 1), (4096, 2), (4096, 8), (4096, 9), (4096, 16)])
@@ -93,6 +112,32 @@ def test_tile_records_and_checkpoint_layout_agree(hidden, inter):
         w.set_decode_impl("auto")
         torch.cuda.synchronize()
         h.b200moe_layer_destroy(bare)
+
+
+# Up to 8 tokens a block has three workers while its ring has two stages for each (hidden sizes up to 6656, 5888 from the checkpoint layout),
+# then two; the largest hidden sizes leave them one stage each: 11264, and 11008 from the checkpoint layout. Above 8 tokens x takes twice the
+# room: 5632 and 5376.
+@pytest.mark.parametrize("hidden,ms", [(5376, (1, 9, 16)), (5504, (16,)), (5632, (9, 16)), (6144, (1, 8)), (7168, (1, 8)), (10496, (1, 8)), (11008, (1, 8)), (11264, (1, 8))])
+def test_widest_layers(hidden, ms):
+    cfg, w, ow = edge_layer(hidden, 128)
+    for m in ms:
+        x, ids, wts = inputs(cfg, m, 20 + m)
+        check_layer_output(run(w, x, ids, wts), O.moe_reference(x.float().numpy(), ow, ids.numpy(), wts.numpy()), f"hidden {hidden}, {m} tokens")
+        bare = bare_forward(w, x, ids, wts)
+        if hidden > (11008 if m <= 8 else 5376):
+            assert bare is None
+        else:
+            assert torch.equal(bare, w.forward(x.cuda(), ids.cuda(), wts.cuda()))
+
+
+@pytest.mark.parametrize("hidden,m", [(11392, 1), (11392, 8), (5760, 9)])
+def test_hidden_sizes_beyond_the_kernel_are_refused(hidden, m):
+    import sm120fp4_b200._lib as L
+    cfg, w, _ = edge_layer(hidden, 64)
+    x, ids, wts = inputs(cfg, m, 3)
+    with pytest.raises(L.B200MoEError):
+        w.forward(x.cuda(), ids.cuda(), wts.cuda())
+    w.status()
 
 
 # Where K is cut and in which order partial sums are added follows from the shares of the tile list alone, not from how many workers deal
