@@ -94,8 +94,11 @@ int b200moe_layer_sm_count(const b200moe_layer* layer);
 /* tcgen05 decode path: the kernel-native weight copy - every (expert, block, K box) tile as one contiguous 18 KB record of
  * codes (shared-memory image) + scale tiles - built once per layer into caller-owned device memory of about the size of
  * the weights (the counterpart of the load-time re-layout in sm120fp4/vllm_backend.py:193-206; the caller may drop the
- * checkpoint-layout codes afterwards if it only decodes). After prepack, b200moe_decode_forward runs the tcgen05 kernel;
- * b200moe_layer_set_decode_impl picks 0 = automatic, 1 = mma.sync kernel, 2 = tcgen05 kernel; b200moe_layer_set_act_scale
+ * checkpoint-layout codes afterwards: b200moe_layer_release_checkpoint). After prepack, b200moe_decode_forward runs the tcgen05
+ * kernel up to hidden size 3072, and b200moe_decode_forward, _mid_forward and _prefill_forward take codes and block scales from
+ * the records at every size: weights changed in place count from the next b200moe_layer_prepack (into the same buffer,
+ * ordered on the stream) on. The alphas are read at every call, and so are codes and scales by b200moe_decode_fc1 / _fc2 and by the
+ * mma.sync kernel under b200moe_layer_set_decode_impl 1. That call picks 0 = automatic, 1 = mma.sync kernel, 2 = tcgen05 kernel; b200moe_layer_set_act_scale
  * sets the global scale of the first NVFP4 term of the FC1->FC2 activations (default 8). */
 long long b200moe_layer_prepack_bytes(const b200moe_layer* layer);
 int b200moe_layer_prepack(b200moe_layer* layer, void* buffer, long long buffer_bytes, void* stream);

@@ -282,7 +282,9 @@ static int decode_common(const b200moe_layer* L, const void* x, const int* ids, 
   DecodeParams p;
   memset(&p, 0, sizeof(p));
   p.tm1 = L->tm1, p.tm2 = L->tm2;
-  p.w1t = L->w1t, p.w2t = L->w2t;
+  // The whole layer runs from the tile records where it takes this kernel by itself. The stand-alone halves, whose callers pass the weights, and
+  // the kernel asked for by b200moe_layer_set_decode_impl read the checkpoint layout as it stands at the call.
+  if (phases == 3 && L->decode_impl != 1) p.w1t = L->w1t, p.w2t = L->w2t;
   p.s1 = (const uint8_t*)L->s1, p.s2 = (const uint8_t*)L->s2;
   p.alpha1 = L->alpha1, p.alpha2 = L->alpha2;
   p.x = (const __nv_bfloat16*)x, p.ids = ids, p.wts = wts, p.out = (__nv_bfloat16*)out;

@@ -111,7 +111,7 @@ class Weights:
         dev = self.device = q1.device
         self.ws_bytes = int(h.b200moe_layer_workspace_bytes(self._h))
         self.workspace = torch.zeros(self.ws_bytes, dtype=torch.uint8, device=dev)
-        # kernel-native copies for the tcgen05 decode kernel (FC1 scale tiles per 64-column block, alpha2 normaliser)
+        # the tile records that `forward` reads: weights changed in place count from the next b200moe_layer_prepack on
         self.prepack = torch.empty(int(h.b200moe_layer_prepack_bytes(self._h)), dtype=torch.uint8, device=dev)
         _lib.check(h.b200moe_layer_prepack(self._h, _lib.ptr(self.prepack), self.prepack.numel(), _lib.stream_ptr()), "prepack")
         if os.environ.get("B200MOE_DECODE", "") in ("mma", "tcgen05"):   # force one decode kernel (default: chosen by batch size)

@@ -87,31 +87,48 @@ def test_nan_values_do_not_set_the_row_scale(m, which):
     assert got == np.float32(1) / (np.float32(2688) / amax)
 
 
-# The mma.sync kernel on a layer that has not been prepacked reads the checkpoint layout instead of the tile records: the same tiles in
-# the same order, so the same bits. Three groups of workers up to 8 tokens, two above; intermediate sizes with a whole and a part
-# 128-row scale run and K box.
-@pytest.mark.parametrize("hidden,inter", [(256, 64), (640, 192), (3200, 192), (4096, 320)])
+# Wide layers decode from the tile records, under set_decode_impl("mma") and without a prepack from the checkpoint layout: the same tiles
+# in the same order, so the same bits. Intermediate sizes with a whole and a part 128-row scale run and K box.
+@pytest.mark.parametrize("hidden,inter", [(3200, 64), (3328, 192), (4096, 320), (6144, 192)])
 def test_tile_records_and_checkpoint_layout_agree(hidden, inter):
-    import ctypes as C
-    from sm120fp4_b200 import _lib
     cfg, w, _ = edge_layer(hidden, inter)
-    h, bare = _lib.lib(), C.c_void_p()
-    _lib.check(h.b200moe_layer_create(C.byref(bare), w.E, w.H, w.I, w.k, _lib.ptr(w.q1), _lib.ptr(w.s1), _lib.ptr(w.alpha1), _lib.ptr(w.q2),
-                                      _lib.ptr(w.s2), _lib.ptr(w.alpha2)), "create")
-    ws = torch.zeros_like(w.workspace)
-    w.set_decode_impl("mma")
-    try:
-        for m in (1, 8, 9, 16):
-            x, ids, wts = (t.cuda() for t in inputs(cfg, m, 50 + m))
-            out = torch.empty_like(x)
-            _lib.check(h.b200moe_decode_forward(bare, _lib.ptr(x), _lib.ptr(ids), _lib.ptr(wts), m, _lib.ptr(out), _lib.ptr(ws), ws.numel(),
-                                                _lib.stream_ptr()), "decode")
-            assert torch.equal(out, w.forward(x, ids, wts)), m
-        w.status()
-    finally:
-        w.set_decode_impl("auto")
-        torch.cuda.synchronize()
-        h.b200moe_layer_destroy(bare)
+    for m in (1, 8, 9, 16) if hidden <= 5376 else (1, 8):
+        x, ids, wts = inputs(cfg, m, 50 + m)
+        out = run(w, x, ids, wts).clone()
+        assert torch.equal(out, bare_forward(w, x, ids, wts)), m
+        w.set_decode_impl("mma")
+        try:
+            assert torch.equal(out, run(w, x, ids, wts)), m
+        finally:
+            w.set_decode_impl("auto")
+
+
+@pytest.mark.parametrize("hidden", [640, 3200])
+def test_weights_changed_in_place(hidden):
+    """The halves and the mma.sync kernel by request compute with the weights as they are at the call; the layer call follows a new prepack."""
+    from sm120fp4_b200 import _lib
+    from sm120fp4_b200.vllm_backend import Weights
+    cfg = dict(experts=16, hidden=hidden, inter=192, top_k=4)
+    w, _ = make_layer(**cfg, seed=12)
+    w.q1.copy_(w.q1.roll(1, 0))
+    w.q2.copy_(w.q2.roll(1, 0))
+    fresh = Weights(w.q1.clone(), w.s1, w.alpha1, w.q2.clone(), w.s2, w.alpha2, w.k, scale_layout="128x4")
+    for m in (3, 12):
+        x, ids, wts = (t.cuda() for t in inputs(cfg, m, 5))
+        act = [torch.zeros(m * w.k, w.I, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        out = [torch.empty_like(x) for _ in range(2)]
+        for i, layer in enumerate((w, fresh)):
+            layer.fc1(x, ids, wts, act[i])
+            layer.fc2(act[0], ids, wts, out[i])
+        assert torch.equal(*act) and torch.equal(*out)
+        for layer in (w, fresh):
+            layer.set_decode_impl("mma")
+        assert torch.equal(w.forward(x, ids, wts), fresh.forward(x, ids, wts))
+        for layer in (w, fresh):
+            layer.set_decode_impl("auto")
+    _lib.check(_lib.lib().b200moe_layer_prepack(w._h, _lib.ptr(w.prepack), w.prepack.numel(), _lib.stream_ptr()), "prepack")
+    assert torch.equal(w.forward(x, ids, wts), fresh.forward(x, ids, wts))
+    w.status()
 
 
 # Up to 8 tokens a block has three workers while its ring has two stages for each (hidden sizes up to 6656, 5888 from the checkpoint layout),
