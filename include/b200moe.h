@@ -103,8 +103,8 @@ int b200moe_layer_sm_count(const b200moe_layer* layer);
 long long b200moe_layer_prepack_bytes(const b200moe_layer* layer);
 int b200moe_layer_prepack(b200moe_layer* layer, void* buffer, long long buffer_bytes, void* stream);
 int b200moe_layer_set_decode_impl(b200moe_layer* layer, int impl);
-/* Forget the checkpoint-layout codes and scales (the caller may free them): from then on only the tcgen05 paths run; the
- * mma.sync kernel and b200moe_decode_fc1 / _fc2 return B200MOE_ERR_ARG. Needs b200moe_layer_prepack. The reference keeps a
+/* Forget the checkpoint-layout codes and scales (the caller may free them): the layer calls go on from the records, at every
+ * size; b200moe_layer_set_decode_impl 1 and b200moe_decode_fc1 / _fc2 return B200MOE_ERR_ARG. Needs b200moe_layer_prepack. The reference keeps a
  * single copy of the weights too: its load-time re-layout is in place (sm120fp4/vllm_backend.py:193-206). */
 int b200moe_layer_release_checkpoint(b200moe_layer* layer);
 int b200moe_layer_set_act_scale(b200moe_layer* layer, float first_term_global_scale);

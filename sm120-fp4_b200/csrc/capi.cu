@@ -180,8 +180,8 @@ extern "C" int b200moe_layer_prepack(b200moe_layer* L, void* buffer, long long b
   return B200MOE_OK;
 }
 
-// After prepack the tcgen05 paths (decode, mid-sized batches, W4A4 prefill) read only the tile records. A caller that does
-// not need the mma.sync kernel or the stand-alone FC1 / FC2 entry points may then free the checkpoint-layout codes and
+// After prepack the layer calls (decode, mid-sized batches, W4A4 prefill) read only the tile records, at every size. A caller that does
+// not need set_decode_impl 1 or the stand-alone FC1 / FC2 entry points may then free the checkpoint-layout codes and
 // scales (about half of the layer's memory); this makes the handle forget them, so that a later call that would need
 // them fails with B200MOE_ERR_ARG instead of reading freed memory.
 extern "C" int b200moe_layer_release_checkpoint(b200moe_layer* L) {
@@ -269,7 +269,7 @@ static int decode_tc(b200moe_layer* L, const void* x, const int* ids, const floa
 static int decode_common(const b200moe_layer* L, const void* x, const int* ids, const float* wts, int M, void* out, void* act_bf16,
                          int phases, int write_tables, void* ws, long long ws_bytes, bool chained, void* stream) {
   if (!L || !ids || !wts || !ws) return B200MOE_ERR_ARG;
-  if (!L->q1) return B200MOE_ERR_ARG;   // the mma.sync kernel reads the checkpoint layout, which the caller released
+  if (!L->q1 && phases != 3) return B200MOE_ERR_ARG;   // the halves read the checkpoint layout, which the caller released
   if ((phases & 1) && !x) return B200MOE_ERR_ARG;
   if ((phases & 2) && !out) return B200MOE_ERR_ARG;
   if (M < 0) return B200MOE_ERR_ARG;

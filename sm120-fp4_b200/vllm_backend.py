@@ -132,8 +132,8 @@ class Weights:
         self._ws_ptr = self.workspace.data_ptr()
 
     def release_checkpoint_layout(self) -> None:
-        """Drop the checkpoint-layout codes and scales (about half of the layer's device memory): every tcgen05 path reads
-        the tile records of the prepack only. Afterwards `set_decode_impl("mma")`, `fc1` and `fc2` raise."""
+        """Drop the checkpoint-layout codes and scales (about half of the layer's device memory): `forward` reads
+        the tile records of the prepack only, at every size. Afterwards `set_decode_impl("mma")`, `fc1` and `fc2` raise."""
         _lib.check(_lib.lib().b200moe_layer_release_checkpoint(self._h), "release_checkpoint_layout")
         self.q1 = self.q2 = self.s1 = self.s2 = self.s1_linear = self.s2_linear = None
 

@@ -103,6 +103,28 @@ def test_tile_records_and_checkpoint_layout_agree(hidden, inter):
             w.set_decode_impl("auto")
 
 
+@pytest.mark.parametrize("hidden,ms", [(3200, (1, 8, 9, 16)), (4096, (1, 8, 9, 16)), (7168, (1, 8))])
+def test_wide_layers_decode_from_the_records_alone(hidden, ms):
+    import sm120fp4_b200._lib as L
+    cfg = dict(experts=16, hidden=hidden, inter=192, top_k=4)
+    w, _ = make_layer(**cfg, seed=13)
+    batches = [inputs(cfg, m, 80 + m) for m in ms]
+    want = [run(w, *b).clone() for b in batches]
+    w.release_checkpoint_layout()
+    for b, o in zip(batches, want):
+        assert torch.equal(run(w, *b), o)
+        pinned = [t.pin_memory() for t in b]
+        host = torch.empty_like(b[0]).pin_memory()
+        w.forward_host(*pinned, host)
+        torch.cuda.synchronize()
+        assert torch.equal(host, o.cpu())
+    x, ids, wts = (t.cuda() for t in batches[0])
+    act = torch.zeros(ms[0] * w.k, w.I, dtype=torch.bfloat16, device="cuda")
+    for refused in (lambda: w.set_decode_impl("mma"), lambda: w.fc1(x, ids, wts, act), lambda: w.fc2(act, ids, wts, torch.empty_like(x))):
+        with pytest.raises(L.B200MoEError):
+            refused()
+
+
 @pytest.mark.parametrize("hidden", [640, 3200])
 def test_weights_changed_in_place(hidden):
     """The halves and the mma.sync kernel by request compute with the weights as they are at the call; the layer call follows a new prepack."""
