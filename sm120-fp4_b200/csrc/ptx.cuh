@@ -176,6 +176,14 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// the same barrier, and whether all of the threads say yes
+__device__ __forceinline__ bool named_bar_and(int id, int threads, bool yes) {
+  uint32_t all;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred p, %2, %3, p;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(all) : "r"((uint32_t)yes), "r"(id), "r"(threads) : "memory");
+  return all != 0;
+}
+
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -379,8 +379,11 @@ constexpr int kQcSmem = kQcSlots * kQcUnit + (int)sizeof(QcShared) + 128;
 // that time is there. Reading the halves in turn and putting them in order takes as long.)
 __device__ __forceinline__ void load_shared(uint32_t at, Raw16<__nv_bfloat16>& v) { v.r[0] = lds128(at), v.r[1] = lds128(at + 16); }
 
+// A wait inside the block gives up after `tries`. The warp that gave up works without what it waited for to the end of the call (a
+// barrier's parity tells only whether the phase before has passed): values come from global memory, group maxima from the worker itself. The
+// bytes are the same, and the block does not leave before its copies have landed.
 __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_bfloat16* x, int groups, int units, QuantGeom q, float* gs_out, uint8_t* packed, uint8_t* sf,
-                                                                     unsigned* scratch, int polls) {
+                                                                     unsigned* scratch, int polls, unsigned tries) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
   QcShared& S = *reinterpret_cast<QcShared*>(smem + kQcSlots * kQcUnit);
@@ -408,14 +411,17 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
       const uint64_t once = policy_evict_first();
       int slot = 0;
       uint32_t ph = 1;   // parity that a free slot's barrier has completed: the first pass finds all slots free
-      for (int k = 0; k < n; ++k) {
+      int k = 0;
+      for (; k < n; ++k) {
         const int2 at = place(k);
         const int i0 = at.y * kUnitBlocks, bytes = min(kUnitBlocks, nblk - i0) * 32;
-        mbar_wait(&S.empty[slot], ph, &S.abort_flag);
+        if (!mbar_wait(&S.empty[slot], ph, &S.abort_flag, tries)) break;
         mbar_expect_tx(&S.full[slot], bytes);
         bulk_load_hint(smem + slot * kQcUnit, x + ((long long)at.x * nblk + i0) * 16, bytes, &S.full[slot], once);
         if (++slot == kQcSlots) { slot = 0; ph ^= 1u; }
       }
+      for (int j = max(0, k - kQcSlots); j < k; ++j)   // the copies that may still be under way
+        for (int i = 0; i < (1 << 20) && !mbar_try_wait(&S.full[j % kQcSlots], (uint32_t)((j / kQcSlots) & 1)); ++i) {}
     }
   } else if (warp == 8 * kQcWorkers + 1) {
     // ============================================================== the maximum of each unit's group, looked at `polls` times
@@ -440,7 +446,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         __nanosleep(50);
       }
       m = __reduce_max_sync(0xffffffffu, m);
-      if (k >= kQcLooks) mbar_wait_warp(smem_u32(&S.taken[k % kQcLooks]), (uint32_t)((k / kQcLooks - 1) & 1), &S.abort_flag);
+      if (k >= kQcLooks && !mbar_wait_warp(smem_u32(&S.taken[k % kQcLooks]), (uint32_t)((k / kQcLooks - 1) & 1), &S.abort_flag, tries)) break;
       if (lane == 0) {
         S.gmax[k % kQcLooks] = ok ? m : kMissing;
         mbar_arrive(&S.known[k % kQcLooks]);
@@ -454,6 +460,28 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     const uint64_t once = policy_evict_first();
     const uint32_t ring = smem_u32(smem);
     float gs_table = -1.f;
+    bool copied = true, told = true;   // this warp has not given up on the copies, on the maxima
+    // body(block) for this thread's blocks i0 + wt + j * threads of a unit, which the slot holds
+    auto blocks = [&](int g, int slot, int i0, auto&& body) {
+      const int left = nblk - i0 - wt;
+      if (copied) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+          if (j * kQcWorkerThreads < left) {
+            Raw16<__nv_bfloat16> v;
+            load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
+            body(j, v);
+          }
+        }
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < kPer && j * kQcWorkerThreads < left; ++j) {
+          Raw16<__nv_bfloat16> v;
+          load_raw(x + ((long long)g * nblk + i0 + wt + j * kQcWorkerThreads) * 16, q.wide, false, v);
+          body(j, v);
+        }
+      }
+    };
     // The maximum of group g by this worker alone, for units whose blocks have not run for a long time (another kernel holds their
     // SMs: nothing says that the grid is resident as a whole). What it finds out it publishes, so that others need not.
     auto group_max = [&](int g) {
@@ -489,17 +517,10 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     for (int k = grp; k < n + kQcWorkers; k += kQcWorkers) {
       if (k < n) {
         const int2 at = place(k);
-        const int slot = k % kQcSlots, left = nblk - at.y * kUnitBlocks - wt;
-        mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag);
+        const int slot = k % kQcSlots;
+        copied = copied && mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries);
         float m = 0.f;
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-          if (j * kQcWorkerThreads < left) {
-            Raw16<__nv_bfloat16> v;
-            load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
-            m = fmaxf(m, amax_raw(v));
-          }
-        }
+        blocks(at.x, slot, at.y * kUnitBlocks, [&](int, const Raw16<__nv_bfloat16>& v) { m = fmaxf(m, amax_raw(v)); });
         __syncwarp();
         unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
         if (lane == 0) S.wm[grp][buf][ww] = mb;
@@ -513,13 +534,13 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
       const int kq = k - kQcWorkers;
       if (kq < 0) continue;
       const int2 at = place(kq);
-      const int g = at.x, u = at.y, slot = kq % kQcSlots, i0 = u * kUnitBlocks, left = nblk - i0 - wt;
-      mbar_wait_warp(smem_u32(&S.known[kq % kQcLooks]), (uint32_t)((kq / kQcLooks) & 1), &S.abort_flag);
-      unsigned m = S.gmax[kq % kQcLooks];
-      if (m == kMissing) m = group_max(g);
+      const int g = at.x, u = at.y, slot = kq % kQcSlots, i0 = u * kUnitBlocks;
+      told = told && mbar_wait_warp(smem_u32(&S.known[kq % kQcLooks]), (uint32_t)((kq / kQcLooks) & 1), &S.abort_flag, tries);
+      unsigned m = told ? S.gmax[kq % kQcLooks] : kMissing;
+      const bool all = named_bar_and(1 + grp, kQcWorkerThreads, m != kMissing);   // (and nobody is at the table any more)
+      if (wt == 0 && told) mbar_arrive(&S.taken[kq % kQcLooks]);
+      if (!all) m = group_max(g);
       const float gs = scale_of(__uint_as_float(m));
-      sync();                                     // nobody is at the table any more, and all have the maximum
-      if (wt == 0) mbar_arrive(&S.taken[kq % kQcLooks]);
       if (gs != gs_table) fill_scale_table(S.table[grp], gs, wt, kQcWorkerThreads);
       gs_table = gs;
       sync();
@@ -531,25 +552,20 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         r = (int)(((unsigned long long)(unsigned)(i0 + wt) * q.bpr_inv) >> q.bpr_shift);
         c = i0 + wt - r * q.bpr;
       }
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) {
-        if (j * kQcWorkerThreads < left) {
-          Raw16<__nv_bfloat16> v;
-          load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
-          uint2 pk;
-          const uint32_t sb = quantize_raw(v, gs, S.table[grp], pk);
-          st_policy(codes + j * kQcWorkerThreads, pk, once);
-          if (q.layout == 0) {
-            sfl[j * kQcWorkerThreads] = (uint8_t)sb;
-          } else {
-            sfg[((r >> 7) * q.nkt + (c >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (c & 3)] = (uint8_t)sb;
-            r += q.step_r, c += q.step_c;
-            if (c >= q.bpr) { c -= q.bpr; ++r; }
-          }
+      blocks(g, slot, i0, [&](int j, const Raw16<__nv_bfloat16>& v) {
+        uint2 pk;
+        const uint32_t sb = quantize_raw(v, gs, S.table[grp], pk);
+        st_policy(codes + j * kQcWorkerThreads, pk, once);
+        if (q.layout == 0) {
+          sfl[j * kQcWorkerThreads] = (uint8_t)sb;
+        } else {
+          sfg[((r >> 7) * q.nkt + (c >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (c & 3)] = (uint8_t)sb;
+          r += q.step_r, c += q.step_c;
+          if (c >= q.bpr) { c -= q.bpr; ++r; }
         }
-      }
+      });
       __syncwarp();
-      if (lane == 0) mbar_arrive(&S.empty[slot]);
+      if (lane == 0 && copied) mbar_arrive(&S.empty[slot]);
       if (u == 0) {
         if (wt == 0) gs_out[g] = gs;
         if (q.layout == 1) zero_padding(sfg, q, wt, kQcWorkerThreads);
@@ -580,6 +596,7 @@ static int quant_units(int dtype, int rows, int K) {
 // Inputs beyond L2 take the resident form. Below, latency is not what the other form waits for: 8 x 1536 x 2048 bf16 (50 MB) 21.4 us against
 // 25.0, 60 x 384 x 768 15.2 against 17.6; above, 128 x 1024 x 1024 (268 MB) 83.4 against 75.9.
 constexpr long long kQResidentFrom = 126ll << 20;
+constexpr unsigned kQTries = 1u << 20;   // of a wait inside a block, for another warp or a copy
 constexpr int kQPolls = 2048;   // looks of ~0.7 us: a unit takes 5 to 10 us, so the words are there long before unless the grid is held up
 
 static bool quant_one_cluster(int groups, int rows, int K) { return groups == 1 && (long long)rows * (K / 16) <= kQSmallMaxBlocks; }
@@ -609,7 +626,7 @@ static int quant_separate(const void* x, int dtype, int groups, int rows, int K,
 // then only ever passed to this function; two calls that may overlap on the GPU (a replay of a captured call is one) need one each.
 // Null where b200moe_quantize_own_scale_workspace_bytes says 0.
 static int quantize_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout, void* workspace,
-                              long long workspace_bytes, int polls, void* stream) {
+                              long long workspace_bytes, int polls, unsigned tries, void* stream) {
   if (!x || !gs_out || !packed || !sf || groups <= 0 || groups > 65535 || rows < 0) return B200MOE_ERR_ARG;
   if (K <= 0 || K % 16) return B200MOE_ERR_SHAPE;
   if ((dtype != 0 && dtype != 1) || (sf_layout != 0 && sf_layout != 1)) return B200MOE_ERR_ARG;
@@ -672,7 +689,7 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
         B200_CUDA_TRY(cudaFuncSetAttribute((const void*)k_quantize_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, kQcSmem));
         if (dev <= 31) configured |= 1u << dev;
       }
-      void* args[] = {(void*)&x, (void*)&groups, (void*)&ru, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&polls};
+      void* args[] = {(void*)&x, (void*)&groups, (void*)&ru, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&polls, (void*)&tries};
       return launch_kernel((const void*)k_quantize_resident, G, kQcThreads, kQcSmem, true, args, st);
     }
   }
@@ -684,11 +701,12 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
 
 extern "C" int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
                                                 void* workspace, long long workspace_bytes, void* stream) {
-  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, kQPolls, stream);
+  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, kQPolls, kQTries, stream);
 }
 
-// The same call that looks `polls` times for a unit's maximum before it works it out again (0: never waits), for tests of that way.
+// The same call that looks `polls` times for a unit's maximum before it works it out again (0: never waits), for tests of that way. Below
+// zero it never waits for other blocks, and a wait inside a block gives up after -1 - polls tries.
 extern "C" int b200moe_quantize_own_scale_probe(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf, int sf_layout,
                                                 void* workspace, long long workspace_bytes, int polls, void* stream) {
-  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, polls, stream);
+  return quantize_own_scale(x, dtype, groups, rows, K, gs_out, packed, sf, sf_layout, workspace, workspace_bytes, polls < 0 ? 0 : polls, polls < 0 ? (unsigned)(-1 - polls) : kQTries, stream);
 }

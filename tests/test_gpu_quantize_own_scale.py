@@ -175,6 +175,24 @@ def test_blocks_that_do_not_wait(groups, rows, k, dtype, polls):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("tries", [0, 1, 2, 70])
+@pytest.mark.parametrize("groups,rows,k", [(45, 1530, 1040), (8400, 500, 16)])
+def test_waits_inside_a_block_that_give_up(groups, rows, k, tries):
+    """More than 126 MB of bf16: a warp whose wait for a copy or a maximum runs out goes on without it. The same bytes."""
+    import sm120fp4_b200 as pkg
+    import sm120fp4_b200._lib as L
+    w = torch.randn(groups, rows, k, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda", dtype=torch.bfloat16)
+    w *= torch.linspace(0.1, 9.0, groups, device="cuda")[:, None, None].to(torch.bfloat16)
+    want = pkg.quantize_nvfp4_experts(w)
+    h = L.lib()
+    ws = torch.zeros(h.b200moe_quantize_own_scale_workspace_bytes(0, groups, rows, k), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        got = [torch.empty_like(t) for t in want]
+        L.check(h.b200moe_quantize_own_scale_probe(L.ptr(w), 0, groups, rows, k, L.ptr(got[2]), L.ptr(got[0]), L.ptr(got[1]), 0, L.ptr(ws), ws.numel(),
+                                                   -1 - tries, L.stream_ptr()), "probe")
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("dtype,groups", [(torch.float32, 24), (torch.bfloat16, 48)])   # (the second stays in shared memory)
 def test_two_calls_at_once(dtype, groups):
     """Two large calls on two streams share the GPU's SMs in whatever way they are scheduled."""
