@@ -427,6 +427,10 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     // ============================================================== the maximum of each unit's group, looked at `polls` times
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
+      // What a worker learns of unit k also tells it that units up to k have landed. It waits for unit k + 7 later on, in the same slot: the parity of
+      // the slot's barrier says something only once the phase before is over. (That the maxima are there does not tell: another block may
+      // have worked them out.)
+      if (!mbar_wait_warp(smem_u32(&S.full[k % kQcSlots]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries)) break;
       const unsigned long long* gw = words + (long long)place(k).x * units;
       unsigned m = 0u;
       bool ok = false;
@@ -518,7 +522,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
       if (k < n) {
         const int2 at = place(k);
         const int slot = k % kQcSlots;
-        copied = copied && mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries);
+        copied = copied && told && mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries);
         float m = 0.f;
         blocks(at.x, slot, at.y * kUnitBlocks, [&](int, const Raw16<__nv_bfloat16>& v) { m = fmaxf(m, amax_raw(v)); });
         __syncwarp();
