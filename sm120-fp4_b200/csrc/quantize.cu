@@ -365,6 +365,11 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
 constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
 constexpr int kQcLooks = 8;        // maxima that may wait for their worker
+// Words of a group that a lane has in flight together, also the last few: a look at a group takes one to three round trips. (With the words of the
+// last incomplete four one after the other it took up to five, and with more than three the blocks waited for it: 320 MB of bf16 in groups
+// of 102 units 107 us, now 91; of 240 units 117, now 93; of 352 units 117, now 100; of 192 units 91 both. All of a group's words at once:
+// 92, 93, 104 and 92; but 128 x 1536 x 2048 with swizzled scales 210 instead of 206.6.)
+constexpr int kQcWords = 4;
 constexpr int kQcBlocks = kQcUnit / 32;   // 16-value blocks of a unit
 struct QcShared {
   uint64_t full[kQcSlots], empty[kQcSlots], known[kQcLooks], taken[kQcLooks];
@@ -438,16 +443,20 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
 #pragma unroll 1
       for (;;) {
         m = 0u, ok = looks > 0;
-#pragma unroll 4
-        for (int w = lane; w < units; w += 32) {
-          const unsigned long long word = ld_relaxed_gpu_u64(gw + w);
-          ok &= (unsigned)(word >> 32) == call;
-          m = max(m, (unsigned)word);
+#pragma unroll 1
+        for (int w0 = lane; w0 < units; w0 += 32 * kQcWords) {
+          unsigned long long word[kQcWords];
+#pragma unroll
+          for (int i = 0; i < kQcWords; ++i)
+            if (w0 + 32 * i < units) word[i] = ld_relaxed_gpu_u64(gw + w0 + 32 * i);
+#pragma unroll
+          for (int i = 0; i < kQcWords; ++i)
+            if (w0 + 32 * i < units) { ok &= (unsigned)(word[i] >> 32) == call; m = max(m, (unsigned)word[i]); }
         }
         ok = __all_sync(0xffffffffu, ok);
         if (ok || looks <= 0) break;
         --looks;
-        __nanosleep(50);
+        __nanosleep(500);
       }
       m = __reduce_max_sync(0xffffffffu, m);
       if (k >= kQcLooks && !mbar_wait_warp(smem_u32(&S.taken[k % kQcLooks]), (uint32_t)((k / kQcLooks - 1) & 1), &S.abort_flag, tries)) break;
@@ -691,7 +700,8 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
         B200_CUDA_TRY(cudaFuncSetAttribute((const void*)k_quantize_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, kQcSmem));
         if (dev <= 31) configured |= 1u << dev;
       }
-      void* args[] = {(void*)&x, (void*)&groups, (void*)&ru, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&polls, (void*)&tries};
+      const int trips = (ru + 32 * kQcWords - 1) / (32 * kQcWords), looks = (polls + trips) / (1 + trips);   // a look takes that much longer here, with its pause
+      void* args[] = {(void*)&x, (void*)&groups, (void*)&ru, (void*)&q, (void*)&gs_out, (void*)&packed, (void*)&sf, (void*)&scratch, (void*)&looks, (void*)&tries};
       return launch_kernel((const void*)k_quantize_resident, G, kQcThreads, kQcSmem, true, args, st);
     }
   }
