@@ -18,10 +18,13 @@ constexpr int kQgThreads = 256;                                  // of the large
 constexpr int kQSmallPerThread = 2;                              // 16-value blocks a thread keeps in registers
 constexpr int kQSmallMaxBlocks = 8 * kQThreads * kQSmallPerThread;
 template <typename T> constexpr int kQPerThread = sizeof(T) == 2 ? 8 : 4;   // 16-value blocks a thread takes of one work unit (64 KB of input)
-// Input bytes between a group's two passes. What is read for the second time and the codes are marked to leave L2 first, so that L2 holds
-// about this and what is in flight: 128 x 1536 x 2048 bf16 take 238 us (20 MB 239, 12 MB 277, 45 MB 243; unmarked 248 to 251), 60 x 1024 x
-// 1536 fp32 91.5 (96, 114, 92.5; unmarked 98 to 100).
+// Input bytes between a group's two passes. Of large inputs what is read for the second time and the codes are marked to leave L2 first, so
+// that L2 holds about this and what is in flight: 60 x 1024 x 1536 fp32 take 91.5 us (20 MB 96, 12 MB 114, 45 MB 92.5; unmarked 98 to 100).
 constexpr long long kQWindowBytes = 30ll << 20;
+// Inputs above this are large: 8192 x 4096 fp32 (128 MB) 58.7 us a call on new inputs with the marks and 63.2 without, 16 x 1536 x 2048 bf16 (96 MB)
+// 35.9 and 37.4. Below, L2 holds everything and the next kernel finds it there: 4096 x 4096 bf16 18.5 and 17.7 us again and again on the
+// same input, 8192 x 2048 fp32 (64 MB) 24.6 and 23.9, 8 x 1536 x 2048 bf16 with another look at the input behind it 56.8 and 55.3.
+constexpr long long kQMarkFrom = 64ll << 20;
 
 struct QuantGeom {
   int rows, bpr;           // rows of a group, 16-value blocks per row
@@ -29,6 +32,7 @@ struct QuantGeom {
   long long sf_stride;     // scale bytes of a group
   int nkt;
   bool wide;               // x is 32-byte aligned
+  bool mark;               // what is not needed again leaves L2 first
   // i / bpr = i * bpr_inv >> bpr_shift with bpr_inv = ceil(2^shift / bpr): exact while i * (bpr_inv * bpr - 2^shift) < 2^shift, which
   // i < 2^30 and shift = 30 + the bits of bpr grant
   unsigned long long bpr_inv;
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
     const T* src = x + ((long long)at.x * nblk + i0 + tid) * 16;
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
-      if (j * kQgThreads < left) load_raw(src + j * kQgThreads * 16, q.wide, at.z != 0, v[j]);
+      if (j * kQgThreads < left) load_raw(src + j * kQgThreads * 16, q.wide, q.mark && at.z != 0, v[j]);
   };
   // The maximum of group g by this block alone, for units whose blocks have not run for a long time (another kernel holds their SMs:
   // nothing says that the grid is resident as a whole). What it finds out it publishes, so that others need not.
@@ -329,7 +333,8 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
       if (j * kQgThreads < left) {
         uint2 pk;
         const uint32_t sb = quantize_raw(v[j], gs, s_table, pk);
-        st_policy(codes + j * kQgThreads, pk, once);
+        if (q.mark) st_policy(codes + j * kQgThreads, pk, once);
+        else __stcg(codes + j * kQgThreads, pk);
         if (q.layout == 0) {
           sfl[j * kQgThreads] = (uint8_t)sb;
         } else {
@@ -650,6 +655,7 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
   q.rows = rows, q.bpr = K / 16, q.layout = sf_layout, q.nkt = (q.bpr + 3) / 4;
   q.sf_stride = sf_layout == 0 ? (long long)rows * q.bpr : ((rows + 127LL) / 128 * 128) * q.nkt * 4;
   q.wide = ((uintptr_t)x & 31) == 0;
+  q.mark = groups * ((long long)rows * K) * (dtype == 0 ? 2 : 4) > kQMarkFrom;
   q.bpr_shift = 30;
   for (int b = q.bpr; b; b >>= 1) ++q.bpr_shift;
   q.bpr_inv = ((1ULL << q.bpr_shift) + q.bpr - 1) / q.bpr;
