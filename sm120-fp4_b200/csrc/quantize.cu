@@ -437,10 +437,6 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     // ============================================================== the maximum of each unit's group, looked at `polls` times
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
-      // What a worker learns of unit k also tells it that units up to k have landed. It waits for unit k + 7 later on, in the same slot: the parity of
-      // the slot's barrier says something only once the phase before is over. (That the maxima are there does not tell: another block may
-      // have worked them out.)
-      if (!mbar_wait_warp(smem_u32(&S.full[k % kQcSlots]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries)) break;
       const unsigned long long* gw = words + (long long)place(k).x * units;
       unsigned m = 0u;
       bool ok = false;
@@ -464,6 +460,10 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         __nanosleep(500);
       }
       m = __reduce_max_sync(0xffffffffu, m);
+      // What a worker learns of unit k also tells it that units up to k have landed. It waits for unit k + 7 later on, in the same slot: the parity of
+      // the slot's barrier says something only once the phase before is over. (That the maxima are there does not tell: another block may
+      // have worked them out. Ahead of the looks this wait holds them up: 16000 x 128 x 64 93.1 us instead of 90.8.)
+      if (!mbar_wait_warp(smem_u32(&S.full[k % kQcSlots]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries)) break;
       if (k >= kQcLooks && !mbar_wait_warp(smem_u32(&S.taken[k % kQcLooks]), (uint32_t)((k / kQcLooks - 1) & 1), &S.abort_flag, tries)) break;
       if (lane == 0) {
         S.gmax[k % kQcLooks] = ok ? m : kMissing;
