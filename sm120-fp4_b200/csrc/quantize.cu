@@ -693,12 +693,13 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
     sms = n;
   }
   if (dtype == 0 && groups * nblk * 32 > kQResidentFrom) {
-    // The resident form where a group's units are at most 2.4 rounds of the grid: its last maximum is then published by the time that
-    // the first unit's worker, three units on, quantises it. (With two more rounds of lag only one slot would be left to fill.)
+    // The resident form where a group's units are at most 1.75 rounds of the grid: beyond, the blocks wait for maxima that stand up to three rounds
+    // ahead of the unit to be quantised, as many as lie between a worker's two passes over it. 320 MB of bf16, us in this form (in the other): groups of 256
+    // units 93.4 (95.6), 272 109.3 (97.6), 288 106.7 (98.2), 320 102.7 (95.1), 352 102.5 (93.7).
     const int ru = quant_resident_units(dtype, rows, K);
     const long long all = (long long)groups * ru;
     const int G = (int)(all < sms ? all : sms);
-    if (5LL * ru <= 12LL * G && all < 0x7fffffffLL) {
+    if (4LL * ru <= 7LL * G && all < 0x7fffffffLL) {
       static thread_local unsigned configured = 0;   // bit d: device d has the attribute
       int dev = 0;
       B200_CUDA_TRY(cudaGetDevice(&dev));

@@ -38,10 +38,10 @@ def test_stacked_matrices(groups, rows, k, swizzle):
         assert np.array_equal(sf[g].cpu().numpy(), O.to_128x4(wsf) if swizzle else wsf)
 
 
-# More than 126 MB of bf16 in groups of up to 11 MB stay in shared memory between the passes, in units of 1024 blocks of 16 values: groups
-# of many units with a ragged last one, of one ragged unit, and the largest that the form takes (2.4 rounds of 148 units) beside the
-# first that it does not. The fp32 copy of the same values goes the other way, and its bytes are the same.
-@pytest.mark.parametrize("groups,rows,k", [(65, 1000, 1040), (8400, 500, 16), (13, 2840, 2048), (13, 2848, 2048)])
+# More than 126 MB of bf16 in groups of up to 8 MB stay in shared memory between the passes, in units of 1024 blocks of 16 values: groups
+# of many units with a ragged last one, of one ragged unit, and the largest that the form takes (1.75 rounds of 148 units) beside the
+# first that it does not and larger ones. The fp32 copy of the same values goes the other way, and its bytes are the same.
+@pytest.mark.parametrize("groups,rows,k", [(65, 1000, 1040), (8400, 500, 16), (16, 2072, 2048), (16, 2080, 2048), (13, 2840, 2048), (13, 2848, 2048)])
 def test_large_inputs_on_chip(groups, rows, k):
     import sm120fp4_b200 as pkg
     g = torch.Generator(device="cuda").manual_seed(rows)
