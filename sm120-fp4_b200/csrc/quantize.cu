@@ -21,9 +21,10 @@ template <typename T> constexpr int kQPerThread = sizeof(T) == 2 ? 8 : 4;   // 1
 // Input bytes between a group's two passes. Of large inputs what is read for the second time and the codes are marked to leave L2 first, so
 // that L2 holds about this and what is in flight: 60 x 1024 x 1536 fp32 take 91.5 us (20 MB 96, 12 MB 114, 45 MB 92.5; unmarked 98 to 100).
 constexpr long long kQWindowBytes = 30ll << 20;
-// Inputs above this are large: 8192 x 4096 fp32 (128 MB) 58.7 us a call on new inputs with the marks and 63.2 without, 16 x 1536 x 2048 bf16 (96 MB)
-// 35.9 and 37.4. Below, L2 holds everything and the next kernel finds it there: 4096 x 4096 bf16 18.5 and 17.7 us again and again on the
-// same input, 8192 x 2048 fp32 (64 MB) 24.6 and 23.9, 8 x 1536 x 2048 bf16 with another look at the input behind it 56.8 and 55.3.
+// Above this an input is large in any case; below, one whose groups do not all lie in a window is (8 x 1472 x 1344 fp32, 60 MB, 21.3 us with the marks and
+// 22.3 without; 16 x 768 x 1024 fp32 behind a copy of it 32.2 and 33.0). 8192 x 4096 fp32 (128 MB) 58.7 us on new inputs with the marks and 63.2
+// without. What is left L2 holds as a whole, and the next kernel finds it there: 2048 x 4096 bf16 again and again on the same input 12.2 us with
+// marks and 10.7 without, 4096 x 4096 18.5 and 18.0, 8192 x 2048 fp32 24.4 and 23.7.
 constexpr long long kQMarkFrom = 64ll << 20;
 
 struct QuantGeom {
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 // when the maxima of its group have normally all been published. A block is three workers of eight warps, a copying warp and one that
 // looks for the maxima. The kernel above reads every value twice into registers and is held up by latency with the 16 warps an SM that
 // its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 190 instructions per 16 values (66 %
-// busy). 128 x 1536 x 2048 bf16: 216 us, 243 above; with two workers 245. (fp32 has half the arithmetic per byte, and its 64-byte blocks
+// busy). 128 x 1536 x 2048 bf16, swizzled scales: 204 us, 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
 // meet a quarter of the banks: 60 x 1024 x 1536 take 96 us either way, or 115 here without instructions that avoid the conflicts.)
 constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
 constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
@@ -609,8 +610,10 @@ static int quant_units(int dtype, int rows, int K) {
   return (int)((nblk + unit - 1) / unit);
 }
 
-// Inputs beyond L2 take the resident form. Below, latency is not what the other form waits for: 8 x 1536 x 2048 bf16 (50 MB) 21.4 us against
-// 25.0, 60 x 384 x 768 15.2 against 17.6; above, 128 x 1024 x 1024 (268 MB) 83.4 against 75.9.
+// Inputs beyond L2 take the resident form: below the line the other one is ahead, but for the smallest groups (new inputs, swizzled scales, us in this form and
+// in the other: 16 x 1536 x 2048, 96 MB, 38.2 and 35.5; 60 x 704 x 1536, 124 MB, 46.5 and 45.5; 4000 x 500 x 16, 61 MB, 40.3 and 66.3), somewhat above it too
+// (64 x 1024 x 1024, 128 MB, 47.6 and 45.0; 24 x 1536 x 2048, 144 MB, 51.0 and 50.1; 8400 x 500 x 16, 128 MB, 76.5 and 144), then this one is (128 x 448
+// x 2048, 224 MB, 71.6 and 74.9; 128 x 1536 x 2048, 768 MB, 204 and 232).
 constexpr long long kQResidentFrom = 126ll << 20;
 constexpr unsigned kQTries = 1u << 20;   // of a wait inside a block, for another warp or a copy
 constexpr int kQPolls = 2048;   // looks of ~0.7 us: a unit takes 5 to 10 us, so the words are there long before unless the grid is held up
@@ -655,7 +658,6 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
   q.rows = rows, q.bpr = K / 16, q.layout = sf_layout, q.nkt = (q.bpr + 3) / 4;
   q.sf_stride = sf_layout == 0 ? (long long)rows * q.bpr : ((rows + 127LL) / 128 * 128) * q.nkt * 4;
   q.wide = ((uintptr_t)x & 31) == 0;
-  q.mark = groups * ((long long)rows * K) * (dtype == 0 ? 2 : 4) > kQMarkFrom;
   q.bpr_shift = 30;
   for (int b = q.bpr; b; b >>= 1) ++q.bpr_shift;
   q.bpr_inv = ((1ULL << q.bpr_shift) + q.bpr - 1) / q.bpr;
@@ -685,6 +687,7 @@ static int quantize_own_scale(const void* x, int dtype, int groups, int rows, in
   if (2LL * groups * units > 0x7fffffffLL) return B200MOE_ERR_LIMIT;
   long long w = kQWindowBytes / (nblk * (dtype == 0 ? 32 : 64));
   const int window = (int)(w < 1 ? 1 : w > groups ? groups : w);
+  q.mark = groups > window || groups * nblk * (dtype == 0 ? 32 : 64) > kQMarkFrom;
   static int sms = 0;   // of the first device used: all devices of a machine are alike, and any grid size is correct
   if (!sms) {
     int dev = 0, n = 0;

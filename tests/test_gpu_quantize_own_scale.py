@@ -58,9 +58,11 @@ def test_large_inputs_on_chip(groups, rows, k):
         assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(got, again))
 
 
-# More than 20 MB in all: the passes of different groups alternate (10 and 5 groups apart here, the last unit of each ragged); a group
-# above 20 MB: its two passes follow one another.
-@pytest.mark.parametrize("dtype,groups,rows,k", [(torch.bfloat16, 16, 1000, 1040), (torch.float32, 12, 1000, 1040), (torch.bfloat16, 2, 6400, 2048)])
+# More than 30 MB in all: the passes of different groups alternate (15 groups apart in bf16, 7 in fp32, the last unit of each ragged), once
+# or, with twice the groups, many times; a group above 30 MB: its two passes follow one another.
+@pytest.mark.parametrize("dtype,groups,rows,k", [(torch.bfloat16, 16, 1000, 1040), (torch.bfloat16, 40, 1000, 1040), (torch.float32, 12, 1000, 1040),
+                                                 (torch.float32, 20, 1000, 1040), (torch.bfloat16, 2, 6400, 2048), (torch.bfloat16, 2, 8200, 2048),
+                                                 (torch.float32, 3, 4100, 2048)])
 def test_groups_in_alternating_order(dtype, groups, rows, k):
     import sm120fp4_b200 as pkg
     scale = torch.linspace(0.01, 9.0, groups, device="cuda")[:, None, None]
