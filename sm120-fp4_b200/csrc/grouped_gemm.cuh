@@ -379,10 +379,11 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
     // Two producers walk the same sequence and issue alternate slots: one thread's wait + issue round is ~430 cycles a copy.
     if (lane == 0) {
       // Weight records are the first to leave L2 again, so that what the layer writes stays there: layers one after the other, each with its
-      // own weights, take 76 us (78 without) at 96 tokens (W4A16), 86.4 (88.1) at 1024, 75.8 (78.3) at 333 of 2816 x 704, 65.9 (68.1) at 24.
-      // Not so in W4A4 the records of an expert with several tiles, which are read again: with those as well 3000 tokens take 167.8 us
-      // instead of 162.5. (W4A16 tiles are small and their expert's others run beside them: 96.4 us with all, 99.1 without those.) Nor the weights of a layer that fits in
-      // L2, which the next call on it may find there (113 MB, one layer again and again: 43.2 us marked, 42.7 not).
+      // own weights, take 76 us (78 without) at 96 tokens (W4A16), 86.4 (88.1) at 1024, 65.9 (68.1) at 24. Not so the records of an
+      // expert with several tiles, which are read again: with those as well 3000 tokens take 167.8 us instead of 162.5, and in W4A16, where a
+      // tile is 16 pairs, skewed batches 178 instead of 145 (195 tokens of 3072 x 1536), 113 instead of 96 (256 of 60 experts of 2304 x 1408) and 120 instead of 104
+      // (150 of 256 experts of 2048 x 1536); at most 3 % were gained with those as well (256 of 2816 x 704: 95.8 instead of 98.5). Nor the weights of a layer that
+      // fits in L2, which the next call on it may find there (113 MB, one layer again and again: 43.2 us marked, 42.7 not).
       const uint64_t once = policy_evict_first();
       int slot = 0;
       uint32_t ph = 1;          // parity that a free slot's `empty` barrier has completed: the first pass finds all slots free
@@ -390,9 +391,10 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
       auto next = [&]() { mine = !mine; if (++slot == NS) { slot = 0; ph ^= 1u; } };
       auto acquire = [&]() { if (!mbar_wait(&S.empty[slot], ph, &S.abort_flag)) *P.status = 2; };
       for_each_segment([&](int t, int n0, int n1, int) {
-        const int expert = __ldcg(P.tile_expert + t);
+        // (the three loads in flight together: nothing else starts before them)
+        const int expert = __ldcg(P.tile_expert + t), before = t > 0 ? __ldcg(P.tile_expert + t - 1) : -1, after = t + 1 < NT ? __ldcg(P.tile_expert + t + 1) : -1;
         const uint8_t* src = P.wrec + ((long long)expert * NBLK + n0) * KB * kRec;   // consecutive column blocks are contiguous
-        const bool stay = !P.stream || (PHASE <= 2 && ((t > 0 && __ldcg(P.tile_expert + t - 1) == expert) || (t + 1 < NT && __ldcg(P.tile_expert + t + 1) == expert)));
+        const bool stay = !P.stream || before == expert || after == expert;
         const uint8_t* asrc = P.arec + (long long)t * KB * kARec;
         const int codes = NR < KB ? tile_rows(t) * 128 : 0;
         for (int n = n0; n < n1; ++n)
