@@ -56,7 +56,8 @@ long long b200moe_quantize_own_scale_workspace_bytes(int dtype, int groups, int 
 int b200moe_quantize_nvfp4_own_scale(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
                                      int sf_layout, void* workspace, long long workspace_bytes, void* stream);
 /* For tests: the same call with the number of looks at a work unit's maximum after which a block that needs it works it out itself
- * (blocks of a grid that is not resident as a whole wait for one another at most that long, about 1.5 ms in the call above). */
+ * (blocks of a grid that is not resident as a whole wait for one another at most that long, about 1.5 ms in the call above).
+ * Below 0: blocks do not wait for one another, and a wait inside a block gives up after -1 - polls tries. */
 int b200moe_quantize_own_scale_probe(const void* x, int dtype, int groups, int rows, int K, float* gs_out, void* packed, void* sf,
                                      int sf_layout, void* workspace, long long workspace_bytes, int polls, void* stream);
 

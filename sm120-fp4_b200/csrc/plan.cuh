@@ -168,7 +168,7 @@ struct alignas(16) BlockPlan {
   uint16_t ids[kBlockPlanPairs];           // expert of every pair, 0xffff: empty slot or an id >= E
   int cnt[kPlanMaxE], off[kPlanMaxE], tb[kPlanMaxE];   // pairs of expert e, its first index in `pairs`, its first tile
   int NT;
-  int found[2];                            // of find_tile
+  int found[2];                            // of block_plan_tile
 };
 
 // tables: this block also writes the tables that are not scattered (experts, offsets, ntiles, tile_*)

@@ -373,8 +373,8 @@ constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
 constexpr int kQcLooks = 8;        // maxima that may wait for their worker
 // Words of a group that a lane has in flight together, also the last few: a look at a group takes one to three round trips. (With the words of the
 // last incomplete four one after the other it took up to five, and with more than three the blocks waited for it: 320 MB of bf16 in groups
-// of 102 units 107 us, now 91; of 240 units 117, now 93; of 352 units 117, now 100; of 192 units 91 both. All of a group's words at once:
-// 92, 93, 104 and 92; but 128 x 1536 x 2048 with swizzled scales 210 instead of 206.6.)
+// of 102 units 107 us, now 91; of 240 units 117, now 93; of 192 units 91 both. All of a group's words at once:
+// 90, 93 and 92, but 128 x 1536 x 2048 with swizzled scales 210 instead of 206.6.)
 constexpr int kQcWords = 4;
 constexpr int kQcBlocks = kQcUnit / 32;   // 16-value blocks of a unit
 struct QcShared {

@@ -2,7 +2,8 @@
 sm120fp4/vllm_backend.py:95-172, on the B200 kernels of this package.
 
 Differences from the reference, all widening: any hidden size that is a multiple of 128 and intermediate size that is a
-multiple of 64 (the reference takes 2048 x {768, 1024} only, vllm_backend.py:44-45,102-103); block scales may be handed
+multiple of 64 (the reference takes 2048 x {768, 1024} only, vllm_backend.py:44-45,102-103; decode batches of 9 to 16 tokens up to a
+hidden size of 5632, of 1 to 8 up to 11264: beyond, `forward` raises); block scales may be handed
 over already in the 128x4 swizzle (`scale_layout="128x4"`) or row-major as the checkpoint stores them (converted once on
 the device); a decode batch (up to 16 tokens) is ONE kernel launch instead of router + FC1 + FC2.
 """
