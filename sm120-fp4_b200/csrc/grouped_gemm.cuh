@@ -53,7 +53,7 @@ struct GroupedParams {
   float gs_out;               // PHASE 1: global scale for the activation re-quantisation
   const float* wts;           // PHASE 2/4: routing weights [P]
   uint8_t* orec;              // PHASE 1/3: FC2 operand records [ntiles][KB2][...]
-  __nv_bfloat16* y;           // PHASE 2: weighted rows [ntiles*128][H]
+  __nv_bfloat16* y;           // PHASE 2: weighted rows [ntiles*128][H], columns ordered as gg_epilogue_fc2 says
   float* yf;                  // PHASE 4: weighted rows [ntiles*16][H] in fp32 (one rounding only, in the combine)
   int* status;
   const float* rowscale;      // PHASE 3: 1 / g_t of every term row of the x operand [ntiles*64]
@@ -73,10 +73,8 @@ struct GgShared {
   volatile int abort_flag;
 };
 
-constexpr int kGgPatch = 32 * 144;   // PHASE 2: one warp's patch for transposed stores (32 rows x 128 bytes, padded)
-
-constexpr int gg_head_bytes(int phase) { return 1024 + (phase == 2 ? 8 * kGgPatch : 0); }   // barriers (+ store patches) ahead of the records
-static_assert(sizeof(GgShared) <= 1024 && (8 * kGgPatch) % 1024 == 0, "the records start on a 1 KB boundary");
+constexpr int kGgHead = 1024;   // barriers ahead of the records
+static_assert(sizeof(GgShared) <= kGgHead, "the records start on a 1 KB boundary");
 
 // How a CTA divides its shared memory, from the most rows its tiles hold: a resident operand record keeps only those rows (rounded
 // up to 8) and its scale tiles; the rest is the ring. A tile of 64 rows over 8 K boxes takes 80 KB and leaves eight slots,
@@ -86,9 +84,9 @@ static_assert(sizeof(GgShared) <= 1024 && (8 * kGgPatch) % 1024 == 0, "the recor
 // + 64 for the rotating weight scales + 64 more for streamed operand scales.
 constexpr int kGgMinRing = 4, kGgMinShared = 6;
 struct GgPlan { int astride, NR, NS; };
-__host__ __device__ inline GgPlan gg_plan(int phase, int KB, int max_rows) {
+__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows) {
   GgPlan p;
-  const int room = kGgSmem - 1024 - gg_head_bytes(phase);
+  const int room = kGgSmem - 1024 - kGgHead;
   p.astride = ((max_rows + 7) & ~7) * 128 + 2048;
   p.NR = KB < 12 ? KB : 12;
   if ((room - p.NR * p.astride) / kRec < kGgMinRing || p.NR < KB) {
@@ -190,37 +188,48 @@ __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float g
   if (store) *reinterpret_cast<uint32_t*>(dst + rec_scale_offset(row, 4 * (n & 3))) = sfw;
 }
 
-// W4A4 FC2: scale, round to bf16, transpose through the warp's patch of shared memory so that every store instruction writes
-// whole 128-byte row segments (four rows per instruction). valid: bit l = row l of the warp holds a pair.
+// W4A4 FC2: scale, round to bf16 and store. The accumulator is read in the fragment layout of mma (eight rows x four lanes), so that the four lanes
+// of a row hold 64 columns between them and an instruction stores 64-byte halves of eight rows' segments; nothing goes through shared
+// memory. The columns of a segment lie as the lanes hold them: 16-byte chunk 4j + q has columns 32j + 8w + 2q + {0, 1}, w = 0..3 (combine_columns
+// puts them right). s[i]: scale of row 8i + lane / 4 of the warp; the first `rows` rows hold a pair. A block's epilogue takes 920 cycles at 1024
+// tokens of the 2048 x 768 layer and 1290 at 8192 (FC2 73 us there); with a thread per row and a transposition through shared memory 2680 and 3170 (84 us, the
+// epilogue was the bound), with that and bulk stores 4040 and 3850: a store waits behind the ring's loads in the copy engine.
 template <class F>
-__device__ __forceinline__ void gg_epilogue_fc2(uint32_t taddr, float s, unsigned valid, uint8_t* patch, __nv_bfloat16* ybase, int H, int lane, F&& release) {
+__device__ __forceinline__ void gg_epilogue_fc2(uint32_t taddr, const float (&s)[4], int rows, __nv_bfloat16* ybase, int H, int lane, F&& release) {
+  __nv_bfloat16* yrow = ybase + (long long)(lane >> 2) * H + (lane & 3) * 8;
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
-    uint32_t r[4][16];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x16(taddr + 64 * half + 16 * c, r[c]);
+    uint32_t r[2][32];
+    tmem_ld_16x256b_x8(taddr + 64 * half, r[0]);
+    tmem_ld_16x256b_x8(taddr + 64 * half + (16u << 16), r[1]);
     tmem_ld_wait();
     if (half == 1) release();
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t o[8];
+    for (int i = 0; i < 4; ++i) {
+      const bool store = 8 * i + (lane >> 2) < rows;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[c][2 * i]) * s, __uint_as_float(r[c][2 * i + 1]) * s);
-        o[i] = *reinterpret_cast<const uint32_t*>(&h);
+      for (int j = 0; j < 2; ++j) {
+        uint32_t o[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t* v = &r[i >> 1][4 * (4 * j + w) + 2 * (i & 1)];
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[0]) * s[i], __uint_as_float(v[1]) * s[i]);
+          o[w] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        if (store) *reinterpret_cast<uint4*>(yrow + (long long)(8 * i) * H + 64 * half + 32 * j) = make_uint4(o[0], o[1], o[2], o[3]);
       }
-      *reinterpret_cast<uint4*>(patch + lane * 144 + 32 * c) = make_uint4(o[0], o[1], o[2], o[3]);
-      *reinterpret_cast<uint4*>(patch + lane * 144 + 32 * c + 16) = make_uint4(o[4], o[5], o[6], o[7]);
     }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int rr = 4 * j + (lane >> 3);   // row of the warp's block this lane stores a 16-byte chunk of
-      const uint4 v4 = *reinterpret_cast<const uint4*>(patch + rr * 144 + (lane & 7) * 16);
-      if ((valid >> rr) & 1u) *reinterpret_cast<uint4*>(ybase + (long long)rr * H + 64 * half + (lane & 7) * 8) = v4;
-    }
-    __syncwarp();
   }
+}
+// The four lanes of a quad hold chunks 4j..4j+3 of a segment: afterwards lane q holds columns 32j + 8q .. + 7 in their order.
+__device__ __forceinline__ void combine_columns(uint32_t (&w)[4], int lane) {
+  const unsigned quad = 0xfu << (lane & 28);
+  uint32_t a = __shfl_xor_sync(quad, lane & 1 ? w[0] : w[1], 1), b = __shfl_xor_sync(quad, lane & 1 ? w[2] : w[3], 1);
+  if (lane & 1) w[0] = a, w[2] = b;
+  else w[1] = a, w[3] = b;
+  a = __shfl_xor_sync(quad, lane & 2 ? w[0] : w[2], 2), b = __shfl_xor_sync(quad, lane & 2 ? w[1] : w[3], 2);
+  if (lane & 2) w[0] = a, w[1] = b;
+  else w[2] = a, w[3] = b;
 }
 
 // W4A16 FC1: rows 4p..4p+3 are the four terms of pair p, each scaled by its 1/g_t. A reduce-scatter over the pair's four lanes
@@ -311,7 +320,6 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   constexpr int kRowsPerPair = PHASE >= 3 ? kTerms : 1;
   const int KB = P.KB, NBLK = P.NBLK;
   GgShared& S = *reinterpret_cast<GgShared*>(smem);
-  uint8_t* patches = smem + 1024;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // (a value from lane 0 is known to be warp-uniform)
   // Without wait_tables the tile tables are read without waiting for the kernel before this one: the tables' own producer is at least
@@ -350,9 +358,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const GgPlan plan = gg_plan(PHASE, KB, __shfl_sync(0xffffffffu, S.max_rows, 0));
+  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0));
   const int NR = plan.NR, NS = plan.NS, astride = plan.astride, acodes = astride - 2048;
-  uint8_t* abuf = smem + gg_head_bytes(PHASE);                  // NR records of the current row tile
+  uint8_t* abuf = smem + kGgHead;                  // NR records of the current row tile
   uint8_t* ring = abuf + NR * astride;                          // NS slots
   const uint32_t tmem = __shfl_sync(0xffffffffu, S.tmem_base, 0);
   const uint32_t tm_acc = tmem, tm_sfa = tmem + 256, tm_sfb = tmem + 256 + 16 * NR, tm_sfs = tm_sfb + 64;   // 2 x 128 | NR x 16 | 4 x 16 | 4 x 16
@@ -519,7 +527,12 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
         for (int q = 0; q < (lane & 3); ++q) g *= 6.0f;
         rs = 1.0f / g;
       }
-      const unsigned valid = PHASE == 2 ? __ballot_sync(0xffffffffu, pr >= 0) : 0u;   // bit l: row quad*32 + l holds a pair
+      const int held = PHASE == 2 ? __popc(__ballot_sync(0xffffffffu, pr >= 0)) : 0;   // rows of this quadrant that hold a pair: the first ones
+      float s4[4];
+      if (PHASE == 2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s4[i] = __shfl_sync(0xffffffffu, s, 8 * i + (lane >> 2));
+      }
       const bool work = quad * 32 < rows;   // warp-uniform: this quadrant holds rows of the tile
 #pragma unroll 1
       for (int n = n0; n < n1; ++n, ++seq) {
@@ -540,7 +553,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
         } else if (PHASE == 1) {
           gg_epilogue_fc1<Ieee>(taddr, s, P.gs_out, S.scale, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kRec, row, row < rows && !dry, n, release);
         } else if (PHASE == 2) {
-          gg_epilogue_fc2(taddr, s, dry ? 0u : valid, patches + warp * kGgPatch, P.y + ((long long)t * 128 + quad * 32) * P.H + 128 * n, P.H, lane, release);
+          gg_epilogue_fc2(taddr, s4, dry ? 0 : held, P.y + ((long long)t * 128 + quad * 32) * P.H + 128 * n, P.H, lane, release);
         } else if (PHASE == 3) {
           if (gg_epilogue_fc1_a16(taddr, s, rs, P.act_g1, P.orec + ((long long)t * P.KB2 + (n >> 2)) * kMidRec, row, row < rows, !dry, n, lane, release))
             P.status[1] = 1;   // beyond the range of the fixed activation scale

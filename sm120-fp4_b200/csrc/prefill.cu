@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(256) k_combine(const void* yv, const int* dst_
       const __nv_bfloat162 h = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
       o[q] = *reinterpret_cast<const uint32_t*>(&h);
     }
+    if (!F32) combine_columns(o, threadIdx.x & 31);
     *reinterpret_cast<uint4*>(out + (long long)tok * H + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }

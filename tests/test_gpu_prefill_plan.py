@@ -165,3 +165,21 @@ def test_quotient_of_wide_layers_is_ieee():
         L.check(L.lib().b200moe_quotient_probe(L.ptr(gate), L.ptr(den), L.ptr(out), n, L.stream_ptr()), "probe")
         want = gate / den
         assert bool(((out.view(torch.int32) == want.view(torch.int32)) | (out.isnan() & want.isnan())).all()), part
+
+
+# FC2's stores and the combine behind them take rows in groups of eight and columns in segments of 64: experts with one row, with whole and ragged
+# groups and quadrants, up to one more than a tile; one segment pair a row (128 columns, an odd number of tokens: half a warp in the combine) and
+# odd numbers of pairs of segments. Against the oracle's W4A4 arithmetic, tolerance as everywhere (2e-2 x RMS from the kernel's own codes).
+@pytest.mark.parametrize("hidden", [128, 384])
+def test_rows_and_segments(hidden):
+    cfg = dict(experts=16, hidden=hidden, inter=64, top_k=2)
+    w, ow = make_layer(**cfg, seed=9)
+    rows = [1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 95, 97, 127, 129]
+    first = np.repeat(np.arange(len(rows)), rows)
+    m = first.size
+    assert m % 2 == 1
+    x, ids, wts = inputs(cfg, m, 7)
+    ids = ids.clone()
+    ids[:, 0], ids[:, 1] = torch.from_numpy(first.astype(np.int32)), 14 + torch.arange(m, dtype=torch.int32) % 2
+    out = run_prefill(w, x, ids, wts, 1024)
+    check_prefill_call(w, ow, x, ids, wts, out, 1024, what=f"rows and segments, hidden {hidden}")
