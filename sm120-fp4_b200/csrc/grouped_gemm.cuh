@@ -9,10 +9,9 @@
 // 128 x 128 x 64 in 64 cycles) plus 8 cycles per tcgen05.cp of a 512-byte scale tile; an SM takes in 63 bytes per cycle from
 // L2 (17.3 TB/s over the chip, from four 18 KB copies in flight on), i.e. 288 cycles per record; HBM delivers a record per
 // SM every ~700 cycles (7.1 TB/s). A batch that touches every expert with few rows is bound by HBM. In a large one no unit is
-// near its peak over the whole kernel (FC1 of 8192 tokens: tensor pipe 48 %, shared memory 51 %, L2 24 %, HBM 30 %; about 530
-// cycles a record). In a loop of its own - four scale copies, four MMAs, records from L2 through four slots, no epilogue - a record takes
-// 345 cycles, 335 without the loads and 267 without the scale copies, so the copies' traffic through shared memory is not the
-// limit. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
+// near its peak over the whole kernel (FC1 of 8192 tokens: tensor pipe 48 %, shared memory 51 %, L2 24 %, HBM 30 %; about 560
+// cycles a record). In a loop of its own - four scale copies and four MMAs, records arriving beside them - a record takes 291 cycles, 257 without the scale
+// copies, so neither the tensor pipe nor shared memory is the limit. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
 // warp to warp between a record's arrival and its math. (Before, four warps moved the scales through registers and handed every
 // record to the MMA warp over a barrier: 870 cycles a record at 8192 tokens.)
 //
@@ -368,65 +367,67 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
 
   if (warp == 8) {
     // ============================================================== resident operand records: once per segment, box by box
-    if (lane == 0) {
-      grid_dependency_wait();   // the records are written by the kernel before this one
-      for_each_segment([&](int t, int, int, int ord) {
-        const int codes = tile_rows(t) * 128;   // only the rows in use, then the scale tiles
-        for (int kb = 0; kb < NR; ++kb) {
-          if (ord >= 1 && !mbar_wait(&S.a_empty[kb], (uint32_t)((ord - 1) & 1), &S.abort_flag)) *P.status = 2;
-          const uint8_t* src = P.arec + ((long long)t * KB + kb) * kARec;
-          mbar_expect_tx(&S.a_full[kb], codes + 2048);
-          bulk_load(abuf + kb * astride, src, codes, &S.a_full[kb]);
-          bulk_load(abuf + kb * astride + acodes, src + kACodes, 2048, &S.a_full[kb]);
-        }
-      });
-    }
+    const uint32_t el = elect_one();
+    const uint32_t full_u = smem_u32(S.a_full), empty_u = smem_u32(S.a_empty), abuf_u = smem_u32(abuf);
+    grid_dependency_wait();   // the records are written by the kernel before this one
+    for_each_segment([&](int t, int, int, int ord) {
+      const int codes = tile_rows(t) * 128;   // only the rows in use, then the scale tiles
+      for (int kb = 0; kb < NR; ++kb) {
+        if (ord >= 1 && !mbar_wait_warp(empty_u + 8 * kb, (uint32_t)((ord - 1) & 1), &S.abort_flag)) *P.status = 2;
+        const uint8_t* src = P.arec + ((long long)t * KB + kb) * kARec;
+        mbar_expect_tx_u32(full_u + 8 * kb, codes + 2048, el);
+        bulk_load_u32(abuf_u + kb * astride, src, codes, full_u + 8 * kb, el);
+        bulk_load_u32(abuf_u + kb * astride + acodes, src + kACodes, 2048, full_u + 8 * kb, el);
+      }
+    });
     __syncwarp();
   } else if (warp == 9 || warp == 10) {
     // ============================================================== ring: weight records (and operand records of boxes >= NR).
-    // Two producers walk the same sequence and issue alternate slots: one thread's wait + issue round is ~430 cycles a copy.
-    if (lane == 0) {
-      // Weight records are the first to leave L2 again, so that what the layer writes stays there: layers one after the other, each with its
-      // own weights, take 76 us (78 without) at 96 tokens (W4A16), 86.4 (88.1) at 1024, 65.9 (68.1) at 24. Not so the records of an
-      // expert with several tiles, which are read again: with those as well 3000 tokens take 167.8 us instead of 162.5, and in W4A16, where a
-      // tile is 16 pairs, skewed batches 178 instead of 145 (195 tokens of 3072 x 1536), 113 instead of 96 (256 of 60 experts of 2304 x 1408) and 120 instead of 104
-      // (150 of 256 experts of 2048 x 1536); at most 3 % were gained with those as well (256 of 2816 x 704: 95.8 instead of 98.5). Nor the weights of a layer that
-      // fits in L2, which the next call on it may find there (113 MB, one layer again and again: 43.2 us marked, 42.7 not).
-      const uint64_t once = policy_evict_first();
-      int slot = 0;
-      uint32_t ph = 1;          // parity that a free slot's `empty` barrier has completed: the first pass finds all slots free
-      bool mine = warp == 9, waited = NR == KB;
-      auto next = [&]() { mine = !mine; if (++slot == NS) { slot = 0; ph ^= 1u; } };
-      auto acquire = [&]() { if (!mbar_wait(&S.empty[slot], ph, &S.abort_flag)) *P.status = 2; };
-      for_each_segment([&](int t, int n0, int n1, int) {
-        // (the three loads in flight together: nothing else starts before them)
-        const int expert = __ldcg(P.tile_expert + t), before = t > 0 ? __ldcg(P.tile_expert + t - 1) : -1, after = t + 1 < NT ? __ldcg(P.tile_expert + t + 1) : -1;
-        const uint8_t* src = P.wrec + ((long long)expert * NBLK + n0) * KB * kRec;   // consecutive column blocks are contiguous
-        const bool stay = !P.stream || before == expert || after == expert;
-        const uint8_t* asrc = P.arec + (long long)t * KB * kARec;
-        const int codes = NR < KB ? tile_rows(t) * 128 : 0;
-        for (int n = n0; n < n1; ++n)
-          for (int kb = 0; kb < KB; ++kb, src += kRec) {
-            if (kb >= NR) {
-              if (mine) {
-                acquire();
-                if (!waited) { grid_dependency_wait(); waited = true; }
-                mbar_expect_tx(&S.full[slot], codes + 2048);
-                bulk_load(ring + slot * kRec, asrc + (long long)kb * kARec, codes, &S.full[slot]);
-                bulk_load(ring + slot * kRec + kACodes, asrc + (long long)kb * kARec + kACodes, 2048, &S.full[slot]);
-              }
-              next();
-            }
+    // Two producers walk the same sequence and issue alternate slots. The warps stay converged and an elected lane issues: a copy takes a producer 320 cycles beside its
+    // wait, 470 from a branch that a single lane takes (8192 tokens of 2048 x 768 348 -> 341 us, 2050 of 4096 x 1536 425 -> 411). What a ring of four
+    // slots gives is bound by its turn-round (MMA, commit, producer, L2): without any MMA, scale copy or epilogue FC1 of 8192 tokens still takes 440 cycles a record.
+    // Weight records are the first to leave L2 again, so that what the layer writes stays there: layers one after the other, each with its
+    // own weights, take 76 us (78 without) at 96 tokens (W4A16), 86.4 (88.1) at 1024, 65.9 (68.1) at 24. Not so the records of an
+    // expert with several tiles, which are read again: with those as well 3000 tokens take 167.8 us instead of 162.5, and in W4A16, where a
+    // tile is 16 pairs, skewed batches 178 instead of 145 (195 tokens of 3072 x 1536), 113 instead of 96 (256 of 60 experts of 2304 x 1408) and 120 instead of 104
+    // (150 of 256 experts of 2048 x 1536); at most 3 % were gained with those as well (256 of 2816 x 704: 95.8 instead of 98.5). Nor the weights of a layer that
+    // fits in L2, which the next call on it may find there (113 MB, one layer again and again: 43.2 us marked, 42.7 not).
+    const uint64_t once = policy_evict_first();
+    const uint32_t el = elect_one();
+    const uint32_t full_u = smem_u32(S.full), empty_u = smem_u32(S.empty), ring_u = smem_u32(ring);
+    int slot = 0;
+    uint32_t ph = 1;          // parity that a free slot's `empty` barrier has completed: the first pass finds all slots free
+    bool mine = warp == 9, waited = NR == KB;
+    auto next = [&]() { mine = !mine; if (++slot == NS) { slot = 0; ph ^= 1u; } };
+    auto acquire = [&]() { if (!mbar_wait_warp(empty_u + 8 * slot, ph, &S.abort_flag)) *P.status = 2; };
+    for_each_segment([&](int t, int n0, int n1, int) {
+      // (the three loads in flight together: nothing else starts before them)
+      const int expert = __ldcg(P.tile_expert + t), before = t > 0 ? __ldcg(P.tile_expert + t - 1) : -1, after = t + 1 < NT ? __ldcg(P.tile_expert + t + 1) : -1;
+      const uint8_t* src = P.wrec + ((long long)__shfl_sync(0xffffffffu, expert, 0) * NBLK + n0) * KB * kRec;   // consecutive column blocks are contiguous
+      const bool stay = __shfl_sync(0xffffffffu, (int)(!P.stream || before == expert || after == expert), 0) != 0;
+      const uint8_t* asrc = P.arec + (long long)t * KB * kARec;
+      const int codes = NR < KB ? tile_rows(t) * 128 : 0;
+      for (int n = n0; n < n1; ++n)
+        for (int kb = 0; kb < KB; ++kb, src += kRec) {
+          if (kb >= NR) {
             if (mine) {
               acquire();
-              mbar_expect_tx(&S.full[slot], kRec);
-              if (stay) bulk_load(ring + slot * kRec, src, kRec, &S.full[slot]);
-              else bulk_load_hint(ring + slot * kRec, src, kRec, &S.full[slot], once);
+              if (!waited) { grid_dependency_wait(); waited = true; }
+              mbar_expect_tx_u32(full_u + 8 * slot, codes + 2048, el);
+              bulk_load_u32(ring_u + slot * kRec, asrc + (long long)kb * kARec, codes, full_u + 8 * slot, el);
+              bulk_load_u32(ring_u + slot * kRec + kACodes, asrc + (long long)kb * kARec + kACodes, 2048, full_u + 8 * slot, el);
             }
             next();
           }
-      });
-    }
+          if (mine) {
+            acquire();
+            mbar_expect_tx_u32(full_u + 8 * slot, kRec, el);
+            if (stay) bulk_load_u32(ring_u + slot * kRec, src, kRec, full_u + 8 * slot, el);
+            else bulk_load_hint_u32(ring_u + slot * kRec, src, kRec, full_u + 8 * slot, once, el);
+          }
+          next();
+        }
+    });
     __syncwarp();
   } else if (warp == 11) {
     // ============================================================== MMA issuer: the warp stays converged (all values are

@@ -99,6 +99,19 @@ __device__ __forceinline__ void bulk_load_hint(void* dst, const void* src, uint3
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
                : "memory");
 }
+// The same from a warp that stays converged: expected bytes and copy are issued by the lane whose `pred` is set, addresses are warp-uniform.
+__device__ __forceinline__ void mbar_expect_tx_u32(uint32_t bar, uint32_t bytes, uint32_t pred) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(bar), "r"(bytes), "r"(pred) : "memory");
+}
+__device__ __forceinline__ void bulk_load_u32(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint32_t pred) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %4, 0;\n @q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n}\n"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "r"(pred) : "memory");
+}
+__device__ __forceinline__ void bulk_load_hint_u32(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t policy, uint32_t pred) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+               " @q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n}\n"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy), "r"(pred) : "memory");
+}
 // 1-D bulk copy shared -> global; returns when the shared memory has been read
 __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n cp.async.bulk.commit_group;\n cp.async.bulk.wait_group.read 0;"
