@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "nvfp4_math.cuh"
 #include "tcgen05.cuh"
+#include <type_traits>
 
 namespace b200 {
 
@@ -76,12 +77,14 @@ __device__ __forceinline__ void st_policy(uint2* p, uint2 v, uint64_t policy) {
 // largest magnitude of the 16 values; NaNs are passed over, as fmaxf does, unless there is nothing else (a block of NaNs then gets the
 // largest block scale, as quantize_block16 gives it)
 __device__ __forceinline__ float amax_raw(const Raw16<__nv_bfloat16>& v) {
-  const uint32_t w[8] = {v.r[0].x, v.r[0].y, v.r[0].z, v.r[0].w, v.r[1].x, v.r[1].y, v.r[1].z, v.r[1].w};
-  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
-#pragma unroll
-  for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
-  const uint32_t b = *reinterpret_cast<const uint32_t*>(&m);
-  return fmaxf(__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u));
+  // the larger magnitude of either half, with the product of the signs: those go at the end
+  auto larger = [](uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  };
+  const uint32_t b = larger(larger(larger(v.r[0].x, v.r[0].y), larger(v.r[0].z, v.r[0].w)), larger(larger(v.r[1].x, v.r[1].y), larger(v.r[1].z, v.r[1].w)));
+  return fmaxf(fabsf(__uint_as_float(b << 16)), fabsf(__uint_as_float(b & 0xffff0000u)));
 }
 __device__ __forceinline__ float amax_raw(const Raw16<float>& v) {
   float m[4];
@@ -119,10 +122,10 @@ __device__ __forceinline__ float sixth(float amax, __nv_bfloat16) {
 }
 __device__ __forceinline__ float sixth(float amax, float) { return __fdiv_rn(amax, 6.0f); }
 
-// quantize_block16 on values as loaded, its second division looked up and two products per instruction
+// quantize_block16 on values as loaded and their largest magnitude, its second division looked up and two products per instruction
 template <typename T>
-__device__ __forceinline__ uint32_t quantize_raw(const Raw16<T>& v, float gs, const float* table, uint2& packed) {
-  const float sf_f = fminf(__fmul_rn(sixth(amax_raw(v), T()), gs), 448.0f);
+__device__ __forceinline__ uint32_t quantize_raw(const Raw16<T>& v, float amax, float gs, const float* table, uint2& packed) {
+  const float sf_f = fminf(__fmul_rn(sixth(amax, T()), gs), 448.0f);
   uint16_t sb;
   asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(sb) : "f"(0.0f), "f"(sf_f));
   const float scale = table[sb & 127];
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
     for (int j = 0; j < kPer; ++j) {
       if (j * kQgThreads < left) {
         uint2 pk;
-        const uint32_t sb = quantize_raw(v[j], gs, s_table, pk);
+        const uint32_t sb = quantize_raw(v[j], amax_raw(v[j]), gs, s_table, pk);
         if (q.mark) st_policy(codes + j * kQgThreads, pk, once);
         else __stcg(codes + j * kQgThreads, pk);
         if (q.layout == 0) {
@@ -366,7 +369,8 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 // when the maxima of its group have normally all been published. A block is three workers of eight warps, a copying warp and one that
 // looks for the maxima. The kernel above reads every value twice into registers and is held up by latency with the 16 warps an SM that
 // its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 190 instructions per 16 values (66 %
-// busy). 128 x 1536 x 2048 bf16, swizzled scales: 204 us, 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
+// busy), less what is kept from one pass to the other: a thread's block maxima and the unit's place stay in registers, and magnitudes are compared without
+// being taken first (220 us before, 208 with them). 128 x 1536 x 2048 bf16, swizzled scales: 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
 // meet a quarter of the banks: 60 x 1024 x 1536 take 96 us either way, or 115 here without instructions that avoid the conflicts.)
 constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
 constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
@@ -480,7 +484,10 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     const uint32_t ring = smem_u32(smem);
     float gs_table = -1.f;
     bool copied = true, told = true;   // this warp has not given up on the copies, on the maxima
-    // body(block) for this thread's blocks i0 + wt + j * threads of a unit, which the slot holds
+    // The largest magnitudes of this thread's blocks, of the unit that is read and of the one before, which is quantised behind it.
+    float seen[kPer] = {}, kept[kPer] = {};
+    // body(j, block, whether it comes from the slot) for this thread's blocks i0 + wt + j * threads of a unit. (Once a warp reads global memory it does so to the
+    // end, and keeps nothing.)
     auto blocks = [&](int g, int slot, int i0, auto&& body) {
       const int left = nblk - i0 - wt;
       if (copied) {
@@ -489,7 +496,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
           if (j * kQcWorkerThreads < left) {
             Raw16<__nv_bfloat16> v;
             load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
-            body(j, v);
+            body(j, v, std::true_type());
           }
         }
       } else {
@@ -497,7 +504,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         for (int j = 0; j < kPer && j * kQcWorkerThreads < left; ++j) {
           Raw16<__nv_bfloat16> v;
           load_raw(x + ((long long)g * nblk + i0 + wt + j * kQcWorkerThreads) * 16, q.wide, false, v);
-          body(j, v);
+          body(j, v, std::false_type());
         }
       }
     };
@@ -532,14 +539,22 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
       return all;
     };
     int buf = 0;
+    int2 next = make_int2(0, 0);
 #pragma unroll 1
     for (int k = grp; k < n + kQcWorkers; k += kQcWorkers) {
+      const int2 last = next;   // of unit k - kQcWorkers
+#pragma unroll
+      for (int j = 0; j < kPer; ++j) kept[j] = seen[j];
       if (k < n) {
-        const int2 at = place(k);
+        const int2 at = next = place(k);
         const int slot = k % kQcSlots;
         copied = copied && told && mbar_wait_warp(smem_u32(&S.full[slot]), (uint32_t)((k / kQcSlots) & 1), &S.abort_flag, tries);
         float m = 0.f;
-        blocks(at.x, slot, at.y * kUnitBlocks, [&](int, const Raw16<__nv_bfloat16>& v) { m = fmaxf(m, amax_raw(v)); });
+        blocks(at.x, slot, at.y * kUnitBlocks, [&](int j, const Raw16<__nv_bfloat16>& v, auto held) {
+          const float a = amax_raw(v);
+          if constexpr (held.value) seen[j] = a;
+          m = fmaxf(m, a);
+        });
         __syncwarp();
         unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
         if (lane == 0) S.wm[grp][buf][ww] = mb;
@@ -552,8 +567,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
       }
       const int kq = k - kQcWorkers;
       if (kq < 0) continue;
-      const int2 at = place(kq);
-      const int g = at.x, u = at.y, slot = kq % kQcSlots, i0 = u * kUnitBlocks;
+      const int g = last.x, u = last.y, slot = kq % kQcSlots, i0 = u * kUnitBlocks;
       told = told && mbar_wait_warp(smem_u32(&S.known[kq % kQcLooks]), (uint32_t)((kq / kQcLooks) & 1), &S.abort_flag, tries);
       unsigned m = told ? S.gmax[kq % kQcLooks] : kMissing;
       const bool all = named_bar_and(1 + grp, kQcWorkerThreads, m != kMissing);   // (and nobody is at the table any more)
@@ -571,9 +585,12 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         r = (int)(((unsigned long long)(unsigned)(i0 + wt) * q.bpr_inv) >> q.bpr_shift);
         c = i0 + wt - r * q.bpr;
       }
-      blocks(g, slot, i0, [&](int j, const Raw16<__nv_bfloat16>& v) {
+      blocks(g, slot, i0, [&](int j, const Raw16<__nv_bfloat16>& v, auto held) {
         uint2 pk;
-        const uint32_t sb = quantize_raw(v, gs, S.table[grp], pk);
+        float amax;
+        if constexpr (held.value) amax = kept[j];
+        else amax = amax_raw(v);
+        const uint32_t sb = quantize_raw(v, amax, gs, S.table[grp], pk);
         st_policy(codes + j * kQcWorkerThreads, pk, once);
         if (q.layout == 0) {
           sfl[j * kQcWorkerThreads] = (uint8_t)sb;
