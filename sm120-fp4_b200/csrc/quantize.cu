@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 // looks for the maxima. The kernel above reads every value twice into registers and is held up by latency with the 16 warps an SM that
 // its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 190 instructions per 16 values (66 %
 // busy), less what is kept from one pass to the other: a thread's block maxima and the unit's place stay in registers, and magnitudes are compared without
-// being taken first (220 us before, 208 with them). 128 x 1536 x 2048 bf16, swizzled scales: 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
+// being taken first (220 us before, 208 with them, 205 with the order of load_shared, which takes 13 of 21 million conflict cycles away). 128 x 1536 x 2048 bf16, swizzled scales: 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
 // meet a quarter of the banks: 60 x 1024 x 1536 take 96 us either way, or 115 here without instructions that avoid the conflicts.)
 constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
 constexpr int kQcThreads = kQcWorkers * kQcWorkerThreads + 64;
@@ -390,9 +390,10 @@ struct QcShared {
 };
 constexpr int kQcSmem = kQcSlots * kQcUnit + (int)sizeof(QcShared) + 128;
 
-// 16 values of a thread from shared memory. (Neighbouring threads' blocks are 32 bytes apart, so eight of them share half of the banks:
-// that time is there. Reading the halves in turn and putting them in order takes as long.)
-__device__ __forceinline__ void load_shared(uint32_t at, Raw16<__nv_bfloat16>& v) { v.r[0] = lds128(at), v.r[1] = lds128(at + 16); }
+// 16 values of a thread from shared memory, the half at `first` (0 or 16) first. Neighbouring threads' blocks are 32 bytes apart: with every second four of a warp's
+// threads starting with the other half, eight threads meet all banks once. A maximum does not mind the order, and two words of codes are put right more cheaply
+// than eight of values.
+__device__ __forceinline__ void load_shared(uint32_t at, uint32_t first, Raw16<__nv_bfloat16>& v) { v.r[0] = lds128(at ^ first), v.r[1] = lds128(at ^ first ^ 16u); }
 
 // A wait inside the block gives up after `tries`. The warp that gave up works without what it waited for to the end of the call (a
 // barrier's parity tells only whether the phase before has passed): values come from global memory, group maxima from the worker itself. The
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
     const int grp = warp >> 3, wt = tid & (kQcWorkerThreads - 1), ww = wt >> 5;
     auto sync = [&]() { named_bar_sync(1 + grp, kQcWorkerThreads); };
     const uint64_t once = policy_evict_first();
-    const uint32_t ring = smem_u32(smem);
+    const uint32_t ring = smem_u32(smem), first_half = (lane & 4) << 2;
     float gs_table = -1.f;
     bool copied = true, told = true;   // this warp has not given up on the copies, on the maxima
     // The largest magnitudes of this thread's blocks, of the unit that is read and of the one before, which is quantised behind it.
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         for (int j = 0; j < kPer; ++j) {
           if (j * kQcWorkerThreads < left) {
             Raw16<__nv_bfloat16> v;
-            load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, v);
+            load_shared(ring + slot * kQcUnit + (wt + j * kQcWorkerThreads) * 32, first_half, v);
             body(j, v, std::true_type());
           }
         }
@@ -591,6 +592,7 @@ __global__ void __launch_bounds__(kQcThreads, 1) k_quantize_resident(const __nv_
         if constexpr (held.value) amax = kept[j];
         else amax = amax_raw(v);
         const uint32_t sb = quantize_raw(v, amax, gs, S.table[grp], pk);
+        if (held.value && first_half) pk = make_uint2(pk.y, pk.x);
         st_policy(codes + j * kQcWorkerThreads, pk, once);
         if (q.layout == 0) {
           sfl[j * kQcWorkerThreads] = (uint8_t)sb;
