@@ -57,7 +57,7 @@ struct GroupedParams {
   int* status;
   const float* rowscale;      // PHASE 3: 1 / g_t of every term row of the x operand [ntiles*64]
   float act_g1;               // PHASE 3/4: global scale of the first term of the SiLU*mul activations
-  int NBLK, KB, KT, KB2, H;
+  int NBLK, KB, KT, KB2, H, E;
   int stream;                 // the layer's weights do not fit in L2
   int wait_tables;            // the kernel before this one writes the tile tables
 };
@@ -81,9 +81,16 @@ static_assert(sizeof(GgShared) <= kGgHead, "the records start on a 1 KB boundary
 // 1.7 us of an SM's share, less than HBM latency plus the hand-offs. NR boxes stay resident; if not all of them do, the
 // ring carries operand records as well and should hold kGgMinShared slots. TMEM: 256 accumulator columns + 16 per resident box
 // + 64 for the rotating weight scales + 64 more for streamed operand scales.
-constexpr int kGgMinRing = 4, kGgMinShared = 6;
+//
+// Once (no more tiles than experts, so hardly a weight record is read twice): the CTAs then share what HBM delivers by the bytes each has in flight, and one
+// with few rows and a deep ring takes from one with many - at 333 tokens of 2816 x 704 a record took 300 ns with ten slots and 420 with four. Six slots a
+// CTA are enough for the stream. us with all slots, eight, seven, six and five: 333 skewed tokens of 2816 x 704 75.7, 74.8, 74.2, 73.7, 72.4; 128 of it 93.7, 92.9, 92.2,
+// 91.8, 91.7; 400 of 256 experts of 2048 x 1536 238.8, 236.0, 230.2, 227.5, 228.8; 700 skewed of 60 experts of 2304 x 1408 64.7, 64.2, 63.4, 62.6, 63.1; 300 skewed of
+// 4096 x 1536 151.5, 149.6, 148.0, 147.8, 147.7. With more tiles than experts records come from L2 as well, and depth is worth something: 2500 of 2048 x 768
+// 147.1, 147.2, 147.4, 147.9, 149.7; W4A16, 200 skewed of the 60 experts 65.8, 65.5, 65.4, 66.0, 68.2.
+constexpr int kGgMinRing = 4, kGgMinShared = 6, kGgMostOnce = 6;
 struct GgPlan { int astride, NR, NS; };
-__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows) {
+__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows, bool once) {
   GgPlan p;
   const int room = kGgSmem - 1024 - kGgHead;
   p.astride = ((max_rows + 7) & ~7) * 128 + 2048;
@@ -93,7 +100,8 @@ __host__ __device__ inline GgPlan gg_plan(int KB, int max_rows) {
     if (p.NR > 8) p.NR = 8;
   }
   p.NS = (room - p.NR * p.astride) / kRec;
-  if (p.NS > kGgMaxRing) p.NS = kGgMaxRing;
+  const int most = once && p.NR == KB ? kGgMostOnce : kGgMaxRing;
+  if (p.NS > most) p.NS = most;
   return p;
 }
 
@@ -357,7 +365,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0));
+  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0), NT <= P.E);
   const int NR = plan.NR, NS = plan.NS, astride = plan.astride, acodes = astride - 2048;
   uint8_t* abuf = smem + kGgHead;                  // NR records of the current row tile
   uint8_t* ring = abuf + NR * astride;                          // NS slots

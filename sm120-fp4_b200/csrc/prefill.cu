@@ -386,7 +386,7 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   }
   GroupedParams p;
   memset(&p, 0, sizeof(p));
-  p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = status, p.H = H;
+  p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = status, p.H = H, p.E = E;
   p.stream = gg_stream_weights(E, H, I);
   // FC1
   p.arec = w + L.xrec, p.wrec = w1t, p.alpha = alpha1, p.gs_in = gs_x, p.gs_out = gs_a, p.orec = w + L.arec;
@@ -488,7 +488,7 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   }
   GroupedParams p;
   memset(&p, 0, sizeof(p));
-  p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = (int*)(w + L.status), p.H = H;
+  p.ntiles = ntiles, p.tile_expert = tile_expert, p.tile_first = tile_first, p.tile_end = tile_end, p.row_pair = row_pair, p.status = (int*)(w + L.status), p.H = H, p.E = E;
   p.stream = gg_stream_weights(E, H, I);
   p.rowscale = rowscale, p.act_g1 = act_g1;
   // FC1
