@@ -79,7 +79,10 @@ static_assert(sizeof(GgShared) <= kGgHead, "the records start on a 1 KB boundary
 // up to 8) and its scale tiles; the rest is the ring. A tile of 64 rows over 8 K boxes takes 80 KB and leaves eight slots,
 // one of 128 rows 144 KB and four. Depth matters when the weights come from HBM: four 18 KB records in flight are worth about
 // 1.7 us of an SM's share, less than HBM latency plus the hand-offs. NR boxes stay resident; if not all of them do, the
-// ring carries operand records as well and should hold kGgMinShared slots. TMEM: 256 accumulator columns + 16 per resident box
+// ring carries operand records as well and should hold kGgMinShared slots, or kGgMinStream where the weights' way from HBM counts for more than the
+// operand's from L2 (up to two tiles an expert): us with 6, 8, 9, 10, 11 slots: 333 skewed tokens of 2816 x 704 73.8, 72.1, 72.4, 71.6, 71.8; 2000 of it 154.5, 152, 151.5, 151, 151.5; 300
+// skewed of 4096 x 1536 148, 141.5, 142.5, 139, 141; 800 of it 262, 254, 254, 253, 254; 2050 of it 371, 362, 360, 359, 356. With more tiles: 5000 of 2816 x 704 288, -, 288, 292, 293.
+// TMEM: 256 accumulator columns + 16 per resident box
 // + 64 for the rotating weight scales + 64 more for streamed operand scales.
 //
 // Once (no more tiles than experts, so hardly a weight record is read twice): the CTAs then share what HBM delivers by the bytes each has in flight, and one
@@ -88,19 +91,19 @@ static_assert(sizeof(GgShared) <= kGgHead, "the records start on a 1 KB boundary
 // 91.8, 91.7; 400 of 256 experts of 2048 x 1536 238.8, 236.0, 230.2, 227.5, 228.8; 700 skewed of 60 experts of 2304 x 1408 64.7, 64.2, 63.4, 62.6, 63.1; 300 skewed of
 // 4096 x 1536 151.5, 149.6, 148.0, 147.8, 147.7. With more tiles than experts records come from L2 as well, and depth is worth something: 2500 of 2048 x 768
 // 147.1, 147.2, 147.4, 147.9, 149.7; W4A16, 200 skewed of the 60 experts 65.8, 65.5, 65.4, 66.0, 68.2.
-constexpr int kGgMinRing = 4, kGgMinShared = 6, kGgMostOnce = 6;
+constexpr int kGgMinRing = 4, kGgMinShared = 6, kGgMinStream = 10, kGgMostOnce = 6;
 struct GgPlan { int astride, NR, NS; };
-__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows, bool once) {
+__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows, int tiles, int experts) {
   GgPlan p;
   const int room = kGgSmem - 1024 - kGgHead;
   p.astride = ((max_rows + 7) & ~7) * 128 + 2048;
   p.NR = KB < 12 ? KB : 12;
   if ((room - p.NR * p.astride) / kRec < kGgMinRing || p.NR < KB) {
-    p.NR = (room - kGgMinShared * kRec) / p.astride;
+    p.NR = (room - (tiles <= 2 * experts ? kGgMinStream : kGgMinShared) * kRec) / p.astride;
     if (p.NR > 8) p.NR = 8;
   }
   p.NS = (room - p.NR * p.astride) / kRec;
-  const int most = once && p.NR == KB ? kGgMostOnce : kGgMaxRing;
+  const int most = tiles <= experts && p.NR == KB ? kGgMostOnce : kGgMaxRing;
   if (p.NS > most) p.NS = most;
   return p;
 }
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0), NT <= P.E);
+  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0), NT, P.E);
   const int NR = plan.NR, NS = plan.NS, astride = plan.astride, acodes = astride - 2048;
   uint8_t* abuf = smem + kGgHead;                  // NR records of the current row tile
   uint8_t* ring = abuf + NR * astride;                          // NS slots
