@@ -132,6 +132,19 @@ def test_streamed_operand_boxes(m):
     check_prefill_call(w, ow, x, ids, wts, run_prefill(w, x, ids, wts), 512, sample_tokens=sample(ids, 8, 1), what=f"13 K boxes, {m} tokens")
 
 
+# How many ring slots a CTA has depends on the number of tiles: up to one an expert, up to two, more; with a resident operand (8 boxes) and a streamed
+# one (13). Rows are the same bits as in calls of at most 64 tokens, whose operand is resident and whose tiles are one an expert.
+@pytest.mark.parametrize("hidden", [2048, 3328])
+@pytest.mark.parametrize("rows", [(128, 100), (129, 100), (256, 200), (257, 250), (300, 400)])
+def test_ring_depth(hidden, rows):
+    cfg = dict(experts=2, hidden=hidden, inter=320, top_k=1)
+    w, _ = make_layer(**cfg, seed=6)
+    m = sum(rows)
+    x, ids, wts = inputs(cfg, m, 8)
+    ids = torch.repeat_interleave(torch.arange(2, dtype=torch.int32), torch.tensor(rows))[torch.randperm(m, generator=torch.Generator().manual_seed(1))][:, None].contiguous()
+    assert torch.equal(run_prefill(w, x, ids, wts, 1024), in_parts(w, x, ids, wts, 1024))
+
+
 @pytest.mark.parametrize("hidden", [2560, 4096])
 def test_silu_division_of_wide_layers(hidden):
     """Above nine K boxes FC1's SiLU divides with IEEE rounding. A gate of -88 shows it: 1 + exp(88) lies between 2^126 and 2^128, where
