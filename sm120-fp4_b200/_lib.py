@@ -12,6 +12,8 @@ _PKG = Path(__file__).resolve().parent
 # B200MOE_LIB: load another build of the same library (the diagnostic build of `build.py --diag`); default: the product build
 LIB_PATH = Path(os.environ["B200MOE_LIB"]) if os.environ.get("B200MOE_LIB") else _PKG / "libb200moe.so"
 _lib = None
+_host = None
+ONE_CLUSTER = 8192 * 16   # values of one matrix up to which the quantiser keeps them in registers and takes no workspace
 
 ERR_ARG, ERR_SHAPE, ERR_CUDA, ERR_DEVICE, ERR_TIMEOUT, ERR_WORKSPACE, ERR_LIMIT, ERR_RANGE, ERR_ORDER = -1, -2, -3, -4, -5, -6, -7, -8, -9
 
@@ -104,6 +106,20 @@ def lib() -> C.CDLL:
                 fn.restype, fn.argtypes = res, args
         _lib = h
     return _lib
+
+
+def host():
+    """The native host side of small calls (csrc/host.cpp), bound to the loaded library."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise ImportError(f"{_PKG / '_host.so'} is missing or stale: build it with `python {_PKG / 'build.py'}`; there is no fallback path") from e
+        h = lib()
+        module.bind(*(C.cast(f, C.c_void_p).value for f in (h.b200moe_quantize_nvfp4_own_scale, h.b200moe_quantize_nvfp4)), ONE_CLUSTER)
+        _host = module
+    return _host
 
 
 def check(code: int, what: str = "") -> None:

@@ -1,8 +1,9 @@
-"""Build recipe of the CUDA library: nvcc, sm_100a only, one shared object next to the package.
+"""Build recipe of the CUDA library: nvcc, sm_100a only, one shared object next to the package; and of the Python extension beside it
+(csrc/host.cpp against torch's C++ interface: the host side of small calls).
 
     python sm120-fp4_b200/build.py [--verbose]
 
-The shared object exports the C ABI declared in include/b200moe.h and nothing else that a caller needs.
+The library exports the C ABI declared in include/b200moe.h and nothing else that a caller needs.
 """
 from __future__ import annotations
 
@@ -10,6 +11,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -39,6 +41,28 @@ def sources() -> list[Path]:
     return [CSRC / s for s in SOURCES if (CSRC / s).exists()] + sorted(p for p in CSRC.glob("*.cu") if p.name not in SOURCES)
 
 
+HOST_SRC, HOST = CSRC / "host.cpp", PKG / "_host.so"
+
+
+def host_command() -> list[str]:
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc()).resolve().parent.parent
+    return [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+            f"-I{root / 'include'}", f"-I{cuda / 'include'}", f"-I{sysconfig.get_paths()['include']}", str(HOST_SRC), "-o", str(HOST),
+            f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
+def build_host(verbose: bool = False, force: bool = False) -> Path:
+    if force or not HOST.exists() or HOST.stat().st_mtime <= HOST_SRC.stat().st_mtime:
+        r = subprocess.run(host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if verbose or r.returncode:
+            print(f"--- {HOST_SRC.name}\n{r.stdout}", file=sys.stderr)
+        if r.returncode:
+            raise RuntimeError(f"{HOST_SRC.name} failed")
+    return HOST
+
+
 def stale() -> bool:
     if not LIB.exists():
         return True
@@ -47,6 +71,7 @@ def stale() -> bool:
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
+    build_host(verbose, force)
     if not force and not stale():
         return LIB
     objs = []

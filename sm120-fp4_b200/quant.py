@@ -36,7 +36,7 @@ def _check_2d(x: torch.Tensor) -> None:
         raise RuntimeError("quantize_nvfp4 runs on the GPU; there is no CPU path in this package")
 
 
-_ONE_CLUSTER = 8192 * BLOCK   # values of one matrix up to which the quantiser keeps them in registers and takes no workspace
+_ONE_CLUSTER = _lib.ONE_CLUSTER
 _WS: dict = {}                # (device index, stream) -> zeroed workspace of eager calls, grown on demand
 
 
@@ -83,6 +83,10 @@ def _scale_on(device: torch.device, gs: torch.Tensor) -> torch.Tensor:
 def quantize_nvfp4(x: torch.Tensor, global_scale: torch.Tensor | None = None):
     """x [M, K] bf16/fp32 -> (packed u8 [M, K/2], sf u8 [M, K/16] E4M3 bits row-major, global_scale f32 [1])
     (sm120fp4/reference.py:74-90)."""
+    if global_scale is None and type(x) is torch.Tensor and x.is_cuda:      # a small plain matrix in one native call (csrc/host.cpp), else None
+        out = (_lib._host or _lib.host()).quantize_own_scale(x)
+        if out is not None:
+            return out if type(out) is tuple else _lib.check(out, "quantize_nvfp4")
     _check_2d(x)
     if x.dtype not in (torch.bfloat16, torch.float32):
         x = x.float()
@@ -105,6 +109,10 @@ def quantize_nvfp4_128x4(x: torch.Tensor, global_scale: torch.Tensor, src_row: t
     """Fused quantizer: packed u8 [R, K/2] and block scales written directly in the 128x4 swizzle ([pad128(R), pad4(K/16)]).
     With `src_row` (int32 [R]) destination row r reads x[src_row[r]] (negative: a zero row), which lays tokens out in
     per-expert segments without a separate gather."""
+    if src_row is None and type(x) is torch.Tensor and x.is_cuda:      # (as in quantize_nvfp4)
+        out = (_lib._host or _lib.host()).quantize_128x4(x, global_scale)
+        if out is not None:
+            return out if type(out) is tuple else _lib.check(out, "quantize_nvfp4_128x4")
     _check_2d(x)
     x = x.contiguous()
     k = x.shape[1]

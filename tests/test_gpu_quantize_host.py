@@ -1,0 +1,83 @@
+"""The native host side of small quantiser calls (csrc/host.cpp) against the general path, which the same call takes without it: same outputs (shapes, strides, types and
+bytes), and None - so that the general path runs, with its checks and errors - for everything that is not a plain contiguous CUDA matrix."""
+import types
+
+import pytest
+import torch
+
+import sm120fp4_b200 as pkg
+from sm120fp4_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def general(monkeypatch, fn):
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "_host", types.SimpleNamespace(quantize_own_scale=lambda *a: None, quantize_128x4=lambda *a: None))
+        return fn()
+
+
+def same(a, b):
+    assert len(a) == len(b) == 3
+    for s, t in zip(a, b):
+        assert s.shape == t.shape and s.stride() == t.stride() and s.dtype == t.dtype and s.device == t.device and s.requires_grad == t.requires_grad
+        assert torch.equal(s.view(torch.uint8), t.view(torch.uint8))
+
+
+# 64 x 2048 is the largest matrix that needs no workspace; 65 x 2048 and all matrices beyond take the general path
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,k", [(1, 16), (3, 80), (16, 2048), (64, 2048), (65, 2048), (8192, 16), (129, 1040)])
+def test_outputs(monkeypatch, rows, k, dtype):
+    x = torch.randn(rows, k, device="cuda", generator=torch.Generator("cuda").manual_seed(rows)).to(dtype).requires_grad_(rows == 3)
+    taken = _lib.host().quantize_own_scale(x)
+    assert (taken is not None) == (rows * k <= 64 * 2048)
+    want = general(monkeypatch, lambda: pkg.quantize_nvfp4(x))
+    same(pkg.quantize_nvfp4(x), want)
+    gs = want[2]
+    assert _lib.host().quantize_128x4(x, gs) is not None
+    got = pkg.quantize_nvfp4_128x4(x, gs)
+    assert got[2] is gs
+    same(got, general(monkeypatch, lambda: pkg.quantize_nvfp4_128x4(x, gs)))
+
+
+def test_what_is_left_to_the_general_path(monkeypatch):
+    h = _lib.host()
+    x, gs = torch.randn(8, 64, device="cuda"), torch.ones(1, device="cuda")
+    views = [x.t()[:16], x[:, :32], x[::2], x[:0], x[:, :0], x[0], x[None], x.half(), x[:, :24].contiguous(), x.cpu(), torch.nn.Parameter(x), x.to_sparse(), None, 3, "x"]
+    for v in views[:10] + views[11:]:
+        assert h.quantize_own_scale(v) is None and h.quantize_128x4(v, gs) is None
+    for g in (torch.ones((), device="cuda"), torch.ones(2, device="cuda"), torch.ones(1), torch.ones(1, device="cuda", dtype=torch.float64), None, 1.0):
+        assert h.quantize_128x4(x, g) is None
+    assert torch.vmap(lambda v: (h.quantize_own_scale(v) is None) * v)(torch.randn(2, 8, 64, device="cuda")).sum() != 0   # inside a transform
+    from torch.overrides import TorchFunctionMode
+
+    class Seen(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    with Seen():
+        assert h.quantize_own_scale(x) is None
+    for v in (x[:, :32], x[::2], x.half()):       # results and errors are the general path's
+        same(pkg.quantize_nvfp4(v), general(monkeypatch, lambda: pkg.quantize_nvfp4(v)))
+    with pytest.raises(ValueError):
+        pkg.quantize_nvfp4(x[:, :24].contiguous())
+    with pytest.raises(TypeError):
+        pkg.quantize_nvfp4_128x4(x.half(), gs)
+    with pytest.raises(TypeError):
+        h.bind(1)
+
+
+def test_streams_and_capture():
+    x = torch.randn(16, 2048, device="cuda", dtype=torch.bfloat16)
+    want = [t.clone() for t in pkg.quantize_nvfp4(x)]
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        same(pkg.quantize_nvfp4(x), want)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        out = pkg.quantize_nvfp4(x)
+    x.mul_(-1)
+    g.replay()
+    torch.cuda.synchronize()
+    same(out, pkg.quantize_nvfp4(x))
