@@ -227,22 +227,28 @@ __device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
   }
 }
 
+// The rows of a thread's first slots are looked up ahead of the wait: dst_row is complete (the kernels of this call start behind the one that has seen its writer complete),
+// and most of the blocks are here before FC2 is.
 template <bool F32>
 __global__ void __launch_bounds__(256) k_combine(const void* yv, const int* dst_row, int M, int top_k, int H, __nv_bfloat16* out) {
   constexpr int kBatch = F32 ? 4 : 8;
-  const int chunks = H / 8;
-  const long long total = (long long)M * chunks;
+  const unsigned chunks = (unsigned)H / 8, total = (unsigned)M * chunks, step = gridDim.x * 256;   // (2^32 chunks are 64 GB of x, as much of out and more of rows)
+  unsigned i = blockIdx.x * 256 + threadIdx.x;
+  int tok = (int)(i / chunks), c = (int)(i % chunks);
+  int r[kBatch];
+  auto look = [&](int j0) {
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) r[j] = j0 + j < top_k ? __ldcg(dst_row + tok * top_k + j0 + j) : -1;   // -1: empty slot
+  };
+  if (i < total) look(0);
   grid_dependency_wait();
   grid_launch_dependents();
 #pragma unroll 1
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int tok = (int)(i / chunks), c = (int)(i % chunks);
+  while (i < total) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int j0 = 0; j0 < top_k; j0 += kBatch) {
-      int r[kBatch];
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) r[j] = j0 + j < top_k ? __ldcg(dst_row + tok * top_k + j0 + j) : -1;   // -1: empty slot
+      if (j0) look(j0);
       uint4 v[kBatch][F32 ? 2 : 1];
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
@@ -271,6 +277,10 @@ __global__ void __launch_bounds__(256) k_combine(const void* yv, const int* dst_
     }
     if (!F32) combine_columns(o, threadIdx.x & 31);
     *reinterpret_cast<uint4*>(out + (long long)tok * H + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    i += step;
+    if (i < step) break;   // (past the end of the type)
+    tok = (int)(i / chunks), c = (int)(i % chunks);
+    if (i < total) look(0);
   }
 }
 
