@@ -215,9 +215,6 @@ __global__ void __launch_bounds__(128) k_expand_scatter(const __nv_bfloat16* __r
 }
 
 // ------------------------------------------------------------------------------------------------ combine
-// out[tok, :] = sum_j y[dst_row[tok*k + j], :] in slot order, fp32 accumulation, one bf16 rounding (for fp32 rows, the W4A16 path,
-// the only one of the layer). A thread sums eight columns; the rows of eight slots are loaded before the first is added, so
-// that the loads of a token overlap (with one row at a time: 88 us at 8192 tokens x 8 rows of 4 KB).
 __device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -227,11 +224,16 @@ __device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
   }
 }
 
+// out[tok, :] = sum_j y[dst_row[tok*k + j], :] in slot order, fp32 accumulation, one bf16 rounding (for fp32 rows, the W4A16 path,
+// the only one of the layer). A thread sums eight columns; the rows of Batch slots are loaded before the first is added, so
+// that the loads of a token overlap (with one row at a time: 88 us at 8192 tokens x 8 rows of 4 KB).
 // The rows of a thread's first slots are looked up ahead of the wait: dst_row is complete (the kernels of this call start behind the one that has seen its writer complete),
 // and most of the blocks are here before FC2 is.
-template <bool F32>
-__global__ void __launch_bounds__(256) k_combine(const void* yv, const int* dst_row, int M, int top_k, int H, __nv_bfloat16* out) {
-  constexpr int kBatch = F32 ? 4 : 8;
+// Blocks: resident per SM, which says how many registers a thread has. The loads are volatile, or the compiler adds as it loads to save registers: with 32
+// of them about four were in flight, and a call of 333 tokens of 2816 x 704 took 71.1 us instead of 68.5, of 512 of 2048 x 768 37.8 instead of 35.2.
+template <bool F32, int Batch, int Blocks>
+__global__ void __launch_bounds__(256, Blocks) k_combine(const void* yv, const int* dst_row, int M, int top_k, int H, __nv_bfloat16* out) {
+  constexpr int kBatch = Batch;
   const unsigned chunks = (unsigned)H / 8, total = (unsigned)M * chunks, step = gridDim.x * 256;   // (2^32 chunks are 64 GB of x, as much of out and more of rows)
   unsigned i = blockIdx.x * 256 + threadIdx.x;
   int tok = (int)(i / chunks), c = (int)(i % chunks);
@@ -254,7 +256,12 @@ __global__ void __launch_bounds__(256) k_combine(const void* yv, const int* dst_
       for (int j = 0; j < kBatch; ++j) {
 #pragma unroll
         for (int q = 0; q < (F32 ? 2 : 1); ++q)
-          v[j][q] = r[j] >= 0 ? __ldcg(reinterpret_cast<const uint4*>(yv) + ((long long)r[j] * H + c * 8) / (F32 ? 4 : 8) + q) : make_uint4(0u, 0u, 0u, 0u);
+        {
+          v[j][q] = make_uint4(0u, 0u, 0u, 0u);
+          if (r[j] >= 0)
+            asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[j][q].x), "=r"(v[j][q].y), "=r"(v[j][q].z), "=r"(v[j][q].w)
+                         : "l"(reinterpret_cast<const uint4*>(yv) + ((long long)r[j] * H + c * 8) / (F32 ? 4 : 8) + q));
+        }
       }
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
@@ -413,7 +420,10 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   if (rc != B200MOE_OK) return rc;
   const uint8_t* y = w + L.y;
   void* args[] = {(void*)&y, (void*)&dst_row, (void*)&M, (void*)&top_k, (void*)&H, (void*)&out};
-  return launch_kernel((const void*)k_combine<false>, sms * 8, 256, 0, true, args, st);
+  // Rows that L2 does not hold come at HBM's rate, and more threads are worth more than more loads of each: 8192 tokens of 2048 x 768 (268 MB) 304.5 us, 306 with
+  // half the threads and twice the loads; 4000 (131 MB) 169 either way, 2500 142.5 and 141.
+  const bool deep = (long long)P * H * 2 <= (126LL << 20);
+  return launch_kernel(deep ? (const void*)k_combine<false, 8, 4> : (const void*)k_combine<false, 8, 8>, sms * 8, 256, 0, true, args, st);
 }
 
 int b200_prefill_status_offset(int E, int H, int I, int top_k, int max_tokens, long long* off) {
@@ -516,7 +526,10 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   if (rc != B200MOE_OK) return rc;
   const uint8_t* y = w + L.y;
   void* args[] = {(void*)&y, (void*)&dst_row, (void*)&M, (void*)&top_k, (void*)&H, (void*)&out};
-  return launch_kernel((const void*)k_combine<true>, sms * 4, 256, 0, true, args, st);
+  // Eight slots at a time where there are more than four and enough columns to fill the SMs: 256 tokens of 2048 x 768 87.1 us (with four at a time 89.9), 200 of
+  // 2816 x 704 99.4 (102.0), 96 of 2048 x 768 74.2 (74.4); 64 of 2816 x 704 91.5 (91.0), 40 of 2048 x 768 67.5 (66.7), 100 of 60 experts with four slots 70.7 (70.0).
+  const bool eight = top_k > 4 && (long long)M * H >= 96 * 2048;
+  return launch_kernel(eight ? (const void*)k_combine<true, 8, 2> : (const void*)k_combine<true, 4, 4>, sms * 4, 256, 0, true, args, st);
 }
 
 // out[i] = g[i] / den[i], den[i] = 1 + exp(-g[i]), as FC1's epilogue divides in wide layers (gg_quotient), for tests.

@@ -145,6 +145,15 @@ def test_ring_depth(hidden, rows):
     assert torch.equal(run_prefill(w, x, ids, wts, 1024), in_parts(w, x, ids, wts, 1024))
 
 
+# Rows that L2 does not hold (4100 tokens of 16 slots and 1024 columns) are added up by more threads with fewer loads each.
+def test_rows_beyond_l2():
+    cfg = dict(experts=24, hidden=1024, inter=64, top_k=16)
+    w, _ = make_layer(**cfg, seed=7)
+    x, ids, wts = inputs(cfg, 4100, 9)
+    assert 4100 * 16 * 1024 * 2 > 126 << 20
+    assert torch.equal(run_prefill(w, x, ids, wts, 4100), in_parts(w, x, ids, wts, 4100))
+
+
 @pytest.mark.parametrize("hidden", [2560, 4096])
 def test_silu_division_of_wide_layers(hidden):
     """Above nine K boxes FC1's SiLU divides with IEEE rounding. A gate of -88 shows it: 1 + exp(88) lies between 2^126 and 2^128, where
