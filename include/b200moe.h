@@ -125,7 +125,10 @@ int b200moe_prefill_status(const b200moe_layer* layer, const void* workspace, in
  * tile_end (128-row tiles: expert, first and end index into pairs), row_pair [tiles*128], dst_row [pairs], x records,
  * activation records, weighted bf16 rows, tile capacity, total bytes. A record is 18,432 bytes per (tile, 256-value K box):
  * row r, 16-value block b at r*128 + (((b>>1) ^ (r&7)) << 4) + (b&1)*8 (8 code bytes), its scale byte at 16384 + (b>>2)*512 +
- * (r&31)*16 + (r>>5)*4 + (b&3) - i.e. four 128x4 scale tiles. */
+ * (r&31)*16 + (r>>5)*4 + (b&3) - i.e. four 128x4 scale tiles. Weighted row dst_row[pair] is what the pair adds to its token's
+ * output, rounded to bf16; its value for column c stands at B200MOE_WEIGHTED_ROW_COLUMN(c), because a row is stored as the lanes
+ * hold the accumulator (stated since version 101; a library of version 100 has it there or at c). */
+#define B200MOE_WEIGHTED_ROW_COLUMN(c) (((c) & ~31) | (((c) >> 1 & 3) << 3) | (((c) >> 3 & 3) << 1) | ((c) & 1))
 int b200moe_prefill_workspace_map(const b200moe_layer* layer, int max_tokens, long long* out14);
 /* For tests: out[i] = gate[i] / den[i], den[i] = 1 + exp(-gate[i]), as the W4A4 FC1 epilogue of hidden sizes above 2304 divides (IEEE
  * rounding). */

@@ -71,7 +71,7 @@ struct b200moe_layer {
 
 static inline long long align_up(long long v, long long a) { return (v + a - 1) / a * a; }
 
-extern "C" int b200moe_version(void) { return 100; }
+extern "C" int b200moe_version(void) { return 101; }
 
 extern "C" const char* b200moe_error_string(int code) {
   switch (code) {
@@ -502,7 +502,7 @@ extern "C" int b200moe_prefill_forward(const b200moe_layer* L, const void* x_bf1
 
 // Where the tables and tile records sit inside a prefill workspace sized for max_tokens (14 values, see the header): lets a
 // tool or a test read back what each stage of the last call wrote (router tables, NVFP4 records of x and of the SiLU*mul
-// activations, weighted rows). Host-side arithmetic only.
+// activations, weighted rows with columns at B200MOE_WEIGHTED_ROW_COLUMN). Host-side arithmetic only.
 extern "C" int b200moe_prefill_workspace_map(const b200moe_layer* L, int max_tokens, long long* out14) {
   if (!L || !out14 || max_tokens <= 0) return B200MOE_ERR_ARG;
   b200_prefill_workspace_map(L->E, L->H, L->I, L->top_k, max_tokens, out14);

@@ -52,7 +52,7 @@ struct GroupedParams {
   float gs_out;               // PHASE 1: global scale for the activation re-quantisation
   const float* wts;           // PHASE 2/4: routing weights [P]
   uint8_t* orec;              // PHASE 1/3: FC2 operand records [ntiles][KB2][...]
-  __nv_bfloat16* y;           // PHASE 2: weighted rows [ntiles*128][H], columns ordered as gg_epilogue_fc2 says
+  __nv_bfloat16* y;           // PHASE 2: weighted rows [ntiles*128][H], columns at B200MOE_WEIGHTED_ROW_COLUMN
   float* yf;                  // PHASE 4: weighted rows [ntiles*16][H] in fp32 (one rounding only, in the combine)
   int* status;
   const float* rowscale;      // PHASE 3: 1 / g_t of every term row of the x operand [ntiles*64]
@@ -201,7 +201,7 @@ __device__ __forceinline__ void gg_epilogue_fc1(uint32_t taddr, float s, float g
 // W4A4 FC2: scale, round to bf16 and store. The accumulator is read in the fragment layout of mma (eight rows x four lanes), so that the four lanes
 // of a row hold 64 columns between them and an instruction stores 64-byte halves of eight rows' segments; nothing goes through shared
 // memory. The columns of a segment lie as the lanes hold them: 16-byte chunk 4j + q has columns 32j + 8w + 2q + {0, 1}, w = 0..3 (combine_columns
-// puts them right). s[i]: scale of row 8i + lane / 4 of the warp; the first `rows` rows hold a pair. A block's epilogue takes 920 cycles at 1024
+// puts them right; B200MOE_WEIGHTED_ROW_COLUMN tells callers). s[i]: scale of row 8i + lane / 4 of the warp; the first `rows` rows hold a pair. A block's epilogue takes 920 cycles at 1024
 // tokens of the 2048 x 768 layer and 1290 at 8192 (FC2 73 us there); with a thread per row and a transposition through shared memory 2680 and 3170 (84 us, the
 // epilogue was the bound), with that and bulk stores 4040 and 3850: a store waits behind the ring's loads in the copy engine.
 template <class F>

@@ -331,7 +331,7 @@ long long b200_prefill_workspace_bytes(int E, int H, int I, int top_k, int max_t
 
 // Byte offsets of the tables and records inside a prefill workspace, for tools and tests that read them back:
 // out[0..11] = experts, offsets, pairs, ntiles, tile_expert, tile_first, tile_end, row_pair, dst_row, x records, activation
-// records, weighted rows; out[12] = tile capacity, out[13] = total bytes.
+// records, weighted rows (columns at B200MOE_WEIGHTED_ROW_COLUMN); out[12] = tile capacity, out[13] = total bytes.
 void b200_prefill_workspace_map(int E, int H, int I, int top_k, int max_tokens, long long* out) {
   const PrefillLayout L = prefill_layout(E, H, I, top_k, max_tokens);
   const long long v[14] = {L.experts, L.offsets, L.pairs, L.ntiles, L.tile_expert, L.tile_tab, L.tile_tab + 4LL * L.max_tiles, L.row_pair,

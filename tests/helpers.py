@@ -66,6 +66,14 @@ def prefill_map(w, max_tokens: int) -> dict:
     return dict(zip(names, [int(v) for v in buf]))
 
 
+def weighted_row_column(c):
+    """Where a weighted row of a prefill workspace keeps column c: the header's B200MOE_WEIGHTED_ROW_COLUMN (its C operators mean the same here)."""
+    import re
+    from pathlib import Path
+    header = (Path(__file__).resolve().parent.parent / "include" / "b200moe.h").read_text()
+    return eval(re.search(r"#define B200MOE_WEIGHTED_ROW_COLUMN\(c\) (.*)", header)[1], {"c": c})
+
+
 def _i32(ws: torch.Tensor, off: int, n: int) -> np.ndarray:
     return ws[off:off + 4 * n].view(torch.int32).cpu().numpy()
 

@@ -23,6 +23,13 @@ def test_header_symbols_are_exported_and_bound():
     assert b"workspace" in h.b200moe_error_string(L.ERR_WORKSPACE)
 
 
+def test_weighted_row_columns_are_a_permutation_of_each_32():
+    from helpers import weighted_row_column
+    at = [weighted_row_column(c) for c in range(128)]
+    assert sorted(at) == list(range(128)) and all(a // 32 == c // 32 for c, a in enumerate(at))
+    assert at[:10] == [0, 1, 8, 9, 16, 17, 24, 25, 2, 3]
+
+
 def test_argument_errors_need_no_gpu():
     import sm120fp4_b200._lib as L
     h = L.lib()

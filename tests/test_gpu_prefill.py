@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import check_prefill_call, check_w4a4_output
+from helpers import _i32, check_prefill_call, check_w4a4_output, prefill_map, read_records, weighted_row_column
+from oracle import conformance as C
 from oracle import nvfp4_oracle as O
 from test_gpu_decode import inputs, layer
 
@@ -69,6 +70,29 @@ def test_prefill_gemma_shape_stage_by_stage():
     r = check_prefill_call(w, ow, x, ids, wts, out, 256, sample_tokens=sample(ids, 8, 1), what="gemma prefill m=256")
     print(f"gemma prefill m=256: own codes {r['max_abs_over_rms_own_codes']:.2e} x rms, {r['max_err_over_bound']:.2f} x bound; "
           f"{r['flips']} code flips in {r['pairs']} rows; plain oracle {r['max_abs_over_rms_plain_oracle']:.2e} x rms")
+
+
+def test_weighted_rows_read_back():
+    """The rows that FC2 leaves in the workspace, one per (token, expert) pair, columns where the header says: every value the bf16 rounding of something inside
+    the accumulation interval of the exact product of the kernel's own activation codes."""
+    cfg, w, ow = layer("mid")
+    x, ids, wts = inputs(cfg, 150, 61)
+    ids, wts = ids.clone(), wts.clone()
+    ids[7, 2], wts[7, 2] = -1, 0
+    run_prefill(w, x, ids, wts)
+    mp, ws, (m, k) = prefill_map(w, 512), w.prefill.workspace, ids.shape
+    h, inter = ow.H, ow.I
+    nt, dst_row = int(_i32(ws, mp["ntiles"], 1)[0]), _i32(ws, mp["dst_row"], m * k)
+    codes, sfs, _ = read_records(ws, mp["arec"], nt, (inter + 255) // 256)
+    y = ws[mp["y"]:mp["y"] + nt * 128 * h * 2].view(torch.bfloat16).view(nt * 128, h).float().cpu().numpy()[:, weighted_row_column(np.arange(h))]
+    for e in range(ow.E):
+        tok, slot = np.nonzero(ids.numpy() == e)
+        rows = dst_row[tok * k + slot]
+        a = C.dequant_exact(codes[rows][:, : inter // 2], sfs[rows][:, : inter // 16], 1.0)
+        c, cb, _ = C.interval_gemm(a, a, C.dequant_exact(ow.q2[e], ow.s2[e].reshape(h, inter // 16), 1.0) * float(ow.alpha2[e]))
+        wf = wts.numpy()[tok, slot].astype(np.float64)[:, None]
+        lo, hi = C._round_bf16_interval((c - cb) * wf, (c + cb) * wf, 4 * C.U32)
+        assert ((lo <= y[rows]) & (y[rows] <= hi)).all(), f"expert {e}"
 
 
 def test_prefill_matches_golden_reference_output(golden):
