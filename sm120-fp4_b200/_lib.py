@@ -1,10 +1,11 @@
-"""ctypes binding of libb200moe.so (the C ABI of include/b200moe.h). There is no fallback: a missing or stale library
+"""ctypes binding of libb200moe.so (the C ABI of include/b200moe.h). There is no fallback for it: a missing or stale library
 raises, and every non-zero return code raises with the library's own message."""
 from __future__ import annotations
 
 import ctypes as C
 import os
 from pathlib import Path
+from types import SimpleNamespace
 
 import torch
 
@@ -14,6 +15,7 @@ LIB_PATH = Path(os.environ["B200MOE_LIB"]) if os.environ.get("B200MOE_LIB") else
 _lib = None
 _host = None
 ONE_CLUSTER = 8192 * 16   # values of one matrix up to which the quantiser keeps them in registers and takes no workspace
+NO_HOST = SimpleNamespace(quantize_own_scale=lambda *args: None, quantize_128x4=lambda *args: None)
 
 ERR_ARG, ERR_SHAPE, ERR_CUDA, ERR_DEVICE, ERR_TIMEOUT, ERR_WORKSPACE, ERR_LIMIT, ERR_RANGE, ERR_ORDER = -1, -2, -3, -4, -5, -6, -7, -8, -9
 
@@ -109,15 +111,17 @@ def lib() -> C.CDLL:
 
 
 def host():
-    """The native host side of small calls (csrc/host.cpp), bound to the loaded library."""
+    """The native host side of small calls (csrc/host.cpp), bound to the loaded library; NO_HOST, which takes no call, beside a library that
+    came without it: every call then takes its general path, to the same kernels."""
     global _host
     if _host is None:
+        h = lib()
         try:
             from . import _host as module
-        except ImportError as e:
-            raise ImportError(f"{_PKG / '_host.so'} is missing or stale: build it with `python {_PKG / 'build.py'}`; there is no fallback path") from e
-        h = lib()
-        module.bind(*(C.cast(f, C.c_void_p).value for f in (h.b200moe_quantize_nvfp4_own_scale, h.b200moe_quantize_nvfp4)), ONE_CLUSTER)
+        except ImportError:
+            module = NO_HOST
+        else:
+            module.bind(*(C.cast(f, C.c_void_p).value for f in (h.b200moe_quantize_nvfp4_own_scale, h.b200moe_quantize_nvfp4)), ONE_CLUSTER)
         _host = module
     return _host
 

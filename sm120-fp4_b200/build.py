@@ -7,6 +7,7 @@ The library exports the C ABI declared in include/b200moe.h and nothing else tha
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -71,7 +72,14 @@ def stale() -> bool:
 
 
 def build(verbose: bool = False, force: bool = False) -> Path:
-    build_host(verbose, force)
+    """The library, and where torch is installed the host extension."""
+    build_library(verbose, force)
+    if importlib.util.find_spec("torch"):
+        build_host(verbose, force)
+    return LIB
+
+
+def build_library(verbose: bool = False, force: bool = False) -> Path:
     if not force and not stale():
         return LIB
     objs = []

@@ -1,7 +1,5 @@
 """The native host side of small quantiser calls (csrc/host.cpp) against the general path, which the same call takes without it: same outputs (shapes, strides, types and
 bytes), and None - so that the general path runs, with its checks and errors - for everything that is not a plain contiguous CUDA matrix."""
-import types
-
 import pytest
 import torch
 
@@ -13,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 def general(monkeypatch, fn):
     with monkeypatch.context() as m:
-        m.setattr(_lib, "_host", types.SimpleNamespace(quantize_own_scale=lambda *a: None, quantize_128x4=lambda *a: None))
+        m.setattr(_lib, "_host", _lib.NO_HOST)
         return fn()
 
 
