@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 from pathlib import Path
 from types import SimpleNamespace
 
@@ -112,15 +113,23 @@ def lib() -> C.CDLL:
 
 def host():
     """The native host side of small calls (csrc/host.cpp), bound to the loaded library; NO_HOST, which takes no call, beside a library that
-    came without it: every call then takes its general path, to the same kernels."""
+    came without it, or with one that was built for another torch: every call then takes its general path, to the same kernels."""
     global _host
     if _host is None:
         h = lib()
         try:
             from . import _host as module
-        except ImportError:
-            module = NO_HOST
+        except ImportError as e:      # not there, or symbols of another torch
+            module, why = NO_HOST, e if any(_PKG.glob("_host.*")) else None
         else:
+            built_for = getattr(module, "torch_version", "unknown")
+            if built_for == torch.__version__:
+                why = None
+            else:
+                module, why = NO_HOST, f"it was built for torch {built_for}, this is {torch.__version__}"
+        if why:
+            warnings.warn(f"the host extension is left out, small quantiser calls take longer: {why}; build it again with `python {_PKG / 'build.py'}`", RuntimeWarning, stacklevel=3)
+        if module is not NO_HOST:
             module.bind(*(C.cast(f, C.c_void_p).value for f in (h.b200moe_quantize_nvfp4_own_scale, h.b200moe_quantize_nvfp4)), ONE_CLUSTER)
         _host = module
     return _host

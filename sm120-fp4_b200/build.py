@@ -42,25 +42,44 @@ def sources() -> list[Path]:
     return [CSRC / s for s in SOURCES if (CSRC / s).exists()] + sorted(p for p in CSRC.glob("*.cu") if p.name not in SOURCES)
 
 
-HOST_SRC, HOST = CSRC / "host.cpp", PKG / "_host.so"
+# The extension inlines torch's C++ interface and knows the interpreter's: its name carries the interpreter's ABI, its code the version of torch (which
+# _lib.host() compares), and it is built again whenever the command would be another one.
+HOST_SRC, HOST = CSRC / "host.cpp", PKG / f"_host{sysconfig.get_config_var('EXT_SUFFIX')}"
+HOST_BUILT_BY = PKG / "build" / "host.command"
 
 
-def host_command() -> list[str]:
+def host_command(out: Path) -> list[str]:
     import torch
     root = Path(torch.__file__).resolve().parent
     cuda = Path(nvcc()).resolve().parent.parent
     return [os.environ.get("CXX") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-            f"-I{root / 'include'}", f"-I{cuda / 'include'}", f"-I{sysconfig.get_paths()['include']}", str(HOST_SRC), "-o", str(HOST),
+            f'-DB200_TORCH_VERSION="{torch.__version__}"',
+            f"-I{root / 'include'}", f"-I{cuda / 'include'}", f"-I{sysconfig.get_paths()['include']}", str(HOST_SRC), "-o", str(out),
             f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
+def host_record() -> str:
+    return "\n".join(host_command(HOST)).replace(str(PKG), ".")      # (the folder may be moved)
+
+
+def host_stale() -> bool:
+    if not HOST.exists() or HOST.stat().st_mtime <= HOST_SRC.stat().st_mtime or not HOST_BUILT_BY.exists():
+        return True
+    return HOST_BUILT_BY.read_text() != host_record()
+
+
 def build_host(verbose: bool = False, force: bool = False) -> Path:
-    if force or not HOST.exists() or HOST.stat().st_mtime <= HOST_SRC.stat().st_mtime:
-        r = subprocess.run(host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if force or host_stale():
+        new = HOST.with_name(HOST.name + f".{os.getpid()}")      # put in place whole: another process may be loading the old one
+        r = subprocess.run(host_command(new), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if verbose or r.returncode:
             print(f"--- {HOST_SRC.name}\n{r.stdout}", file=sys.stderr)
         if r.returncode:
             raise RuntimeError(f"{HOST_SRC.name} failed")
+        HOST_BUILT_BY.parent.mkdir(exist_ok=True)
+        HOST_BUILT_BY.unlink(missing_ok=True)
+        os.replace(new, HOST)
+        HOST_BUILT_BY.write_text(host_record())
     return HOST
 
 

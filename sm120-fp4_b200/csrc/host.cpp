@@ -121,4 +121,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host(void) {   // (nothing of torch: the caller compares the version before anything else)
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch_version", B200_TORCH_VERSION)) Py_CLEAR(m);
+  return m;
+}
