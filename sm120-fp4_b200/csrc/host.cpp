@@ -44,6 +44,12 @@ bool plain_matrix(const at::Tensor& x) {
 
 at::Tensor bytes(int64_t rows, int64_t cols, const at::Tensor& like) { return at::empty({rows, cols}, at::TensorOptions().dtype(at::kByte).device(like.device())); }
 
+// Python runs on meanwhile, as under torch's own calls: an allocation may wait for the device, and the device for a callback that wants the interpreter.
+struct Released {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Released() { PyEval_RestoreThread(state); }
+};
+
 PyObject* outputs(int rc, const at::Tensor& packed, const at::Tensor& sf, PyObject* scale) {   // takes over the reference to scale
   if (rc) {
     Py_XDECREF(scale);
@@ -75,18 +81,17 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_quantize_own_scale(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 1 || !own_scale || !THPVariable_CheckExact(args[0]) || !plain_call()) Py_RETURN_NONE;
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const at::Tensor x = THPVariable_Unpack(args[0]);
   if (!plain_matrix(x) || x.numel() > one_cluster) Py_RETURN_NONE;
   const int64_t rows = x.size(0), k = x.size(1);
-  const at::Tensor packed = bytes(rows, k / 2, x), sf = bytes(rows, k / 16, x), gs = at::empty({1}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
-  const void* src = x.data_ptr();
-  void *d = packed.data_ptr(), *s = sf.data_ptr(), *g = gs.data_ptr();
-  void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
-  const int dtype = x.scalar_type() == at::kFloat;
+  at::Tensor packed, sf, gs;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = own_scale(src, dtype, 1, (int)rows, (int)k, g, d, s, 0, nullptr, 0, stream);
-  Py_END_ALLOW_THREADS
+  {
+    Released released;
+    packed = bytes(rows, k / 2, x), sf = bytes(rows, k / 16, x), gs = at::empty({1}, at::TensorOptions().dtype(at::kFloat).device(x.device()));
+    rc = own_scale(x.data_ptr(), x.scalar_type() == at::kFloat, 1, (int)rows, (int)k, gs.data_ptr(), packed.data_ptr(), sf.data_ptr(), 0, nullptr, 0,
+                   (void*)c10::cuda::getCurrentCUDAStream().stream());
+  }
   return outputs(rc, packed, sf, THPVariable_Wrap(gs));
   END_HANDLE_TH_ERRORS
 }
@@ -95,19 +100,18 @@ PyObject* py_quantize_own_scale(PyObject*, PyObject* const* args, Py_ssize_t n) 
 PyObject* py_quantize_128x4(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 2 || !quantize || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !plain_call()) Py_RETURN_NONE;
-  const at::Tensor &x = THPVariable_Unpack(args[0]), &gs = THPVariable_Unpack(args[1]);
+  const at::Tensor x = THPVariable_Unpack(args[0]), gs = THPVariable_Unpack(args[1]);
   if (!plain_matrix(x) || !plain_tensor(gs) || gs.scalar_type() != at::kFloat || gs.dim() != 1 || gs.size(0) != 1 || gs.device() != x.device()) Py_RETURN_NONE;
   const int64_t rows = x.size(0), k = x.size(1);
   if (rows > 0x7fffffff - 128 || k > 0x7fffffff) Py_RETURN_NONE;
-  const at::Tensor packed = bytes(rows, k / 2, x), sf = bytes((rows + 127) / 128 * 128, (k / 16 + 3) / 4 * 4, x);
-  const void *src = x.data_ptr(), *g = gs.data_ptr();
-  void *d = packed.data_ptr(), *s = sf.data_ptr();
-  void* stream = (void*)c10::cuda::getCurrentCUDAStream().stream();
-  const int dtype = x.scalar_type() == at::kFloat;
+  at::Tensor packed, sf;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = quantize(src, dtype, nullptr, (int)rows, (int)k, g, 0, d, s, 1, stream);
-  Py_END_ALLOW_THREADS
+  {
+    Released released;
+    packed = bytes(rows, k / 2, x), sf = bytes((rows + 127) / 128 * 128, (k / 16 + 3) / 4 * 4, x);
+    rc = quantize(x.data_ptr(), x.scalar_type() == at::kFloat, nullptr, (int)rows, (int)k, gs.data_ptr(), 0, packed.data_ptr(), sf.data_ptr(), 1,
+                  (void*)c10::cuda::getCurrentCUDAStream().stream());
+  }
   Py_INCREF(args[1]);
   return outputs(rc, packed, sf, args[1]);
   END_HANDLE_TH_ERRORS

@@ -1,9 +1,13 @@
 """The native host side of small quantiser calls (csrc/host.cpp) against the general path, which the same call takes without it: same outputs (shapes, strides, types and
 bytes), and None - so that the general path runs, with its checks and errors - for everything that is not a plain contiguous CUDA matrix."""
+import subprocess
+import sys
+
 import pytest
 import torch
 
 import sm120fp4_b200 as pkg
+from conftest import ROOT
 from sm120fp4_b200 import _lib
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +83,41 @@ def test_streams_and_capture():
     g.replay()
     torch.cuda.synchronize()
     same(out, pkg.quantize_nvfp4(x))
+
+
+ALLOCATOR = """#include <stddef.h>
+int (*held)(void); char* memory; size_t used; int calls, calls_held;
+void* take(size_t n, int device, void* stream) { (void)device, (void)stream; ++calls; calls_held += held(); void* p = memory + used; used += n; return p; }
+void give(void* p, size_t n, int device, void* stream) { (void)p, (void)n, (void)device, (void)stream; }
+"""
+ALLOCATE = """
+import ctypes, os, sys
+import torch
+import sm120fp4_b200 as pkg
+a = ctypes.CDLL(sys.argv[1])
+memory = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")      # (a segment of small blocks is 2 MB, of large ones 20 MB)
+x, y, gs = torch.randn(16, 2048, device="cuda"), torch.randn(2048, 2048, device="cuda"), torch.ones(1, device="cuda")
+ctypes.c_void_p.in_dll(a, "held").value = ctypes.cast(ctypes.pythonapi.PyGILState_Check, ctypes.c_void_p).value
+ctypes.c_void_p.in_dll(a, "memory").value = memory.data_ptr()
+calls, held = ctypes.c_int.in_dll(a, "calls"), ctypes.c_int.in_dll(a, "calls_held")
+allocator = torch.cuda.memory.CUDAPluggableAllocator(sys.argv[1], "take", "give")
+pool = torch.cuda.MemPool(allocator.allocator())
+with torch.cuda.use_mem_pool(pool):
+    out = pkg.quantize_nvfp4(x)
+    first = calls.value
+    more = pkg.quantize_nvfp4_128x4(y, gs)
+torch.cuda.synchronize()
+print(first, calls.value - first, held.value, flush=True)
+os._exit(0)      # (the pool's memory is another tensor's: nothing takes it apart)
+"""
+
+
+def test_allocations_leave_the_interpreter_to_other_threads(tmp_path):
+    """An allocation that has to wait for the device must not hold the interpreter, which a callback on the device's way may want. An allocator that looks
+    whether its caller holds it, and hands out memory that another tensor owns."""
+    (tmp_path / "a.c").write_text(ALLOCATOR)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(tmp_path / "a.so"), str(tmp_path / "a.c")], check=True)
+    r = subprocess.run([sys.executable, "-c", ALLOCATE, str(tmp_path / "a.so")], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    first, second, held = map(int, r.stdout.split())
+    assert first > 0 and second > 0 and held == 0
