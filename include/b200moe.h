@@ -121,7 +121,7 @@ int b200moe_prefill_forward(const b200moe_layer* layer, const void* x_bf16, cons
 int b200moe_prefill_status(const b200moe_layer* layer, const void* workspace, int max_tokens, void* stream);
 /* Byte offsets inside a prefill workspace sized for max_tokens, so that a tool or a test can read back what each stage of the
  * last call wrote (the reference exposes its intermediates the same way, as tensors: sm120fp4/kernels/bench_moe_baseline.py:
- * 53-74 returns them from `reference`). out14 = experts, offsets, pairs (router tables), ntiles, tile_expert, tile_first,
+ * 53-74 returns them from `reference`). out14 = experts, offsets, pairs (router tables), ntiles (then how many experts they are of), tile_expert, tile_first,
  * tile_end (128-row tiles: expert, first and end index into pairs), row_pair [tiles*128], dst_row [pairs], x records,
  * activation records, weighted bf16 rows, tile capacity, total bytes. A record is 18,432 bytes per (tile, 256-value K box):
  * row r, 16-value block b at r*128 + (((b>>1) ^ (r&7)) << 4) + (b&1)*8 (8 code bytes), its scale byte at 16384 + (b>>2)*512 +

@@ -42,7 +42,7 @@ __device__ __forceinline__ int rec_scale_offset(int r, int b16) { return 16384 +
 struct GroupedParams {
   const uint8_t* arec;        // operand records [ntiles][KB][kRec or kMidRec]
   const uint8_t* wrec;        // weight records [E][NBLK][KB][kRec]
-  const int* ntiles;
+  const int* ntiles;          // tiles, experts that they are of
   const int* tile_expert;
   const int* tile_first;      // first and end index of the tile's rows in the router's pair list
   const int* tile_end;
@@ -80,26 +80,33 @@ static_assert(sizeof(GgShared) <= kGgHead, "the records start on a 1 KB boundary
 // one of 128 rows 144 KB and four. Depth matters when the weights come from HBM: four 18 KB records in flight are worth about
 // 1.7 us of an SM's share, less than HBM latency plus the hand-offs. NR boxes stay resident; if not all of them do, the
 // ring carries operand records as well and should hold kGgMinShared slots, or kGgMinStream where the weights' way from HBM counts for more than the
-// operand's from L2 (up to two tiles an expert): us with 6, 8, 9, 10, 11 slots: 333 skewed tokens of 2816 x 704 73.8, 72.1, 72.4, 71.6, 71.8; 2000 of it 154.5, 152, 151.5, 151, 151.5; 300
-// skewed of 4096 x 1536 148, 141.5, 142.5, 139, 141; 800 of it 262, 254, 254, 253, 254; 2050 of it 371, 362, 360, 359, 356. With more tiles: 5000 of 2816 x 704 288, -, 288, 292, 293.
+// operand's from L2: us with 6, 8, 9, 10, 11 slots: 333 skewed tokens of 2816 x 704 73.8, 72.1, 72.4, 71.6, 71.8; 2000 of it 154.5, 152, 151.5, 151, 151.5; 300
+// skewed of 4096 x 1536 148, 141.5, 142.5, 139, 141; 800 of it 262, 254, 254, 253, 254; 2050 of it 371, 362, 360, 359, 356.
+// That goes by how often a weight record is read (tiles by the experts they are of) and by what the four boxes fewer add to a column block's copies (a third at
+// nine boxes, 15 % at 16). us with 6 and 10 slots, at tiles / experts: 10 boxes 1.47 137.8 / 136.7, 1.65 146.5 / 146.7, 1.99 162.5 / 165.6; 11 boxes 1.52 161.6 / 159.5, 2.0 219.7 / 221.4, 3.0
+// 152.8 / 156.2, 8.0 61.0 / 62.4; 12 boxes 1.98 146.3 / 145.0, 2.25 53.2 / 52.5, 8.0 75.6 / 77.1; 14 boxes 2.33 74.0 / 71.9, 3.0 192.0 / 187.3, 8.0 67.7 / 69.1; 16 boxes
+// 1.98 513 / 508, 3.0 61.0 / 60.2, 8.0 131.5 / 132.4. (By the layer's experts alone a batch on a few of them streamed: 3500 tokens on eight of 2816 x 704 190.2 instead of 184.4.)
+// Where every expert has three tiles six slots are the better ones at all sizes (12 boxes 210.4 / 216.0, 16 boxes 761 / 770): at most two a layer's expert.
 // TMEM: 256 accumulator columns + 16 per resident box
 // + 64 for the rotating weight scales + 64 more for streamed operand scales.
 //
-// Once (no more tiles than experts, so hardly a weight record is read twice): the CTAs then share what HBM delivers by the bytes each has in flight, and one
+// Once (no more tiles than the layer has experts): most weight records are then read once or twice, and the CTAs share what HBM delivers by the bytes each has in flight; one
 // with few rows and a deep ring takes from one with many - at 333 tokens of 2816 x 704 a record took 300 ns with ten slots and 420 with four. Six slots a
-// CTA are enough for the stream. us with all slots, eight, seven, six and five: 333 skewed tokens of 2816 x 704 75.7, 74.8, 74.2, 73.7, 72.4; 128 of it 93.7, 92.9, 92.2,
+// CTA are enough for the stream. (A batch on few experts, whose records are read many times, is indifferent: on eight of 128, 512 tokens of 2048 x 768 34.5 and 34.3 with all slots, W4A16 96 tokens
+// 39.0 and 39.3.) us with all slots, eight, seven, six and five: 333 skewed tokens of 2816 x 704 75.7, 74.8, 74.2, 73.7, 72.4; 128 of it 93.7, 92.9, 92.2,
 // 91.8, 91.7; 400 of 256 experts of 2048 x 1536 238.8, 236.0, 230.2, 227.5, 228.8; 700 skewed of 60 experts of 2304 x 1408 64.7, 64.2, 63.4, 62.6, 63.1; 300 skewed of
 // 4096 x 1536 151.5, 149.6, 148.0, 147.8, 147.7. With more tiles than experts records come from L2 as well, and depth is worth something: 2500 of 2048 x 768
 // 147.1, 147.2, 147.4, 147.9, 149.7; W4A16, 200 skewed of the 60 experts 65.8, 65.5, 65.4, 66.0, 68.2.
 constexpr int kGgMinRing = 4, kGgMinShared = 6, kGgMinStream = 10, kGgMostOnce = 6;
 struct GgPlan { int astride, NR, NS; };
-__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows, int tiles, int experts) {
+__host__ __device__ inline GgPlan gg_plan(int KB, int max_rows, int tiles, int touched, int experts) {   // touched: experts that the tiles are of
   GgPlan p;
+  const bool stream = tiles <= 2 * experts && 2 * tiles <= touched * (KB > 10 ? KB - 7 : 3);
   const int room = kGgSmem - 1024 - kGgHead;
   p.astride = ((max_rows + 7) & ~7) * 128 + 2048;
   p.NR = KB < 12 ? KB : 12;
   if ((room - p.NR * p.astride) / kRec < kGgMinRing || p.NR < KB) {
-    p.NR = (room - (tiles <= 2 * experts ? kGgMinStream : kGgMinShared) * kRec) / p.astride;
+    p.NR = (room - (stream ? kGgMinStream : kGgMinShared) * kRec) / p.astride;
     if (p.NR > 8) p.NR = 8;
   }
   p.NS = (room - p.NR * p.astride) / kRec;
@@ -334,7 +341,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);       // (a value from lane 0 is known to be warp-uniform)
   // Without wait_tables the tile tables are read without waiting for the kernel before this one: the tables' own producer is at least
   // two kernels back, and the kernel in between lets this one start only after it has seen that producer complete.
-  int ntiles = P.wait_tables ? 0 : __ldcg(P.ntiles);
+  int2 ntiles = P.wait_tables ? make_int2(0, 0) : __ldcg(reinterpret_cast<const int2*>(P.ntiles));
   if (tid == 0) {
     for (int k = 0; k < 12; ++k) { mbar_init(&S.a_full[k], 1); mbar_init(&S.a_empty[k], 1); }
     for (int s = 0; s < kGgMaxRing; ++s) { mbar_init(&S.full[s], 1); mbar_init(&S.empty[s], 1); }
@@ -344,9 +351,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   }
   if (warp == 11) { tmem_alloc(&S.tmem_base, 512); tmem_relinquish(); }
   if (PHASE == 1) fill_scale_table(S.scale, P.gs_out, tid, kGgThreads);
-  if (P.wait_tables) { grid_dependency_wait(); ntiles = __ldcg(P.ntiles); }
+  if (P.wait_tables) { grid_dependency_wait(); ntiles = __ldcg(reinterpret_cast<const int2*>(P.ntiles)); }
   grid_launch_dependents();   // the next kernel of the chain may take over SMs as this one's CTAs leave
-  const int NT = __shfl_sync(0xffffffffu, ntiles, 0);
+  const int NT = __shfl_sync(0xffffffffu, ntiles.x, 0), touched = __shfl_sync(0xffffffffu, ntiles.y, 0);
   const GgSplit split(NT, NBLK, (int)gridDim.x, (int)blockIdx.x);
   const int nseg = split.nseg;
   auto for_each_segment = [&](auto&& body) {   // body(t, n0, n1, ordinal), one call site: a copy of a role's code per launch is enough
@@ -368,7 +375,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0), NT, P.E);
+  const GgPlan plan = gg_plan(KB, __shfl_sync(0xffffffffu, S.max_rows, 0), NT, touched, P.E);
   const int NR = plan.NR, NS = plan.NS, astride = plan.astride, acodes = astride - 2048;
   uint8_t* abuf = smem + kGgHead;                  // NR records of the current row tile
   uint8_t* ring = abuf + NR * astride;                          // NS slots

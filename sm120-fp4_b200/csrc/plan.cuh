@@ -26,7 +26,7 @@ __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
 // TILE pairs per row tile (at most P / TILE + Umax tiles: the tables have room for them), ROWS operand rows per pair. row_pair
 // [tiles*TILE*ROWS] = pair of every operand row of a tile (-1: none),
 // dst_row[pair] = tile * TILE + slot (-1: empty slot, or an id >= E). tile_first / tile_end: first and end index into `pairs`.
-struct PlanTables {
+struct PlanTables {   // ntiles: how many tiles, and how many experts they are of
   int *experts, *offsets, *ntiles, *tile_expert, *tile_first, *tile_end, *dst_row;
 };
 
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(1024) k_plan(const int* ids, int P, int E, int
       for (int u = U + lane; u < Umax; u += 32) { T.experts[u] = -1; T.offsets[u + 1] = routed; }
       if (lane == 0) {
         if (U <= Umax) T.offsets[U] = routed;
-        T.ntiles[0] = NT;
+        T.ntiles[0] = NT, T.ntiles[1] = U;
       }
     }
   }
@@ -214,7 +214,7 @@ __device__ __forceinline__ void block_plan(const int* ids, int P, int E, int Uma
       for (int u = U + lane; u < Umax; u += 32) { T.experts[u] = -1; T.offsets[u + 1] = routed; }
       if (lane == 0) {
         if (U <= Umax) T.offsets[U] = routed;
-        T.ntiles[0] = NT;
+        T.ntiles[0] = NT, T.ntiles[1] = U;
       }
     }
   }

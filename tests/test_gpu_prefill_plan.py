@@ -145,6 +145,19 @@ def test_ring_depth(hidden, rows):
     assert torch.equal(run_prefill(w, x, ids, wts, 1024), in_parts(w, x, ids, wts, 1024))
 
 
+# Beside a streamed operand it also goes by the tiles of an expert that has any (ten boxes: 1.5, thirteen: 3), however many experts the layer has: rows on two
+# experts of sixteen, on both sides.
+@pytest.mark.parametrize("hidden,rows", [(2560, (128, 200)), (2560, (200, 200)), (3328, (300, 300)), (3328, (300, 400))])
+def test_ring_depth_on_few_experts(hidden, rows):
+    cfg = dict(experts=16, hidden=hidden, inter=128, top_k=1)
+    w, _ = make_layer(**cfg, seed=6)
+    m = sum(rows)
+    x, ids, wts = inputs(cfg, m, 8)
+    ids = torch.repeat_interleave(torch.tensor([3, 11], dtype=torch.int32), torch.tensor(rows))[torch.randperm(m, generator=torch.Generator().manual_seed(1))][:, None].contiguous()
+    assert torch.equal(run_prefill(w, x, ids, wts, 1024), in_parts(w, x, ids, wts, 1024))
+    assert _i32(w.prefill.workspace, prefill_map(w, 1024)["ntiles"], 2)[1] == 2
+
+
 # Rows that L2 does not hold (4100 tokens of 16 slots and 1024 columns) are added up by more threads with fewer loads each.
 def test_rows_beyond_l2():
     cfg = dict(experts=24, hidden=1024, inter=64, top_k=16)
