@@ -526,9 +526,12 @@ int b200_mid_forward(int E, int H, int I, int top_k, const uint8_t* w1t, const u
   if (rc != B200MOE_OK) return rc;
   const uint8_t* y = w + L.y;
   void* args[] = {(void*)&y, (void*)&dst_row, (void*)&M, (void*)&top_k, (void*)&H, (void*)&out};
-  // Eight slots at a time where there are more than four and enough columns to fill the SMs: 256 tokens of 2048 x 768 87.1 us (with four at a time 89.9), 200 of
-  // 2816 x 704 99.4 (102.0), 96 of 2048 x 768 74.2 (74.4); 64 of 2816 x 704 91.5 (91.0), 40 of 2048 x 768 67.5 (66.7), 100 of 60 experts with four slots 70.7 (70.0).
-  const bool eight = top_k > 4 && (long long)M * H >= 96 * 2048;
+  // Eight slots at a time where the blocks that have work are more than one an SM and all of them fit (two an SM have the registers). Fewer leave an SM's loads short of what
+  // it can have in flight either way, and looking four rows up is done sooner; of more blocks, four an SM run side by side in the form for four. us with four and eight slots at a time, by
+  // blocks an SM: 2048 wide 0.99 77.5 / 78.0, 1.08 81.7 / 79.0, 1.73 96.0 / 92.6, 1.97 93.8 / 90.9, 2.4 108.6 / 109.1, 4.7 166.1 / 168.8; 2816 wide 0.66 94.9 / 95.4, 0.98 96.7 / 97.2, 1.05 100.1 / 97.3, 1.97 112.4 / 109.2, 2.4 120.8 / 121.2;
+  // 3072 wide 0.98 79.9 / 80.2, 1.06 81.1 / 79.2, 1.97 117.4 / 116.1, 2.6 119.8 / 120.6. Four slots or fewer are one round of the form for four.
+  const int blocks = (int)(((long long)M * (H / 8) + 255) / 256);
+  const bool eight = top_k > 4 && blocks > sms && blocks <= 2 * sms;
   return launch_kernel(eight ? (const void*)k_combine<true, 8, 2> : (const void*)k_combine<true, 4, 4>, sms * 4, 256, 0, true, args, st);
 }
 

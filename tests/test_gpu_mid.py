@@ -62,17 +62,19 @@ def test_mid_batches_on_both_sides_of_the_plan_kernel(hidden, m, more):
     assert torch.equal(run_mid(w, x[:m], ids[:m], wts[:m]), whole[:m])
 
 
-# The last kernel takes eight slots at a time above four slots and 96 x 2048 values, else four: numbers of slots that are no multiple of either, on both sides (the
-# same bits; the form for four is what the tests above hold to the oracle).
+# The last kernel takes eight slots at a time above four slots where it has one to two blocks an SM (a token of 2048 columns is a block), else four: numbers of slots
+# that are no multiple of either, on both sides of both ends (the same bits; the form for four is what the tests above hold to the oracle).
 @pytest.mark.parametrize("top_k", [3, 5, 8, 9, 16])
 def test_mid_batches_on_both_sides_of_the_combine(top_k):
     cfg = dict(experts=24, hidden=2048, inter=64, top_k=top_k)
     w, _ = make_layer(**cfg, seed=6)
-    x, ids, wts = inputs(cfg, 101, 80 + top_k)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x, ids, wts = inputs(cfg, 2 * sms + 1, 80 + top_k)
     ids, wts = ids.clone(), wts.clone()
     ids[50, top_k - 1], wts[50, top_k - 1] = -1, 0
-    whole = run_mid(w, x, ids, wts).clone()
-    assert torch.equal(run_mid(w, x[:95], ids[:95], wts[:95]), whole[:95])
+    whole = run_mid(w, x, ids, wts, 512).clone()
+    for m in (2 * sms, sms + 1, sms):
+        assert torch.equal(run_mid(w, x[:m], ids[:m], wts[:m], 512), whole[:m])
 
 
 def test_qwen_shape_mid_batches():
