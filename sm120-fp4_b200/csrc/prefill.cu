@@ -227,10 +227,11 @@ __device__ __forceinline__ void add8(float (&acc)[8], const uint4& v) {
 // out[tok, :] = sum_j y[dst_row[tok*k + j], :] in slot order, fp32 accumulation, one bf16 rounding (for fp32 rows, the W4A16 path,
 // the only one of the layer). A thread sums eight columns; the rows of Batch slots are loaded before the first is added, so
 // that the loads of a token overlap (with one row at a time: 88 us at 8192 tokens x 8 rows of 4 KB).
-// The rows of a thread's first slots are looked up ahead of the wait: dst_row is complete (the kernels of this call start behind the one that has seen its writer complete),
-// and most of the blocks are here before FC2 is.
+// The rows of a thread's first slots are looked up ahead of the wait: dst_row is complete (the kernels of this call start behind the one that has seen its writer complete).
+// That is worth something where a block is there before FC2 has ended, on an SM that FC2's CTA has left: beside one there are no registers for a block.
 // Blocks: resident per SM, which says how many registers a thread has. The loads are volatile, or the compiler adds as it loads to save registers: with 32
-// of them about four were in flight, and a call of 333 tokens of 2816 x 704 took 71.1 us instead of 68.5, of 512 of 2048 x 768 37.8 instead of 35.2.
+// of them about four were in flight, and a call of 333 tokens of 2816 x 704 took 71.1 us instead of 68.5, of 512 of 2048 x 768 37.8 instead of 35.2. (Volatile keeps them in their
+// order; that the additions stand behind them is what the compiler does where the registers allow it. 32 registers hold the rows of four slots at most.)
 template <bool F32, int Batch, int Blocks>
 __global__ void __launch_bounds__(256, Blocks) k_combine(const void* yv, const int* dst_row, int M, int top_k, int H, __nv_bfloat16* out) {
   constexpr int kBatch = Batch;
@@ -421,9 +422,9 @@ int b200_prefill_forward(int E, int H, int I, int top_k, const uint8_t* w1t, con
   const uint8_t* y = w + L.y;
   void* args[] = {(void*)&y, (void*)&dst_row, (void*)&M, (void*)&top_k, (void*)&H, (void*)&out};
   // Rows that L2 does not hold come at HBM's rate, and more threads are worth more than more loads of each: 8192 tokens of 2048 x 768 (268 MB) 304.5 us, 306 with
-  // half the threads and twice the loads; 4000 (131 MB) 169 either way, 2500 142.5 and 141.
+  // half the threads and twice the loads; 4000 (131 MB) 169 either way, 2500 142.5 and 141. (Four slots or fewer: 7500 tokens of 60 experts of 2304 x 1408 280.5, with lookups for eight 290.7.)
   const bool deep = (long long)P * H * 2 <= (126LL << 20);
-  return launch_kernel(deep ? (const void*)k_combine<false, 8, 4> : (const void*)k_combine<false, 8, 8>, sms * 8, 256, 0, true, args, st);
+  return launch_kernel(deep ? (const void*)k_combine<false, 8, 4> : (const void*)k_combine<false, 4, 8>, sms * 8, 256, 0, true, args, st);
 }
 
 int b200_prefill_status_offset(int E, int H, int I, int top_k, int max_tokens, long long* off) {
