@@ -9,9 +9,12 @@
 // 128 x 128 x 64 in 64 cycles) plus 8 cycles per tcgen05.cp of a 512-byte scale tile; an SM takes in 63 bytes per cycle from
 // L2 (17.3 TB/s over the chip, from four 18 KB copies in flight on), i.e. 288 cycles per record; HBM delivers a record per
 // SM every ~700 cycles (7.1 TB/s). A batch that touches every expert with few rows is bound by HBM. In a large one no unit is
-// near its peak over the whole kernel (FC1 of 8192 tokens: tensor pipe 48 %, shared memory 51 %, L2 24 %, HBM 30 %; about 560
-// cycles a record). In a loop of its own - four scale copies and four MMAs, records arriving beside them - a record takes 291 cycles, 257 without the scale
-// copies, so neither the tensor pipe nor shared memory is the limit. Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
+// near its peak over the whole kernel (FC1 of 8192 tokens: tensor pipe 48 %, shared memory 51 %, L2 24 %, HBM 30 %), but two streams of nearly the same length share the SM. Cycles a record of
+// FC1 at 8192 tokens and seven boxes: 560 as it is, 500 without the epilogue, 430 with the ring alone (no MMA, scale copy or epilogue; 305 if every CTA reads one expert's records), 420 with
+// the MMAs alone on one expert's records. In a loop of its own a round of four scale copies and four MMAs takes 290 (257 without the copies) with 100 bytes a cycle landing beside it, so
+// neither the tensor pipe nor shared memory is the limit; where the ring's waits lengthen it to 420 is not known. The clock counts too: 1965 MHz without MMAs, 1750 in FC1, 1350 in that loop. Slots
+// count for little: launch time at four to eight boxes 78.5, 87.3, 99.1, 111.9 and 131.0 us with eight, seven, six, five and four; the same with five, 2 to 5 % more with four, 13 to 19 % with three.
+// Everything else has to stay out of the way of that stream: ONE warp waits for a record, copies its scale tiles into TMEM (tcgen05.cp) and issues its MMAs - operations of one lane execute in order, so nothing is handed from
 // warp to warp between a record's arrival and its math. (Before, four warps moved the scales through registers and handed every
 // record to the MMA warp over a barrier: 870 cycles a record at 8192 tokens.)
 //
@@ -402,8 +405,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) k_grouped_gemm(const __grid_con
   } else if (warp == 9 || warp == 10) {
     // ============================================================== ring: weight records (and operand records of boxes >= NR).
     // Two producers walk the same sequence and issue alternate slots. The warps stay converged and an elected lane issues: a copy takes a producer 320 cycles beside its
-    // wait, 470 from a branch that a single lane takes (8192 tokens of 2048 x 768 348 -> 341 us, 2050 of 4096 x 1536 425 -> 411). What a ring of four
-    // slots gives is bound by its turn-round (MMA, commit, producer, L2): without any MMA, scale copy or epilogue FC1 of 8192 tokens still takes 440 cycles a record.
+    // wait, 470 from a branch that a single lane takes (8192 tokens of 2048 x 768 348 -> 341 us, 2050 of 4096 x 1536 425 -> 411).
     // Weight records are the first to leave L2 again, so that what the layer writes stays there: layers one after the other, each with its
     // own weights, take 76 us (78 without) at 96 tokens (W4A16), 86.4 (88.1) at 1024, 65.9 (68.1) at 24. Not so the records of an
     // expert with several tiles, which are read again: with those as well 3000 tokens take 167.8 us instead of 162.5, and in W4A16, where a

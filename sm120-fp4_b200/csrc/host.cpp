@@ -1,5 +1,5 @@
 // Host side of the quantiser calls that are host time for the most part (16 x 2048 bf16: 2.4 us on the GPU, 11.5 us from Python, of which three allocations
-// 4.8, the ctypes call 1.1 and the launch 2.5; 6.3 us this way): argument checks, allocations and the library call in one call into native code. Each function takes plain CUDA
+// 4.8, the ctypes call 1.1 and the launch 2.5; 5.7 us this way): argument checks, allocations and the library call in one call into native code. Each function takes plain CUDA
 // tensors on the current device only and returns None for whatever it does not take - the caller's general path, with its checks and errors, is then
 // the one that runs -, the error code of the library as an int, or the outputs.
 #include <Python.h>

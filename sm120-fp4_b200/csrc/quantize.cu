@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(kQgThreads, 2) k_quantize_grouped(const T* x, 
 // unit is copied into shared memory once, its maximum is published, and it is quantised from there one unit of its worker later,
 // when the maxima of its group have normally all been published. A block is three workers of eight warps, a copying warp and one that
 // looks for the maxima. The kernel above reads every value twice into registers and is held up by latency with the 16 warps an SM that
-// its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 190 instructions per 16 values (66 %
-// busy), less what is kept from one pass to the other: a thread's block maxima and the unit's place stay in registers, and magnitudes are compared without
+// its registers allow (issue slots 50 % busy, DRAM 47 %); here what bounds it is the issue of about 165 instructions per 16 values (61 to 67 %
+// busy), 190 before what is kept from one pass to the other: a thread's block maxima and the unit's place stay in registers, and magnitudes are compared without
 // being taken first (220 us before, 208 with them, 205 with the order of load_shared, which takes 13 of 21 million conflict cycles away). 128 x 1536 x 2048 bf16, swizzled scales: 232 above; with two workers 13 % more. (fp32 has half the arithmetic per byte, and its 64-byte blocks
 // meet a quarter of the banks: 60 x 1024 x 1536 take 96 us either way, or 115 here without instructions that avoid the conflicts.)
 constexpr int kQcUnit = 32768, kQcSlots = 7, kQcWorkers = 3, kQcWorkerThreads = 256;
